@@ -29,6 +29,7 @@
 #include "efwi_fuse.cuh"
 #include "efwi_kernels.h"
 #include "efwi_revolve.h"
+#include "efwi_vec.cuh"
 
 using namespace efwi;
 
@@ -97,7 +98,7 @@ struct Pending {
 };
 
 // CUDA graph of one time loop, replayed while the launch parameters the
-// loop bakes in (buffer addresses, tensor maps, tuning, time axis: the key)
+// loop bakes in (buffer addresses, tuning, time axis: the key)
 // are unchanged -- across the shots of a call and across calls.
 struct GraphCache {
   std::string key;
@@ -112,7 +113,7 @@ struct GraphCache {
 };
 
 // Byte image of the values that make up a graph's key: scalars, pointers
-// and padding-free structs (Fields, Psi, tensor maps) as they are; the
+// and padding-free structs (Fields, Psi) as they are; the
 // structs with padding field by field.
 struct KeyBytes {
   std::string s;
@@ -146,9 +147,8 @@ struct EfwiHandle {
   long long N = 0;  // cells of one pitched volume
   int py = 0;       // y pitch
   int if_win = 0, bx = 4, zchunk = 8, max_batch = 4;
-  int variant = 1;  // 0: L1-served stencils, 1: TMA-staged planes
-  int fcfg = 0, rcfg = 0;  // launch configurations of the TMA kernels
-  int zchunk_rev = 8;      // z planes per CTA of the reverse kernels
+  int variant = 1;  // 0: L1-served stencils, 1: four cells per thread (exact: TMA-staged)
+  int zchunk_rev = 8;  // z planes per CTA of the exact adjoint kernels
   int nt_limit = 0;        // > 0: time loops stop early (timing probes)
   std::string err;
 
@@ -161,8 +161,8 @@ struct EfwiHandle {
 
   DevBuf pts;
   int npts = 0;
-  // row table of the shell points for the save/restore fused into the TMA
-  // stencil kernels (efwi_fuse.cuh); shell_fused false: separate kernels
+  // row table of the shell points for the save/restore fused into the
+  // vector stencil kernels (efwi_fuse.cuh); shell_fused false: separate kernels
   DevBuf shell_rows;
   ShellMap shm{};
   bool shell_fused = false;
@@ -181,7 +181,7 @@ struct EfwiHandle {
   DevBuf wobs, wimg, wsel;
   std::vector<float> stf_host;  // untapered source-time functions [nshot][nt]
   cudaStream_t cap_stream = nullptr;
-  // shot windows on the TMA kernels: window groups run on their own streams
+  // shot windows on the vector kernels: window groups run on their own streams
   cudaStream_t wst[8] = {};
   cudaEvent_t wev[9] = {};
   // shot lanes of reference-mode calls: sub-handles with their own
@@ -529,11 +529,6 @@ int status_check(EfwiHandle *h, cudaStream_t st) {
   return EFWI_OK;
 }
 
-struct FwdMaps {
-  Maps<11> s;  // vz vx vy | szz sxx syy sxz sxy syz | lam mu
-  Maps<9> v;   // sxz syz sxx sxy syy | vz vx vy | buoy
-};
-
 Fields fields_at(float *base, long long N, int S) {
   // volumes of a batch of S shots: 9 arrays of S*N floats
   Fields f;
@@ -608,7 +603,7 @@ int upload_receivers(EfwiHandle *h, const RecHost &r, cudaStream_t st, RecArgs *
   out->nrec = (const int *)(p + b0 + b1 + b2 + b3 + b4);
   out->ncell = (int)r.ucell.size();
   // Per-plane maps of the unique receiver cells for the gather / injection
-  // fused into the TMA stencil kernels; none for the L1 kernels, or when
+  // fused into the vector stencil kernels; none for the L1 kernels, or when
   // the receivers spread over so many planes that the maps would pass
   // 64 Mi cells (the separate kernels run then).
   out->plane = nullptr;
@@ -662,21 +657,26 @@ int nt_eff(const EfwiHandle *h) {
   return h->nt_limit > 0 && h->nt_limit < h->grid.nt ? std::max(h->nt_limit, 2) : h->grid.nt;
 }
 
+// Whether a launch over S shots of grid g runs on the vector kernels: variant
+// 1, within the grid limits of a launch (65535 CTAs along x rows and along
+// planes; larger grids take the L1-served kernels, whose CTAs march z).
+bool use_vec(const EfwiHandle *h, const Geo &g, int S) {
+  return h->variant == 1 && vec_fits(g, S);
+}
+
 // One forward time step of a batch: stress (+ source), velocity, receivers.
 // With `shell` set (one shot), the boundary shell of the step's starting
-// state is stored there first.  On the TMA kernels the shell store and the
-// receiver gather run in the stencil kernels' epilogues; otherwise as
+// state is stored there first.  On the vector kernels (variant 1) the shell
+// store and the receiver gather run in the stencil kernels; otherwise as
 // separate launches.
 int forward_step(EfwiHandle *h, Fields f, Psi ps, int S, const SrcArgs &src, const RecArgs &rec,
-                 float *traces_tm, cudaStream_t st, int it, const FwdMaps *maps,
-                 float *shell = nullptr) {
+                 float *traces_tm, cudaStream_t st, int it, float *shell = nullptr) {
+  const bool vec = use_vec(h, h->geo, S);
   int nzc;
-  const int bx = maps ? fwd_tma_tile(h->fcfg) : h->bx;
-  const dim3 grid = stencil_grid(h, S, bx, h->zchunk, &nzc);
-  int *status = h->status.as<int>();
+  const dim3 grid = stencil_grid(h, S, h->bx, h->zchunk, &nzc);
   ShellMap shm{};
   if (shell && h->npts > 0) {
-    if (maps && h->shell_fused) {
+    if (vec && h->shell_fused) {
       shm = h->shm;
       shm.store = shell;
     } else {
@@ -685,22 +685,20 @@ int forward_step(EfwiHandle *h, Fields f, Psi ps, int S, const SrcArgs &src, con
     }
   }
   RecFuse rf{};
-  const bool rec_fused = maps && rec.ncell > 0 && rec.plane;
+  const bool rec_fused = vec && rec.ncell > 0 && rec.plane;
   if (rec_fused) rf = RecFuse{rec, traces_tm, it + 1};
   {
     Timer t(h, K_STRESS_FWD, st, it);
-    if (maps)
-      launch_stress_fwd_tma(h->fcfg, grid, st, maps->s, h->geo, f, ps, h->zchunk, nzc, src, shm,
-                            status);
+    if (vec)
+      launch_stress_fwd_vec(S, st, h->geo, f, ps, h->lam.as<float>(), h->mu.as<float>(), src, shm);
     else
       launch_stress_fwd(h->bx, grid, st, h->geo, f, ps, h->lam.as<float>(), h->mu.as<float>(),
                         h->zchunk, nzc, src);
   }
   {
     Timer t(h, K_VELOCITY_FWD, st, it);
-    if (maps)
-      launch_velocity_fwd_tma(h->fcfg, grid, st, maps->v, h->geo, f, ps, h->zchunk, nzc, rf,
-                              status);
+    if (vec)
+      launch_velocity_fwd_vec(S, st, h->geo, f, ps, h->buoy.as<float>(), rf);
     else
       launch_velocity_fwd(h->bx, grid, st, h->geo, f, ps, h->buoy.as<float>(), h->zchunk, nzc);
   }
@@ -711,32 +709,13 @@ int forward_step(EfwiHandle *h, Fields f, Psi ps, int S, const SrcArgs &src, con
   return check_launch(h, "forward step");
 }
 
-// Tensor maps of the forward kernels over the batch volumes f.
-int make_fwd_maps(EfwiHandle *h, const Fields &f, int S, FwdMaps *maps) {
-  const float *sm[11] = {f.vz, f.vx, f.vy, f.szz, f.sxx, f.syy, f.sxz, f.sxy, f.syz,
-                         h->lam.as<float>(), h->mu.as<float>()};
-  const float *vm[9] = {f.sxz, f.syz, f.sxx, f.sxy, f.syy, f.vz, f.vx, f.vy, h->buoy.as<float>()};
-  const int bxf = fwd_tma_tile(h->fcfg);
-  for (int k = 0; k < 11; ++k) {
-    int rc = make_map(h, &maps->s.m[k], sm[k], k < 9 ? S : 1, k < 3, bxf);
-    if (rc) return rc;
-  }
-  for (int k = 0; k < 9; ++k) {
-    int rc = make_map(h, &maps->v.m[k], vm[k], k < 8 ? S : 1, k < 5, bxf);
-    if (rc) return rc;
-  }
-  return EFWI_OK;
-}
-
-// Zeroed state, receivers, source rows and tensor maps of a batch of S
-// shots (ids) whose traces go to traces_tm (time-major, zeroed here).
+// Zeroed state, receivers and source rows of a batch of S shots
+// (ids) whose traces go to traces_tm (time-major, zeroed here).
 struct Batch {
   Fields f;
   Psi ps;
   RecArgs rec;
   SrcArgs src;
-  FwdMaps maps;
-  const FwdMaps *mp = nullptr;
 };
 
 int prepare_batch(EfwiHandle *h, const int *ids, int S, float *traces_tm, long long ntr,
@@ -767,12 +746,6 @@ int prepare_batch(EfwiHandle *h, const int *ids, int S, float *traces_tm, long l
     CK_CUDA(h, cudaMemcpyAsync(dstf + (size_t)s * nt, h->stf.as<float>() + (size_t)ids[s] * nt,
                                sizeof(float) * nt, cudaMemcpyDeviceToDevice, st));
   b->src = SrcArgs{dcell, dstf, nt, 0};
-  b->mp = nullptr;
-  if (h->variant == 1) {
-    rc = make_fwd_maps(h, b->f, S, &b->maps);
-    if (rc) return rc;
-    b->mp = &b->maps;
-  }
   return EFWI_OK;
 }
 
@@ -790,7 +763,7 @@ int run_forward_batch(EfwiHandle *h, const int *ids, int S, float *traces_tm, lo
   auto loop = [&](cudaStream_t s) -> int {
     for (int it = 0; it <= ntl - 2; ++it) {
       b.src.it = it;
-      const int r = forward_step(h, b.f, b.ps, S, b.src, b.rec, traces_tm, s, it, b.mp,
+      const int r = forward_step(h, b.f, b.ps, S, b.src, b.rec, traces_tm, s, it,
                                  shell ? shell + (size_t)it * 9 * npts : nullptr);
       if (r) return r;
     }
@@ -798,10 +771,8 @@ int run_forward_batch(EfwiHandle *h, const int *ids, int S, float *traces_tm, lo
   };
   KeyBytes key;
   key.add(b.f).add(b.ps).rec(b.rec).src(b.src).add(S).add(ntl).add(traces_tm).add(shell)
-      .add(npts).add(h->fcfg).add(h->zchunk).add(h->bx).add(h->variant).geo(h->geo)
-      .shell(h->shm).add(h->shell_fused).add(h->status.p).add(h->lam.p).add(h->mu.p)
-      .add(h->buoy.p);
-  if (b.mp) key.add(b.maps);
+      .add(npts).add(h->zchunk).add(h->bx).add(h->variant).geo(h->geo)
+      .shell(h->shm).add(h->shell_fused).add(h->lam.p).add(h->mu.p).add(h->buoy.p);
   return run_graphed(h, h->g_fwd, key.s, st, loop);
 }
 
@@ -962,7 +933,7 @@ int exact_shot(EfwiHandle *h, int id, const float *obs, double *jdev, float *res
       for (int it = act.a; it < act.b; ++it) {
         b.src.it = it;
         rc = forward_step(h, b.f, b.ps, 1, b.src, first ? b.rec : norec, h->traces_tm.as<float>(),
-                          st, it, b.mp);
+                          st, it);
         if (rc) return rc;
       }
     } else if (act.op == CK_STORE) {
@@ -1052,46 +1023,19 @@ int window_traces(EfwiHandle *h, const std::vector<Domain> &dom, float *traces, 
   return EFWI_OK;
 }
 
-// Tensor maps of the forward TMA kernels over one window's state and
-// sliced model.
-int make_window_maps(EfwiHandle *h, const Domain &d, int bxf, FwdMaps *maps) {
-  const Fields &f = d.f;
-  const float *sm[11] = {f.vz, f.vx, f.vy, f.szz, f.sxx, f.syy, f.sxz, f.sxy, f.syz, d.lam, d.mu};
-  const float *vm[9] = {f.sxz, f.syz, f.sxx, f.sxy, f.syy, f.vz, f.vx, f.vy, d.buoy};
-  for (int k = 0; k < 11; ++k) {
-    int rc = make_map_dims(h, &maps->s.m[k], sm[k], d.g.sx, d.g.nx, d.g.nz, k < 3, bxf);
-    if (rc) return rc;
-  }
-  for (int k = 0; k < 9; ++k) {
-    int rc = make_map_dims(h, &maps->v.m[k], vm[k], d.g.sx, d.g.nx, d.g.nz, k < 5, bxf);
-    if (rc) return rc;
-  }
-  return EFWI_OK;
-}
-
-// Time loop of the windows on the TMA kernels.  Each window is its own
-// single-domain grid with its own tensor maps (kernel parameters, which a
-// table of many domains in one launch cannot carry).  Contiguous groups of
-// windows, balanced by cells, advance on up to 8 streams (the default
-// number of hardware queues); every group records its own receivers after
-// its velocity updates, so the groups never wait on one another inside the
-// loop.  Each launch covers a whole window, so one stream already fills the
-// GPU; the other streams fill the tails between launches.
-int window_loop_tma(EfwiHandle *h, const std::vector<Domain> &dom, const std::vector<int> &rec_dom,
+// Time loop of the windows on the vector kernels, each window a grid of its
+// own.  Contiguous groups of windows, balanced by cells, advance on up to 8
+// streams (the default number of hardware queues); every group records its
+// own receivers after its velocity updates, so the groups never wait on one
+// another inside the loop.  Each launch covers a whole window, so one stream
+// already fills the GPU; the other streams fill the tails between launches.
+int window_loop_vec(EfwiHandle *h, const std::vector<Domain> &dom, const std::vector<int> &rec_dom,
                     const Domain *ddom, const int *drd, const int *drc, const int *drr,
                     long long *dsrc, float *ttm, int ntl, bool use_graph, cudaStream_t st) {
   const int n = (int)dom.size();
-  int rc = status_reset(h, st);
-  if (rc) return rc;
   std::vector<long long> srcs(n);
   for (int k = 0; k < n; ++k) srcs[k] = dom[k].src_cell;
   CK_CUDA(h, cudaMemcpyAsync(dsrc, srcs.data(), sizeof(long long) * n, cudaMemcpyHostToDevice, st));
-  const int bxf = fwd_tma_tile(h->fcfg);
-  std::vector<FwdMaps> maps(n);
-  for (int k = 0; k < n; ++k) {
-    rc = make_window_maps(h, dom[k], bxf, &maps[k]);
-    if (rc) return rc;
-  }
   // groups [gbeg[g], gbeg[g+1]) of at least one window each
   const int G = std::min(n, 8);
   std::vector<long long> cum(n + 1, 0);
@@ -1113,15 +1057,7 @@ int window_loop_tma(EfwiHandle *h, const std::vector<Domain> &dom, const std::ve
     if (!h->wev[e]) CK_CUDA(h, cudaEventCreateWithFlags(&h->wev[e], cudaEventDisableTiming));
   CK_CUDA(h, cudaEventRecord(h->wev[8], st));
   for (int g = 0; g < G; ++g) CK_CUDA(h, cudaStreamWaitEvent(h->wst[g], h->wev[8], 0));
-  int *status = h->status.as<int>();
   const int nt = h->grid.nt;
-  std::vector<dim3> grids(n);
-  std::vector<int> nzcs(n);
-  for (int k = 0; k < n; ++k) {
-    const Geo &g = dom[k].g;
-    nzcs[k] = (g.nz + h->zchunk - 1) / h->zchunk;
-    grids[k] = dim3((g.ny + 31) / 32, (g.nx + bxf - 1) / bxf, nzcs[k]);
-  }
   long long nrec_launch = 0;
   // one time step of every group (it_dev: the step read from device memory)
   auto step = [&](int it, const int *it_dev) {
@@ -1130,10 +1066,8 @@ int window_loop_tma(EfwiHandle *h, const std::vector<Domain> &dom, const std::ve
       for (int k = gbeg[g]; k < gbeg[g + 1]; ++k) {
         const Domain &d = dom[k];
         const SrcArgs src{dsrc + k, d.stf, nt, it, it_dev};
-        launch_stress_fwd_tma(h->fcfg, grids[k], s, maps[k].s, d.g, d.f, d.ps, h->zchunk, nzcs[k],
-                              src, ShellMap{}, status);
-        launch_velocity_fwd_tma(h->fcfg, grids[k], s, maps[k].v, d.g, d.f, d.ps, h->zchunk,
-                                nzcs[k], RecFuse{}, status);
+        launch_stress_fwd_vec(1, s, d.g, d.f, d.ps, d.lam, d.mu, src, ShellMap{});
+        launch_velocity_fwd_vec(1, s, d.g, d.f, d.ps, d.buoy, RecFuse{});
       }
       const int r0 = rstart[gbeg[g]], r1 = rstart[gbeg[g + 1]];
       if (r1 > r0) {
@@ -1188,9 +1122,7 @@ int window_loop_tma(EfwiHandle *h, const std::vector<Domain> &dom, const std::ve
   h->launches[K_STRESS_FWD] += steps * n;
   h->launches[K_VELOCITY_FWD] += steps * n;
   h->launches[K_RECORD] += nrec_launch;
-  rc = check_launch(h, "window forward (TMA)");
-  if (rc) return rc;
-  return status_check(h, st);
+  return check_launch(h, "window forward");
 }
 
 }  // namespace
@@ -1232,28 +1164,28 @@ int efwi_create(const EfwiGrid *g, EfwiHandle **out) {
   G.slab_x = (long long)g->nz * 2 * g->npml * g->ny;
   G.slab_y = (long long)g->nz * g->nx * 2 * g->npml;
   *out = h;
-  const int nmax = g->nz + g->nx + g->ny;
-  std::vector<float> c(6 * nmax);
+  // each axis's rows start on a 16-byte boundary
+  const int oz = (6 * g->nz + 3) & ~3, ox = oz + ((6 * g->nx + 3) & ~3);
+  std::vector<float> c(ox + 6 * g->ny);
   cpml_profile(g->nz, g->npml, g->dz, g->f0, g->dt, c.data());
-  cpml_profile(g->nx, g->npml, g->dx, g->f0, g->dt, c.data() + 6 * g->nz);
-  cpml_profile(g->ny, g->npml, g->dy, g->f0, g->dt, c.data() + 6 * (g->nz + g->nx));
+  cpml_profile(g->nx, g->npml, g->dx, g->f0, g->dt, c.data() + oz);
+  cpml_profile(g->ny, g->npml, g->dy, g->f0, g->dt, c.data() + ox);
   // The kernels multiply by 1/K and 1/K_half instead of dividing by K.
   {
-    const int ns[3] = {g->nz, g->nx, g->ny};
-    float *row = c.data();
+    const int ns[3] = {g->nz, g->nx, g->ny}, at[3] = {0, oz, ox};
     for (int ax = 0; ax < 3; ++ax) {
+      float *row = c.data() + at[ax];
       for (int i = 0; i < ns[ax]; ++i) {
         row[CK * ns[ax] + i] = 1.0f / row[CK * ns[ax] + i];
         row[CKH * ns[ax] + i] = 1.0f / row[CKH * ns[ax] + i];
       }
-      row += 6 * ns[ax];
     }
   }
   CK_CUDA(h, h->coef.ensure(sizeof(float) * c.size()));
   CK_CUDA(h, cudaMemcpy(h->coef.p, c.data(), sizeof(float) * c.size(), cudaMemcpyHostToDevice));
   G.cz = h->coef.as<float>();
-  G.cx = G.cz + 6 * g->nz;
-  G.cy = G.cx + 6 * g->nx;
+  G.cx = G.cz + oz;
+  G.cy = G.cz + ox;
   std::vector<int> pts = shell_points(*g, h->py);
   h->npts = (int)pts.size();
   if (!pts.empty()) {
@@ -1301,8 +1233,6 @@ int efwi_set_tuning(EfwiHandle *h, int fwd_cfg, int zchunk_fwd, int rev_cfg, int
   if (!h) return EFWI_ERR_ARG;
   if (fwd_cfg < 0 || fwd_cfg > 3 || rev_cfg < 0 || rev_cfg > 7 || zchunk_fwd < 0 || zchunk_rev < 0)
     return fail(h, EFWI_ERR_ARG, "invalid tuning (forward cfg 0-3, reverse cfg 0-7, zchunk >= 0)");
-  h->fcfg = fwd_cfg;
-  h->rcfg = rev_cfg;
   if (zchunk_fwd) h->zchunk = zchunk_fwd;
   if (zchunk_rev) h->zchunk_rev = zchunk_rev;
   return EFWI_OK;
@@ -1539,47 +1469,15 @@ static int gradient_impl(EfwiHandle *h, int n, const int *ids, const float *obs,
     SrcArgs src{dcell, dstf, nt, 0};
     const int npts = h->npts;
     const float *shell = h->shell.as<float>();
-    // Reverse kernels: TMA-staged (tile 32 x 4) or L1-served.
-    Maps<21> m1;
-    Maps<23> m2;
-    Maps<13> m1r;
-    Maps<12> m1a;
-    const bool split = h->rcfg == 6 || h->rcfg == 7;
-    const bool tma = h->variant == 1;
-    const EfwiGrid &G = h->grid;
-    if (tma) {
-      const float *h1[11] = {f.sxz, f.syz, f.sxx, f.sxy, f.syy, a.sxz, a.syz, a.sxx, a.sxy, a.syy, a.szz};
-      const float *p1[10] = {f.vz, f.vx, f.vy, a.vz, a.vx, a.vy, h->buoy.as<float>(),
-                             h->lam.as<float>(), h->mu.as<float>(), grho};
-      const float *h2[6] = {f.vz, f.vx, f.vy, a.vz, a.vx, a.vy};
-      const float *p2[17] = {f.szz, f.sxx, f.syy, f.sxz, f.sxy, f.syz, a.szz, a.sxx, a.syy,
-                             a.sxz, a.sxy, a.syz, h->lam.as<float>(), h->mu.as<float>(),
-                             h->buoy.as<float>(), glam, gmu};
-      const int bxm = rev_tma_tile(h->rcfg);
-      for (int k2 = 0; k2 < 21 && rc == 0; ++k2)
-        rc = make_map(h, &m1.m[k2], k2 < 11 ? h1[k2] : p1[k2 - 11], 1, k2 < 11, bxm);
-      if (split) {
-        const float *r1[13] = {f.sxz, f.syz, f.sxx, f.sxy, f.syy, f.vz, f.vx, f.vy,
-                               a.vz, a.vx, a.vy, h->buoy.as<float>(), grho};
-        const float *a1[12] = {a.sxz, a.syz, a.sxx, a.sxy, a.syy, a.szz, a.vz, a.vx, a.vy,
-                               h->buoy.as<float>(), h->lam.as<float>(), h->mu.as<float>()};
-        for (int k2 = 0; k2 < 13 && rc == 0; ++k2) rc = make_map(h, &m1r.m[k2], r1[k2], 1, k2 < 5, 4);
-        for (int k2 = 0; k2 < 12 && rc == 0; ++k2) rc = make_map(h, &m1a.m[k2], a1[k2], 1, k2 < 6, 4);
-      }
-      for (int k2 = 0; k2 < 23 && rc == 0; ++k2)
-        rc = make_map(h, &m2.m[k2], k2 < 6 ? h2[k2] : p2[k2 - 6], 1, k2 < 6, bxm);
-      if (rc) return rc;
-    }
+    // Reverse kernels: four cells per thread (variant 1) or L1-served.
+    const bool vec = use_vec(h, h->geo, 1);
     int nzc;
-    const int bxr = tma ? rev_tma_tile(h->rcfg) : h->bx;
-    const int zcr = tma ? h->zchunk_rev : h->zchunk;
-    const dim3 grid = stencil_grid(h, 1, bxr, zcr, &nzc);
-    (void)G;
-    int *status = h->status.as<int>();
-    // On the TMA kernels the shell restore and the adjoint-source injection
-    // run in K1's and K2's epilogues; otherwise as separate launches.
-    const bool shell_fused = tma && h->shell_fused && npts > 0;
-    const bool inj_fused = tma && rec.ncell > 0 && rec.plane;
+    const int zcr = h->zchunk;
+    const dim3 grid = stencil_grid(h, 1, h->bx, zcr, &nzc);
+    // On the vector kernels the shell restore and the adjoint-source
+    // injection run inside K1 and K2; otherwise as separate launches.
+    const bool shell_fused = vec && h->shell_fused && npts > 0;
+    const bool inj_fused = vec && rec.ncell > 0 && rec.plane;
     auto shell_at = [&](int rev, int it) {
       ShellMap m{};
       if (shell_fused && rev) {
@@ -1593,12 +1491,9 @@ static int gradient_impl(EfwiHandle *h, int n, const int *ids, const float *obs,
       const ShellMap sm = shell_at(rev, it);
       RecFuse inj{};
       if (inj_fused && adj) inj = RecFuse{rec, h->res_tm.as<float>(), it};
-      if (tma && split)
-        launch_rev_velocity_split_tma(h->rcfg, grid, st, m1r, m1a, h->geo, f, a, ps, grho, zcr,
-                                      nzc, rev, adj, sm, inj, status);
-      else if (tma)
-        launch_rev_velocity_tma(h->rcfg, grid, st, m1, h->geo, f, a, ps, grho, zcr, nzc, rev, adj,
-                                sm, inj, status);
+      if (vec)
+        launch_rev_velocity_vec(st, h->geo, f, a, ps, h->lam.as<float>(), h->mu.as<float>(),
+                                h->buoy.as<float>(), grho, rev, adj, sm, inj);
       else
         launch_rev_velocity(h->bx, grid, st, h->geo, f, a, ps, h->lam.as<float>(),
                             h->mu.as<float>(), h->buoy.as<float>(), grho, zcr, nzc, rev, adj);
@@ -1606,9 +1501,9 @@ static int gradient_impl(EfwiHandle *h, int n, const int *ids, const float *obs,
     auto K2 = [&](int rev, int adj, int it) {
       Timer t(h, K_REV_STRESS, st, it);
       src.it = it;
-      if (tma)
-        launch_rev_stress_tma(h->rcfg, grid, st, m2, h->geo, f, a, ps, glam, gmu, zcr, nzc, rev,
-                              adj, src, shell_at(rev, it), status);
+      if (vec)
+        launch_rev_stress_vec(st, h->geo, f, a, ps, h->lam.as<float>(), h->mu.as<float>(),
+                              h->buoy.as<float>(), glam, gmu, rev, adj, src, shell_at(rev, it));
       else
         launch_rev_stress(h->bx, grid, st, h->geo, f, a, ps, h->lam.as<float>(), h->mu.as<float>(),
                           h->buoy.as<float>(), glam, gmu, zcr, nzc, rev, adj, src);
@@ -1641,11 +1536,9 @@ static int gradient_impl(EfwiHandle *h, int n, const int *ids, const float *obs,
     };
     KeyBytes key;
     key.add(f).add(a).add(ps).add(grho).add(glam).add(gmu).add(shell).add(npts).rec(rec)
-        .src(src).add(h->res_tm.p).add(h->rcfg).add(zcr).add(bxr).add(h->bx).add(tma)
-        .add(split).add(shell_fused).add(inj_fused).add(ntl).geo(h->geo).shell(h->shm)
-        .add(h->status.p).add(h->lam.p).add(h->mu.p).add(h->buoy.p);
-    if (tma) key.add(m1).add(m2);
-    if (tma && split) key.add(m1r).add(m1a);
+        .src(src).add(h->res_tm.p).add(zcr).add(h->bx).add(vec).add(shell_fused)
+        .add(inj_fused).add(ntl).geo(h->geo).shell(h->shm).add(h->lam.p).add(h->mu.p)
+        .add(h->buoy.p);
     cudaStream_t caller = st;
     rc = run_graphed(h, h->g_rev, key.s, caller, loop);
     st = caller;
@@ -1683,7 +1576,7 @@ static int lane_sync(EfwiHandle *h, EfwiHandle *c) {
   c->N = h->N;
   c->py = h->py;
   c->if_win = h->if_win; c->bx = h->bx; c->zchunk = h->zchunk; c->max_batch = h->max_batch;
-  c->variant = h->variant; c->fcfg = h->fcfg; c->rcfg = h->rcfg; c->zchunk_rev = h->zchunk_rev;
+  c->variant = h->variant; c->zchunk_rev = h->zchunk_rev;
   c->nt_limit = h->nt_limit;
   c->use_graphs = h->use_graphs;
   c->prof_sample = 0;  // lane 0 alone records kernel events (the others count launches)
@@ -1992,9 +1885,11 @@ int efwi_forward_windows(EfwiHandle *h, int n, const int *ids, const EfwiWindow 
   const Domain *ddom = (const Domain *)tab;
   const int ntl = nt_eff(h);
   float *ttm = h->traces_tm.as<float>();
-  if (h->variant == 1) {
+  bool vec = true;
+  for (const Domain &d : dom) vec = vec && use_vec(h, d.g, 1);
+  if (vec) {
     long long *dsrc = (long long *)((char *)drr + b_rec);
-    rc = window_loop_tma(h, dom, rec_dom, ddom, drd, drc, drr, dsrc, ttm, ntl,
+    rc = window_loop_vec(h, dom, rec_dom, ddom, drd, drc, drr, dsrc, ttm, ntl,
                          use_graph && h->prof_sample == 0, st);
     if (rc) return rc;
     return window_traces(h, dom, traces, st);
@@ -2076,7 +1971,7 @@ int efwi_gradient_windows(EfwiHandle *h, int n, const int *ids, const EfwiWindow
       }
     }
     W->if_win = h->if_win; W->bx = h->bx; W->zchunk = h->zchunk; W->max_batch = 1;
-    W->variant = h->variant; W->fcfg = h->fcfg; W->rcfg = h->rcfg; W->zchunk_rev = h->zchunk_rev;
+    W->variant = h->variant; W->zchunk_rev = h->zchunk_rev;
     W->nt_limit = h->nt_limit; W->use_graphs = h->use_graphs; W->ck_budget = h->ck_budget;
     W->lanes = 1;
     // model: the window of the resident model volumes (as efwi_forward_windows)
@@ -2195,7 +2090,7 @@ int efwi_illumination(EfwiHandle *h, int n, const int *ids, float *h_lam, float 
     const dim3 grid((h->grid.ny + 31) / 32, (h->grid.nx + 3) / 4, (h->grid.nz - 4 + 7) / 8);
     for (int it = 0; it <= ntl - 2; ++it) {
       b.src.it = it;
-      rc = forward_step(h, b.f, b.ps, S, b.src, norec, nullptr, st, it, b.mp);
+      rc = forward_step(h, b.f, b.ps, S, b.src, norec, nullptr, st, it);
       if (rc) return rc;
       Timer t(h, K_OTHER, st, it);
       k_illumination<<<grid, dim3(32, 4), 0, st>>>(h->geo, b.f, b.ps, S, h->buoy.as<float>(),
@@ -2278,16 +2173,9 @@ int efwi_step(EfwiHandle *h, float *state, int transpose, void *stream) {
   if (rc) return rc;
   if (!transpose) {
     k_state_convert<<<1184, 256, 0, st>>>(h->geo, state, f, ps, 1);
-    FwdMaps maps;
-    const FwdMaps *mp = nullptr;
-    if (h->variant == 1) {
-      rc = make_fwd_maps(h, f, 1, &maps);
-      if (rc) return rc;
-      mp = &maps;
-    }
     RecArgs norec{};
     SrcArgs nosrc{nullptr, nullptr, h->grid.nt, 0};
-    rc = forward_step(h, f, ps, 1, nosrc, norec, nullptr, st, 0, mp);
+    rc = forward_step(h, f, ps, 1, nosrc, norec, nullptr, st, 0);
     if (rc) return rc;
     k_state_convert<<<1184, 256, 0, st>>>(h->geo, state, f, ps, 0);
   } else {

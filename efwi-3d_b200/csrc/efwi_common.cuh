@@ -63,11 +63,38 @@ __device__ __forceinline__ long long cell(const Geo &g, int z, int x, int y) {
 
 __device__ __forceinline__ float dminus(float m2, float m1, float p0, float p1) {
   // c1 (f[i] - f[i-1]) - c2 (f[i+1] - f[i-2])
-  return EFWI_C1 * (p0 - m1) - EFWI_C2 * (p1 - m2);
+  return __fmaf_rn(EFWI_C1, p0 - m1, -__fmul_rn(EFWI_C2, p1 - m2));
 }
 __device__ __forceinline__ float dplus(float m1, float p0, float p1, float p2) {
   // c1 (f[i+1] - f[i]) - c2 (f[i+2] - f[i-1])
-  return EFWI_C1 * (p1 - p0) - EFWI_C2 * (p2 - m1);
+  return __fmaf_rn(EFWI_C1, p1 - p0, -__fmul_rn(EFWI_C2, p2 - m1));
+}
+// Quirk Q1 (velocity.cu:79): c1 (f[i] - f[i-1]) - c2 (f[i-1] - f[i-2]).
+__device__ __forceinline__ float dquirk(float m2, float m1, float p0) {
+  return __fmaf_rn(EFWI_C1, p0 - m1, -__fmul_rn(EFWI_C2, m1 - m2));
+}
+
+// Arithmetic of the reverse sweep, rounded as written (the compiler would
+// fuse the products of a sum differently from kernel to kernel): both kernel
+// families use these, so their images are the same bits.
+__device__ __forceinline__ float sum3(float a, float b, float c) {
+  return __fadd_rn(__fadd_rn(a, b), c);
+}
+// v - d b dt
+__device__ __forceinline__ float undo(float v, float d, float b, float dt) {
+  return __fmaf_rn(-__fmul_rn(d, b), dt, v);
+}
+// s + a d K dt
+__device__ __forceinline__ float add4(float s, float a, float d, float K, float dt) {
+  return __fmaf_rn(__fmul_rn(__fmul_rn(a, d), K), dt, s);
+}
+// s + a b dt
+__device__ __forceinline__ float add3(float s, float a, float b, float dt) {
+  return __fmaf_rn(__fmul_rn(a, b), dt, s);
+}
+// c1 e1 + c2 e2 + c3 e3
+__device__ __forceinline__ float dot3(float c1, float e1, float c2, float e2, float c3, float e3) {
+  return __fmaf_rn(c3, e3, __fmaf_rn(c2, e2, __fmul_rn(c1, e1)));
 }
 
 __device__ __forceinline__ bool slab_s(int i, int n, int np) { return i < np || i > n - np - 1; }

@@ -13,6 +13,7 @@
 #pragma once
 #include "efwi_common.cuh"
 #include "efwi_kernels.h"
+#include "efwi_vec.cuh"
 
 namespace efwi {
 
@@ -26,6 +27,20 @@ __host__ __device__ __forceinline__ int shell_index(const ShellMap &s, int row, 
   if (y >= s.ya0 && y <= s.ya1) return base + y - s.ya0;
   if (y >= s.yb0 && y <= s.yb1) return base + (s.ya1 - s.ya0 + 1) + y - s.yb0;
   return -1;
+}
+
+// Shell point indices of the four cells of a vector in a row with entry
+// `row` (-1: none, or a cell that the thread does not update); true when
+// there is one.
+__device__ __forceinline__ bool shell_cells(const ShellMap &s, int row, const VecCell &c,
+                                            int k[VEC]) {
+  bool any = false;
+#pragma unroll
+  for (int e = 0; e < VEC; ++e) {
+    k[e] = c.act[e] ? shell_index(s, row, c.y + e) : -1;
+    any = any || k[e] >= 0;
+  }
+  return any;
 }
 
 // Unique receiver cell at (shot, z, x, y), or -1.

@@ -1,0 +1,370 @@
+// Forward half-steps, one thread per four cells (efwi_vec.cuh); the same
+// arithmetic as efwi_fwd.cu.
+//
+// K_S  stress update + C-PML (slabs only) + point-source injection
+//      (restates stress.cu:36-97 and add_source, utilities.cu:442-479)
+// K_V  velocity update + C-PML (slabs only) + receiver gather
+//      (restates velocity.cu:35-96, quirks Q1 and Q2 kept)
+//
+// Fused epilogues (efwi_fuse.cuh): K_S stores the step's starting state at
+// the boundary-shell points (gradient sweeps, from_bnd); K_V records the
+// receivers (recording).
+#include "efwi_common.cuh"
+#include "efwi_fuse.cuh"
+#include "efwi_kernels.h"
+#include "efwi_vec.cuh"
+
+namespace efwi {
+
+// Both kernels form one output (K_S: the normal stresses together) at a time,
+// each from its own differences, so that few values are live: registers, not
+// bandwidth, hold these kernels' occupancy down, and the rows read again for
+// the next output come from L1.
+template <bool VA, int MINB>
+__global__ void __launch_bounds__(VEC_THREADS, MINB)
+k_stress_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ lam,
+                 const float *__restrict__ mu, int nzb, SrcArgs src, ShellMap shell) {
+  const int shot = blockIdx.z / nzb;
+  const int z = 2 + (blockIdx.z - shot * nzb) * VEC_TZ + threadIdx.z;
+  const int x = 2 + blockIdx.y * VEC_TX + threadIdx.y;
+  const int y = VEC * (blockIdx.x * VEC_TY + threadIdx.x);
+  const int nz = g.nz, nx = g.nx, ny = g.ny;
+  if (z > nz - 3 || x > nx - 3 || y > ny - 3) return;
+  const VecCell c = vec_cell(g, z, x, y);
+  const long long so = (long long)shot * g.N + c.i;
+  const float *__restrict__ vz = f.vz + so;
+  const float *__restrict__ vx = f.vx + so;
+  const float *__restrict__ vy = f.vy + so;
+  const int sz = (int)g.sz, sx = g.sx;
+  const float dt = g.dt, idz = g.idz, idx = g.idx, idy = g.idy;
+  float *szz = f.szz + so, *sxx = f.sxx + so, *syy = f.syy + so;
+  float *sxz = f.sxz + so, *sxy = f.sxy + so, *syz = f.syz + so;
+  __shared__ float4 stash[8 * VEC_THREADS];
+  Stash own{stash + vec_thread()};
+  own.fetch(0, szz); own.fetch(1, sxx); own.fetch(2, syy);
+  own.fetch(3, sxz); own.fetch(4, sxy); own.fetch(5, syz);
+  own.fetch(6, lam + c.i); own.fetch(7, mu + c.i);
+
+  const Pml<VA> m = pml_of<VA>(g, c, false);
+  float *pz = ps.z + (long long)shot * 6 * g.slab_z;
+  float *px = ps.x + (long long)shot * 6 * g.slab_x;
+  float *py = ps.y + (long long)shot * 6 * g.slab_y;
+  if (shell.rows) {  // from_bnd: the state at the start of the step
+    const int srow = shell.rows[z * nx + x];
+    int sk[VEC];
+    if (srow >= 0 && shell_cells(shell, srow, c, sk)) {
+      const float *src9[9] = {szz, sxz, sxx, syy, sxy, syz, vz, vx, vy};
+#pragma unroll
+      for (int q = 0; q < 9; ++q) {
+        const Row r = ld_row(src9[q]);
+        float *st = shell.store + (size_t)q * shell.npts;
+#pragma unroll
+        for (int e = 0; e < VEC; ++e)
+          if (sk[e] >= 0) st[sk[e]] = r[e];
+      }
+    }
+  }
+  // memory variables `slot` of one axis, and their derivative's update (half:
+  // the coefficients at half points)
+  auto ld_z = [&](int slot) { return m.zs ? ld_psi<VA>(pz + slot * g.slab_z, m.kz, c) : Row{}; };
+  auto ld_x = [&](int slot) { return m.xs ? ld_psi<VA>(px + slot * g.slab_x, m.kx, c) : Row{}; };
+  auto ld_y = [&](int slot) { return m.yany ? ld_psi_y(py + slot * g.slab_y, g, m, c) : Row{}; };
+  auto pml_z = [&](int slot, int half, Row &r, float d[VEC]) {
+    if (m.zs) pml_row<VA>(pz + slot * g.slab_z, m.kz, r, c, g.cz + 3 * half * nz + z, nz, d);
+  };
+  auto pml_x = [&](int slot, int half, Row &r, float d[VEC]) {
+    if (m.xs) pml_row<VA>(px + slot * g.slab_x, m.kx, r, c, g.cx + 3 * half * nx + x, nx, d);
+  };
+  auto pml_y = [&](int slot, int half, Row &r, float d[VEC]) {
+    if (m.yany) pml_row_y(py + slot * g.slab_y, r, g, m, c, half, d);
+  };
+
+  {  // normal stresses
+    Row qz = ld_z(PSI_VA), qx = ld_x(PSI_VA), qy = ld_y(PSI_VA);
+    float ezz[VEC], exx[VEC], eyy[VEC];
+    const Row z0 = ld_row(vz), x0 = ld_row(vx), y0 = ld_row(vy);
+    {
+      const Row a = ld_row(vz - 2 * sz), b = ld_row(vz - sz), d = ld_row(vz + sz);
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) ezz[e] = dminus(a[e], b[e], z0[e], d[e]) * idz;
+    }
+    {
+      const Row a = ld_row(vx - 2 * sx), b = ld_row(vx - sx), d = ld_row(vx + sx);
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) exx[e] = dminus(a[e], b[e], x0[e], d[e]) * idx;
+    }
+    {
+      const Span w = ld_span(vy, y0, c);
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) eyy[e] = dminus(w(e, -2), w(e, -1), y0[e], w(e, 1)) * idy;
+    }
+    pml_z(PSI_VA, 0, qz, ezz);
+    pml_x(PSI_VA, 0, qx, exx);
+    pml_y(PSI_VA, 0, qy, eyy);
+    own.wait();
+    const Row l = own.get(6), u = own.get(7);
+    Row nzz = own.get(0), nxx = own.get(1), nyy = own.get(2);
+#pragma unroll
+    for (int e = 0; e < VEC; ++e) {
+      if (!c.act[e]) continue;
+      const float le = l[e], ue = u[e], l2u = le + 2.0f * ue;
+      nzz.v[e] += (l2u * ezz[e] + le * exx[e] + le * eyy[e]) * dt;
+      nxx.v[e] += (le * ezz[e] + l2u * exx[e] + le * eyy[e]) * dt;
+      nyy.v[e] += (le * ezz[e] + le * exx[e] + l2u * eyy[e]) * dt;
+    }
+    const long long hit = src.cell ? src.cell[shot] - c.i : -1;
+    if (hit >= 0 && hit < VEC) {
+      // add_source follows the stress kernel; amplitude formed in double
+      // from pow(1500, 2) (utilities.cu:450-461).
+      const int sit = src.it_dev ? *src.it_dev : src.it;
+      const float src_amp = src.stf ? src.stf[(long long)shot * src.nt + sit] : 0.f;
+      const double a = 2250000.0 * (double)src_amp * (double)dt;
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) {
+        if (hit != e) continue;
+        nzz.v[e] = (float)((double)nzz[e] + a);
+        nxx.v[e] = (float)((double)nxx[e] + a);
+        nyy.v[e] = (float)((double)nyy[e] + a);
+      }
+    }
+    st_row(szz, nzz); st_row(sxx, nxx); st_row(syy, nyy);
+  }
+  // one shear stress from its two derivatives
+  auto shear = [&](int r, float *dst, const float d0[VEC], const float d1[VEC]) {
+    Row n = own.get(r);
+    const Row u = own.get(7);
+#pragma unroll
+    for (int e = 0; e < VEC; ++e)
+      if (c.act[e]) n.v[e] += u[e] * (d0[e] + d1[e]) * dt;
+    st_row(dst, n);
+  };
+  {  // sxz
+    Row qz = ld_z(PSI_VB1), qx = ld_x(PSI_VB1);
+    float dvx_dz[VEC], dvz_dx[VEC];
+    {
+      const Row a = ld_row(vx - sz), m = ld_row(vx), b = ld_row(vx + sz), d = ld_row(vx + 2 * sz);
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) dvx_dz[e] = dplus(a[e], m[e], b[e], d[e]) * idz;
+    }
+    {
+      const Row a = ld_row(vz - sx), m = ld_row(vz), b = ld_row(vz + sx), d = ld_row(vz + 2 * sx);
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) dvz_dx[e] = dplus(a[e], m[e], b[e], d[e]) * idx;
+    }
+    pml_z(PSI_VB1, 1, qz, dvx_dz);
+    pml_x(PSI_VB1, 1, qx, dvz_dx);
+    shear(3, sxz, dvx_dz, dvz_dx);
+  }
+  {  // sxy
+    Row qx = ld_x(PSI_VB2), qy = ld_y(PSI_VB2);
+    float dvx_dy[VEC], dvy_dx[VEC];
+    {
+      const Row m = ld_row(vx);
+      const Span w = ld_span(vx, m, c);
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) dvx_dy[e] = dplus(w(e, -1), m[e], w(e, 1), w(e, 2)) * idy;
+    }
+    {
+      const Row a = ld_row(vy - sx), m = ld_row(vy), b = ld_row(vy + sx), d = ld_row(vy + 2 * sx);
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) dvy_dx[e] = dplus(a[e], m[e], b[e], d[e]) * idx;
+    }
+    pml_x(PSI_VB2, 1, qx, dvy_dx);
+    pml_y(PSI_VB2, 1, qy, dvx_dy);
+    shear(4, sxy, dvx_dy, dvy_dx);
+  }
+  {  // syz
+    Row qz = ld_z(PSI_VB2), qy = ld_y(PSI_VB1);
+    float dvy_dz[VEC], dvz_dy[VEC];
+    {
+      const Row a = ld_row(vy - sz), m = ld_row(vy), b = ld_row(vy + sz), d = ld_row(vy + 2 * sz);
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) dvy_dz[e] = dplus(a[e], m[e], b[e], d[e]) * idz;
+    }
+    {
+      const Row m = ld_row(vz);
+      const Span w = ld_span(vz, m, c);
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) dvz_dy[e] = dplus(w(e, -1), m[e], w(e, 1), w(e, 2)) * idy;
+    }
+    pml_z(PSI_VB2, 1, qz, dvy_dz);
+    pml_y(PSI_VB1, 1, qy, dvz_dy);
+    shear(5, syz, dvy_dz, dvz_dy);
+  }
+}
+
+template <bool VA, int MINB>
+__global__ void __launch_bounds__(VEC_THREADS, MINB)
+k_velocity_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ buoy, int nzb, RecFuse rec) {
+  const int shot = blockIdx.z / nzb;
+  const int z = 2 + (blockIdx.z - shot * nzb) * VEC_TZ + threadIdx.z;
+  const int x = 2 + blockIdx.y * VEC_TX + threadIdx.y;
+  const int y = VEC * (blockIdx.x * VEC_TY + threadIdx.x);
+  const int nz = g.nz, nx = g.nx, ny = g.ny;
+  if (z > nz - 3 || x > nx - 3 || y > ny - 3) return;
+  const VecCell c = vec_cell(g, z, x, y);
+  const long long so = (long long)shot * g.N + c.i;
+  const float *__restrict__ szz = f.szz + so;
+  const float *__restrict__ sxx = f.sxx + so;
+  const float *__restrict__ syy = f.syy + so;
+  const float *__restrict__ sxz = f.sxz + so;
+  const float *__restrict__ sxy = f.sxy + so;
+  const float *__restrict__ syz = f.syz + so;
+  const int sz = (int)g.sz, sx = g.sx;
+  const float idz = g.idz, idx = g.idx, idy = g.idy, dt = g.dt;
+  float *vz = f.vz + so, *vx = f.vx + so, *vy = f.vy + so;
+  __shared__ float4 stash[4 * VEC_THREADS];
+  Stash own{stash + vec_thread()};
+  own.fetch(0, vz); own.fetch(1, vx); own.fetch(2, vy); own.fetch(3, buoy + c.i);
+  // receiver map of this plane, loaded first so that its latency overlaps
+  const int rmap = rec.a.plane ? rec.a.plane[shot * nz + z] : -1;
+
+  const Pml<VA> m = pml_of<VA>(g, c, true);
+  float *pz = ps.z + (long long)shot * 6 * g.slab_z;
+  float *px = ps.x + (long long)shot * 6 * g.slab_x;
+  float *py = ps.y + (long long)shot * 6 * g.slab_y;
+  // memory variables `slot` of one axis, and their derivative's update (half:
+  // the coefficients at half points)
+  auto ld_z = [&](int slot) { return m.zs ? ld_psi<VA>(pz + slot * g.slab_z, m.kz, c) : Row{}; };
+  auto ld_x = [&](int slot) { return m.xs ? ld_psi<VA>(px + slot * g.slab_x, m.kx, c) : Row{}; };
+  auto ld_y = [&](int slot) { return m.yany ? ld_psi_y(py + slot * g.slab_y, g, m, c) : Row{}; };
+  auto pml_z = [&](int slot, int half, Row &r, float d[VEC]) {
+    if (m.zs) pml_row<VA>(pz + slot * g.slab_z, m.kz, r, c, g.cz + 3 * half * nz + z, nz, d);
+  };
+  auto pml_x = [&](int slot, int half, Row &r, float d[VEC]) {
+    if (m.xs) pml_row<VA>(px + slot * g.slab_x, m.kx, r, c, g.cx + 3 * half * nx + x, nx, d);
+  };
+  auto pml_y = [&](int slot, int half, Row &r, float d[VEC]) {
+    if (m.yany) pml_row_y(py + slot * g.slab_y, r, g, m, c, half, d);
+  };
+
+  // one velocity from its three derivatives
+  auto update = [&](int r, const float d0[VEC], const float d1[VEC], const float d2[VEC]) {
+    Row n = own.get(r);
+    const Row b = own.get(3);
+#pragma unroll
+    for (int e = 0; e < VEC; ++e)
+      if (c.act[e]) n.v[e] += (d0[e] + d1[e] + d2[e]) * b[e] * dt;
+    return n;
+  };
+  Row nvz, nvx, nvy;
+  {  // vz
+    Row qz = ld_z(PSI_SAA), qx = ld_x(PSI_SAB1), qy = ld_y(PSI_SAB1);
+    float dszz_dz[VEC], dsxz_dx[VEC], dsyz_dy[VEC];
+    {
+      const Row a = ld_row(szz - sz), b = ld_row(szz), d = ld_row(szz + sz),
+                h = ld_row(szz + 2 * sz);
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) dszz_dz[e] = dplus(a[e], b[e], d[e], h[e]) * idz;
+    }
+    {
+      const Row a = ld_row(sxz - 2 * sx), b = ld_row(sxz - sx), m = ld_row(sxz),
+                d = ld_row(sxz + sx);
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) dsxz_dx[e] = dminus(a[e], b[e], m[e], d[e]) * idx;
+    }
+    {
+      const Row m = ld_row(syz);
+      const Span w = ld_span(syz, m, c);
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) dsyz_dy[e] = dminus(w(e, -2), w(e, -1), m[e], w(e, 1)) * idy;
+    }
+    pml_z(PSI_SAA, 1, qz, dszz_dz);
+    pml_x(PSI_SAB1, 0, qx, dsxz_dx);
+    pml_y(PSI_SAB1, 0, qy, dsyz_dy);
+    own.wait();
+    nvz = update(0, dszz_dz, dsxz_dx, dsyz_dy);
+    st_row(vz, nvz);
+  }
+  {  // vx
+    Row qz = ld_z(PSI_SAB1), qx = ld_x(PSI_SAA), qy = ld_y(PSI_SAB2);
+    float dsxz_dz[VEC], dsxx_dx[VEC], dsxy_dy[VEC];
+    {
+      const Row h = ld_row(sxz - 2 * sz), k = ld_row(sxz - sz), m = ld_row(sxz),
+                l = ld_row(sxz + sz);
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) dsxz_dz[e] = dminus(h[e], k[e], m[e], l[e]) * idz;
+    }
+    {
+      const Row a = ld_row(sxx - sx), m = ld_row(sxx), b = ld_row(sxx + sx),
+                d = ld_row(sxx + 2 * sx);
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) dsxx_dx[e] = dplus(a[e], m[e], b[e], d[e]) * idx;
+    }
+    {
+      const Row m = ld_row(sxy);
+      const Span w = ld_span(sxy, m, c);
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) dsxy_dy[e] = dminus(w(e, -2), w(e, -1), m[e], w(e, 1)) * idy;
+    }
+    pml_z(PSI_SAB1, 0, qz, dsxz_dz);
+    pml_x(PSI_SAA, 1, qx, dsxx_dx);
+    pml_y(PSI_SAB2, 0, qy, dsxy_dy);
+    nvx = update(1, dsxz_dz, dsxx_dx, dsxy_dy);
+    st_row(vx, nvx);
+  }
+  {  // vy
+    Row qz = ld_z(PSI_SAB2), qx = ld_x(PSI_SAB2), qy = ld_y(PSI_SAA);
+    float dsyz_dz[VEC], dsxy_dx[VEC], dsyy_dy[VEC];
+    {
+      const Row h = ld_row(syz - 2 * sz), k = ld_row(syz - sz), m = ld_row(syz),
+                l = ld_row(syz + sz);
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) dsyz_dz[e] = dminus(h[e], k[e], m[e], l[e]) * idz;
+    }
+    {
+      const Row m = ld_row(sxy), a = ld_row(sxy - sx), b = ld_row(sxy - 2 * sx);
+      // Quirk Q1 (velocity.cu:79): c2 * (sxy[i-1] - sxy[i-2]) along x.
+#pragma unroll
+      for (int e = 0; e < VEC; ++e)
+        dsxy_dx[e] = (EFWI_C1 * (m[e] - a[e]) - EFWI_C2 * (a[e] - b[e])) * idx;
+    }
+    {
+      const Row m = ld_row(syy);
+      const Span w = ld_span(syy, m, c);
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) dsyy_dy[e] = dplus(w(e, -1), m[e], w(e, 1), w(e, 2)) * idy;
+    }
+    pml_z(PSI_SAB2, 0, qz, dsyz_dz);
+    pml_x(PSI_SAB2, 0, qx, dsxy_dx);
+    pml_y(PSI_SAA, 1, qy, dsyy_dy);
+    nvy = update(2, dsyz_dz, dsxy_dx, dsyy_dy);
+    st_row(vy, nvy);
+  }
+  if (rmap >= 0) {
+    const int4 u = *reinterpret_cast<const int4 *>(rec.a.map + (long long)rmap * rec.a.nxpy +
+                                                   x * g.sx + y);
+    const int us[VEC] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+    for (int e = 0; e < VEC; ++e)
+      if (c.act[e] && us[e] >= 0)
+        record_cell(rec.a, rec.tm, rec.it, us[e], nvz[e], nvx[e], nvy[e]);
+  }
+}
+
+// Registers decide the resident CTAs per SM: K_S 6 (80 registers), K_V 5 (96).
+// At 152^3, one shot of a gradient (microseconds, event overhead of 6 in all):
+// K_S 94 / 82 / 79 / 89 and K_V 68 / 64 / 62 / 68 with 4 / 5 / 6 / 7 CTAs; K_V
+// with 6 is no faster where a launch has few waves (75 x 109 x 91).
+void launch_stress_fwd_vec(int S, cudaStream_t st, const Geo &g, const Fields &f, const Psi &ps,
+                           const float *lam, const float *mu, const SrcArgs &src,
+                           const ShellMap &shell) {
+  const dim3 grid = vec_grid(g, S);
+  const int nzb = grid.z / S;
+  if (psi_vectors(g))
+    k_stress_fwd_vec<true, 6><<<grid, vec_block(), 0, st>>>(g, f, ps, lam, mu, nzb, src, shell);
+  else
+    k_stress_fwd_vec<false, 6><<<grid, vec_block(), 0, st>>>(g, f, ps, lam, mu, nzb, src, shell);
+}
+
+void launch_velocity_fwd_vec(int S, cudaStream_t st, const Geo &g, const Fields &f, const Psi &ps,
+                             const float *buoy, const RecFuse &rec) {
+  const dim3 grid = vec_grid(g, S);
+  const int nzb = grid.z / S;
+  if (psi_vectors(g))
+    k_velocity_fwd_vec<true, 5><<<grid, vec_block(), 0, st>>>(g, f, ps, buoy, nzb, rec);
+  else
+    k_velocity_fwd_vec<false, 5><<<grid, vec_block(), 0, st>>>(g, f, ps, buoy, nzb, rec);
+}
+
+}  // namespace efwi

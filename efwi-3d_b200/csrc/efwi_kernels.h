@@ -109,53 +109,28 @@ void launch_rev_stress(int bx, dim3 grid, cudaStream_t st, const Geo &g, const F
                        const float *buoy, float *glam, float *gmu, int zchunk, int nzc,
                        int do_rev, int do_adj, const SrcArgs &src);
 
-// TMA-staged variants (efwi_fwd_tma.cu); `status` receives
-// EFWI_STATUS_TIMEOUT if a pipeline wait ran out of time.
-// cfg selects (tile, ring depth, min CTAs/SM); fwd_tma_tile(cfg) is the
-// tile's x extent.
-int fwd_tma_tile(int cfg);
-// K_S maps: halo vz vx vy | point szz sxx syy sxz sxy syz | model lambda mu.
-// With shell.rows set (one shot per launch), the state at the start of the
-// step is stored into shell.store at the shell points.
-void launch_stress_fwd_tma(int cfg, dim3 grid, cudaStream_t st, const Maps<11> &maps,
-                           const Geo &g, const Fields &f, const Psi &ps, int zchunk, int nzc,
-                           const SrcArgs &src, const ShellMap &shell, int *status);
-// K_V maps: halo sxz syz sxx sxy syy | point vz vx vy | model buoyancy.
-// With rec.a.plane set, the new velocities of receiver cells are recorded
-// at sample rec.it.
-void launch_velocity_fwd_tma(int cfg, dim3 grid, cudaStream_t st, const Maps<9> &maps,
-                             const Geo &g, const Fields &f, const Psi &ps, int zchunk, int nzc,
-                             const RecFuse &rec, int *status);
+// One thread per four cells (efwi_fwd_vec.cu), S shots per launch.  With
+// shell.rows set (one shot), K_S stores the state at the start of the step
+// into shell.store at the shell points; with rec.a.plane set, K_V records the
+// new velocities of the receiver cells at sample rec.it.
+void launch_stress_fwd_vec(int S, cudaStream_t st, const Geo &g, const Fields &f, const Psi &ps,
+                           const float *lam, const float *mu, const SrcArgs &src,
+                           const ShellMap &shell);
+void launch_velocity_fwd_vec(int S, cudaStream_t st, const Geo &g, const Fields &f, const Psi &ps,
+                             const float *buoy, const RecFuse &rec);
 
-// Reverse sweep with TMA-staged planes (efwi_rev_tma.cu); rev_tma_tile(cfg)
-// is the tile's x extent (4 or 8; the tile is 32 x that).
-int rev_tma_tile(int cfg);
-// K1 maps: halo sxz syz sxx sxy syy asxz asyz asxx asxy asyy aszz |
-//          point vz vx vy avz avx avy | model buoyancy lambda mu grho.
-// With shell.rows set (do_rev), the reverse velocities are restored at the
-// shell points from shell.store; with inj.a.plane set (do_adj), the adjoint
-// source inj.tm at sample inj.it is added to the adjoint velocities.
-void launch_rev_velocity_tma(int cfg, dim3 grid, cudaStream_t st, const Maps<21> &maps,
-                             const Geo &g, const Fields &f, const Fields &a, const Psi &ps,
-                             float *grho, int zchunk, int nzc, int do_rev, int do_adj,
-                             const ShellMap &shell, const RecFuse &inj, int *status);
-// K1 as two launches (cfg 6, 7): reverse half maps halo sxz syz sxx sxy syy |
-// point vz vx vy avz avx avy | model buoyancy rho-image; adjoint half maps
-// halo asxz asyz asxx asxy asyy aszz | point avz avx avy | model buoyancy
-// lambda mu.
-void launch_rev_velocity_split_tma(int cfg, dim3 grid, cudaStream_t st, const Maps<13> &rev_maps,
-                                   const Maps<12> &adj_maps, const Geo &g, const Fields &f,
-                                   const Fields &a, const Psi &ps, float *grho, int zchunk,
-                                   int nzc, int do_rev, int do_adj, const ShellMap &shell,
-                                   const RecFuse &inj, int *status);
-// K2 maps: halo vz vx vy avz avx avy | point szz sxx syy sxz sxy syz aszz
-//          asxx asyy asxz asxy asyz | model lambda mu buoyancy glam gmu.
-// With shell.rows set (do_rev), the reverse stresses are restored at the
-// shell points from shell.store.
-void launch_rev_stress_tma(int cfg, dim3 grid, cudaStream_t st, const Maps<23> &maps,
-                           const Geo &g, const Fields &f, const Fields &a, const Psi &ps,
-                           float *glam, float *gmu, int zchunk, int nzc, int do_rev, int do_adj,
-                           const SrcArgs &src, const ShellMap &shell, int *status);
+// Reverse sweep, one thread per four cells (efwi_rev_vec.cu).  With shell.rows
+// set (do_rev), the reverse velocities (K1) and stresses (K2) are restored at
+// the shell points from shell.store; with inj.a.plane set (do_adj), K1 adds
+// the adjoint source inj.tm at sample inj.it to the adjoint velocities.
+void launch_rev_velocity_vec(cudaStream_t st, const Geo &g, const Fields &f, const Fields &a,
+                             const Psi &ps, const float *lam, const float *mu, const float *buoy,
+                             float *grho, int do_rev, int do_adj, const ShellMap &shell,
+                             const RecFuse &inj);
+void launch_rev_stress_vec(cudaStream_t st, const Geo &g, const Fields &f, const Fields &a,
+                           const Psi &ps, const float *lam, const float *mu, const float *buoy,
+                           float *glam, float *gmu, int do_rev, int do_adj, const SrcArgs &src,
+                           const ShellMap &shell);
 
 __global__ void k_prep_buoyancy(const float *rho, float *buoy, int nz, int nx, int ny, int py);
 __global__ void k_window_slice(const float *src, float *dst, int nz, int nx, int pyg, int x0,

@@ -102,20 +102,21 @@ k_rev_velocity(Geo g, Fields f, Fields a, Psi ps, const float *__restrict__ lam,
     const float b = buoy[i];
     const float avz0 = a.vz[i], avx0 = a.vx[i], avy0 = a.vy[i];
     if (do_rev && xin && yin && z >= np && z <= nz - 1 - np) {
-      const float dz_ = dplus(szz[i - sz], szz[i], szz[i + sz], szz[i + 2 * sz]) * idz +
-                        dminus(sxz[i - 2 * sx], sxz[i - sx], sxz[i], sxz[i + sx]) * idx +
-                        dminus(syz[i - 2], syz[i - 1], syz[i], syz[i + 1]) * idy;
-      const float dx_ = dminus(sxz[i - 2 * sz], sxz[i - sz], sxz[i], sxz[i + sz]) * idz +
-                        dplus(sxx[i - sx], sxx[i], sxx[i + sx], sxx[i + 2 * sx]) * idx +
-                        dminus(sxy[i - 2], sxy[i - 1], sxy[i], sxy[i + 1]) * idy;
-      const float dy_ = dminus(syz[i - 2 * sz], syz[i - sz], syz[i], syz[i + sz]) * idz +
-                        (EFWI_C1 * (sxy[i] - sxy[i - sx]) - EFWI_C2 * (sxy[i - sx] - sxy[i - 2 * sx])) * idx +
-                        dplus(syy[i - 1], syy[i], syy[i + 1], syy[i + 2]) * idy;
-      f.vz[i] = f.vz[i] - dz_ * b * dt;
-      f.vx[i] = f.vx[i] - dx_ * b * dt;
-      f.vy[i] = f.vy[i] - dy_ * b * dt;
+      const float dz_ = sum3(__fmul_rn(dplus(szz[i - sz], szz[i], szz[i + sz], szz[i + 2 * sz]), idz),
+                             __fmul_rn(dminus(sxz[i - 2 * sx], sxz[i - sx], sxz[i], sxz[i + sx]), idx),
+                             __fmul_rn(dminus(syz[i - 2], syz[i - 1], syz[i], syz[i + 1]), idy));
+      const float dx_ = sum3(__fmul_rn(dminus(sxz[i - 2 * sz], sxz[i - sz], sxz[i], sxz[i + sz]), idz),
+                             __fmul_rn(dplus(sxx[i - sx], sxx[i], sxx[i + sx], sxx[i + 2 * sx]), idx),
+                             __fmul_rn(dminus(sxy[i - 2], sxy[i - 1], sxy[i], sxy[i + 1]), idy));
+      const float dy_ = sum3(__fmul_rn(dminus(syz[i - 2 * sz], syz[i - sz], syz[i], syz[i + sz]), idz),
+                             __fmul_rn(dquirk(sxy[i - 2 * sx], sxy[i - sx], sxy[i]), idx),
+                             __fmul_rn(dplus(syy[i - 1], syy[i], syy[i + 1], syy[i + 2]), idy));
+      f.vz[i] = undo(f.vz[i], dz_, b, dt);
+      f.vx[i] = undo(f.vx[i], dx_, b, dt);
+      f.vy[i] = undo(f.vy[i], dy_, b, dt);
       const float nb2 = -(b * b);
-      grho[i] = grho[i] - (avz0 * dz_ * dt * nb2 + avx0 * dx_ * dt * nb2 + avy0 * dy_ * dt * nb2);
+      grho[i] = __fadd_rn(grho[i], -add4(add4(add4(0.f, avz0, dz_, dt, nb2), avx0, dx_, dt, nb2),
+                                         avy0, dy_, dt, nb2));
     }
     if (!do_adj) continue;
     const bool zs = slab_s(z, nz, np);
@@ -123,57 +124,69 @@ k_rev_velocity(Geo g, Fields f, Fields a, Psi ps, const float *__restrict__ lam,
     const float l = lam[i], u = mu[i], l2u = l + 2.0f * u;
     // ---- adjoint vx
     {
-      const float dszz_dx = -dplus(aszz[i - sx], aszz[i], aszz[i + sx], aszz[i + 2 * sx]) * idx;
-      const float dsxx_dx = -dplus(asxx[i - sx], asxx[i], asxx[i + sx], asxx[i + 2 * sx]) * idx;
-      const float dsyy_dx = -dplus(asyy[i - sx], asyy[i], asyy[i + sx], asyy[i + 2 * sx]) * idx;
-      const float dsxz_dz = -dminus(asxz[i - 2 * sz], asxz[i - sz], asxz[i], asxz[i + sz]) * idz;
-      const float dsxy_dy = -dminus(asxy[i - 2], asxy[i - 1], asxy[i], asxy[i + 1]) * idy;
-      float acc = l2u * dsxx_dx * cx.K * dt + l * dszz_dx * cx.K * dt + l * dsyy_dx * cx.K * dt +
-                  u * cz.Kh * dsxz_dz * dt + u * cy.Kh * dsxy_dy * dt;
-      if (xs) acc += cx.a * (nxp(g, psx + PSI_VA * g.slab_x, z, x, y) * idx);
-      if (zs) acc += cz.ah * (nzm(g, psz + PSI_VB1 * g.slab_z, z, x, y) * idz);
-      if (ys) acc += cy.ah * (nym(g, psy + PSI_VB2 * g.slab_y, z, x, y) * idy);
-      const float v = avx0 + acc;
+      const float dszz_dx = __fmul_rn(-dplus(aszz[i - sx], aszz[i], aszz[i + sx], aszz[i + 2 * sx]), idx);
+      const float dsxx_dx = __fmul_rn(-dplus(asxx[i - sx], asxx[i], asxx[i + sx], asxx[i + 2 * sx]), idx);
+      const float dsyy_dx = __fmul_rn(-dplus(asyy[i - sx], asyy[i], asyy[i + sx], asyy[i + 2 * sx]), idx);
+      const float dsxz_dz = __fmul_rn(-dminus(asxz[i - 2 * sz], asxz[i - sz], asxz[i], asxz[i + sz]), idz);
+      const float dsxy_dy = __fmul_rn(-dminus(asxy[i - 2], asxy[i - 1], asxy[i], asxy[i + 1]), idy);
+      float acc = 0.f;
+      acc = add4(acc, l2u, dsxx_dx, cx.K, dt);
+      acc = add4(acc, l, dszz_dx, cx.K, dt);
+      acc = add4(acc, l, dsyy_dx, cx.K, dt);
+      acc = add4(acc, u, cz.Kh, dsxz_dz, dt);
+      acc = add4(acc, u, cy.Kh, dsxy_dy, dt);
+      if (xs) acc = __fmaf_rn(cx.a, __fmul_rn(nxp(g, psx + PSI_VA * g.slab_x, z, x, y), idx), acc);
+      if (zs) acc = __fmaf_rn(cz.ah, __fmul_rn(nzm(g, psz + PSI_VB1 * g.slab_z, z, x, y), idz), acc);
+      if (ys) acc = __fmaf_rn(cy.ah, __fmul_rn(nym(g, psy + PSI_VB2 * g.slab_y, z, x, y), idy), acc);
+      const float v = __fadd_rn(avx0, acc);
       a.vx[i] = v;
-      if (xs) { const long long k = PSI_SAA * g.slab_x + psi_x_idx(g, z, x, y); px[k] = cx.bh * px[k] + b * v * dt; }
-      if (zs) { const long long k = PSI_SAB1 * g.slab_z + psi_z_idx(g, z, x, y); pz[k] = cz.b * pz[k] + b * v * dt; }
-      if (ys) { const long long k = PSI_SAB2 * g.slab_y + psi_y_idx(g, z, x, y); py[k] = cy.b * py[k] + b * v * dt; }
+      if (xs) { const long long k = PSI_SAA * g.slab_x + psi_x_idx(g, z, x, y); px[k] = __fmaf_rn(cx.bh, px[k], __fmul_rn(__fmul_rn(b, v), dt)); }
+      if (zs) { const long long k = PSI_SAB1 * g.slab_z + psi_z_idx(g, z, x, y); pz[k] = __fmaf_rn(cz.b, pz[k], __fmul_rn(__fmul_rn(b, v), dt)); }
+      if (ys) { const long long k = PSI_SAB2 * g.slab_y + psi_y_idx(g, z, x, y); py[k] = __fmaf_rn(cy.b, py[k], __fmul_rn(__fmul_rn(b, v), dt)); }
     }
     // ---- adjoint vz
     {
-      const float dszz_dz = -dplus(aszz[i - sz], aszz[i], aszz[i + sz], aszz[i + 2 * sz]) * idz;
-      const float dsxx_dz = -dplus(asxx[i - sz], asxx[i], asxx[i + sz], asxx[i + 2 * sz]) * idz;
-      const float dsyy_dz = -dplus(asyy[i - sz], asyy[i], asyy[i + sz], asyy[i + 2 * sz]) * idz;
-      const float dsxz_dx = -dminus(asxz[i - 2 * sx], asxz[i - sx], asxz[i], asxz[i + sx]) * idx;
-      const float dsyz_dy = -dminus(asyz[i - 2], asyz[i - 1], asyz[i], asyz[i + 1]) * idy;
-      float acc = l2u * dszz_dz * cz.K * dt + l * dsxx_dz * cz.K * dt + l * dsyy_dz * cz.K * dt +
-                  u * cy.Kh * dsyz_dy * dt + u * cx.Kh * dsxz_dx * dt;
-      if (zs) acc += cz.a * (nzp(g, psz + PSI_VA * g.slab_z, z, x, y) * idz);
-      if (ys) acc += cy.ah * (nym(g, psy + PSI_VB1 * g.slab_y, z, x, y) * idy);
-      if (xs) acc += cx.ah * (nxm(g, psx + PSI_VB1 * g.slab_x, z, x, y) * idx);
-      const float v = avz0 + acc;
+      const float dszz_dz = __fmul_rn(-dplus(aszz[i - sz], aszz[i], aszz[i + sz], aszz[i + 2 * sz]), idz);
+      const float dsxx_dz = __fmul_rn(-dplus(asxx[i - sz], asxx[i], asxx[i + sz], asxx[i + 2 * sz]), idz);
+      const float dsyy_dz = __fmul_rn(-dplus(asyy[i - sz], asyy[i], asyy[i + sz], asyy[i + 2 * sz]), idz);
+      const float dsxz_dx = __fmul_rn(-dminus(asxz[i - 2 * sx], asxz[i - sx], asxz[i], asxz[i + sx]), idx);
+      const float dsyz_dy = __fmul_rn(-dminus(asyz[i - 2], asyz[i - 1], asyz[i], asyz[i + 1]), idy);
+      float acc = 0.f;
+      acc = add4(acc, l2u, dszz_dz, cz.K, dt);
+      acc = add4(acc, l, dsxx_dz, cz.K, dt);
+      acc = add4(acc, l, dsyy_dz, cz.K, dt);
+      acc = add4(acc, u, cy.Kh, dsyz_dy, dt);
+      acc = add4(acc, u, cx.Kh, dsxz_dx, dt);
+      if (zs) acc = __fmaf_rn(cz.a, __fmul_rn(nzp(g, psz + PSI_VA * g.slab_z, z, x, y), idz), acc);
+      if (ys) acc = __fmaf_rn(cy.ah, __fmul_rn(nym(g, psy + PSI_VB1 * g.slab_y, z, x, y), idy), acc);
+      if (xs) acc = __fmaf_rn(cx.ah, __fmul_rn(nxm(g, psx + PSI_VB1 * g.slab_x, z, x, y), idx), acc);
+      const float v = __fadd_rn(avz0, acc);
       a.vz[i] = v;
-      if (xs) { const long long k = PSI_SAB1 * g.slab_x + psi_x_idx(g, z, x, y); px[k] = cx.b * px[k] + b * v * dt; }
-      if (zs) { const long long k = PSI_SAA * g.slab_z + psi_z_idx(g, z, x, y); pz[k] = cz.bh * pz[k] + b * v * dt; }
-      if (ys) { const long long k = PSI_SAB1 * g.slab_y + psi_y_idx(g, z, x, y); py[k] = cy.b * py[k] + b * v * dt; }
+      if (xs) { const long long k = PSI_SAB1 * g.slab_x + psi_x_idx(g, z, x, y); px[k] = __fmaf_rn(cx.b, px[k], __fmul_rn(__fmul_rn(b, v), dt)); }
+      if (zs) { const long long k = PSI_SAA * g.slab_z + psi_z_idx(g, z, x, y); pz[k] = __fmaf_rn(cz.bh, pz[k], __fmul_rn(__fmul_rn(b, v), dt)); }
+      if (ys) { const long long k = PSI_SAB1 * g.slab_y + psi_y_idx(g, z, x, y); py[k] = __fmaf_rn(cy.b, py[k], __fmul_rn(__fmul_rn(b, v), dt)); }
     }
     // ---- adjoint vy
     {
-      const float dsyy_dy = -dplus(asyy[i - 1], asyy[i], asyy[i + 1], asyy[i + 2]) * idy;
-      const float dsxx_dy = -dplus(asxx[i - 1], asxx[i], asxx[i + 1], asxx[i + 2]) * idy;
-      const float dszz_dy = -dplus(aszz[i - 1], aszz[i], aszz[i + 1], aszz[i + 2]) * idy;
-      const float dsxy_dx = -dminus(asxy[i - 2 * sx], asxy[i - sx], asxy[i], asxy[i + sx]) * idx;
-      const float dsyz_dz = -dminus(asyz[i - 2 * sz], asyz[i - sz], asyz[i], asyz[i + sz]) * idz;
-      float acc = l2u * dsyy_dy * cy.K * dt + l * dsxx_dy * cy.K * dt + l * dszz_dy * cy.K * dt +
-                  u * cx.Kh * dsxy_dx * dt + u * cz.Kh * dsyz_dz * dt;
-      if (ys) acc += cy.a * (nyp(g, psy + PSI_VA * g.slab_y, z, x, y) * idy);
-      if (xs) acc += cx.ah * (nxm(g, psx + PSI_VB2 * g.slab_x, z, x, y) * idx);
-      if (zs) acc += cz.ah * (nzm(g, psz + PSI_VB2 * g.slab_z, z, x, y) * idz);
-      const float v = avy0 + acc;
+      const float dsyy_dy = __fmul_rn(-dplus(asyy[i - 1], asyy[i], asyy[i + 1], asyy[i + 2]), idy);
+      const float dsxx_dy = __fmul_rn(-dplus(asxx[i - 1], asxx[i], asxx[i + 1], asxx[i + 2]), idy);
+      const float dszz_dy = __fmul_rn(-dplus(aszz[i - 1], aszz[i], aszz[i + 1], aszz[i + 2]), idy);
+      const float dsxy_dx = __fmul_rn(-dminus(asxy[i - 2 * sx], asxy[i - sx], asxy[i], asxy[i + sx]), idx);
+      const float dsyz_dz = __fmul_rn(-dminus(asyz[i - 2 * sz], asyz[i - sz], asyz[i], asyz[i + sz]), idz);
+      float acc = 0.f;
+      acc = add4(acc, l2u, dsyy_dy, cy.K, dt);
+      acc = add4(acc, l, dsxx_dy, cy.K, dt);
+      acc = add4(acc, l, dszz_dy, cy.K, dt);
+      acc = add4(acc, u, cx.Kh, dsxy_dx, dt);
+      acc = add4(acc, u, cz.Kh, dsyz_dz, dt);
+      if (ys) acc = __fmaf_rn(cy.a, __fmul_rn(nyp(g, psy + PSI_VA * g.slab_y, z, x, y), idy), acc);
+      if (xs) acc = __fmaf_rn(cx.ah, __fmul_rn(nxm(g, psx + PSI_VB2 * g.slab_x, z, x, y), idx), acc);
+      if (zs) acc = __fmaf_rn(cz.ah, __fmul_rn(nzm(g, psz + PSI_VB2 * g.slab_z, z, x, y), idz), acc);
+      const float v = __fadd_rn(avy0, acc);
       a.vy[i] = v;
-      if (xs) { const long long k = PSI_SAB2 * g.slab_x + psi_x_idx(g, z, x, y); px[k] = cx.b * px[k] + b * v * dt; }
-      if (zs) { const long long k = PSI_SAB2 * g.slab_z + psi_z_idx(g, z, x, y); pz[k] = cz.bh * pz[k] + b * v * dt; }
-      if (ys) { const long long k = PSI_SAA * g.slab_y + psi_y_idx(g, z, x, y); py[k] = cy.b * py[k] + b * v * dt; }
+      if (xs) { const long long k = PSI_SAB2 * g.slab_x + psi_x_idx(g, z, x, y); px[k] = __fmaf_rn(cx.b, px[k], __fmul_rn(__fmul_rn(b, v), dt)); }
+      if (zs) { const long long k = PSI_SAB2 * g.slab_z + psi_z_idx(g, z, x, y); pz[k] = __fmaf_rn(cz.bh, pz[k], __fmul_rn(__fmul_rn(b, v), dt)); }
+      if (ys) { const long long k = PSI_SAA * g.slab_y + psi_y_idx(g, z, x, y); py[k] = __fmaf_rn(cy.b, py[k], __fmul_rn(__fmul_rn(b, v), dt)); }
     }
   }
 }
@@ -223,25 +236,27 @@ k_rev_stress(Geo g, Fields f, Fields a, Psi ps, const float *__restrict__ lam,
         syy = (float)((double)syy - am);
       }
       if (xin && yin && z >= np && z <= nz - 1 - np) {
-        const float ezz = dminus(vz[i - 2 * sz], vz[i - sz], vz[i], vz[i + sz]) * idz;
-        const float exx = dminus(vx[i - 2 * sx], vx[i - sx], vx[i], vx[i + sx]) * idx;
-        const float eyy = dminus(vy[i - 2], vy[i - 1], vy[i], vy[i + 1]) * idy;
-        szz = szz - (l2u * ezz + l * exx + l * eyy) * dt;
-        sxx = sxx - (l * ezz + l2u * exx + l * eyy) * dt;
-        syy = syy - (l * ezz + l * exx + l2u * eyy) * dt;
-        const float dvx_dz = dplus(vx[i - sz], vx[i], vx[i + sz], vx[i + 2 * sz]) * idz;
-        const float dvx_dy = dplus(vx[i - 1], vx[i], vx[i + 1], vx[i + 2]) * idy;
-        const float dvz_dx = dplus(vz[i - sx], vz[i], vz[i + sx], vz[i + 2 * sx]) * idx;
-        const float dvz_dy = dplus(vz[i - 1], vz[i], vz[i + 1], vz[i + 2]) * idy;
-        const float dvy_dx = dplus(vy[i - sx], vy[i], vy[i + sx], vy[i + 2 * sx]) * idx;
-        const float dvy_dz = dplus(vy[i - sz], vy[i], vy[i + sz], vy[i + 2 * sz]) * idz;
-        f.sxz[i] = f.sxz[i] - u * (dvx_dz + dvz_dx) * dt;
-        f.sxy[i] = f.sxy[i] - u * (dvx_dy + dvy_dx) * dt;
-        f.syz[i] = f.syz[i] - u * (dvy_dz + dvz_dy) * dt;
-        glam[i] = glam[i] - (azz0 + axx0 + ayy0) * (ezz + exx + eyy) * dt;
-        gmu[i] = gmu[i] - (2.0f * azz0 * ezz + 2.0f * axx0 * exx + 2.0f * ayy0 * eyy +
-                           axz0 * (dvx_dz + dvz_dx) + ayz0 * (dvy_dz + dvz_dy) +
-                           axy0 * (dvy_dx + dvx_dy)) * dt;
+        const float ezz = __fmul_rn(dminus(vz[i - 2 * sz], vz[i - sz], vz[i], vz[i + sz]), idz);
+        const float exx = __fmul_rn(dminus(vx[i - 2 * sx], vx[i - sx], vx[i], vx[i + sx]), idx);
+        const float eyy = __fmul_rn(dminus(vy[i - 2], vy[i - 1], vy[i], vy[i + 1]), idy);
+        szz = __fmaf_rn(-dot3(l2u, ezz, l, exx, l, eyy), dt, szz);
+        sxx = __fmaf_rn(-dot3(l, ezz, l2u, exx, l, eyy), dt, sxx);
+        syy = __fmaf_rn(-dot3(l, ezz, l, exx, l2u, eyy), dt, syy);
+        const float dvx_dz = __fmul_rn(dplus(vx[i - sz], vx[i], vx[i + sz], vx[i + 2 * sz]), idz);
+        const float dvx_dy = __fmul_rn(dplus(vx[i - 1], vx[i], vx[i + 1], vx[i + 2]), idy);
+        const float dvz_dx = __fmul_rn(dplus(vz[i - sx], vz[i], vz[i + sx], vz[i + 2 * sx]), idx);
+        const float dvz_dy = __fmul_rn(dplus(vz[i - 1], vz[i], vz[i + 1], vz[i + 2]), idy);
+        const float dvy_dx = __fmul_rn(dplus(vy[i - sx], vy[i], vy[i + sx], vy[i + 2 * sx]), idx);
+        const float dvy_dz = __fmul_rn(dplus(vy[i - sz], vy[i], vy[i + sz], vy[i + 2 * sz]), idz);
+        f.sxz[i] = undo(f.sxz[i], __fadd_rn(dvx_dz, dvz_dx), u, dt);
+        f.sxy[i] = undo(f.sxy[i], __fadd_rn(dvx_dy, dvy_dx), u, dt);
+        f.syz[i] = undo(f.syz[i], __fadd_rn(dvy_dz, dvz_dy), u, dt);
+        glam[i] = undo(glam[i], sum3(azz0, axx0, ayy0), sum3(ezz, exx, eyy), dt);
+        float gm = dot3(2.0f * azz0, ezz, 2.0f * axx0, exx, 2.0f * ayy0, eyy);
+        gm = __fmaf_rn(axz0, __fadd_rn(dvx_dz, dvz_dx), gm);
+        gm = __fmaf_rn(ayz0, __fadd_rn(dvy_dz, dvz_dy), gm);
+        gm = __fmaf_rn(axy0, __fadd_rn(dvx_dy, dvy_dx), gm);
+        gmu[i] = __fmaf_rn(-gm, dt, gmu[i]);
       }
       f.szz[i] = szz; f.sxx[i] = sxx; f.syy[i] = syy;
     }
@@ -251,55 +266,61 @@ k_rev_stress(Geo g, Fields f, Fields a, Psi ps, const float *__restrict__ lam,
     const float b = buoy[i];
     // ---- sxz
     {
-      const float dvz_dx = -dplus(avz[i - sx], avz[i], avz[i + sx], avz[i + 2 * sx]) * idx;
-      const float dvx_dz = -dplus(avx[i - sz], avx[i], avx[i + sz], avx[i + 2 * sz]) * idz;
-      float acc = dvz_dx * cx.K * b * dt + dvx_dz * cz.K * b * dt;
-      if (xs) acc += cx.a * (nxp(g, psx + PSI_SAB1 * g.slab_x, z, x, y) * idx);
-      if (zs) acc += cz.a * (nzp(g, psz + PSI_SAB1 * g.slab_z, z, x, y) * idz);
-      const float s = axz0 + acc;
+      const float dvz_dx = __fmul_rn(-dplus(avz[i - sx], avz[i], avz[i + sx], avz[i + 2 * sx]), idx);
+      const float dvx_dz = __fmul_rn(-dplus(avx[i - sz], avx[i], avx[i + sz], avx[i + 2 * sz]), idz);
+      float acc = 0.f;
+      acc = add4(acc, dvz_dx, cx.K, b, dt);
+      acc = add4(acc, dvx_dz, cz.K, b, dt);
+      if (xs) acc = __fmaf_rn(cx.a, __fmul_rn(nxp(g, psx + PSI_SAB1 * g.slab_x, z, x, y), idx), acc);
+      if (zs) acc = __fmaf_rn(cz.a, __fmul_rn(nzp(g, psz + PSI_SAB1 * g.slab_z, z, x, y), idz), acc);
+      const float s = __fadd_rn(axz0, acc);
       a.sxz[i] = s;
-      if (xs) { const long long k = PSI_VB1 * g.slab_x + psi_x_idx(g, z, x, y); px[k] = cx.bh * px[k] + s * u * dt; }
-      if (zs) { const long long k = PSI_VB1 * g.slab_z + psi_z_idx(g, z, x, y); pz[k] = cz.bh * pz[k] + s * u * dt; }
+      if (xs) { const long long k = PSI_VB1 * g.slab_x + psi_x_idx(g, z, x, y); px[k] = __fmaf_rn(cx.bh, px[k], __fmul_rn(__fmul_rn(s, u), dt)); }
+      if (zs) { const long long k = PSI_VB1 * g.slab_z + psi_z_idx(g, z, x, y); pz[k] = __fmaf_rn(cz.bh, pz[k], __fmul_rn(__fmul_rn(s, u), dt)); }
     }
     // ---- sxy
     {
-      const float dvy_dx = -dplus(avy[i - sx], avy[i], avy[i + sx], avy[i + 2 * sx]) * idx;
-      const float dvx_dy = -dplus(avx[i - 1], avx[i], avx[i + 1], avx[i + 2]) * idy;
-      float acc = dvy_dx * cx.K * b * dt + dvx_dy * cy.K * b * dt;
-      if (xs) acc += cx.a * (nxp(g, psx + PSI_SAB2 * g.slab_x, z, x, y) * idx);
-      if (ys) acc += cy.a * (nyp(g, psy + PSI_SAB2 * g.slab_y, z, x, y) * idy);
-      const float s = axy0 + acc;
+      const float dvy_dx = __fmul_rn(-dplus(avy[i - sx], avy[i], avy[i + sx], avy[i + 2 * sx]), idx);
+      const float dvx_dy = __fmul_rn(-dplus(avx[i - 1], avx[i], avx[i + 1], avx[i + 2]), idy);
+      float acc = 0.f;
+      acc = add4(acc, dvy_dx, cx.K, b, dt);
+      acc = add4(acc, dvx_dy, cy.K, b, dt);
+      if (xs) acc = __fmaf_rn(cx.a, __fmul_rn(nxp(g, psx + PSI_SAB2 * g.slab_x, z, x, y), idx), acc);
+      if (ys) acc = __fmaf_rn(cy.a, __fmul_rn(nyp(g, psy + PSI_SAB2 * g.slab_y, z, x, y), idy), acc);
+      const float s = __fadd_rn(axy0, acc);
       a.sxy[i] = s;
-      if (ys) { const long long k = PSI_VB2 * g.slab_y + psi_y_idx(g, z, x, y); py[k] = cy.bh * py[k] + s * u * dt; }
-      if (xs) { const long long k = PSI_VB2 * g.slab_x + psi_x_idx(g, z, x, y); px[k] = cx.bh * px[k] + s * u * dt; }
+      if (ys) { const long long k = PSI_VB2 * g.slab_y + psi_y_idx(g, z, x, y); py[k] = __fmaf_rn(cy.bh, py[k], __fmul_rn(__fmul_rn(s, u), dt)); }
+      if (xs) { const long long k = PSI_VB2 * g.slab_x + psi_x_idx(g, z, x, y); px[k] = __fmaf_rn(cx.bh, px[k], __fmul_rn(__fmul_rn(s, u), dt)); }
     }
     // ---- syz
     {
-      const float dvz_dy = -dplus(avz[i - 1], avz[i], avz[i + 1], avz[i + 2]) * idy;
-      const float dvy_dz = -dplus(avy[i - sz], avy[i], avy[i + sz], avy[i + 2 * sz]) * idz;
-      float acc = dvz_dy * cy.K * b * dt + dvy_dz * cz.K * b * dt;
-      if (ys) acc += cy.a * (nyp(g, psy + PSI_SAB1 * g.slab_y, z, x, y) * idy);
-      if (zs) acc += cz.a * (nzp(g, psz + PSI_SAB2 * g.slab_z, z, x, y) * idz);
-      const float s = ayz0 + acc;
+      const float dvz_dy = __fmul_rn(-dplus(avz[i - 1], avz[i], avz[i + 1], avz[i + 2]), idy);
+      const float dvy_dz = __fmul_rn(-dplus(avy[i - sz], avy[i], avy[i + sz], avy[i + 2 * sz]), idz);
+      float acc = 0.f;
+      acc = add4(acc, dvz_dy, cy.K, b, dt);
+      acc = add4(acc, dvy_dz, cz.K, b, dt);
+      if (ys) acc = __fmaf_rn(cy.a, __fmul_rn(nyp(g, psy + PSI_SAB1 * g.slab_y, z, x, y), idy), acc);
+      if (zs) acc = __fmaf_rn(cz.a, __fmul_rn(nzp(g, psz + PSI_SAB2 * g.slab_z, z, x, y), idz), acc);
+      const float s = __fadd_rn(ayz0, acc);
       a.syz[i] = s;
-      if (ys) { const long long k = PSI_VB1 * g.slab_y + psi_y_idx(g, z, x, y); py[k] = cy.bh * py[k] + s * u * dt; }
-      if (zs) { const long long k = PSI_VB2 * g.slab_z + psi_z_idx(g, z, x, y); pz[k] = cz.bh * pz[k] + s * u * dt; }
+      if (ys) { const long long k = PSI_VB1 * g.slab_y + psi_y_idx(g, z, x, y); py[k] = __fmaf_rn(cy.bh, py[k], __fmul_rn(__fmul_rn(s, u), dt)); }
+      if (zs) { const long long k = PSI_VB2 * g.slab_z + psi_z_idx(g, z, x, y); pz[k] = __fmaf_rn(cz.bh, pz[k], __fmul_rn(__fmul_rn(s, u), dt)); }
     }
     // ---- normal stresses
     {
-      const float dvx_dx = -dminus(avx[i - 2 * sx], avx[i - sx], avx[i], avx[i + sx]) * idx;
-      const float dvz_dz = -dminus(avz[i - 2 * sz], avz[i - sz], avz[i], avz[i + sz]) * idz;
-      const float dvy_dy = -dminus(avy[i - 2], avy[i - 1], avy[i], avy[i + 1]) * idy;
-      float sxx = axx0 + b * dvx_dx * cx.Kh * dt;
-      float szz = azz0 + b * dvz_dz * cz.Kh * dt;
-      float syy = ayy0 + b * dvy_dy * cy.Kh * dt;
-      if (xs) sxx += cx.ah * (nxm(g, psx + PSI_SAA * g.slab_x, z, x, y) * idx);
-      if (zs) szz += cz.ah * (nzm(g, psz + PSI_SAA * g.slab_z, z, x, y) * idz);
-      if (ys) syy += cy.ah * (nym(g, psy + PSI_SAA * g.slab_y, z, x, y) * idy);
+      const float dvx_dx = __fmul_rn(-dminus(avx[i - 2 * sx], avx[i - sx], avx[i], avx[i + sx]), idx);
+      const float dvz_dz = __fmul_rn(-dminus(avz[i - 2 * sz], avz[i - sz], avz[i], avz[i + sz]), idz);
+      const float dvy_dy = __fmul_rn(-dminus(avy[i - 2], avy[i - 1], avy[i], avy[i + 1]), idy);
+      float sxx = add4(axx0, b, dvx_dx, cx.Kh, dt);
+      float szz = add4(azz0, b, dvz_dz, cz.Kh, dt);
+      float syy = add4(ayy0, b, dvy_dy, cy.Kh, dt);
+      if (xs) sxx = __fmaf_rn(cx.ah, __fmul_rn(nxm(g, psx + PSI_SAA * g.slab_x, z, x, y), idx), sxx);
+      if (zs) szz = __fmaf_rn(cz.ah, __fmul_rn(nzm(g, psz + PSI_SAA * g.slab_z, z, x, y), idz), szz);
+      if (ys) syy = __fmaf_rn(cy.ah, __fmul_rn(nym(g, psy + PSI_SAA * g.slab_y, z, x, y), idy), syy);
       a.sxx[i] = sxx; a.szz[i] = szz; a.syy[i] = syy;
-      if (xs) { const long long k = PSI_VA * g.slab_x + psi_x_idx(g, z, x, y); px[k] = cx.b * px[k] + l * szz * dt + l2u * sxx * dt + l * syy * dt; }
-      if (zs) { const long long k = PSI_VA * g.slab_z + psi_z_idx(g, z, x, y); pz[k] = cz.b * pz[k] + l2u * szz * dt + l * sxx * dt + l * syy * dt; }
-      if (ys) { const long long k = PSI_VA * g.slab_y + psi_y_idx(g, z, x, y); py[k] = cy.b * py[k] + l * szz * dt + l * sxx * dt + l2u * syy * dt; }
+      if (xs) { const long long k = PSI_VA * g.slab_x + psi_x_idx(g, z, x, y); px[k] = add3(add3(add3(__fmul_rn(cx.b, px[k]), l, szz, dt), l2u, sxx, dt), l, syy, dt); }
+      if (zs) { const long long k = PSI_VA * g.slab_z + psi_z_idx(g, z, x, y); pz[k] = add3(add3(add3(__fmul_rn(cz.b, pz[k]), l2u, szz, dt), l, sxx, dt), l, syy, dt); }
+      if (ys) { const long long k = PSI_VA * g.slab_y + psi_y_idx(g, z, x, y); py[k] = add3(add3(add3(__fmul_rn(cy.b, py[k]), l, szz, dt), l, sxx, dt), l2u, syy, dt); }
     }
   }
 }

@@ -1,11 +1,12 @@
-"""Launch-configuration autotuner of the TMA stencil kernels.
+"""Launch-configuration autotuner.
 
-The kernels' results do not depend on the configuration (tile, ring depth,
-occupancy target, z planes per CTA); only their speed does.  For one
+Results do not depend on the configuration; only speed can.  For one
 problem the tuner runs short gradient probes (the time loops stopped after
 `nt_probe` steps) on the handle's real grid, model and survey, reads the
-per-kernel CUDA-event timings of the engine, and keeps the fastest forward
-and reverse configurations.
+per-kernel CUDA-event timings of the engine, and keeps the fastest.  The
+vector kernels of variant 1 choose their own launch shape, so by default one
+configuration of each knob is probed; callers may pass more (zchunk_rev is
+the z march of the exact adjoint kernels, zchunk_fwd that of variant 0).
 """
 from __future__ import annotations
 
@@ -14,9 +15,9 @@ from typing import Dict, Sequence
 
 import torch
 
-FWD_CFGS = (0, 1, 2, 3)
-REV_CFGS = (0, 1, 2, 3, 4, 5, 6, 7)
-ZCHUNKS = (2, 3, 4, 6, 8)
+FWD_CFGS = (0,)
+REV_CFGS = (0,)
+ZCHUNKS = (8,)
 
 
 def _probe(P, shot_ids, obs, names) -> float:
@@ -105,11 +106,11 @@ def autotune(P, shot_id: int, obs_shot: torch.Tensor, nt_probe: int = 16,
 
 
 def autotune_windows(P, shot_ids, windows, nt_probe: int = 16, bxs=(4, 8), zchunks=(4, 8, 16),
-                     fwd_cfgs: Sequence[int] = FWD_CFGS, tma_zchunks=(2, 4, 8)):
+                     fwd_cfgs: Sequence[int] = FWD_CFGS, tma_zchunks=(8,)):
     """Stencil variant and launch shape of the window forward, the fastest
     over short probes (time loop stopped after `nt_probe` steps, CUDA events
     on the current stream): the L1-served multi-domain launch over
-    (tile_bx, zchunk) and the per-window TMA kernels over (fwd_cfg, zchunk).
+    (tile_bx, zchunk) and the per-window vector kernels (reported as "tma").
     Sets the choice on P (its variant included: the windows' results do not
     depend on it)."""
     def probe():

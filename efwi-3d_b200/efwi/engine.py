@@ -115,12 +115,12 @@ class Propagator:
         check(self._h, self._L.efwi_set_graphs(self._h, int(bool(on))))
 
     def set_variant(self, variant: int) -> None:
-        """1: TMA-staged stencil planes (default); 0: L1-served stencils."""
+        """1: four cells per thread (default); 0: L1-served z marches."""
         check(self._h, self._L.efwi_set_variant(self._h, int(variant)))
 
     def set_tuning(self, fwd_cfg: int = 0, zchunk_fwd: int = 0, rev_cfg: int = 0,
                    zchunk_rev: int = 0) -> None:
-        """Launch configuration of the TMA kernels (see efwi_set_tuning)."""
+        """Launch configuration (see efwi_set_tuning)."""
         check(self._h, self._L.efwi_set_tuning(self._h, int(fwd_cfg), int(zchunk_fwd),
                                                int(rev_cfg), int(zchunk_rev)))
         self.tuning = (fwd_cfg, zchunk_fwd, rev_cfg, zchunk_rev)
@@ -283,7 +283,7 @@ class Propagator:
 
     def forward_windows(self, shot_ids, windows, use_graph: bool = True) -> torch.Tensor:
         """Traces of shots each on its own window (x0, y0, nx, ny) of the
-        padded grid: per-window TMA launches on several streams (variant 1)
+        padded grid: per-window launches on several streams (variant 1)
         or one persistent multi-domain launch per half-step (variant 0)."""
         ids = self._ids(shot_ids)
         if len(windows) != len(ids):

@@ -69,9 +69,10 @@ const char *efwi_version(void);
  * per CTA; 0 keeps), max_batch >= 1 shots per forward launch (0 keeps). */
 int efwi_set_options(EfwiHandle *h, int if_win, int tile_bx, int zchunk, int max_batch);
 
-/* Kernel family of the stencil sweeps: 1 (default) stages the x/y-halo
- * operands of every z plane in shared memory with bulk tensor copies
- * (TMA); 0 reads them through L1.  Both give identical results.  No
+/* Kernel family of the stencil sweeps: 1 (default) updates four cells per
+ * thread with 16-byte accesses (exact gradients: planes staged in shared
+ * memory by bulk tensor copies); 0 marches z one cell per thread.  Both give
+ * identical results; grids beyond 65535 CTAs along x or z run as 0.  No
  * reference counterpart (the reference has one plain kernel per update). */
 int efwi_set_variant(EfwiHandle *h, int variant);
 
@@ -85,11 +86,11 @@ int efwi_set_variant(EfwiHandle *h, int variant);
  * host, libCUFD.cu:312-354, 532-612). */
 int efwi_set_graphs(EfwiHandle *h, int on);
 
-/* Launch configuration of the TMA kernels (the autotuner's knobs; results
- * do not depend on them): fwd_cfg in 0..3 and rev_cfg in 0..7 select tile,
- * ring depth and occupancy target (rev_cfg 6, 7 run the reverse-velocity
- * kernel as two launches); zchunk_* > 0 sets the z planes per CTA (0 keeps).
- * No reference counterpart. */
+/* Launch configuration (the autotuner's knobs; results do not depend on
+ * them): zchunk_fwd > 0 sets the z planes per CTA of variant 0, zchunk_rev
+ * > 0 those of the exact adjoint kernels (0 keeps).  fwd_cfg in 0..3 and
+ * rev_cfg in 0..7 are accepted and have no effect: the vector kernels choose
+ * their own launch shape.  No reference counterpart. */
 int efwi_set_tuning(EfwiHandle *h, int fwd_cfg, int zchunk_fwd, int rev_cfg, int zchunk_rev);
 
 /* Shot lanes of reference-mode efwi_misfit / efwi_gradient calls of two or
@@ -150,13 +151,12 @@ int efwi_gradient(EfwiHandle *h, int n, const int *shot_ids, const float *obs, i
  * window of the padded grid,
  * x in [x0, x0 + nx), y in [y0, y0 + ny), all z, with its own C-PML of npml
  * cells inside the window edges; receivers outside the window record
- * zeros.  With the TMA variant (efwi_set_variant 1, the default) every
- * window runs the forward TMA kernels as its own grid (forward cfg and
- * zchunk of efwi_set_tuning), groups of windows on up to 8 internal
- * streams; use_graph is ignored.  With the L1 variant all windows of a
+ * zeros.  With variant 1 (efwi_set_variant, the default) every window runs
+ * the vector kernels as its own grid, groups of windows on up to 8 internal
+ * streams.  With the L1 variant all windows of a
  * call advance together in one persistent launch per half-step (tile_bx
  * and zchunk of efwi_set_options); use_graph = 1 captures the whole time
- * loop in a CUDA graph and launches it once.  With the TMA variant,
+ * loop in a CUDA graph and launches it once.  With variant 1,
  * use_graph = 1 captures one time step (every group, as parallel branches)
  * in a CUDA graph and replays it once per step, the step index read from a
  * device word.  All forms give the same bits.

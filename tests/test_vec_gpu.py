@@ -1,0 +1,57 @@
+"""Vector kernels (variant 1, four cells per thread) against the one-cell
+L1 kernels (variant 0): the same bits, at the edges of their vectors, tiles
+and slabs.  ny runs over every remainder by the vector length; C-PML widths
+and ny that are not multiples of it take the single-cell memory variables,
+the others the vector ones; nx and nz run over the remainders of the 4 x 4
+row and plane tile; the smallest grid has one updated cell."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module", autouse=True)
+def _ready():
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+
+
+def _run(g, shots, stf, model, obs, variant, graphs):
+    from efwi.engine import Propagator
+    P = Propagator(g)
+    P.set_variant(variant)
+    P.set_graphs(graphs)
+    P.set_survey(shots, stf)
+    P.set_model(*model)
+    ids = list(range(len(shots)))
+    tr = P.forward(ids)
+    out = [tr] + list(P.gradient(ids, obs if obs is not None else 0.5 * tr + 1e-4)[1:])
+    return out + list(P.illumination(ids))
+
+
+@pytest.mark.parametrize("nz,nx,ny,npml", [
+    (5, 5, 5, 2), (14, 13, 12, 4), (15, 14, 33, 4), (16, 17, 34, 5), (17, 18, 35, 6),
+    (18, 19, 36, 8), (23, 22, 40, 4), (22, 23, 64, 8), (13, 24, 69, 6)])
+@pytest.mark.parametrize("graphs", [True, False])
+def test_vector_kernels_match_single_cell_kernels(nz, nx, ny, npml, graphs):
+    from efwi.engine import Grid, Shot
+    nt = 40
+    g = Grid(nz, nx, ny, npml, nt, 10.0, 11.0, 9.0, 8e-4, 25.0)
+    rng = np.random.default_rng(nz + ny)
+    rho = (1.5 + rng.random((nz, nx, ny))).astype(np.float32)
+    mu = (1e6 * (1.0 + rng.random((nz, nx, ny)))).astype(np.float32)
+    model = [torch.from_numpy(a) for a in ((1.2 * mu).astype(np.float32), mu, rho)]
+    shots = []
+    for k in range(2):
+        # receivers over all updated cells, C-PML and shared cells among them
+        z, x, y = (rng.integers(2, n - 2, 40).astype(np.int32) for n in (nz, nx, ny))
+        z[:5], x[:5], y[:5] = nz // 2, nx // 2, ny // 2
+        shots.append(Shot(src=(2 + k * (nz - 5), nx // 2, 2 + (1 - k) * (ny - 5)), z_rec=z, x_rec=x,
+                          y_rec=y))
+    stf = rng.standard_normal((2, nt)).astype(np.float32)
+    a = _run(g, shots, stf, model, None, 0, graphs)
+    b = _run(g, shots, stf, model, None, 1, graphs)
+    assert float(a[0].abs().max()) > 0
+    for u, v in zip(a, b):
+        assert torch.equal(u, v)
