@@ -199,13 +199,27 @@ k_conv3d_wgrad(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restr
   }
 }
 
-__global__ void k_reduce_partials(const float *__restrict__ partial, int nparts, int n,
-                                  float *__restrict__ out) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
+// out[i] = sum over the CTAs' partial sums, in a fixed order: warp w of a CTA
+// adds the partials w, w + 8, ... of 32 outputs (one 128-byte line each), the
+// eight warps' sums are added in warp order.  One thread per output, reading
+// all partials one after the other, took 40 us for 592 of them.
+constexpr int kRedWarps = 8;
+__global__ void __launch_bounds__(32 * kRedWarps)
+k_reduce_partials(const float *__restrict__ partial, int nparts, int n, float *__restrict__ out) {
+  __shared__ float sum[kRedWarps][32];
+  const int i = blockIdx.x * 32 + threadIdx.x, w = threadIdx.y;
   float s = 0.f;
-  for (int p = 0; p < nparts; ++p) s += partial[(long long)p * n + i];
-  out[i] = s;
+  if (i < n) {
+#pragma unroll 8
+    for (int p = w; p < nparts; p += kRedWarps) s += partial[(long long)p * n + i];
+  }
+  sum[w][threadIdx.x] = s;
+  __syncthreads();
+  if (w == 0 && i < n) {
+#pragma unroll
+    for (int k = 1; k < kRedWarps; ++k) s += sum[k][threadIdx.x];
+    out[i] = s;
+  }
 }
 
 
@@ -752,164 +766,220 @@ k_conv3d_fwd_ws(const __grid_constant__ CUtensorMap xmap, const __nv_bfloat16 *_
   if (warp == 0)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 32;" ::"r"(tmem) : "memory");
 }
-// Weight gradient on tcgen05: dW[t][co][ci] = sum_u dy[u - off_t][co] x[u][ci]
-// (u = v + off_t).  A unit is 8 (x) x 16 (y) voxels u on each of up to 8
-// consecutive z planes (the dy planes of one z are reused for the next);
-// its K = 16 slices are two staged rows of 8 voxels.  B = x[u][ci] staged as
-// [row][ci][8 x] (256-byte row blocks: ci halves 128 B apart, the second K
-// row one block on).  A stacks taps on M: rows (j, co), j = 3a + b standing
-// for dy = 1 - a, dz = 1 - b, read from dy staged as [row][plane][co][8 x]
-// with the three planes z-1, z, z+1 in consecutive 256-byte blocks, so the
-// 16 row groups of taps j = 0..7 lie 128 B apart (a uniform stride) and the
-// second K row is three blocks on.  One staged copy per x shift dx keeps the
-// operands 16-byte aligned; per K slice and shift one MMA covers taps 0..7
-// and a second, one block later, taps 1..8 (only its last 16 rows, tap 8,
-// are kept).  Six accumulators of 16 TMEM columns sum over all units of a
-// CTA; the CTA's 27 x 16 x 16 sums go to partial[cta] for the fixed-order
-// reduction.  Every wait is bounded; on a timeout the CTA sets the status
-// flag and writes NaN partial sums.
-constexpr int kWgRows = 16;                           // y rows of a unit
-constexpr int kWgZ = 8;                               // z planes a unit marches
-constexpr int kWgX = 8;                               // x voxels of a unit
-constexpr int kWgXBytes = kWgRows * 256;              // staged x: [row][ci][8]
-constexpr int kWgDyBytes = (kWgRows + 2) * 3 * 256;   // staged dy per shift
-constexpr int kWgSmem = kWgXBytes + 3 * kWgDyBytes + 128;
-constexpr int kWgThreads = 128;
+// Weight gradient on tcgen05: dW[t][co][ci] = sum_w dy[w - dx][co]
+// x[w + (dy, dz)][ci], the y and z shifts of a tap on x and its x shift on dy.
+// K runs over voxels w, so both operands are "MN-major": a voxel's 16
+// channels are contiguous, as in memory, and bulk tensor copies bring them
+// to shared memory without a transposition (32-byte swizzle: rows of one
+// voxel, blocks of 8 voxels of 256 bytes).
+// A unit is 8 (x) x 16 (y) x 2 (z) voxels.  x is staged as [y 18][z 4][8 x],
+// so the blocks of the taps (dy, dz) of one voxel row follow one another:
+// block 4 dy' + dz' (dy' = dy + 1, dz' = dz + 1), the fourth of each four
+// unused.  One MMA with M = 128 takes blocks 0-7, a second blocks 8-15 (of
+// which 8-10 are taps).  dy is staged three times, moved by the three x
+// shifts, so that N = 48 = (dx', co).  K = 16: two voxel rows.
+// Two accumulators of 48 TMEM columns sum over a group of kWgGroup units;
+// four warps then add them to sums in registers while the next group runs in
+// a second pair: the tensor cores' accumulation truncates, so its error grows
+// with the number of MMAs added in one go (at 93 x 117 x 141 the sums are
+// 6e-6 off when a CTA's units stay in TMEM to the end).  The CTA's 27 x 16
+// x 16 sums go to partial[cta] for the fixed-order reduction.  One thread of a
+// fifth warp runs the copies (two stages) and the MMAs; every wait is
+// bounded, and on a timeout the CTA sets the status flag and writes NaN
+// partial sums.
+constexpr int kWgX = 8, kWgY = 16, kWgZ = 2;          // voxels of a unit
+constexpr int kWgZs = kWgZ + 2;                       // staged x planes
+constexpr int kWgABytes = (kWgY + 2) * kWgZs * 256;   // staged x
+constexpr int kWgBCopy = kWgZ * kWgY * 256;           // one shifted copy of dy
+constexpr int kWgCopied = kWgABytes + 3 * kWgBCopy;   // bytes of a stage's copies
+constexpr int kWgStage = kWgCopied;
+constexpr int kWgStages = 2;
+constexpr int kWgSmem = kWgStages * kWgStage + 1024;  // + alignment slack
+constexpr int kWgThreads = 160;
+constexpr int kWgGroup = 4;   // units per accumulator hand-over
+constexpr int kWgCol2 = 64;  // first TMEM column of the second accumulator
+// the second MMA of a unit's last rows reads past the staged x, into dy
+static_assert(((kWgY - 2 + 1) * kWgZs + kWgZ - 1 + 16) * 256 <= kWgCopied, "in the stage");
+
+// Both operands MN-major, N = 48, M = 128.
+constexpr uint32_t kWgIdesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) |
+                              ((48u >> 3) << 17) | ((128u >> 4) << 24);
+
+// MN-major operand with 32-byte swizzle: blocks of 16 M/N elements `lbo`
+// bytes apart, blocks of 8 K rows `sbo` apart.
+__device__ __forceinline__ uint64_t tc_desc_mn32(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
+  return tc_desc(saddr, lbo, sbo) | (6ull << 61);
+}
+
+__device__ __forceinline__ void tc_mma_idesc(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc,
+                                             uint32_t acc) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d),
+      "l"(a), "l"(b), "r"(idesc), "r"(acc));
+}
+
+__device__ __forceinline__ void tma_load_4d(void *dst, const CUtensorMap *map, uint64_t *bar,
+                                            int c0, int c1, int c2, int c3) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+      " [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(smem_u32(dst)),
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(c3),
+      "r"(smem_u32(bar))
+      : "memory");
+}
 
 __global__ void __launch_bounds__(kWgThreads)
-k_conv3d_wgrad_tc(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restrict__ dy,
+k_conv3d_wgrad_tc(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap gmap,
                   int D, int H, int W, float *__restrict__ partial) {
   extern __shared__ unsigned char smem_raw[];
-  __shared__ __align__(8) uint64_t bar;
+  __shared__ __align__(8) uint64_t full[kWgStages], done[kWgStages], tfull[2], tempty[2];
   __shared__ uint32_t tmem_slot;
-  unsigned char *smem = smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u);
-  unsigned char *sxs = smem;                  // [row][ci][8 x]
-  unsigned char *sdy = smem + kWgXBytes;      // [dx][row][plane][co][8 x]
+  __shared__ volatile int s_abort;
+  unsigned char *smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int nxw = (W + kWgX - 1) / kWgX, nyb = (H + kWgRows - 1) / kWgRows;
+  const int nxw = (W + kWgX - 1) / kWgX, nyb = (H + kWgY - 1) / kWgY;
   const long long nunits = (long long)nxw * nyb * ((D + kWgZ - 1) / kWgZ);
+  const long long nj =
+      (long long)blockIdx.x < nunits ? (nunits - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
+  const long long ng = (nj + kWgGroup - 1) / kWgGroup;
   if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 128;" ::"r"(
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 256;" ::"r"(
                      smem_u32(&tmem_slot))
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   if (tid == 0) {
-    mbar_init(&bar, 1);
+    for (int s = 0; s < kWgStages; ++s) {
+      mbar_init(&full[s], 1);
+      mbar_init(&done[s], 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&tfull[b], 1);
+      mbar_init(&tempty[b], 4);
+    }
     fence_mbar_init();
+    s_abort = 0;
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = tmem_slot;
-  const uint32_t xa = smem_u32(sxs), da = smem_u32(sdy);
-  int phase = 0;
-  bool ok = true, any = false;
-  // dy of plane gz into plane slot b of every shift copy (zeros outside)
-  auto stage_dy_plane = [&](int b, int gz, int x0, int y0) {
-    for (int c = tid; c < 3 * (kWgRows + 2) * kWgX * 2; c += blockDim.x) {
-      const int h = c & 1;
-      int rest = c >> 1;
-      const int k = rest % kWgX;
-      rest /= kWgX;
-      const int r = rest % (kWgRows + 2), sh = rest / (kWgRows + 2);
-      const int gy = y0 - 1 + r, gx = x0 + k - (sh - 1);
-      uint4 v = make_uint4(0u, 0u, 0u, 0u);
-      if (gz >= 0 && gz < D && gy >= 0 && gy < H && gx >= 0 && gx < W)
-        v = *reinterpret_cast<const uint4 *>(dy + (((long long)gz * H + gy) * W + gx) * kC + h * 8);
-      const unsigned short *e = reinterpret_cast<const unsigned short *>(&v);
-      unsigned short *dst =
-          reinterpret_cast<unsigned short *>(sdy + sh * kWgDyBytes + (r * 3 + b) * 256) + k;
-#pragma unroll
-      for (int q = 0; q < 8; ++q) dst[(h * 8 + q) * kWgX] = e[q];
-    }
+  auto give_up = [&]() {
+    s_abort = 1;
+    atomicExch(&g_conv_status, EFWI_STATUS_TIMEOUT);
   };
-  for (long long unit = blockIdx.x; unit < nunits && ok; unit += gridDim.x) {
-    const int xw = (int)(unit % nxw);
-    const long long r0 = unit / nxw;
-    const int yb = (int)(r0 % nyb), zc = (int)(r0 / nyb);
-    const int x0 = xw * kWgX, y0 = yb * kWgRows;
-    const int zb = zc * kWgZ, ze = min(zb + kWgZ, D);
-    for (int z = zb; z < ze && ok; ++z) {
-      if (z == zb) {
-        for (int b = 0; b < 3; ++b) stage_dy_plane(b, z - 1 + b, x0, y0);
-      } else {
-        // planes z-1, z of the new window are planes 1, 2 of the last one:
-        // each thread moves its own 16-byte pieces, then plane z+1 arrives
-        for (int c = tid; c < 3 * (kWgRows + 2) * 16; c += blockDim.x) {
-          const int piece = c & 15, rs = c >> 4;  // rs = shift * (rows) + row
-          uint4 *blk = reinterpret_cast<uint4 *>(sdy + (rs / (kWgRows + 2)) * kWgDyBytes +
-                                                 (rs % (kWgRows + 2)) * 3 * 256);
-          const uint4 p1 = blk[16 + piece], p2 = blk[32 + piece];
-          blk[piece] = p1;
-          blk[16 + piece] = p2;
+  float sum[6][16];  // [2 accumulators x 3 shifts][co] of this thread's row
+#pragma unroll
+  for (int k = 0; k < 6; ++k)
+#pragma unroll
+    for (int q = 0; q < 16; ++q) sum[k][q] = 0.f;
+  if (warp == 4) {
+    if (lane == 0) {
+      auto issue = [&](long long j) {
+        const long long unit = blockIdx.x + j * gridDim.x;
+        const int x0 = (int)(unit % nxw) * kWgX;
+        const long long r = unit / nxw;
+        const int y0 = (int)(r % nyb) * kWgY, z0 = (int)(r / nyb) * kWgZ;
+        const int s = (int)(j % kWgStages);
+        unsigned char *dst = smem + s * kWgStage;
+        mbar_arrive_expect_tx(&full[s], kWgCopied);
+        tma_load_4d(dst, &xmap, &full[s], 0, x0, z0 - 1, y0 - 1);
+        for (int k = 0; k < 3; ++k)
+          tma_load_4d(dst + kWgABytes + k * kWgBCopy, &gmap, &full[s], 0, x0 - (k - 1), y0, z0);
+      };
+      long long nt = 0, nm = 0;  // units whose copies / MMAs were issued
+      for (; nt < kWgStages && nt < nj; ++nt) issue(nt);
+      for (long long j = 0; j < nj && !s_abort; ++j) {
+        const int s = (int)(j % kWgStages);
+        const long long grp = j / kWgGroup;
+        const int b = (int)(grp & 1);
+        const bool first = j % kWgGroup == 0;
+        // the accumulators of group grp - 2 have been drained
+        if (first && grp >= 2 && !mbar_wait_bounded(&tempty[b], (uint32_t)(((grp - 2) >> 1) & 1))) {
+          give_up();
+          break;
         }
-        __syncthreads();  // plane slot 2 is rewritten below by other threads
-        stage_dy_plane(2, z + 1, x0, y0);
-      }
-      // x: voxel (row, k) of plane z, 8 channels per item
-      for (int c = tid; c < kWgRows * kWgX * 2; c += blockDim.x) {
-        const int h = c & 1, k = (c >> 1) % kWgX, row = (c >> 1) / kWgX;
-        const int gy = y0 + row, gx = x0 + k;
-        uint4 v = make_uint4(0u, 0u, 0u, 0u);
-        if (gy < H && gx < W)
-          v = *reinterpret_cast<const uint4 *>(x + (((long long)z * H + gy) * W + gx) * kC + h * 8);
-        const unsigned short *e = reinterpret_cast<const unsigned short *>(&v);
-        unsigned short *dst = reinterpret_cast<unsigned short *>(sxs + row * 256) + k;
-#pragma unroll
-        for (int q = 0; q < 8; ++q) dst[(h * 8 + q) * kWgX] = e[q];
-      }
-      fence_proxy_async_smem();  // staged by the threads, read by the tensor cores
-      __syncthreads();
-      if (tid == 0) {
+        if (!mbar_wait_bounded(&full[s], (uint32_t)((j / kWgStages) & 1))) { give_up(); break; }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t a0 = smem_u32(smem + s * kWgStage), b0 = a0 + kWgABytes;
+        const uint32_t acc0 = tmem + (uint32_t)(2 * kWgCol2 * b);
 #pragma unroll 1
-        for (int r = 0; r < kWgRows; r += 2) {
-          const uint64_t bd = tc_desc(xa + (uint32_t)(r * 256), 256, 128);
+        for (int z = 0; z < kWgZ; ++z) {
+          const uint64_t ad = tc_desc_mn32(a0 + z * 256, 256, kWgZs * 256);
+          const uint64_t bd = tc_desc_mn32(b0 + z * kWgY * 256, kWgBCopy, 256);
 #pragma unroll
-          for (int sh = 0; sh < 3; ++sh) {
-            const uint32_t a0 = da + (uint32_t)(sh * kWgDyBytes + r * 3 * 256);
-            const uint32_t acc = (any || r > 0) ? 1u : 0u;
-            tc_mma(tmem + (uint32_t)(2 * sh * kC), tc_desc(a0, 768, 128), bd, acc);
-            tc_mma(tmem + (uint32_t)((2 * sh + 1) * kC), tc_desc(a0 + 256, 768, 128), bd, acc);
+          for (int r = 0; r < kWgY; r += 2) {
+            const uint32_t acc = (!first || z > 0 || r > 0) ? 1u : 0u;
+            const uint64_t da = ad + (uint64_t)(r * kWgZs * 16), db = bd + (uint64_t)(r * 16);
+            tc_mma_idesc(acc0, da, db, kWgIdesc, acc);
+            tc_mma_idesc(acc0 + kWgCol2, da + 8 * 16, db, kWgIdesc, acc);
           }
         }
-        tc_commit(&bar);
+        tc_commit(&done[s]);
+        if (j % kWgGroup == kWgGroup - 1 || j + 1 == nj) tc_commit(&tfull[b]);
+        nm = j + 1;
+        if (j >= 1 && nt < nj) {  // refill the stage of unit j-1 once its MMAs are done
+          const long long p = j - 1;
+          if (!mbar_wait_bounded(&done[p % kWgStages], (uint32_t)((p / kWgStages) & 1))) {
+            give_up();
+            break;
+          }
+          issue(nt);
+          ++nt;
+        }
       }
-      any = true;
-      // the staged planes are read by the MMAs: wait before changing them
-      ok = __syncthreads_and(mbar_wait_bounded(&bar, (uint32_t)phase));
-      phase ^= 1;
+      // what is still in flight, bounded: copies that no MMA waited for, and
+      // the last unit's MMAs (whose commit covers all before it)
+      for (long long j = nm; j < nt; ++j)
+        mbar_wait_bounded(&full[j % kWgStages], (uint32_t)((j / kWgStages) & 1));
+      if (nm > 0 &&
+          !mbar_wait_bounded(&done[(nm - 1) % kWgStages], (uint32_t)(((nm - 1) / kWgStages) & 1)))
+        give_up();
+    }
+  } else {
+    for (long long grp = 0; grp < ng && !s_abort; ++grp) {
+      const int b = (int)(grp & 1);
+      bool ok = mbar_wait_bounded(&tfull[b], (uint32_t)((grp >> 1) & 1));
+      ok = __all_sync(0xffffffffu, ok);  // tcgen05.ld is warp-collective
+      if (!ok) {
+        if (lane == 0) give_up();
+        break;
+      }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const uint32_t t0 = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(2 * kWgCol2 * b);
+#pragma unroll
+      for (int k = 0; k < 6; ++k) {
+        float v[16];
+        tc_ld16(t0 + (uint32_t)(kWgCol2 * (k / 3) + 16 * (k % 3)), v);
+#pragma unroll
+        for (int q = 0; q < 16; ++q) sum[k][q] += v[q];
+      }
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive1(&tempty[b]);
     }
   }
-  if (!ok && tid == 0) {
-    atomicExch(&g_conv_status, EFWI_STATUS_TIMEOUT);
-    mbar_wait_bounded(&bar, (uint32_t)(phase ^ 1));  // the MMAs still in flight, bounded
-  }
-  // the CTA's sums: accumulator 2s holds taps j = 0..7 of shift s in rows
-  // 16 j + co, accumulator 2s + 1 tap j = 8 in rows 112..127; column = ci
-  float *out = partial + (long long)blockIdx.x * 27 * kC * kC;
-  const float nan = __int_as_float(0x7fc00000);
-#pragma unroll 1
-  for (int acc = 0; acc < 6; ++acc) {
-    float v[16];
+  __syncthreads();
+  // accumulator k / 3, row (block, ci), column (dx', co): tap block 8 (k/3) + row / 16
+  if (warp < 4) {
+    const bool ok = !s_abort;
+    float *out = partial + (long long)blockIdx.x * 27 * kC * kC;
+    const float nan = __int_as_float(0x7fc00000);
+    const int row = warp * 32 + lane, ci = row & 15;
 #pragma unroll
-    for (int q = 0; q < 16; ++q) v[q] = 0.f;
-    if (any && ok) tc_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(acc * kC), v);
-    const int row = warp * 32 + lane, co = row & 15;
-    const int j = (acc & 1) ? 8 : row >> 4;
-    if ((acc & 1) && row < 112) continue;
-    const int a = j / 3, b = j % 3, s = acc >> 1;
-    const int t = (2 - b) * 9 + (2 - a) * 3 + s;  // (dz+1)*9 + (dy+1)*3 + (dx+1)
-    float *o = out + ((long long)t * kC + co) * kC;
+    for (int k = 0; k < 6; ++k) {
+      const int blk = 8 * (k / 3) + (row >> 4), dyp = blk >> 2, dzp = blk & 3;
+      if (dyp > 2 || dzp > 2) continue;
+      float *o = out + (long long)(dzp * 9 + dyp * 3 + k % 3) * kC * kC + ci;
 #pragma unroll
-    for (int q = 0; q < 16; ++q) o[q] = ok ? v[q] : nan;
+      for (int q = 0; q < 16; ++q) o[q * kC] = ok ? sum[k][q] : nan;
+    }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (warp == 0)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 128;" ::"r"(tmem) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 256;" ::"r"(tmem) : "memory");
 }
 
 }  // namespace
@@ -954,6 +1024,36 @@ bool conv_map(CUtensorMap *m, const void *x, int D, int H, int W) {
              es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
+
+// Maps of the weight gradient, a voxel's 32 bytes innermost: x with boxes of
+// 8 x, 4 z, 18 y (in that order in shared memory), dy of 8 x, 16 y, 2 z.
+bool wgrad_maps(CUtensorMap *xm, CUtensorMap *gm, const void *x, const void *dy, int D, int H,
+                int W) {
+  PFN_cuTensorMapEncodeTiled_v12000 enc = conv_encoder();
+  if (!enc) return false;
+  const cuuint64_t w = W, h = H, d = D;
+  cuuint64_t xd[4] = {kC, w, d, h}, xs[3] = {32, 32 * w * h, 32 * w};
+  cuuint64_t gd[4] = {kC, w, h, d}, gs[3] = {32, 32 * w, 32 * w * h};
+  cuuint32_t xb[4] = {kC, kWgX, kWgZs, kWgY + 2}, gb[4] = {kC, kWgX, kWgY, kWgZ};
+  cuuint32_t es[4] = {1, 1, 1, 1};
+  auto one = [&](CUtensorMap *m, const void *p, cuuint64_t *dims, cuuint64_t *str, cuuint32_t *box) {
+    return enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void *>(p), dims, str, box, es,
+               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_32B,
+               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+  };
+  return one(xm, x, xd, xs, xb) && one(gm, dy, gd, gs, gb);
+}
+
+// SM count of the current device.
+bool conv_sms(int *out) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return false;
+  int &sms = g_sm_count[dev & 63];
+  if (!sms && cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    return false;
+  *out = sms;
+  return true;
+}
 }  // namespace
 
 extern "C" int efwi_conv3d_set_kernel(int form) {
@@ -984,11 +1084,8 @@ extern "C" int efwi_conv3d_forward(const void *x, const void *w, const float *bi
   const int form = g_conv_kernel.load();
   if (form != 0 && ((uintptr_t)w & 15) == 0 && ((uintptr_t)y_bf16 & 15) == 0 &&
       ((uintptr_t)y_f32 & 15) == 0) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return 2;
-    int &sms = g_sm_count[dev & 63];
-    if (!sms && cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-      return 2;
+    int sms = 0;
+    if (!conv_sms(&sms)) return 2;
     const long long tiles = (long long)((W + kTcX - 1) / kTcX) * ((H + kTcY - 1) / kTcY) * D;
     if (form >= 2) {
       CUtensorMap map;
@@ -1047,16 +1144,24 @@ extern "C" int efwi_conv3d_wgrad(const void *x, const void *dy, int D, int H, in
                                  float *partial, int nparts, float *dw, void *stream) {
   if (!x || !dy || !partial || !dw || D < 1 || H < 1 || W < 1 || nparts < 1) return 1;
   cudaStream_t st = (cudaStream_t)stream;
-  // the tcgen05 form stages with 16-byte loads; unaligned inputs take mma.sync
+  // the bulk copies need 16-byte aligned volumes; others take mma.sync
+  int parts = nparts;
   if (g_wgrad_kernel.load() == 1 && ((uintptr_t)x & 15) == 0 && ((uintptr_t)dy & 15) == 0) {
+    int sms = 0;
+    if (!conv_sms(&sms)) return 2;
+    CUtensorMap xmap, gmap;
+    if (!wgrad_maps(&xmap, &gmap, x, dy, D, H, W)) return 2;
     set_smem_once(k_conv3d_wgrad_tc, kWgSmem, g_wg_smem_set);
-    k_conv3d_wgrad_tc<<<nparts, kWgThreads, kWgSmem, st>>>(
-        (const __nv_bfloat16 *)x, (const __nv_bfloat16 *)dy, D, H, W, partial);
+    // two resident CTAs per SM (87 KB of shared memory each)
+    const long long units = (long long)((W + kWgX - 1) / kWgX) * ((H + kWgY - 1) / kWgY) *
+                            ((D + kWgZ - 1) / kWgZ);
+    parts = (int)std::min<long long>(std::min<long long>(nparts, 2LL * sms), units);
+    k_conv3d_wgrad_tc<<<parts, kWgThreads, kWgSmem, st>>>(xmap, gmap, D, H, W, partial);
   } else {
     k_conv3d_wgrad<<<nparts, 27 * 32, 0, st>>>((const __nv_bfloat16 *)x,
                                                (const __nv_bfloat16 *)dy, D, H, W, partial);
   }
   const int n = 27 * kC * kC;
-  k_reduce_partials<<<(n + 255) / 256, 256, 0, st>>>(partial, nparts, n, dw);
+  k_reduce_partials<<<(n + 31) / 32, dim3(32, kRedWarps), 0, st>>>(partial, parts, n, dw);
   return cudaGetLastError() == cudaSuccess ? 0 : 2;
 }
