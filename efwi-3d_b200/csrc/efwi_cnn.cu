@@ -204,22 +204,104 @@ k_conv3d_wgrad(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restr
 // eight warps' sums are added in warp order.  One thread per output, reading
 // all partials one after the other, took 40 us for 592 of them.
 constexpr int kRedWarps = 8;
-__global__ void __launch_bounds__(32 * kRedWarps)
-k_reduce_partials(const float *__restrict__ partial, int nparts, int n, float *__restrict__ out) {
+struct Partials {
+  const float *p;  // [parts][n]
+  int parts, n;
+  float *out;
+};
+// Blocks [0, ceil(a.n / 32)) reduce a, the rest b.
+__global__ void __launch_bounds__(32 * kRedWarps) k_reduce_partials(Partials a, Partials b) {
   __shared__ float sum[kRedWarps][32];
-  const int i = blockIdx.x * 32 + threadIdx.x, w = threadIdx.y;
+  const int na = (a.n + 31) / 32;
+  const bool second = (int)blockIdx.x >= na;
+  const Partials r = second ? b : a;
+  const int i = ((int)blockIdx.x - (second ? na : 0)) * 32 + threadIdx.x, w = threadIdx.y;
   float s = 0.f;
-  if (i < n) {
+  if (i < r.n) {
 #pragma unroll 8
-    for (int p = w; p < nparts; p += kRedWarps) s += partial[(long long)p * n + i];
+    for (int p = w; p < r.parts; p += kRedWarps) s += r.p[(long long)p * r.n + i];
   }
   sum[w][threadIdx.x] = s;
   __syncthreads();
-  if (w == 0 && i < n) {
+  if (w == 0 && i < r.n) {
 #pragma unroll
     for (int k = 1; k < kRedWarps; ++k) s += sum[k][threadIdx.x];
-    out[i] = s;
+    r.out[i] = s;
   }
+}
+
+// What the backward pass of a layer needs before its two convolutions, in one
+// pass over the volume: the gradient behind the ReLU, g = gy * (y > 0) in
+// float32 (rounded to BF16 into `dy`), per-CTA sums of g over the voxels (the
+// bias gradient) and the weights of the transposed convolution,
+// wt[t][a][b] = w[26-t][b][a].  A thread takes 8 channels of a voxel, the same
+// half for all its voxels (an even number of threads).
+constexpr int kPrepThreads = 256;
+template <class T>
+__device__ __forceinline__ void ld8(const T *p, float v[8]);
+template <>
+__device__ __forceinline__ void ld8(const __nv_bfloat16 *p, float v[8]) {
+  const uint4 r = *reinterpret_cast<const uint4 *>(p);
+  const uint32_t u[4] = {r.x, r.y, r.z, r.w};
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    v[2 * k] = __uint_as_float(u[k] << 16);
+    v[2 * k + 1] = __uint_as_float(u[k] & 0xffff0000u);
+  }
+}
+template <>
+__device__ __forceinline__ void ld8(const float *p, float v[8]) {
+  const float4 a = *reinterpret_cast<const float4 *>(p), b = *reinterpret_cast<const float4 *>(p + 4);
+  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+  v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+}
+template <class TG, class TY>
+__global__ void __launch_bounds__(kPrepThreads)
+k_conv3d_grad_prep(const TG *__restrict__ gy, const TY *__restrict__ y, long long nhalf,
+                   __nv_bfloat16 *__restrict__ dy, float *__restrict__ dbp,
+                   const __nv_bfloat16 *__restrict__ w, __nv_bfloat16 *__restrict__ wt) {
+  __shared__ float red[kPrepThreads][9];
+  const int tid = threadIdx.x;
+  if (wt)
+    for (int k = blockIdx.x * kPrepThreads + tid; k < 27 * kC * kC; k += gridDim.x * kPrepThreads) {
+      const int t = k / (kC * kC), a = k / kC % kC, b = k % kC;
+      wt[k] = w[((26 - t) * kC + b) * kC + a];
+    }
+  float s[8];
+#pragma unroll
+  for (int q = 0; q < 8; ++q) s[q] = 0.f;
+  for (long long i = blockIdx.x * (long long)kPrepThreads + tid; i < nhalf;
+       i += (long long)gridDim.x * kPrepThreads) {
+    float g[8];
+    ld8(gy + 8 * i, g);
+    if (y) {
+      float v[8];
+      ld8(y + 8 * i, v);
+#pragma unroll
+      for (int q = 0; q < 8; ++q) g[q] *= v[q] > 0.f ? 1.f : 0.f;
+    }
+#pragma unroll
+    for (int q = 0; q < 8; ++q) s[q] += g[q];
+    if (dy) {
+      uint32_t pk[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const __nv_bfloat162 b2 = __floats2bfloat162_rn(g[2 * q], g[2 * q + 1]);
+        pk[q] = *reinterpret_cast<const uint32_t *>(&b2);
+      }
+      *reinterpret_cast<uint4 *>(dy + 8 * i) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < 8; ++q) red[tid][q] = s[q];
+  __syncthreads();
+  for (int n = kPrepThreads / 2; n >= 2; n >>= 1) {  // even strides keep the channel half
+    if (tid < n)
+#pragma unroll
+      for (int q = 0; q < 8; ++q) red[tid][q] += red[tid + n][q];
+    __syncthreads();
+  }
+  if (tid < kC) dbp[(long long)blockIdx.x * kC + tid] = red[tid >> 3][tid & 7];
 }
 
 
@@ -592,6 +674,198 @@ k_conv3d_fwd_tc2(const __grid_constant__ CUtensorMap xmap, const __nv_bfloat16 *
 }
 
 
+// z-marching form (the default).  What bounds the forms above is the operand
+// path: every input voxel is read 27 times, for an MMA of N = 16.  Here a CTA
+// marches the 8 x 16 tile through z, one staged input plane z' at a time, and
+// one MMA per (dy, dx) multiplies it with the weights of all three dz at once:
+// N = 48 = (output planes z'-1, z', z'+1) x 16 channels, so that a voxel is
+// read 9 times.  Output plane p accumulates in TMEM columns 16 (p mod 3); the
+// weights of one (dy, dx) lie in blocks of 16 rows in the dz order 2 1 0 2 1,
+// of which an MMA takes three from block (1 - z') mod 3.  After plane z' the
+// tile of plane z'-1 is complete: the warps read it, set its columns to zero
+// for plane z'+2 and hand over to the next MMAs before they store.  A plane's
+// sums see the taps in the same order as in the forms above (the same bits).
+// Waits inside a CTA are filled by the other CTAs of the SM (six: 35 KB of
+// shared memory and 64 TMEM columns each).
+constexpr int kZmStages = 2;
+constexpr int kZmPlane = kTcSY * kTcSX * 32;                     // a staged plane
+constexpr int kZmStage = (kZmPlane + 255) / 256 * 256;
+constexpr int kZmWTap = 2 * 5 * kC * 16;                         // weights of one (dy, dx)
+constexpr int kZmWBytes = 9 * kZmWTap;
+constexpr int kZmSmem = kZmStages * kZmStage + kZmWBytes + 256;  // + alignment slack
+
+// kind::f16, FP32 accumulator, BF16 K-major operands, N = 48, M = 128.
+constexpr uint32_t kZmIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((48u >> 3) << 17) |
+                              ((128u >> 4) << 24);
+
+__device__ __forceinline__ void tc_mma_idesc(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc,
+                                             uint32_t acc) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d),
+      "l"(a), "l"(b), "r"(idesc), "r"(acc));
+}
+
+// Operand staged with the 32-byte swizzle of the bulk copies.  The pattern
+// lies on 256-byte boundaries of shared memory, so an operand may start at
+// any row of 32 bytes.
+__device__ __forceinline__ uint64_t tc_desc_sw32(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
+  return tc_desc(saddr, lbo, sbo) | (6ull << 61);
+}
+
+__device__ __forceinline__ void tma_load_4d(void *dst, const CUtensorMap *map, uint64_t *bar,
+                                            int c0, int c1, int c2, int c3) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+      " [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(smem_u32(dst)),
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(c3),
+      "r"(smem_u32(bar))
+      : "memory");
+}
+
+// Zeros in 16 TMEM columns of the warp's 32 lanes.
+__device__ __forceinline__ void tc_zero16(uint32_t taddr) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %1, %1, %1, %1, %1, %1, %1, %1, %1, "
+      "%1, %1, %1, %1, %1, %1};" ::"r"(taddr),
+      "r"(0)
+      : "memory");
+  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+
+__global__ void __launch_bounds__(128)
+k_conv3d_fwd_zm(const __grid_constant__ CUtensorMap xmap, const __nv_bfloat16 *__restrict__ w,
+                const float *__restrict__ bias, int D, int H, int W, int zlen, int relu,
+                __nv_bfloat16 *__restrict__ yb, float *__restrict__ yf) {
+  extern __shared__ unsigned char smem_raw[];
+  __shared__ __align__(8) uint64_t full[kZmStages], done;
+  __shared__ uint32_t tmem_slot;
+  __shared__ int s_abort;
+  unsigned char *smem = smem_raw + ((256u - (smem_u32(smem_raw) & 255u)) & 255u);
+  unsigned char *swt = smem + kZmStages * kZmStage;  // [dy][dx][half][5 dz blocks][co] x 16 B
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int ntx = (W + kTcX - 1) / kTcX, nty = (H + kTcY - 1) / kTcY;
+  const int x0 = (int)(blockIdx.x % ntx) * kTcX;
+  const int rest = (int)(blockIdx.x / ntx);
+  const int y0 = rest % nty * kTcY, zb = rest / nty * zlen, ze = min(zb + zlen, D);
+  const int nj = ze - zb + 2;  // input planes zb-1 .. ze
+  auto issue = [&](int j) {    // thread 0: input plane zb-1+j into stage j % kZmStages
+    const int s = j % kZmStages;
+    mbar_arrive_expect_tx(&full[s], kZmPlane);
+    tma_load_4d(smem + s * kZmStage, &xmap, &full[s], 0, x0 - 1, y0 - 1, zb - 1 + j);
+  };
+  int n_tma = 0;
+  if (tid == 0) {
+    for (int s = 0; s < kZmStages; ++s) mbar_init(&full[s], 1);
+    mbar_init(&done, 1);
+    fence_mbar_init();
+    s_abort = 0;
+    for (; n_tma < kZmStages && n_tma < nj; ++n_tma) issue(n_tma);
+  }
+  for (int k = tid; k < 9 * 2 * 5 * kC; k += blockDim.x) {
+    const int co = k % kC, b = k / kC % 5, h = k / (kC * 5) % 2, t = k / (kC * 10);
+    const int dz = (5 - b) % 3;  // blocks in the order 2 1 0 2 1
+    *reinterpret_cast<uint4 *>(swt + k * 16) =
+        *reinterpret_cast<const uint4 *>(w + ((dz * 9 + t) * kC + co) * kC + h * 8);
+  }
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 64;" ::"r"(
+                     smem_u32(&tmem_slot))
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  fence_proxy_async_smem();  // the staged weights are read by the tensor cores
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = tmem_slot, tlane = tmem + ((uint32_t)(warp * 32) << 16);
+  const uint32_t swa = smem_u32(swt);
+  for (int s = 0; s < 3; ++s) tc_zero16(tlane + (uint32_t)(s * kC));
+  float bv[16];
+#pragma unroll
+  for (int q = 0; q < 16; ++q) bv[q] = bias ? bias[q] : 0.f;
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+
+  const int m = warp * 32 + lane;
+  const int xv = x0 + (m & 7), yv = y0 + (m >> 3);
+  const bool inside = xv < W && yv < H;
+  int n_mma = 0;
+  // thread 0: the nine MMAs of input plane j, once its stage landed
+  auto mma = [&](int j) {
+    const int s = j % kZmStages, z = zb - 1 + j;
+    if (!mbar_wait_bounded(&full[s], (uint32_t)((j / kZmStages) & 1))) { s_abort = 1; return; }
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const int b0 = ((1 - z) % 3 + 3) % 3;  // first weight block
+    const uint64_t a = tc_desc_sw32(smem_u32(smem + s * kZmStage), 16, kTcSX * 32);
+    const uint64_t b = tc_desc(swa + (uint32_t)(b0 * kC * 16), 5 * kC * 16, 8 * 16);
+#pragma unroll
+    for (int t = 0; t < 9; ++t)
+      tc_mma_idesc(tmem, a + (uint64_t)(2 * ((t / 3) * kTcSX + t % 3)), b + (uint64_t)(t * (kZmWTap / 16)),
+                   kZmIdesc, 1u);
+    tc_commit(&done);
+    n_mma = j + 1;
+  };
+  if (tid == 0) mma(0);
+  bool ok = true;
+  for (int j = 0; j < nj; ++j) {
+    // every thread takes the same branch: tcgen05.ld is warp-collective
+    ok = __syncthreads_and(!s_abort && mbar_wait_bounded(&done, (uint32_t)(j & 1)));
+    if (!ok) break;
+    if (tid == 0 && n_tma < nj) { issue(n_tma); ++n_tma; }  // into plane j's stage
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const int p = zb - 2 + j;  // the plane that is complete
+    const uint32_t col = tlane + (uint32_t)((p + 3) % 3 * kC);
+    float v[16];
+    tc_ld16(col, v);
+    if (j + 1 < nj) {
+      tc_zero16(col);
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncthreads();
+      if (tid == 0) mma(j + 1);
+    }
+    if (p >= zb && inside) {
+      const long long off = (((long long)p * H + yv) * W + xv) * kC;
+      float o[16];
+#pragma unroll
+      for (int q = 0; q < 16; ++q) {
+        o[q] = v[q] + bv[q];
+        if (relu) o[q] = fmaxf(o[q], 0.f);
+      }
+      if (yb) {
+        uint32_t pk[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          const __nv_bfloat162 b2 = __floats2bfloat162_rn(o[2 * q], o[2 * q + 1]);
+          pk[q] = *reinterpret_cast<const uint32_t *>(&b2);
+        }
+        uint4 *dst = reinterpret_cast<uint4 *>(yb + off);
+        dst[0] = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+        dst[1] = make_uint4(pk[4], pk[5], pk[6], pk[7]);
+      }
+      if (yf) {
+        float4 *dst = reinterpret_cast<float4 *>(yf + off);
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          dst[q] = make_float4(o[4 * q], o[4 * q + 1], o[4 * q + 2], o[4 * q + 3]);
+      }
+    }
+  }
+  if (!ok && tid == 0) {
+    atomicExch(&g_conv_status, EFWI_STATUS_TIMEOUT);
+    // bounded waits for what may still be in flight: the copies of planes
+    // whose MMAs were never issued, and the last MMAs issued
+    for (int j = n_mma; j < n_tma; ++j)
+      mbar_wait_bounded(&full[j % kZmStages], (uint32_t)((j / kZmStages) & 1));
+    if (n_mma > 0) mbar_wait_bounded(&done, (uint32_t)((n_mma - 1) & 1));
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 0)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 64;" ::"r"(tmem) : "memory");
+}
+
+
 // Warp-specialised form of the copy-staged kernel: warp 0 (one elected
 // thread) fills NS stages with bulk tensor copies and issues each tile's 27
 // MMAs into one of two accumulators; warps 1-4 drain the accumulators
@@ -776,8 +1050,9 @@ k_conv3d_fwd_ws(const __grid_constant__ CUtensorMap xmap, const __nv_bfloat16 *_
 // so the blocks of the taps (dy, dz) of one voxel row follow one another:
 // block 4 dy' + dz' (dy' = dy + 1, dz' = dz + 1), the fourth of each four
 // unused.  One MMA with M = 128 takes blocks 0-7, a second blocks 8-15 (of
-// which 8-10 are taps).  dy is staged three times, moved by the three x
-// shifts, so that N = 48 = (dx', co).  K = 16: two voxel rows.
+// which 8-10 are taps).  dy is staged as [z][y][10 x]: the three x shifts are
+// operands that start one voxel (32 bytes) apart, so that N = 48 = (2 - dx',
+// co).  K = 16: two voxel rows.
 // Two accumulators of 48 TMEM columns sum over a group of kWgGroup units;
 // four warps then add them to sums in registers while the next group runs in
 // a second pair: the tensor cores' accumulation truncates, so its error grows
@@ -790,10 +1065,10 @@ k_conv3d_fwd_ws(const __grid_constant__ CUtensorMap xmap, const __nv_bfloat16 *_
 constexpr int kWgX = 8, kWgY = 16, kWgZ = 2;          // voxels of a unit
 constexpr int kWgZs = kWgZ + 2;                       // staged x planes
 constexpr int kWgABytes = (kWgY + 2) * kWgZs * 256;   // staged x
-constexpr int kWgBCopy = kWgZ * kWgY * 256;           // one shifted copy of dy
-constexpr int kWgCopied = kWgABytes + 3 * kWgBCopy;   // bytes of a stage's copies
-constexpr int kWgStage = kWgCopied;
-constexpr int kWgStages = 2;
+constexpr int kWgGX = kWgX + 2;                       // staged dy: x with the shifts
+constexpr int kWgCopied = kWgABytes + kWgZ * kWgY * kWgGX * 32;  // bytes of a stage
+constexpr int kWgStage = (kWgCopied + 255) / 256 * 256;
+constexpr int kWgStages = 3;
 constexpr int kWgSmem = kWgStages * kWgStage + 1024;  // + alignment slack
 constexpr int kWgThreads = 160;
 constexpr int kWgGroup = 4;   // units per accumulator hand-over
@@ -804,30 +1079,6 @@ static_assert(((kWgY - 2 + 1) * kWgZs + kWgZ - 1 + 16) * 256 <= kWgCopied, "in t
 // Both operands MN-major, N = 48, M = 128.
 constexpr uint32_t kWgIdesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) |
                               ((48u >> 3) << 17) | ((128u >> 4) << 24);
-
-// MN-major operand with 32-byte swizzle: blocks of 16 M/N elements `lbo`
-// bytes apart, blocks of 8 K rows `sbo` apart.
-__device__ __forceinline__ uint64_t tc_desc_mn32(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
-  return tc_desc(saddr, lbo, sbo) | (6ull << 61);
-}
-
-__device__ __forceinline__ void tc_mma_idesc(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc,
-                                             uint32_t acc) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d),
-      "l"(a), "l"(b), "r"(idesc), "r"(acc));
-}
-
-__device__ __forceinline__ void tma_load_4d(void *dst, const CUtensorMap *map, uint64_t *bar,
-                                            int c0, int c1, int c2, int c3) {
-  asm volatile(
-      "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(smem_u32(dst)),
-      "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(c3),
-      "r"(smem_u32(bar))
-      : "memory");
-}
 
 __global__ void __launch_bounds__(kWgThreads)
 k_conv3d_wgrad_tc(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap gmap,
@@ -885,8 +1136,7 @@ k_conv3d_wgrad_tc(const __grid_constant__ CUtensorMap xmap, const __grid_constan
         unsigned char *dst = smem + s * kWgStage;
         mbar_arrive_expect_tx(&full[s], kWgCopied);
         tma_load_4d(dst, &xmap, &full[s], 0, x0, z0 - 1, y0 - 1);
-        for (int k = 0; k < 3; ++k)
-          tma_load_4d(dst + kWgABytes + k * kWgBCopy, &gmap, &full[s], 0, x0 - (k - 1), y0, z0);
+        tma_load_4d(dst + kWgABytes, &gmap, &full[s], 0, x0 - 1, y0, z0);
       };
       long long nt = 0, nm = 0;  // units whose copies / MMAs were issued
       for (; nt < kWgStages && nt < nj; ++nt) issue(nt);
@@ -906,12 +1156,12 @@ k_conv3d_wgrad_tc(const __grid_constant__ CUtensorMap xmap, const __grid_constan
         const uint32_t acc0 = tmem + (uint32_t)(2 * kWgCol2 * b);
 #pragma unroll 1
         for (int z = 0; z < kWgZ; ++z) {
-          const uint64_t ad = tc_desc_mn32(a0 + z * 256, 256, kWgZs * 256);
-          const uint64_t bd = tc_desc_mn32(b0 + z * kWgY * 256, kWgBCopy, 256);
+          const uint64_t ad = tc_desc_sw32(a0 + z * 256, 256, kWgZs * 256);
+          const uint64_t bd = tc_desc_sw32(b0 + z * kWgY * kWgGX * 32, 32, kWgGX * 32);
 #pragma unroll
           for (int r = 0; r < kWgY; r += 2) {
             const uint32_t acc = (!first || z > 0 || r > 0) ? 1u : 0u;
-            const uint64_t da = ad + (uint64_t)(r * kWgZs * 16), db = bd + (uint64_t)(r * 16);
+            const uint64_t da = ad + (uint64_t)(r * kWgZs * 16), db = bd + (uint64_t)(r * kWgGX * 2);
             tc_mma_idesc(acc0, da, db, kWgIdesc, acc);
             tc_mma_idesc(acc0 + kWgCol2, da + 8 * 16, db, kWgIdesc, acc);
           }
@@ -961,7 +1211,7 @@ k_conv3d_wgrad_tc(const __grid_constant__ CUtensorMap xmap, const __grid_constan
     }
   }
   __syncthreads();
-  // accumulator k / 3, row (block, ci), column (dx', co): tap block 8 (k/3) + row / 16
+  // accumulator k / 3, row (block, ci), column (2 - dx', co): tap block 8 (k/3) + row / 16
   if (warp < 4) {
     const bool ok = !s_abort;
     float *out = partial + (long long)blockIdx.x * 27 * kC * kC;
@@ -971,7 +1221,7 @@ k_conv3d_wgrad_tc(const __grid_constant__ CUtensorMap xmap, const __grid_constan
     for (int k = 0; k < 6; ++k) {
       const int blk = 8 * (k / 3) + (row >> 4), dyp = blk >> 2, dzp = blk & 3;
       if (dyp > 2 || dzp > 2) continue;
-      float *o = out + (long long)(dzp * 9 + dyp * 3 + k % 3) * kC * kC + ci;
+      float *o = out + (long long)(dzp * 9 + dyp * 3 + 2 - k % 3) * kC * kC + ci;
 #pragma unroll
       for (int q = 0; q < 16; ++q) o[q * kC] = ok ? sum[k][q] : nan;
     }
@@ -1025,8 +1275,20 @@ bool conv_map(CUtensorMap *m, const void *x, int D, int H, int W) {
              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// x with boxes of one plane of 10 x 18 voxels of 32 bytes.
+bool plane_map(CUtensorMap *m, const void *x, int D, int H, int W) {
+  PFN_cuTensorMapEncodeTiled_v12000 enc = conv_encoder();
+  if (!enc) return false;
+  const cuuint64_t w = W, h = H, d = D;
+  cuuint64_t dims[4] = {kC, w, h, d}, strides[3] = {32, 32 * w, 32 * w * h};
+  cuuint32_t box[4] = {kC, kTcSX, kTcSY, 1}, es[4] = {1, 1, 1, 1};
+  return enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void *>(x), dims, strides, box, es,
+             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_32B,
+             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 // Maps of the weight gradient, a voxel's 32 bytes innermost: x with boxes of
-// 8 x, 4 z, 18 y (in that order in shared memory), dy of 8 x, 16 y, 2 z.
+// 8 x, 4 z, 18 y (in that order in shared memory), dy of 10 x, 16 y, 2 z.
 bool wgrad_maps(CUtensorMap *xm, CUtensorMap *gm, const void *x, const void *dy, int D, int H,
                 int W) {
   PFN_cuTensorMapEncodeTiled_v12000 enc = conv_encoder();
@@ -1034,7 +1296,7 @@ bool wgrad_maps(CUtensorMap *xm, CUtensorMap *gm, const void *x, const void *dy,
   const cuuint64_t w = W, h = H, d = D;
   cuuint64_t xd[4] = {kC, w, d, h}, xs[3] = {32, 32 * w * h, 32 * w};
   cuuint64_t gd[4] = {kC, w, h, d}, gs[3] = {32, 32 * w, 32 * w * h};
-  cuuint32_t xb[4] = {kC, kWgX, kWgZs, kWgY + 2}, gb[4] = {kC, kWgX, kWgY, kWgZ};
+  cuuint32_t xb[4] = {kC, kWgX, kWgZs, kWgY + 2}, gb[4] = {kC, kWgGX, kWgY, kWgZ};
   cuuint32_t es[4] = {1, 1, 1, 1};
   auto one = [&](CUtensorMap *m, const void *p, cuuint64_t *dims, cuuint64_t *str, cuuint32_t *box) {
     return enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void *>(p), dims, str, box, es,
@@ -1089,7 +1351,7 @@ extern "C" int efwi_conv3d_forward(const void *x, const void *w, const float *bi
     const long long tiles = (long long)((W + kTcX - 1) / kTcX) * ((H + kTcY - 1) / kTcY) * D;
     if (form >= 2) {
       CUtensorMap map;
-      if (!conv_map(&map, x, D, H, W)) return 2;
+      if (!(form == 2 ? plane_map(&map, x, D, H, W) : conv_map(&map, x, D, H, W))) return 2;
       if (form >= 4) {  // warp-specialised: two stages at 4 CTAs per SM, or three at 3
         const __nv_bfloat16 *wb = (const __nv_bfloat16 *)w;
         if (form == 4) {
@@ -1103,11 +1365,25 @@ extern "C" int efwi_conv3d_forward(const void *x, const void *w, const float *bi
           k_conv3d_fwd_ws<3><<<blocks, kWsThreads, tc2_smem<3>(), st>>>(
               map, wb, bias, D, H, W, relu, (__nv_bfloat16 *)y_bf16, y_f32);
         }
-      } else if (form == 2) {  // two stages, 49 KB of shared memory: 4 CTAs per SM
-        set_smem_once(k_conv3d_fwd_tc2<2>, tc2_smem<2>(), g_tc2_smem_set);
-        const int blocks = (int)std::min<long long>(tiles, 4LL * sms);
-        k_conv3d_fwd_tc2<2><<<blocks, 128, tc2_smem<2>(), st>>>(
-            map, (const __nv_bfloat16 *)w, bias, D, H, W, relu, (__nv_bfloat16 *)y_bf16, y_f32);
+      } else if (form == 2) {
+        // planes per CTA: the fewest steps (waves of 6 CTAs per SM times the
+        // planes that a CTA reads)
+        const long long cols = tiles / D, slots = 6LL * sms;
+        long long best = -1;
+        int zlen = D;
+        for (int n = 1; n <= D; ++n) {
+          const int len = (D + n - 1) / n;
+          const long long ctas = cols * ((D + len - 1) / len);
+          const long long steps = ((ctas + slots - 1) / slots) * (len + 2);
+          if (best < 0 || steps < best) { best = steps; zlen = len; }
+          if (ctas > 8 * slots) break;
+        }
+        const long long ctas = cols * ((D + zlen - 1) / zlen);
+        if (ctas > 0x7fffffffLL) return 1;
+        set_smem_once(k_conv3d_fwd_zm, kZmSmem, g_tc2_smem_set);
+        k_conv3d_fwd_zm<<<(unsigned)ctas, 128, kZmSmem, st>>>(
+            map, (const __nv_bfloat16 *)w, bias, D, H, W, zlen, relu, (__nv_bfloat16 *)y_bf16,
+            y_f32);
       } else {  // three stages, 66 KB: 3 CTAs per SM
         set_smem_once(k_conv3d_fwd_tc2<3>, tc2_smem<3>(), g_tc3_smem_set);
         const int blocks = (int)std::min<long long>(tiles, 3LL * sms);
@@ -1140,28 +1416,89 @@ extern "C" int efwi_conv3d_set_wgrad_kernel(int tcgen05) {
   return 0;
 }
 
-extern "C" int efwi_conv3d_wgrad(const void *x, const void *dy, int D, int H, int W,
-                                 float *partial, int nparts, float *dw, void *stream) {
-  if (!x || !dy || !partial || !dw || D < 1 || H < 1 || W < 1 || nparts < 1) return 1;
-  cudaStream_t st = (cudaStream_t)stream;
+namespace {
+// Partial sums of the weight gradient; *parts: how many were written.
+int wgrad_partials(const void *x, const void *dy, int D, int H, int W, float *partial, int nparts,
+                   int *parts, cudaStream_t st) {
+  *parts = nparts;
   // the bulk copies need 16-byte aligned volumes; others take mma.sync
-  int parts = nparts;
   if (g_wgrad_kernel.load() == 1 && ((uintptr_t)x & 15) == 0 && ((uintptr_t)dy & 15) == 0) {
     int sms = 0;
     if (!conv_sms(&sms)) return 2;
     CUtensorMap xmap, gmap;
     if (!wgrad_maps(&xmap, &gmap, x, dy, D, H, W)) return 2;
     set_smem_once(k_conv3d_wgrad_tc, kWgSmem, g_wg_smem_set);
-    // two resident CTAs per SM (87 KB of shared memory each)
+    // two resident CTAs per SM (87 KB of shared memory, half of TMEM each)
     const long long units = (long long)((W + kWgX - 1) / kWgX) * ((H + kWgY - 1) / kWgY) *
                             ((D + kWgZ - 1) / kWgZ);
-    parts = (int)std::min<long long>(std::min<long long>(nparts, 2LL * sms), units);
-    k_conv3d_wgrad_tc<<<parts, kWgThreads, kWgSmem, st>>>(xmap, gmap, D, H, W, partial);
+    *parts = (int)std::min<long long>(std::min<long long>(nparts, 2LL * sms), units);
+    k_conv3d_wgrad_tc<<<*parts, kWgThreads, kWgSmem, st>>>(xmap, gmap, D, H, W, partial);
   } else {
     k_conv3d_wgrad<<<nparts, 27 * 32, 0, st>>>((const __nv_bfloat16 *)x,
                                                (const __nv_bfloat16 *)dy, D, H, W, partial);
   }
-  const int n = 27 * kC * kC;
-  k_reduce_partials<<<(n + 31) / 32, dim3(32, kRedWarps), 0, st>>>(partial, parts, n, dw);
+  return 0;
+}
+
+void reduce_partials(const Partials &a, const Partials &b, cudaStream_t st) {
+  k_reduce_partials<<<(a.n + 31) / 32 + (b.n + 31) / 32, dim3(32, kRedWarps), 0, st>>>(a, b);
+}
+}  // namespace
+
+extern "C" int efwi_conv3d_wgrad(const void *x, const void *dy, int D, int H, int W,
+                                 float *partial, int nparts, float *dw, void *stream) {
+  if (!x || !dy || !partial || !dw || D < 1 || H < 1 || W < 1 || nparts < 1) return 1;
+  cudaStream_t st = (cudaStream_t)stream;
+  int parts = 0;
+  const int rc = wgrad_partials(x, dy, D, H, W, partial, nparts, &parts, st);
+  if (rc) return rc;
+  reduce_partials({partial, parts, 27 * kC * kC, dw}, {nullptr, 0, 0, nullptr}, st);
+  return cudaGetLastError() == cudaSuccess ? 0 : 2;
+}
+
+extern "C" long long efwi_conv3d_backward_scratch(int D, int H, int W, int nparts, int gy_f32,
+                                                  int relu) {
+  if (D < 1 || H < 1 || W < 1 || nparts < 1) return -1;
+  const long long vox = (long long)D * H * W;
+  const bool own = gy_f32 || relu;  // a BF16 copy of the gradient is written
+  return (own ? vox * kC * 2 : 0) + 27LL * kC * kC * 2 + (27LL * kC * kC + kC) * 4 * nparts;
+}
+
+extern "C" int efwi_conv3d_backward(const void *x, const void *w, const void *gy, int gy_f32,
+                                    const void *y, int y_f32, int D, int H, int W, void *scratch,
+                                    int nparts, void *dx, float *dw, float *db, void *stream) {
+  if (!x || !w || !gy || !scratch || !dw || !db || D < 1 || H < 1 || W < 1 || nparts < 1) return 1;
+  if ((((uintptr_t)x | (uintptr_t)gy | (uintptr_t)y | (uintptr_t)scratch | (uintptr_t)dx) & 15) != 0)
+    return 1;
+  cudaStream_t st = (cudaStream_t)stream;
+  const long long vox = (long long)D * H * W;
+  const bool own = gy_f32 || y;
+  char *p = (char *)scratch;
+  __nv_bfloat16 *dyb = own ? (__nv_bfloat16 *)p : nullptr;
+  if (own) p += vox * kC * 2;
+  __nv_bfloat16 *wt = (__nv_bfloat16 *)p;
+  p += 27 * kC * kC * 2;
+  float *dbp = (float *)p, *partial = dbp + (long long)kC * nparts;
+  const int blocks = (int)std::min<long long>(nparts, (2 * vox + kPrepThreads - 1) / kPrepThreads);
+  const __nv_bfloat16 *wb = (const __nv_bfloat16 *)w;
+  auto prep = [&](auto g, auto yy) {
+    k_conv3d_grad_prep<<<blocks, kPrepThreads, 0, st>>>(g, yy, 2 * vox, dyb, dbp, wb,
+                                                        dx ? wt : nullptr);
+  };
+  const __nv_bfloat16 *gb = (const __nv_bfloat16 *)gy, *ybf = (const __nv_bfloat16 *)y;
+  const float *gf = (const float *)gy, *yf = (const float *)y;
+  if (gy_f32 && y_f32) prep(gf, yf);
+  else if (gy_f32) prep(gf, ybf);
+  else if (y_f32) prep(gb, yf);
+  else prep(gb, ybf);
+  const void *dy = own ? (const void *)dyb : gy;
+  if (dx) {
+    const int rc = efwi_conv3d_forward(dy, wt, nullptr, D, H, W, 0, dx, nullptr, stream);
+    if (rc) return rc;
+  }
+  int parts = 0;
+  const int rc = wgrad_partials(x, dy, D, H, W, partial, nparts, &parts, st);
+  if (rc) return rc;
+  reduce_partials({partial, parts, 27 * kC * kC, dw}, {dbp, blocks, kC, db}, st);
   return cudaGetLastError() == cudaSuccess ? 0 : 2;
 }

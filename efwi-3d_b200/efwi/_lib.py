@@ -103,6 +103,10 @@ _SIGS = {
                                       C.c_int, C.c_int, C.c_void_p, C.c_void_p, C.c_void_p]),
     "efwi_conv3d_wgrad": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int,
                                     C.c_void_p, C.c_int, C.c_void_p, C.c_void_p]),
+    "efwi_conv3d_backward_scratch": (C.c_longlong, [C.c_int] * 6),
+    "efwi_conv3d_backward": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_void_p,
+                                       C.c_int, C.c_int, C.c_int, C.c_int, C.c_void_p, C.c_int,
+                                       C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]),
     "efwi_conv3d_set_kernel": (C.c_int, [C.c_int]),
     "efwi_conv3d_status": (C.c_int, [C.POINTER(C.c_int), C.c_void_p]),
     "efwi_conv3d_set_wgrad_kernel": (C.c_int, [C.c_int]),

@@ -51,9 +51,9 @@ def set_conv_kernel(form: str) -> None:
     """Kernel of every later forward / input-gradient convolution of this
     process: 'mma' (mma.sync m16n8k16), 'tcgen05' (tensor-memory accumulator,
     one MMA per tap for 128 voxels, tile staged by loads), 'tcgen05-tma'
-    (the same MMAs, tiles staged by bulk tensor copies two stages deep, the
-    next tile's MMAs overlapping this tile's epilogue; the default),
-    'tcgen05-tma3' (three stages, fewer CTAs per SM), 'tcgen05-ws' /
+    (z-marching, one MMA per (dy, dx) for the three dz, planes staged by bulk
+    tensor copies; the default), 'tcgen05-tma3' (one MMA per tap, tiles staged
+    by bulk tensor copies three stages deep), 'tcgen05-ws' /
     'tcgen05-ws3' (warp-specialised: one warp issues the copies and MMAs,
     four drain the accumulators, mbarriers between them; two / three
     stages)."""
@@ -96,6 +96,30 @@ def conv3d_wgrad(x: torch.Tensor, dy: torch.Tensor, nparts: int = 592) -> torch.
     return dw
 
 
+def conv3d_backward(x: torch.Tensor, wb: torch.Tensor, gy: torch.Tensor, y, want_dx: bool,
+                    nparts: int = 592):
+    """(dx or None, dw, db) of one layer: g = gy * (y > 0) in float32 (y None:
+    no ReLU), dx and dw from g in BF16, db = sum of g over the voxels."""
+    D, H, W = x.shape[:3]
+    gy = gy.contiguous() if gy.dtype in (torch.bfloat16, torch.float32) else gy.float().contiguous()
+    if gy.data_ptr() & 15:
+        gy = gy.clone()
+    gf, relu = int(gy.dtype == torch.float32), int(y is not None)
+    L = lib()
+    n = L.efwi_conv3d_backward_scratch(D, H, W, nparts, gf, relu)
+    scratch = torch.empty(n, device=x.device, dtype=torch.uint8)
+    dx = torch.empty_like(x) if want_dx else None
+    dw = torch.empty(27, C16, C16, device=x.device, dtype=torch.float32)
+    db = torch.empty(C16, device=x.device, dtype=torch.float32)
+    with torch.cuda.device(x.device):
+        rc = L.efwi_conv3d_backward(_ptr(x), _ptr(wb), _ptr(gy), gf, _ptr(y),
+                                    int(relu and y.dtype == torch.float32), D, H, W, _ptr(scratch),
+                                    nparts, _ptr(dx), _ptr(dw), _ptr(db), _stream(x.device))
+    if rc:
+        raise RuntimeError(f"efwi_conv3d_backward failed ({rc})")
+    return dx, dw, db
+
+
 class Conv3dBF16(torch.autograd.Function):
     """One layer: y = relu?(conv(x, w) + b) with BF16 operands."""
 
@@ -110,15 +134,8 @@ class Conv3dBF16(torch.autograd.Function):
     @staticmethod
     def backward(ctx, gy):
         x, wb, y = ctx.saved_tensors
-        g = gy.float()
-        if ctx.relu:
-            g = g * (y > 0)
-        dyb = g.to(torch.bfloat16).contiguous()
-        wt = wb.flip(0).transpose(1, 2).contiguous()  # w'[t][a][b] = w[26-t][b][a]
-        dx = conv3d_raw(dyb, wt, None, False) if ctx.needs_input_grad[0] else None
-        dw = conv3d_wgrad(x, dyb)
-        db = g.sum(dim=(0, 1, 2))
-        return dx, dw, db, None, None
+        return (*conv3d_backward(x, wb, gy, y if ctx.relu else None, ctx.needs_input_grad[0]),
+                None, None)
 
 
 def to_channels_last(feats: torch.Tensor) -> torch.Tensor:

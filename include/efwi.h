@@ -275,12 +275,23 @@ int efwi_conv3d_forward(const void *x, const void *w, const float *bias, int D, 
                         int relu, void *y_bf16, float *y_f32, void *stream);
 int efwi_conv3d_wgrad(const void *x, const void *dy, int D, int H, int W, float *partial,
                       int nparts, float *dw, void *stream);
+/* Backward pass of one layer y = relu?(conv(x, w) + bias) in four launches:
+ * with g = gy (y > 0) in float32 (y NULL: no ReLU, g = gy), dx = the input
+ * gradient of bf16(g) (bf16; NULL: not wanted), dw as efwi_conv3d_wgrad of
+ * x and bf16(g), db[co] = sum over voxels of g.  gy and y are bf16, or f32
+ * where gy_f32 / y_f32 is set; all pointers 16-byte aligned.  scratch:
+ * efwi_conv3d_backward_scratch bytes (relu: whether y is given). */
+long long efwi_conv3d_backward_scratch(int D, int H, int W, int nparts, int gy_f32, int relu);
+int efwi_conv3d_backward(const void *x, const void *w, const void *gy, int gy_f32, const void *y,
+                         int y_f32, int D, int H, int W, void *scratch, int nparts, void *dx,
+                         float *dw, float *db, void *stream);
 /* Kernel form of efwi_conv3d_forward for this process: 0 = mma.sync;
  * 1 = tcgen05.mma with the accumulator in tensor memory (128 voxels x 16
- * channels per tile, one MMA per tap), tile staged by loads; 2 / 3 = the
- * same MMAs with the tiles staged by bulk tensor copies two / three stages
- * deep and the next tile's MMAs overlapping this tile's epilogue; 4 / 5 =
- * the same warp-specialised (one warp issues the copies and MMAs, four
+ * channels per tile, one MMA per tap), tile staged by loads; 2 = z-marching,
+ * one MMA per (dy, dx) for the three dz, planes staged by bulk tensor
+ * copies; 3 = the MMAs of 1 with the tiles staged by bulk tensor copies three
+ * stages deep and the next tile's MMAs overlapping this tile's epilogue; 4 /
+ * 5 = the same warp-specialised (one warp issues the copies and MMAs, four
  * drain the accumulators; mbarriers between them), two / three stages.  All
  * give the same sums up to FP32 rounding order.  The tcgen05 forms need w
  * and the outputs 16-byte aligned and fall back to mma.sync otherwise.
