@@ -255,6 +255,20 @@ __device__ __forceinline__ void ld8(const float *p, float v[8]) {
   v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
   v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
 }
+// A gradient of channel 0 alone, [voxel] f32: the others are zero.
+struct Head {
+  float v;
+};
+template <class T>
+__device__ __forceinline__ void ld8_at(const T *p, long long i, float v[8]) {
+  ld8(p + 8 * i, v);
+}
+template <>
+__device__ __forceinline__ void ld8_at(const Head *p, long long i, float v[8]) {
+#pragma unroll
+  for (int q = 0; q < 8; ++q) v[q] = 0.f;
+  if ((i & 1) == 0) v[0] = p[i >> 1].v;
+}
 template <class TG, class TY>
 __global__ void __launch_bounds__(kPrepThreads)
 k_conv3d_grad_prep(const TG *__restrict__ gy, const TY *__restrict__ y, long long nhalf,
@@ -273,7 +287,7 @@ k_conv3d_grad_prep(const TG *__restrict__ gy, const TY *__restrict__ y, long lon
   for (long long i = blockIdx.x * (long long)kPrepThreads + tid; i < nhalf;
        i += (long long)gridDim.x * kPrepThreads) {
     float g[8];
-    ld8(gy + 8 * i, g);
+    ld8_at(gy, i, g);
     if (y) {
       float v[8];
       ld8(y + 8 * i, v);
@@ -736,7 +750,7 @@ __device__ __forceinline__ void tc_zero16(uint32_t taddr) {
 __global__ void __launch_bounds__(128)
 k_conv3d_fwd_zm(const __grid_constant__ CUtensorMap xmap, const __nv_bfloat16 *__restrict__ w,
                 const float *__restrict__ bias, int D, int H, int W, int zlen, int relu,
-                __nv_bfloat16 *__restrict__ yb, float *__restrict__ yf) {
+                __nv_bfloat16 *__restrict__ yb, float *__restrict__ yf, float *__restrict__ y0c) {
   extern __shared__ unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t full[kZmStages], done;
   __shared__ uint32_t tmem_slot;
@@ -832,6 +846,7 @@ k_conv3d_fwd_zm(const __grid_constant__ CUtensorMap xmap, const __nv_bfloat16 *_
         o[q] = v[q] + bv[q];
         if (relu) o[q] = fmaxf(o[q], 0.f);
       }
+      if (y0c) y0c[((long long)p * H + yv) * W + xv] = o[0];
       if (yb) {
         uint32_t pk[8];
 #pragma unroll
@@ -1232,6 +1247,23 @@ k_conv3d_wgrad_tc(const __grid_constant__ CUtensorMap xmap, const __grid_constan
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 256;" ::"r"(tmem) : "memory");
 }
 
+// out[v] = channels [v][16] of feats [c][v], zeros from c on.
+__global__ void __launch_bounds__(256)
+k_channels_last(const float *__restrict__ feats, int c, long long vox, __nv_bfloat16 *__restrict__ out) {
+  for (long long v = blockIdx.x * 256LL + threadIdx.x; v < vox; v += gridDim.x * 256LL) {
+    uint32_t pk[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const float a = 2 * q < c ? feats[(2 * q) * vox + v] : 0.f;
+      const float b = 2 * q + 1 < c ? feats[(2 * q + 1) * vox + v] : 0.f;
+      const __nv_bfloat162 b2 = __floats2bfloat162_rn(a, b);
+      pk[q] = *reinterpret_cast<const uint32_t *>(&b2);
+    }
+    uint4 *dst = reinterpret_cast<uint4 *>(out + v * kC);
+    dst[0] = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+    dst[1] = make_uint4(pk[4], pk[5], pk[6], pk[7]);
+  }
+}
 }  // namespace
 }  // namespace efwi
 
@@ -1338,6 +1370,56 @@ extern "C" int efwi_conv3d_status(int *timed_out, void *stream) {
   return 0;
 }
 
+namespace {
+// The z-marching form; y0c: channel 0 alone, [D][H][W] f32.
+int zm_launch(const CUtensorMap &map, const void *w, const float *bias, int D, int H, int W,
+              int relu, void *y_bf16, float *y_f32, float *y0c, cudaStream_t st) {
+  int sms = 0;
+  if (!conv_sms(&sms)) return 2;
+  // planes per CTA: the fewest steps (waves of 6 CTAs per SM times the planes
+  // that a CTA reads)
+  const long long cols = (long long)((W + kTcX - 1) / kTcX) * ((H + kTcY - 1) / kTcY);
+  const long long slots = 6LL * sms;
+  long long best = -1;
+  int zlen = D;
+  for (int n = 1; n <= D; ++n) {
+    const int len = (D + n - 1) / n;
+    const long long ctas = cols * ((D + len - 1) / len);
+    const long long steps = ((ctas + slots - 1) / slots) * (len + 2);
+    if (best < 0 || steps < best) { best = steps; zlen = len; }
+    if (ctas > 8 * slots) break;
+  }
+  const long long ctas = cols * ((D + zlen - 1) / zlen);
+  if (ctas > 0x7fffffffLL) return 1;
+  set_smem_once(k_conv3d_fwd_zm, kZmSmem, g_tc2_smem_set);
+  k_conv3d_fwd_zm<<<(unsigned)ctas, 128, kZmSmem, st>>>(map, (const __nv_bfloat16 *)w, bias, D, H,
+                                                        W, zlen, relu, (__nv_bfloat16 *)y_bf16,
+                                                        y_f32, y0c);
+  return 0;
+}
+
+}  // namespace
+
+extern "C" int efwi_channels_last(const float *feats, int c, long long voxels, void *out,
+                                  void *stream) {
+  if (!feats || !out || c < 1 || c > kC || voxels < 1 || ((uintptr_t)out & 15) != 0) return 1;
+  const int blocks = (int)std::min<long long>((voxels + 255) / 256, 16384);
+  k_channels_last<<<blocks, 256, 0, (cudaStream_t)stream>>>(feats, c, voxels, (__nv_bfloat16 *)out);
+  return cudaGetLastError() == cudaSuccess ? 0 : 2;
+}
+
+extern "C" int efwi_conv3d_forward_head(const void *x, const void *w, const float *bias, int D,
+                                        int H, int W, int relu, float *y, void *stream) {
+  if (!x || !w || !y || D < 1 || H < 1 || W < 1 || D > 65535) return 1;
+  if ((((uintptr_t)x | (uintptr_t)w) & 15) != 0) return 1;
+  if (g_conv_kernel.load() != 2) return 3;
+  CUtensorMap map;
+  if (!plane_map(&map, x, D, H, W)) return 2;
+  const int rc = zm_launch(map, w, bias, D, H, W, relu, nullptr, nullptr, y, (cudaStream_t)stream);
+  if (rc) return rc;
+  return cudaGetLastError() == cudaSuccess ? 0 : 2;
+}
+
 extern "C" int efwi_conv3d_forward(const void *x, const void *w, const float *bias, int D, int H,
                                    int W, int relu, void *y_bf16, float *y_f32, void *stream) {
   if (!x || !w || D < 1 || H < 1 || W < 1 || D > 65535 || (!y_bf16 && !y_f32)) return 1;
@@ -1366,24 +1448,8 @@ extern "C" int efwi_conv3d_forward(const void *x, const void *w, const float *bi
               map, wb, bias, D, H, W, relu, (__nv_bfloat16 *)y_bf16, y_f32);
         }
       } else if (form == 2) {
-        // planes per CTA: the fewest steps (waves of 6 CTAs per SM times the
-        // planes that a CTA reads)
-        const long long cols = tiles / D, slots = 6LL * sms;
-        long long best = -1;
-        int zlen = D;
-        for (int n = 1; n <= D; ++n) {
-          const int len = (D + n - 1) / n;
-          const long long ctas = cols * ((D + len - 1) / len);
-          const long long steps = ((ctas + slots - 1) / slots) * (len + 2);
-          if (best < 0 || steps < best) { best = steps; zlen = len; }
-          if (ctas > 8 * slots) break;
-        }
-        const long long ctas = cols * ((D + zlen - 1) / zlen);
-        if (ctas > 0x7fffffffLL) return 1;
-        set_smem_once(k_conv3d_fwd_zm, kZmSmem, g_tc2_smem_set);
-        k_conv3d_fwd_zm<<<(unsigned)ctas, 128, kZmSmem, st>>>(
-            map, (const __nv_bfloat16 *)w, bias, D, H, W, zlen, relu, (__nv_bfloat16 *)y_bf16,
-            y_f32);
+        const int rc = zm_launch(map, w, bias, D, H, W, relu, y_bf16, y_f32, nullptr, st);
+        if (rc) return rc;
       } else {  // three stages, 66 KB: 3 CTAs per SM
         set_smem_once(k_conv3d_fwd_tc2<3>, tc2_smem<3>(), g_tc3_smem_set);
         const int blocks = (int)std::min<long long>(tiles, 3LL * sms);
@@ -1468,6 +1534,7 @@ extern "C" int efwi_conv3d_backward(const void *x, const void *w, const void *gy
                                     const void *y, int y_f32, int D, int H, int W, void *scratch,
                                     int nparts, void *dx, float *dw, float *db, void *stream) {
   if (!x || !w || !gy || !scratch || !dw || !db || D < 1 || H < 1 || W < 1 || nparts < 1) return 1;
+  if (gy_f32 < 0 || gy_f32 > 2 || (gy_f32 == 2 && y)) return 1;
   if ((((uintptr_t)x | (uintptr_t)gy | (uintptr_t)y | (uintptr_t)scratch | (uintptr_t)dx) & 15) != 0)
     return 1;
   cudaStream_t st = (cudaStream_t)stream;
@@ -1487,7 +1554,8 @@ extern "C" int efwi_conv3d_backward(const void *x, const void *w, const void *gy
   };
   const __nv_bfloat16 *gb = (const __nv_bfloat16 *)gy, *ybf = (const __nv_bfloat16 *)y;
   const float *gf = (const float *)gy, *yf = (const float *)y;
-  if (gy_f32 && y_f32) prep(gf, yf);
+  if (gy_f32 == 2) prep((const Head *)gy, ybf);
+  else if (gy_f32 && y_f32) prep(gf, yf);
   else if (gy_f32) prep(gf, ybf);
   else if (y_f32) prep(gb, yf);
   else prep(gb, ybf);

@@ -103,6 +103,9 @@ _SIGS = {
                                       C.c_int, C.c_int, C.c_void_p, C.c_void_p, C.c_void_p]),
     "efwi_conv3d_wgrad": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int,
                                     C.c_void_p, C.c_int, C.c_void_p, C.c_void_p]),
+    "efwi_conv3d_forward_head": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_int,
+                                           C.c_int, C.c_int, C.c_void_p, C.c_void_p]),
+    "efwi_channels_last": (C.c_int, [C.c_void_p, C.c_int, C.c_longlong, C.c_void_p, C.c_void_p]),
     "efwi_conv3d_backward_scratch": (C.c_longlong, [C.c_int] * 6),
     "efwi_conv3d_backward": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_void_p,
                                        C.c_int, C.c_int, C.c_int, C.c_int, C.c_void_p, C.c_int,

@@ -9,6 +9,7 @@ optimizer trains them.  No reference counterpart.
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes as C
 import math
 
@@ -20,11 +21,18 @@ C16 = 16
 
 
 def _ptr(t):
-    return C.c_void_p(t.data_ptr()) if t is not None else C.c_void_p(0)
+    return t.data_ptr() if t is not None else None
 
 
 def _stream(dev):
     return C.c_void_p(torch.cuda.current_stream(dev).cuda_stream)
+
+
+def _on(dev):
+    """The device as the current one (nothing to do where it is already)."""
+    if torch.cuda.current_device() == dev.index:
+        return contextlib.nullcontext()
+    return torch.cuda.device(dev)
 
 
 def conv3d_raw(x: torch.Tensor, wb: torch.Tensor, bias, relu: bool, out_f32: bool = False):
@@ -35,7 +43,7 @@ def conv3d_raw(x: torch.Tensor, wb: torch.Tensor, bias, relu: bool, out_f32: boo
     yb = None if out_f32 else torch.empty_like(x)
     yf = torch.empty(x.shape, device=x.device, dtype=torch.float32) if out_f32 else None
     b = bias.float().contiguous() if bias is not None else None
-    with torch.cuda.device(x.device):
+    with _on(x.device):
         rc = lib().efwi_conv3d_forward(_ptr(x), _ptr(wb), _ptr(b), D, H, W, int(relu), _ptr(yb),
                                        _ptr(yf), _stream(x.device))
     if rc:
@@ -88,7 +96,7 @@ def conv3d_wgrad(x: torch.Tensor, dy: torch.Tensor, nparts: int = 592) -> torch.
     D, H, W = x.shape[:3]
     partial = torch.empty(nparts * 27 * C16 * C16, device=x.device, dtype=torch.float32)
     dw = torch.empty(27, C16, C16, device=x.device, dtype=torch.float32)
-    with torch.cuda.device(x.device):
+    with _on(x.device):
         rc = lib().efwi_conv3d_wgrad(_ptr(x), _ptr(dy), D, H, W, _ptr(partial), nparts, _ptr(dw),
                                      _stream(x.device))
     if rc:
@@ -99,20 +107,26 @@ def conv3d_wgrad(x: torch.Tensor, dy: torch.Tensor, nparts: int = 592) -> torch.
 def conv3d_backward(x: torch.Tensor, wb: torch.Tensor, gy: torch.Tensor, y, want_dx: bool,
                     nparts: int = 592):
     """(dx or None, dw, db) of one layer: g = gy * (y > 0) in float32 (y None:
-    no ReLU), dx and dw from g in BF16, db = sum of g over the voxels."""
+    no ReLU), dx and dw from g in BF16, db = sum of g over the voxels.  A gy
+    [D, H, W] is the gradient of channel 0 alone."""
     D, H, W = x.shape[:3]
-    gy = gy.contiguous() if gy.dtype in (torch.bfloat16, torch.float32) else gy.float().contiguous()
+    if gy.dim() == 3:
+        gy, kind = gy.float().contiguous(), 2
+    else:
+        if gy.dtype != torch.bfloat16:
+            gy = gy.float()
+        gy, kind = gy.contiguous(), int(gy.dtype == torch.float32)
     if gy.data_ptr() & 15:
         gy = gy.clone()
-    gf, relu = int(gy.dtype == torch.float32), int(y is not None)
+    relu = int(y is not None)
     L = lib()
-    n = L.efwi_conv3d_backward_scratch(D, H, W, nparts, gf, relu)
+    n = L.efwi_conv3d_backward_scratch(D, H, W, nparts, kind, relu)
     scratch = torch.empty(n, device=x.device, dtype=torch.uint8)
     dx = torch.empty_like(x) if want_dx else None
     dw = torch.empty(27, C16, C16, device=x.device, dtype=torch.float32)
     db = torch.empty(C16, device=x.device, dtype=torch.float32)
-    with torch.cuda.device(x.device):
-        rc = L.efwi_conv3d_backward(_ptr(x), _ptr(wb), _ptr(gy), gf, _ptr(y),
+    with _on(x.device):
+        rc = L.efwi_conv3d_backward(_ptr(x), _ptr(wb), _ptr(gy), kind, _ptr(y),
                                     int(relu and y.dtype == torch.float32), D, H, W, _ptr(scratch),
                                     nparts, _ptr(dx), _ptr(dw), _ptr(db), _stream(x.device))
     if rc:
@@ -138,9 +152,76 @@ class Conv3dBF16(torch.autograd.Function):
                 None, None)
 
 
+class _Network(torch.autograd.Function):
+    """The network's layers as one node: ReLU layers, then channel 0 of the
+    last layer, [D, H, W] f32 (its other channels are neither written nor
+    differentiated).  Same kernels and sums as a chain of Conv3dBF16; what
+    it saves is the host work between their launches."""
+
+    @staticmethod
+    def forward(ctx, x, n, *params):
+        ws, bs = params[:n], params[n:]
+        if any(p.device != x.device for p in params):
+            raise ValueError("the network's parameters and input are on different devices")
+        wb = torch.stack([w.detach() for w in ws]).to(torch.bfloat16)
+        assert tuple(wb.shape) == (n, 27, C16, C16)
+        bias = [b.detach().float().contiguous() for b in bs]
+        D, H, W = x.shape[:3]
+        L, acts, h, rc = lib(), [], x, 0
+        with _on(x.device):
+            st = _stream(x.device)
+            for k in range(n - 1):
+                y = torch.empty_like(x)
+                rc = rc or L.efwi_conv3d_forward(_ptr(h), _ptr(wb[k]), _ptr(bias[k]), D, H, W, 1,
+                                                 _ptr(y), None, st)
+                acts.append(y)
+                h = y
+            out = torch.empty(D, H, W, device=x.device, dtype=torch.float32)
+            head = rc or L.efwi_conv3d_forward_head(_ptr(h), _ptr(wb[n - 1]), _ptr(bias[n - 1]), D,
+                                                    H, W, 0, _ptr(out), st)
+        if rc or head not in (0, 3):
+            raise RuntimeError(f"a convolution of the network failed ({rc or head})")
+        if head == 3:  # another kernel form is selected
+            out = conv3d_raw(h, wb[n - 1], bs[n - 1], False, True)[..., 0].contiguous()
+        ctx.save_for_backward(x, wb, *acts)
+        return out
+
+    @staticmethod
+    def backward(ctx, gy):
+        x, wb, *acts = ctx.saved_tensors
+        n = wb.shape[0]
+        dws, dbs, g = [None] * n, [None] * n, gy
+        for k in range(n - 1, -1, -1):
+            g, dws[k], dbs[k] = conv3d_backward(acts[k - 1] if k else x, wb[k], g,
+                                                acts[k] if k < n - 1 else None,
+                                                k > 0 or ctx.needs_input_grad[0])
+        return (g, None, *dws, *dbs)
+
+
+class _ChannelsLast(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, feats):
+        ctx.c = feats.shape[0]
+        f = feats.contiguous()
+        x = torch.empty(feats.shape[1:] + (C16,), device=feats.device, dtype=torch.bfloat16)
+        with _on(f.device):
+            rc = lib().efwi_channels_last(_ptr(f), ctx.c, x.numel() // C16, _ptr(x),
+                                          _stream(f.device))
+        if rc:
+            raise RuntimeError(f"efwi_channels_last failed ({rc})")
+        return x
+
+    @staticmethod
+    def backward(ctx, gx):
+        return gx[..., :ctx.c].permute(3, 0, 1, 2).to(torch.float32)
+
+
 def to_channels_last(feats: torch.Tensor) -> torch.Tensor:
     """[C, D, H, W] f32 -> [D, H, W, 16] bf16 (channels zero-padded)."""
     c = feats.shape[0]
+    if (feats.is_cuda and feats.dtype == torch.float32 and feats.dim() == 4 and 1 <= c <= C16
+            and feats.numel() > 0):
+        return _ChannelsLast.apply(feats)
     x = torch.zeros(feats.shape[1:] + (C16,), device=feats.device, dtype=torch.bfloat16)
     x[..., :c] = feats.permute(1, 2, 3, 0).to(torch.bfloat16)
     return x
@@ -169,8 +250,4 @@ class Preconditioner(torch.nn.Module):
     def forward(self, feats: torch.Tensor) -> torch.Tensor:
         """feats [C, D, H, W] f32 on a GPU -> [D, H, W] f32."""
         h = to_channels_last(feats)
-        n = len(self.w)
-        for k in range(n):
-            last = k == n - 1
-            h = Conv3dBF16.apply(h, self.w[k], self.b[k], not last, last)
-        return h[..., 0]
+        return _Network.apply(h, len(self.w), *self.w, *self.b)

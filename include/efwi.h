@@ -279,12 +279,21 @@ int efwi_conv3d_wgrad(const void *x, const void *dy, int D, int H, int W, float 
  * with g = gy (y > 0) in float32 (y NULL: no ReLU, g = gy), dx = the input
  * gradient of bf16(g) (bf16; NULL: not wanted), dw as efwi_conv3d_wgrad of
  * x and bf16(g), db[co] = sum over voxels of g.  gy and y are bf16, or f32
- * where gy_f32 / y_f32 is set; all pointers 16-byte aligned.  scratch:
+ * where gy_f32 / y_f32 is 1; gy_f32 = 2 (y NULL): gy is [D][H][W] f32, the
+ * gradient of channel 0 alone.  All pointers 16-byte aligned.  scratch:
  * efwi_conv3d_backward_scratch bytes (relu: whether y is given). */
 long long efwi_conv3d_backward_scratch(int D, int H, int W, int nparts, int gy_f32, int relu);
 int efwi_conv3d_backward(const void *x, const void *w, const void *gy, int gy_f32, const void *y,
                          int y_f32, int D, int H, int W, void *scratch, int nparts, void *dx,
                          float *dw, float *db, void *stream);
+/* Channel 0 of efwi_conv3d_forward's output alone, y: [D][H][W] f32 (the
+ * z-marching form; x and w 16-byte aligned).  Returns 3 while another form is
+ * selected. */
+int efwi_conv3d_forward_head(const void *x, const void *w, const float *bias, int D, int H, int W,
+                             int relu, float *y, void *stream);
+/* out [voxels][16] bf16 (16-byte aligned) from feats [c][voxels] f32, c <= 16;
+ * channels from c on are zero. */
+int efwi_channels_last(const float *feats, int c, long long voxels, void *out, void *stream);
 /* Kernel form of efwi_conv3d_forward for this process: 0 = mma.sync;
  * 1 = tcgen05.mma with the accumulator in tensor memory (128 voxels x 16
  * channels per tile, one MMA per tap), tile staged by loads; 2 = z-marching,

@@ -75,3 +75,37 @@ def test_z_march_matches_single_tap_form(shape):
     for u, v in zip(out["tcgen05"], out["tcgen05-tma"]):
         assert torch.equal(u, v)
     assert not conv3d_status()
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 1), (5, 17, 9), (20, 16, 8)])
+@pytest.mark.parametrize("form", ["tcgen05-tma", "mma"])
+def test_network_node_matches_chain_of_layers(shape, form):
+    """One autograd node for the network, its channel-0 head and its input
+    copy against Conv3dBF16 layer by layer: the same bits, gradients of the
+    input and all parameters included."""
+    from efwi.cnn import Conv3dBF16, Preconditioner, set_conv_kernel
+    g = torch.Generator(device="cuda").manual_seed(7)
+    feats = torch.randn(3, *shape, device="cuda", generator=g)
+    gy = torch.randn(*shape, device="cuda", generator=g)
+    net = Preconditioner(seed=3).cuda()
+    with torch.no_grad():
+        for p in net.b:
+            p += 0.1
+    try:
+        set_conv_kernel(form)
+        a = feats.clone().requires_grad_(True)
+        ya = net(a)
+        ga = torch.autograd.grad(ya, [a, *net.parameters()], gy)
+        b = feats.clone().requires_grad_(True)
+        h = torch.zeros(shape + (16,), device="cuda", dtype=torch.bfloat16)
+        h[..., :3] = b.permute(1, 2, 3, 0).to(torch.bfloat16)
+        n = len(net.w)
+        for k in range(n):
+            h = Conv3dBF16.apply(h, net.w[k], net.b[k], k < n - 1, k == n - 1)
+        yb = h[..., 0]
+        gb = torch.autograd.grad(yb, [b, *net.parameters()], gy)
+    finally:
+        set_conv_kernel("tcgen05-tma")
+    assert torch.equal(ya, yb)
+    for u, v in zip(ga, gb):
+        assert torch.equal(u, v)
