@@ -10,8 +10,6 @@
 //     stored in HBM, and accumulates the images in shot order;
 //   - the exact gradient runs shot by shot with binomial checkpoints of the
 //     whole state in HBM under a byte budget (efwi_revolve.h).
-#include <cuda.h>
-#include <cudaTypedefs.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -135,7 +133,7 @@ struct KeyBytes {
   KeyBytes &geo(const Geo &g) {
     return add(g.nz).add(g.nx).add(g.ny).add(g.np).add(g.N).add(g.sz).add(g.sx).add(g.dt)
         .add(g.idz).add(g.idx).add(g.idy).add(g.slab_z).add(g.slab_x).add(g.slab_y).add(g.cz)
-        .add(g.cx).add(g.cy);
+        .add(g.cx).add(g.cy).add(g.far);
   }
 };
 
@@ -169,7 +167,6 @@ struct EfwiHandle {
   DevBuf recmap;  // per-plane receiver maps of the current batch
 
   DevBuf fields, psi, adj, traces_tm, res_tm, shell, partial, jdev, recbuf, winbuf, scalar, grad;
-  DevBuf status;  // pipeline status word (EFWI_STATUS_*)
 
   // exact gradient: checkpoint slots and the two adjoint memory-variable sets
   DevBuf ckpt, apsi;
@@ -472,60 +469,6 @@ int run_graphed(EfwiHandle *h, GraphCache &gc, const std::string &key, cudaStrea
   }
   CK_CUDA(h, cudaGraphLaunch(gc.exec, st));
   for (int k = 0; k < K_NCLASS; ++k) h->launches[k] += gc.launches[k];
-  return EFWI_OK;
-}
-
-PFN_cuTensorMapEncodeTiled_v12000 g_encode = nullptr;
-
-int get_encoder(EfwiHandle *h) {
-  if (g_encode) return EFWI_OK;
-  void *fn = nullptr;
-  cudaDriverEntryPointQueryResult q;
-  cudaError_t e = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q);
-  if (e != cudaSuccess || q != cudaDriverEntryPointSuccess || !fn)
-    return fail(h, EFWI_ERR_CUDA, "cuTensorMapEncodeTiled is not available");
-  g_encode = (PFN_cuTensorMapEncodeTiled_v12000)fn;
-  return EFWI_OK;
-}
-
-// Tensor map of S stacked pitched volumes [S*nz][nx][py]; halo boxes of
-// 40 (y) x (bx + 4) (x) x 1 plane, or point boxes of 32 x bx x 1.
-// Tensor map of one field over volumes of pitch py, nx rows and nzs planes.
-int make_map_dims(EfwiHandle *h, CUtensorMap *m, const float *base, int py, int nx, long long nzs,
-                  bool halo, int bx) {
-  int rc = get_encoder(h);
-  if (rc) return rc;
-  if (((uintptr_t)base & 15) != 0 || (py & 3) != 0)
-    return fail(h, EFWI_ERR_ARG, "tensor map base or pitch not 16-byte aligned");
-  cuuint64_t dims[3] = {(cuuint64_t)py, (cuuint64_t)nx, (cuuint64_t)nzs};
-  cuuint64_t strides[2] = {(cuuint64_t)py * 4, (cuuint64_t)nx * py * 4};
-  cuuint32_t box[3] = {halo ? (cuuint32_t)TMA_BOXY : 32u,
-                       (cuuint32_t)(halo ? bx + 2 * TMA_HX : bx), 1};
-  cuuint32_t es[3] = {1, 1, 1};
-  CUresult r = g_encode(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, (void *)base, dims, strides, box, es,
-                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                        CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) return fail(h, EFWI_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d)", (int)r);
-  return EFWI_OK;
-}
-
-int make_map(EfwiHandle *h, CUtensorMap *m, const float *base, int S, bool halo, int bx) {
-  return make_map_dims(h, m, base, h->py, h->grid.nx, (long long)h->grid.nz * S, halo, bx);
-}
-
-// Resets the status word at the start of a call.
-int status_reset(EfwiHandle *h, cudaStream_t st) {
-  CK_CUDA(h, h->status.ensure(sizeof(int)));
-  CK_CUDA(h, cudaMemsetAsync(h->status.p, 0, sizeof(int), st));
-  return EFWI_OK;
-}
-
-// Reads the status word (synchronises the stream).
-int status_check(EfwiHandle *h, cudaStream_t st) {
-  int v = 0;
-  CK_CUDA(h, cudaMemcpyAsync(&v, h->status.p, sizeof(int), cudaMemcpyDeviceToHost, st));
-  CK_CUDA(h, cudaStreamSynchronize(st));
-  if (v != EFWI_STATUS_OK) return fail(h, EFWI_ERR_CUDA, "a bulk-copy pipeline wait timed out");
   return EFWI_OK;
 }
 
@@ -911,21 +854,7 @@ int exact_shot(EfwiHandle *h, int id, const float *obs, double *jdev, float *res
   const int zc = h->zchunk_rev;
   const int bxe = h->bx;
   const dim3 grid = stencil_grid(h, 1, bxe, zc, &nzc);
-  // adjoint kernels with bulk-copy staged planes (TMA variant): tensor maps
-  // over this shot's buffers
-  const bool etma = h->variant == 1 && (bxe == 4 || bxe == 8);
-  Maps<11> mes;
-  Maps<10> mev;
-  if (etma) {
-    const float *hs[11] = {a.szz, a.sxx, a.syy, a.sxz, a.sxy, a.syz, h->lam.as<float>(),
-                           h->mu.as<float>(), b.f.vz, b.f.vx, b.f.vy};
-    const float *hv[10] = {a.vz, a.vx, a.vy, h->buoy.as<float>(), b.f.sxz, b.f.sxx, b.f.sxy,
-                           b.f.syz, b.f.syy, b.f.szz};
-    for (int k2 = 0; k2 < 11 && rc == 0; ++k2) rc = make_map(h, &mes.m[k2], hs[k2], 1, true, bxe);
-    for (int k2 = 0; k2 < 10 && rc == 0; ++k2) rc = make_map(h, &mev.m[k2], hv[k2], 1, true, bxe);
-    if (rc) return rc;
-  }
-  int *status = h->status.as<int>();
+  const bool vec = use_vec(h, h->geo, 1);
   int par_s = 0, par_v = 0;
   bool first = true;
   for (const CkAction &act : plan.actions) {
@@ -982,7 +911,7 @@ int exact_shot(EfwiHandle *h, int id, const float *obs, double *jdev, float *res
       if (k <= ntl - 2) {
         Timer t(h, K_ADJ_STRESS, st, k);
         const ExactArgs A = exact_args(h, b.f, b.ps, a, par_s, glam, gmu);
-        if (etma) launch_adj_stress_tma(bxe, grid, st, mes, A, zc, status);
+        if (vec) launch_adj_stress_vec(st, A);
         else launch_adj_stress_exact(bxe, grid, st, A, zc, nzc);
         par_s ^= 1;
       }
@@ -994,7 +923,7 @@ int exact_shot(EfwiHandle *h, int id, const float *obs, double *jdev, float *res
         }
         Timer t(h, K_ADJ_VELOCITY, st, k);
         const ExactArgs A = exact_args(h, b.f, b.ps, a, par_v, gB, nullptr);
-        if (etma) launch_adj_velocity_tma(bxe, grid, st, mev, A, zc, status);
+        if (vec) launch_adj_velocity_vec(st, A);
         else launch_adj_velocity_exact(bxe, grid, st, A, zc, nzc);
         par_v ^= 1;
       }
@@ -1163,6 +1092,7 @@ int efwi_create(const EfwiGrid *g, EfwiHandle **out) {
   G.slab_z = 2LL * g->npml * g->nx * g->ny;
   G.slab_x = (long long)g->nz * 2 * g->npml * g->ny;
   G.slab_y = (long long)g->nz * g->nx * 2 * g->npml;
+  G.far = geo_far(h->N);
   *out = h;
   // each axis's rows start on a 16-byte boundary
   const int oz = (6 * g->nz + 3) & ~3, ox = oz + ((6 * g->nx + 3) & ~3);
@@ -1365,8 +1295,6 @@ int efwi_forward(EfwiHandle *h, int n, const int *ids, float *traces, void *stre
   cudaStream_t st = (cudaStream_t)stream;
   const int nt = h->grid.nt;
   long long out_off = 0;
-  rc = status_reset(h, st);
-  if (rc) return rc;
   for (int b0 = 0; b0 < n; b0 += h->max_batch) {
     const int S = std::min(h->max_batch, n - b0);
     long long ntr = 0;
@@ -1388,7 +1316,8 @@ int efwi_forward(EfwiHandle *h, int n, const int *ids, float *traces, void *stre
     rc = check_launch(h, "traces");
     if (rc) return rc;
   }
-  return status_check(h, st);
+  CK_CUDA(h, cudaStreamSynchronize(st));
+  return EFWI_OK;
 }
 
 // Misfit (and, with glam set, the images) of shots ids on stream st.  With
@@ -1402,10 +1331,6 @@ static int gradient_impl(EfwiHandle *h, int n, const int *ids, const float *obs,
   const int nt = h->grid.nt;
   const long long N = h->N;
   const bool grad = glam != nullptr;
-  {
-    int rc0 = status_reset(h, st);
-    if (rc0) return rc0;
-  }
   float *out_lam = glam, *out_mu = gmu, *out_rho = grho;
   if (grad) {
     // images accumulate in pitched volumes, copied out at the end
@@ -1560,10 +1485,6 @@ static int gradient_impl(EfwiHandle *h, int n, const int *ids, const float *obs,
   for (int k = 0; k < n; ++k) J += js[k];
   if (misfit) *misfit = J;
   if (js_out) std::copy(js.begin(), js.begin() + n, js_out);
-  {
-    int rc1 = status_check(h, st);
-    if (rc1) return rc1;
-  }
   if (h->prof_sample > 0) return resolve_profile(h);
   return EFWI_OK;
 }
@@ -1641,10 +1562,6 @@ static int gradient_lanes(EfwiHandle *h, int n, const int *ids, const float *obs
   const bool grad = glam != nullptr;
   const int nt = h->grid.nt;
   int L = std::min(h->lanes, n);
-  if (h->variant == 1) {
-    int rc = get_encoder(h);  // once, before any thread needs it
-    if (rc) return rc;
-  }
   // exact mode: every lane takes an equal share of the checkpoint budget
   const long long budget = h->ck_budget;
   auto share = [&](int lanes) { return budget / std::max(lanes, 1); };
@@ -1812,6 +1729,7 @@ int efwi_forward_windows(EfwiHandle *h, int n, const int *ids, const EfwiWindow 
     g.slab_z = 2LL * np * w.nx * w.ny;
     g.slab_x = (long long)nz * 2 * np * w.ny;
     g.slab_y = (long long)nz * w.nx * 2 * np;
+    g.far = geo_far(g.N);
     for (int ax = 0; ax < 2; ++ax) {
       const int m = ax == 0 ? w.nx : w.ny;
       std::vector<float> c(6 * m);
@@ -2071,8 +1989,6 @@ int efwi_illumination(EfwiHandle *h, int n, const int *ids, float *h_lam, float 
   cudaStream_t st = (cudaStream_t)stream;
   const long long N = h->N;
   const int nt = h->grid.nt;
-  rc = status_reset(h, st);
-  if (rc) return rc;
   CK_CUDA(h, h->grad.ensure(sizeof(float) * 3 * N));
   CK_CUDA(h, cudaMemsetAsync(h->grad.p, 0, sizeof(float) * 3 * N, st));
   float *il = h->grad.as<float>(), *im = il + N, *ib = il + 2 * N;
@@ -2105,7 +2021,8 @@ int efwi_illumination(EfwiHandle *h, int n, const int *ids, float *h_lam, float 
   h->launches[K_OTHER] += 4;
   rc = check_launch(h, "illumination");
   if (rc) return rc;
-  return status_check(h, st);
+  CK_CUDA(h, cudaStreamSynchronize(st));
+  return EFWI_OK;
 }
 
 int efwi_set_stf_gradient(EfwiHandle *h, float *g_stf) {
@@ -2169,8 +2086,7 @@ int efwi_step(EfwiHandle *h, float *state, int transpose, void *stream) {
   CK_CUDA(h, cudaMemsetAsync(h->psi.p, 0, sizeof(float) * P, st));
   Fields f = fields_at(h->fields.as<float>(), N, 1);
   Psi ps = psi_at(h->psi.as<float>(), h->geo, 1);
-  int rc = status_reset(h, st);
-  if (rc) return rc;
+  int rc = EFWI_OK;
   if (!transpose) {
     k_state_convert<<<1184, 256, 0, st>>>(h->geo, state, f, ps, 1);
     RecArgs norec{};
@@ -2194,7 +2110,8 @@ int efwi_step(EfwiHandle *h, float *state, int transpose, void *stream) {
   h->launches[K_OTHER] += 2;
   rc = check_launch(h, "step");
   if (rc) return rc;
-  return status_check(h, st);
+  CK_CUDA(h, cudaStreamSynchronize(st));
+  return EFWI_OK;
 }
 
 int efwi_profile(EfwiHandle *h, int sample) {

@@ -47,7 +47,13 @@ struct Geo {
   float dt, idz, idx, idy;
   long long slab_z, slab_x, slab_y;  // elements per variable of each slab
   const float *cz, *cx, *cy;         // [6][n] coefficient rows
+  int far;  // a step's working set exceeds L2: rows of later use are prefetched
 };
+
+// A step reads and writes about 20 volumes.  Where these stay in L2 (126 MB)
+// the requests only cost issue slots: 5 % of a 84^3 forward step, against 10
+// % gained by K_V at 152^3.
+inline int geo_far(long long N) { return 20 * 4 * N > (64LL << 20); }
 
 struct Fields {
   float *vz, *vx, *vy, *szz, *sxx, *syy, *sxz, *sxy, *syz;

@@ -1,9 +1,19 @@
 // Exact discrete adjoint kernels (efwi_exact.cu).
 #pragma once
 #include "efwi_common.cuh"
-#include "efwi_tma.cuh"
 
 namespace efwi {
+
+// Adjoint of one C-PML-modified derivative (see efwi_exact.cu).
+__device__ __forceinline__ float qpml(float G, bool slab, float L, float kinv, float a) {
+  return slab ? G * kinv + a * (L + G) : G;
+}
+
+// Transpose of the quirk-Q1 difference over the rows x, x+1, x+2.
+__device__ __forceinline__ float dq_t(float p0, float p1, float p2) {
+  return EFWI_C1 * p0 - (EFWI_C1 + EFWI_C2) * p1 + EFWI_C2 * p2;
+}
+
 
 struct ExactArgs {
   Geo g;
@@ -22,14 +32,9 @@ void launch_adj_stress_exact(int bx, dim3 grid, cudaStream_t st, const ExactArgs
                              int nzc);
 void launch_adj_velocity_exact(int bx, dim3 grid, cudaStream_t st, const ExactArgs &A, int zchunk,
                                int nzc);
-// The same with every plane's operands staged by bulk tensor copies (bitwise
-// the same results).  Stress stage maps (halo boxes): adjoint szz sxx syy sxz
-// sxy syz, lambda, mu, forward vz vx vy.  Velocity stage maps: adjoint vz vx
-// vy, buoyancy, forward sxz sxx sxy syz syy szz.
-void launch_adj_stress_tma(int bx, dim3 grid, cudaStream_t st, const Maps<11> &maps,
-                           const ExactArgs &A, int zchunk, int *status);
-void launch_adj_velocity_tma(int bx, dim3 grid, cudaStream_t st, const Maps<10> &maps,
-                             const ExactArgs &A, int zchunk, int *status);
+// One thread per four cells (efwi_exact_vec.cu).
+void launch_adj_stress_vec(cudaStream_t st, const ExactArgs &A);
+void launch_adj_velocity_vec(cudaStream_t st, const ExactArgs &A);
 
 __global__ void k_buoy_to_rho(const float *gB, const float *buoy, float *grho, int nz, int nx,
                               int ny, int py);

@@ -31,6 +31,7 @@ k_stress_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ lam,
   const int nz = g.nz, nx = g.nx, ny = g.ny;
   if (z > nz - 3 || x > nx - 3 || y > ny - 3) return;
   const VecCell c = vec_cell(g, z, x, y);
+  vec_begin();
   const long long so = (long long)shot * g.N + c.i;
   const float *__restrict__ vz = f.vz + so;
   const float *__restrict__ vx = f.vx + so;
@@ -46,6 +47,8 @@ k_stress_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ lam,
   own.fetch(6, lam + c.i); own.fetch(7, mu + c.i);
 
   const Pml<VA> m = pml_of<VA>(g, c, false);
+  prefetch_psi<3>(g, Psi{ps.z + (long long)shot * 6 * g.slab_z, ps.x + (long long)shot * 6 * g.slab_x,
+                         ps.y + (long long)shot * 6 * g.slab_y}, m, c, PSI_VA);
   float *pz = ps.z + (long long)shot * 6 * g.slab_z;
   float *px = ps.x + (long long)shot * 6 * g.slab_x;
   float *py = ps.y + (long long)shot * 6 * g.slab_y;
@@ -203,6 +206,7 @@ k_velocity_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ buoy, int 
   const int nz = g.nz, nx = g.nx, ny = g.ny;
   if (z > nz - 3 || x > nx - 3 || y > ny - 3) return;
   const VecCell c = vec_cell(g, z, x, y);
+  vec_begin();
   const long long so = (long long)shot * g.N + c.i;
   const float *__restrict__ szz = f.szz + so;
   const float *__restrict__ sxx = f.sxx + so;
@@ -216,10 +220,14 @@ k_velocity_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ buoy, int 
   __shared__ float4 stash[4 * VEC_THREADS];
   Stash own{stash + vec_thread()};
   own.fetch(0, vz); own.fetch(1, vx); own.fetch(2, vy); own.fetch(3, buoy + c.i);
+  if (g.far)
+    for (const float *p : {sxx, sxy, syy}) prefetch_row(p);
   // receiver map of this plane, loaded first so that its latency overlaps
   const int rmap = rec.a.plane ? rec.a.plane[shot * nz + z] : -1;
 
   const Pml<VA> m = pml_of<VA>(g, c, true);
+  prefetch_psi<3>(g, Psi{ps.z + (long long)shot * 6 * g.slab_z, ps.x + (long long)shot * 6 * g.slab_x,
+                         ps.y + (long long)shot * 6 * g.slab_y}, m, c, PSI_SAA);
   float *pz = ps.z + (long long)shot * 6 * g.slab_z;
   float *px = ps.x + (long long)shot * 6 * g.slab_x;
   float *py = ps.y + (long long)shot * 6 * g.slab_y;
@@ -352,9 +360,9 @@ void launch_stress_fwd_vec(int S, cudaStream_t st, const Geo &g, const Fields &f
   const dim3 grid = vec_grid(g, S);
   const int nzb = grid.z / S;
   if (psi_vectors(g))
-    k_stress_fwd_vec<true, 6><<<grid, vec_block(), 0, st>>>(g, f, ps, lam, mu, nzb, src, shell);
+    vec_launch(k_stress_fwd_vec<true, 6>, grid, st, g, f, ps, lam, mu, nzb, src, shell);
   else
-    k_stress_fwd_vec<false, 6><<<grid, vec_block(), 0, st>>>(g, f, ps, lam, mu, nzb, src, shell);
+    vec_launch(k_stress_fwd_vec<false, 6>, grid, st, g, f, ps, lam, mu, nzb, src, shell);
 }
 
 void launch_velocity_fwd_vec(int S, cudaStream_t st, const Geo &g, const Fields &f, const Psi &ps,
@@ -362,9 +370,9 @@ void launch_velocity_fwd_vec(int S, cudaStream_t st, const Geo &g, const Fields 
   const dim3 grid = vec_grid(g, S);
   const int nzb = grid.z / S;
   if (psi_vectors(g))
-    k_velocity_fwd_vec<true, 5><<<grid, vec_block(), 0, st>>>(g, f, ps, buoy, nzb, rec);
+    vec_launch(k_velocity_fwd_vec<true, 5>, grid, st, g, f, ps, buoy, nzb, rec);
   else
-    k_velocity_fwd_vec<false, 5><<<grid, vec_block(), 0, st>>>(g, f, ps, buoy, nzb, rec);
+    vec_launch(k_velocity_fwd_vec<false, 5>, grid, st, g, f, ps, buoy, nzb, rec);
 }
 
 }  // namespace efwi

@@ -1,7 +1,6 @@
 // Kernel declarations shared by the kernel translation units and the C-ABI.
 #pragma once
 #include "efwi_common.cuh"
-#include "efwi_tma.cuh"
 
 namespace efwi {
 

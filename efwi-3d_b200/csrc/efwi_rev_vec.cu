@@ -84,6 +84,7 @@ k_rev_velocity_vec(Geo g, Fields f, Fields a, Psi ps, const float *__restrict__ 
   const int nz = g.nz, nx = g.nx, ny = g.ny;
   if (z > nz - 3 || x > nx - 3 || y > ny - 3) return;
   const VecCell c = vec_cell(g, z, x, y);
+  vec_begin();
   const Diff D{c};
   const int i = c.i, sz = (int)g.sz, sx = g.sx;
   const float dt = g.dt, idz = g.idz, idx = g.idx, idy = g.idy;
@@ -93,8 +94,13 @@ k_rev_velocity_vec(Geo g, Fields f, Fields a, Psi ps, const float *__restrict__ 
   own.fetch(AVZ, a.vz + i); own.fetch(AVX, a.vx + i); own.fetch(AVY, a.vy + i);
   own.fetch(BU, buoy + i);
   if (do_adj) { own.fetch(LA, lam + i); own.fetch(MU, mu + i); }
+  const Pml<VA> m = pml_of<VA>(g, c, false);
+  if (do_adj && g.far)
+    for (const float *p : {a.szz, a.sxx, a.syy, a.sxz, a.sxy, a.syz}) prefetch_row(p + i);
   bool in[VEC];
   const bool any_in = do_rev && inner_cells(g, c, in);
+  if (any_in && g.far)
+    for (const float *p : {f.sxx, f.sxy, f.syy}) prefetch_row(p + i);
   // to_bnd: the shell points take the stored velocities of the step
   int sk[VEC] = {-1, -1, -1, -1};
   bool any_sk = false;
@@ -156,7 +162,6 @@ k_rev_velocity_vec(Geo g, Fields f, Fields a, Psi ps, const float *__restrict__ 
   }
   if (!do_adj) { own.wait(); return; }
 
-  const Pml<VA> m = pml_of<VA>(g, c, false);
   const PsiGather<VA> G{g, c, m};
   float *pz = ps.z, *px = ps.x, *py = ps.y;
   const int lz = (int)g.slab_z, lx = (int)g.slab_x, ly = (int)g.slab_y;
@@ -299,6 +304,7 @@ k_rev_stress_vec(Geo g, Fields f, Fields a, Psi ps, const float *__restrict__ la
   const int nz = g.nz, nx = g.nx, ny = g.ny;
   if (z > nz - 3 || x > nx - 3 || y > ny - 3) return;
   const VecCell c = vec_cell(g, z, x, y);
+  vec_begin();
   const Diff D{c};
   const int i = c.i, sz = (int)g.sz, sx = g.sx;
   const float dt = g.dt, idz = g.idz, idx = g.idx, idy = g.idy;
@@ -308,6 +314,9 @@ k_rev_stress_vec(Geo g, Fields f, Fields a, Psi ps, const float *__restrict__ la
   own.fetch(LA, lam + i); own.fetch(MU, mu + i);
   own.fetch(AZZ, a.szz + i); own.fetch(AXX, a.sxx + i); own.fetch(AYY, a.syy + i);
   own.fetch(AXZ, a.sxz + i); own.fetch(AXY, a.sxy + i); own.fetch(AYZ, a.syz + i);
+  const Pml<VA> m = pml_of<VA>(g, c, false);
+  if (do_adj && g.far)
+    for (const float *p : {a.vz, a.vx, a.vy}) prefetch_row(p + i);
   bool in[VEC];
   const bool any_in = do_rev && inner_cells(g, c, in);
   // to_bnd: the shell points take the stored stresses of the step
@@ -406,7 +415,6 @@ k_rev_stress_vec(Geo g, Fields f, Fields a, Psi ps, const float *__restrict__ la
   }
   if (!do_adj) { own.wait(); return; }
 
-  const Pml<VA> m = pml_of<VA>(g, c, false);
   const PsiGather<VA> G{g, c, m};
   float *pz = ps.z, *px = ps.x, *py = ps.y;
   const int lz = (int)g.slab_z, lx = (int)g.slab_x, ly = (int)g.slab_y;
@@ -549,11 +557,9 @@ void launch_rev_velocity_vec(cudaStream_t st, const Geo &g, const Fields &f, con
                              float *grho, int do_rev, int do_adj, const ShellMap &shell,
                              const RecFuse &inj) {
   if (psi_vectors(g))
-    k_rev_velocity_vec<true, 6><<<vec_grid(g), vec_block(), 0, st>>>(
-        g, f, a, ps, lam, mu, buoy, grho, do_rev, do_adj, shell, inj);
+    vec_launch(k_rev_velocity_vec<true, 6>, vec_grid(g), st, g, f, a, ps, lam, mu, buoy, grho, do_rev, do_adj, shell, inj);
   else
-    k_rev_velocity_vec<false, 6><<<vec_grid(g), vec_block(), 0, st>>>(
-        g, f, a, ps, lam, mu, buoy, grho, do_rev, do_adj, shell, inj);
+    vec_launch(k_rev_velocity_vec<false, 6>, vec_grid(g), st, g, f, a, ps, lam, mu, buoy, grho, do_rev, do_adj, shell, inj);
 }
 
 void launch_rev_stress_vec(cudaStream_t st, const Geo &g, const Fields &f, const Fields &a,
@@ -561,11 +567,9 @@ void launch_rev_stress_vec(cudaStream_t st, const Geo &g, const Fields &f, const
                            float *glam, float *gmu, int do_rev, int do_adj, const SrcArgs &src,
                            const ShellMap &shell) {
   if (psi_vectors(g))
-    k_rev_stress_vec<true, 5><<<vec_grid(g), vec_block(), 0, st>>>(
-        g, f, a, ps, lam, mu, buoy, glam, gmu, do_rev, do_adj, src, shell);
+    vec_launch(k_rev_stress_vec<true, 5>, vec_grid(g), st, g, f, a, ps, lam, mu, buoy, glam, gmu, do_rev, do_adj, src, shell);
   else
-    k_rev_stress_vec<false, 5><<<vec_grid(g), vec_block(), 0, st>>>(
-        g, f, a, ps, lam, mu, buoy, glam, gmu, do_rev, do_adj, src, shell);
+    vec_launch(k_rev_stress_vec<false, 5>, vec_grid(g), st, g, f, a, ps, lam, mu, buoy, glam, gmu, do_rev, do_adj, src, shell);
 }
 
 }  // namespace efwi

@@ -37,6 +37,13 @@ __device__ __forceinline__ void st_row(float *p, const Row &r) {
   *reinterpret_cast<float4 *>(p) = make_float4(r.v[0], r.v[1], r.v[2], r.v[3]);
 }
 
+// Asks for the thread's row of a field that a later part of the kernel reads:
+// into L2, so that the part waits for L2 and not for DRAM.  One lane per
+// 128-byte line.
+__device__ __forceinline__ void prefetch_row(const float *p) {
+  if (threadIdx.x == 0) asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
+}
+
 // Cells y-2 .. y+5 of a row around the vector c at y: (e, k) is cell y+e+k.
 struct Span {
   float v[VEC + 4];
@@ -158,6 +165,20 @@ __device__ __forceinline__ Row coef_y(const Geo &g, const VecCell &c, int which)
   return r;
 }
 __device__ __forceinline__ Row fill(float v) { return Row{{v, v, v, v}}; }
+
+// prefetch_row of the memory variables s0 .. s0 + N - 1 at the thread's row.
+template <int N, bool VA>
+__device__ __forceinline__ void prefetch_psi(const Geo &g, const Psi &ps, const Pml<VA> &m,
+                                             const VecCell &c, int s0) {
+  if (!g.far) return;
+  const bool ys = c.y < g.np || c.y + VEC * VEC_TY > g.ny - g.np;  // of lane 0: the CTA's row
+#pragma unroll
+  for (int k = 0; k < N; ++k) {
+    if (m.zs) prefetch_row(ps.z + (s0 + k) * g.slab_z + m.kz);
+    if (m.xs) prefetch_row(ps.x + (s0 + k) * g.slab_x + m.kx);
+    if (ys) prefetch_row(ps.y + (s0 + k) * g.slab_y + (c.z * g.nx + c.x) * (2 * g.np));
+  }
+}
 
 // m = b m + a d,  d = d / K + m  of one cell.
 __device__ __forceinline__ void pml_step(float Ki, float a, float b, float &m, float &d) {
@@ -318,6 +339,32 @@ inline bool vec_fits(const Geo &g, int S) {
   return (g.nx - 4 + VEC_TX - 1) / VEC_TX <= 65535 &&
          (long long)S * ((g.nz - 4 + VEC_TZ - 1) / VEC_TZ) <= 65535;
 }
-inline dim3 vec_block() { return dim3(VEC_TY, VEC_TX, VEC_TZ); }
+
+// Launch of a stencil kernel that may begin while the kernel before it in
+// the stream drains (programmatic dependent launch): the kernels order their
+// reads and writes with vec_begin().  What overlaps is the launch itself and
+// the index arithmetic, 1-2 us of a launch that takes 4 on the smallest
+// grids.
+template <class... P, class... T>
+inline void vec_launch(void (*kernel)(P...), dim3 grid, cudaStream_t st, T... args) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cf{};
+  cf.gridDim = grid;
+  cf.blockDim = dim3(VEC_TY, VEC_TX, VEC_TZ);
+  cf.stream = st;
+  cf.attrs = &at;
+  cf.numAttrs = 1;
+  cudaLaunchKernelEx(&cf, kernel, static_cast<P>(args)...);
+}
+// Waits until the kernels before this one are complete and their writes
+// visible, then lets the next kernel's CTAs start (once all of this grid's
+// have come here or left).  Nothing that a kernel of the time loop writes is
+// touched before it.
+__device__ __forceinline__ void vec_begin() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
 
 }  // namespace efwi
