@@ -51,18 +51,14 @@ __device__ __forceinline__ int receiver_at(const RecArgs &r, int nz, int py, int
   return r.map[(long long)mp * r.nxpy + x * py + y];
 }
 
-// recording (utilities.cu:481-495) of unique receiver cell u at sample it.
+// recording (utilities.cu:481-495) of one component (0 vx, 1 vy, 2 vz) of
+// unique receiver cell u at sample it.
 __device__ __forceinline__ void record_cell(const RecArgs &rec, float *traces_tm, int it, int u,
-                                            float vz, float vx, float vy) {
+                                            int comp, float v) {
   const int s = rec.ushot[u];
   const int nr = rec.nrec[s];
-  float *t = traces_tm + rec.trace_off[s] + (long long)it * 3 * nr;
-  for (int k = rec.uptr[u]; k < rec.uptr[u + 1]; ++k) {
-    const int r = rec.rec[k];
-    t[r] = vx;
-    t[nr + r] = vy;
-    t[2 * nr + r] = vz;
-  }
+  float *t = traces_tm + rec.trace_off[s] + ((long long)it * 3 + comp) * nr;
+  for (int k = rec.uptr[u]; k < rec.uptr[u + 1]; ++k) t[rec.rec[k]] = v;
 }
 
 // res_injection (utilities.cu:497-507) at unique receiver cell u: the

@@ -19,13 +19,17 @@ namespace efwi {
 // Both kernels form one output (K_S: the normal stresses together) at a time,
 // each from its own differences, so that few values are live: registers, not
 // bandwidth, hold these kernels' occupancy down, and the rows read again for
-// the next output come from L1.
-template <bool VA, int MINB>
-__global__ void __launch_bounds__(VEC_THREADS, MINB)
+// the next output come from L1.  PARTS > 1: the outputs lie on different warps
+// instead (vec_split); a memory variable belongs to one derivative and so to one
+// part, and the shell's copy of an output is taken by the part that updates it.
+template <bool VA, int PARTS, int MINB>
+__global__ void __launch_bounds__(vec_threads(PARTS), MINB)
 k_stress_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ lam,
                  const float *__restrict__ mu, int nzb, SrcArgs src, ShellMap shell) {
   const int shot = blockIdx.z / nzb;
-  const int z = 2 + (blockIdx.z - shot * nzb) * VEC_TZ + threadIdx.z;
+  constexpr int TZ = vec_tz(PARTS), T = vec_threads(PARTS);
+  const int part = PARTS > 1 ? threadIdx.z / TZ : 0;
+  const int z = 2 + (blockIdx.z - shot * nzb) * TZ + threadIdx.z % TZ;
   const int x = 2 + blockIdx.y * VEC_TX + threadIdx.y;
   const int y = VEC * (blockIdx.x * VEC_TY + threadIdx.x);
   const int nz = g.nz, nx = g.nx, ny = g.ny;
@@ -40,11 +44,17 @@ k_stress_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ lam,
   const float dt = g.dt, idz = g.idz, idx = g.idx, idy = g.idy;
   float *szz = f.szz + so, *sxx = f.sxx + so, *syy = f.syy + so;
   float *sxz = f.sxz + so, *sxy = f.sxy + so, *syz = f.syz + so;
-  __shared__ float4 stash[8 * VEC_THREADS];
-  Stash own{stash + vec_thread()};
-  own.fetch(0, szz); own.fetch(1, sxx); own.fetch(2, syy);
-  own.fetch(3, sxz); own.fetch(4, sxy); own.fetch(5, syz);
-  own.fetch(6, lam + c.i); own.fetch(7, mu + c.i);
+  __shared__ float4 stash[8 * T];
+  Stash<T> own{stash + vec_thread()};
+  // outputs of the thread: 0 the normal stresses, 1 sxz, 2 sxy, 3 syz
+  auto mine = [&](int k) { return PARTS == 1 || part == k; };
+  if (mine(0)) {
+    own.fetch(0, szz); own.fetch(1, sxx); own.fetch(2, syy); own.fetch(6, lam + c.i);
+  }
+  if (mine(1)) own.fetch(3, sxz);
+  if (mine(2)) own.fetch(4, sxy);
+  if (mine(3)) own.fetch(5, syz);
+  own.fetch(7, mu + c.i);
 
   const Pml<VA> m = pml_of<VA>(g, c, false);
   prefetch_psi<3>(g, Psi{ps.z + (long long)shot * 6 * g.slab_z, ps.x + (long long)shot * 6 * g.slab_x,
@@ -56,15 +66,17 @@ k_stress_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ lam,
     const int srow = shell.rows[z * nx + x];
     int sk[VEC];
     if (srow >= 0 && shell_cells(shell, srow, c, sk)) {
-      const float *src9[9] = {szz, sxz, sxx, syy, sxy, syz, vz, vx, vy};
-#pragma unroll
-      for (int q = 0; q < 9; ++q) {
-        const Row r = ld_row(src9[q]);
+      auto keep = [&](int q, const float *p) {
+        const Row r = ld_row(p);
         float *st = shell.store + (size_t)q * shell.npts;
 #pragma unroll
         for (int e = 0; e < VEC; ++e)
           if (sk[e] >= 0) st[sk[e]] = r[e];
-      }
+      };
+      if (mine(0)) { keep(0, szz); keep(2, sxx); keep(3, syy); }
+      if (mine(1)) { keep(1, sxz); keep(6, vz); }
+      if (mine(2)) { keep(4, sxy); keep(7, vx); }
+      if (mine(3)) { keep(5, syz); keep(8, vy); }
     }
   }
   // memory variables `slot` of one axis, and their derivative's update (half:
@@ -82,7 +94,7 @@ k_stress_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ lam,
     if (m.yany) pml_row_y(py + slot * g.slab_y, r, g, m, c, half, d);
   };
 
-  {  // normal stresses
+  if (mine(0)) {  // normal stresses
     Row qz = ld_z(PSI_VA), qx = ld_x(PSI_VA), qy = ld_y(PSI_VA);
     float ezz[VEC], exx[VEC], eyy[VEC];
     const Row z0 = ld_row(vz), x0 = ld_row(vx), y0 = ld_row(vy);
@@ -134,6 +146,7 @@ k_stress_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ lam,
   }
   // one shear stress from its two derivatives
   auto shear = [&](int r, float *dst, const float d0[VEC], const float d1[VEC]) {
+    if (PARTS > 1) own.wait();
     Row n = own.get(r);
     const Row u = own.get(7);
 #pragma unroll
@@ -141,7 +154,7 @@ k_stress_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ lam,
       if (c.act[e]) n.v[e] += u[e] * (d0[e] + d1[e]) * dt;
     st_row(dst, n);
   };
-  {  // sxz
+  if (mine(1)) {  // sxz
     Row qz = ld_z(PSI_VB1), qx = ld_x(PSI_VB1);
     float dvx_dz[VEC], dvz_dx[VEC];
     {
@@ -158,7 +171,7 @@ k_stress_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ lam,
     pml_x(PSI_VB1, 1, qx, dvz_dx);
     shear(3, sxz, dvx_dz, dvz_dx);
   }
-  {  // sxy
+  if (mine(2)) {  // sxy
     Row qx = ld_x(PSI_VB2), qy = ld_y(PSI_VB2);
     float dvx_dy[VEC], dvy_dx[VEC];
     {
@@ -176,7 +189,7 @@ k_stress_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ lam,
     pml_y(PSI_VB2, 1, qy, dvx_dy);
     shear(4, sxy, dvx_dy, dvy_dx);
   }
-  {  // syz
+  if (mine(3)) {  // syz
     Row qz = ld_z(PSI_VB2), qy = ld_y(PSI_VB1);
     float dvy_dz[VEC], dvz_dy[VEC];
     {
@@ -196,11 +209,13 @@ k_stress_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ lam,
   }
 }
 
-template <bool VA, int MINB>
-__global__ void __launch_bounds__(VEC_THREADS, MINB)
+template <bool VA, int PARTS, int MINB>
+__global__ void __launch_bounds__(vec_threads(PARTS), MINB)
 k_velocity_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ buoy, int nzb, RecFuse rec) {
   const int shot = blockIdx.z / nzb;
-  const int z = 2 + (blockIdx.z - shot * nzb) * VEC_TZ + threadIdx.z;
+  constexpr int TZ = vec_tz(PARTS), T = vec_threads(PARTS);
+  const int part = PARTS > 1 ? threadIdx.z / TZ : 0;
+  const int z = 2 + (blockIdx.z - shot * nzb) * TZ + threadIdx.z % TZ;
   const int x = 2 + blockIdx.y * VEC_TX + threadIdx.y;
   const int y = VEC * (blockIdx.x * VEC_TY + threadIdx.x);
   const int nz = g.nz, nx = g.nx, ny = g.ny;
@@ -217,9 +232,14 @@ k_velocity_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ buoy, int 
   const int sz = (int)g.sz, sx = g.sx;
   const float idz = g.idz, idx = g.idx, idy = g.idy, dt = g.dt;
   float *vz = f.vz + so, *vx = f.vx + so, *vy = f.vy + so;
-  __shared__ float4 stash[4 * VEC_THREADS];
-  Stash own{stash + vec_thread()};
-  own.fetch(0, vz); own.fetch(1, vx); own.fetch(2, vy); own.fetch(3, buoy + c.i);
+  __shared__ float4 stash[4 * T];
+  Stash<T> own{stash + vec_thread()};
+  // outputs of the thread: 0 vz, 1 vx, 2 vy
+  auto mine = [&](int k) { return PARTS == 1 || part == k; };
+  if (mine(0)) own.fetch(0, vz);
+  if (mine(1)) own.fetch(1, vx);
+  if (mine(2)) own.fetch(2, vy);
+  own.fetch(3, buoy + c.i);
   if (g.far)
     for (const float *p : {sxx, sxy, syy}) prefetch_row(p);
   // receiver map of this plane, loaded first so that its latency overlaps
@@ -248,6 +268,7 @@ k_velocity_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ buoy, int 
 
   // one velocity from its three derivatives
   auto update = [&](int r, const float d0[VEC], const float d1[VEC], const float d2[VEC]) {
+    if (PARTS > 1) own.wait();
     Row n = own.get(r);
     const Row b = own.get(3);
 #pragma unroll
@@ -255,8 +276,8 @@ k_velocity_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ buoy, int 
       if (c.act[e]) n.v[e] += (d0[e] + d1[e] + d2[e]) * b[e] * dt;
     return n;
   };
-  Row nvz, nvx, nvy;
-  {  // vz
+  Row nvz{}, nvx{}, nvy{};
+  if (mine(0)) {  // vz
     Row qz = ld_z(PSI_SAA), qx = ld_x(PSI_SAB1), qy = ld_y(PSI_SAB1);
     float dszz_dz[VEC], dsxz_dx[VEC], dsyz_dy[VEC];
     {
@@ -284,7 +305,7 @@ k_velocity_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ buoy, int 
     nvz = update(0, dszz_dz, dsxz_dx, dsyz_dy);
     st_row(vz, nvz);
   }
-  {  // vx
+  if (mine(1)) {  // vx
     Row qz = ld_z(PSI_SAB1), qx = ld_x(PSI_SAA), qy = ld_y(PSI_SAB2);
     float dsxz_dz[VEC], dsxx_dx[VEC], dsxy_dy[VEC];
     {
@@ -311,7 +332,7 @@ k_velocity_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ buoy, int 
     nvx = update(1, dsxz_dz, dsxx_dx, dsxy_dy);
     st_row(vx, nvx);
   }
-  {  // vy
+  if (mine(2)) {  // vy
     Row qz = ld_z(PSI_SAB2), qx = ld_x(PSI_SAB2), qy = ld_y(PSI_SAA);
     float dsyz_dz[VEC], dsxy_dx[VEC], dsyy_dy[VEC];
     {
@@ -345,8 +366,11 @@ k_velocity_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ buoy, int 
     const int us[VEC] = {u.x, u.y, u.z, u.w};
 #pragma unroll
     for (int e = 0; e < VEC; ++e)
-      if (c.act[e] && us[e] >= 0)
-        record_cell(rec.a, rec.tm, rec.it, us[e], nvz[e], nvx[e], nvy[e]);
+      if (c.act[e] && us[e] >= 0) {
+        if (mine(1)) record_cell(rec.a, rec.tm, rec.it, us[e], 0, nvx[e]);
+        if (mine(2)) record_cell(rec.a, rec.tm, rec.it, us[e], 1, nvy[e]);
+        if (mine(0)) record_cell(rec.a, rec.tm, rec.it, us[e], 2, nvz[e]);
+      }
   }
 }
 
@@ -357,22 +381,22 @@ k_velocity_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ buoy, int 
 void launch_stress_fwd_vec(int S, cudaStream_t st, const Geo &g, const Fields &f, const Psi &ps,
                            const float *lam, const float *mu, const SrcArgs &src,
                            const ShellMap &shell) {
-  const dim3 grid = vec_grid(g, S);
+  const int parts = vec_split(g, S) ? 4 : 1;
+  const dim3 grid = vec_grid(g, S, parts);
   const int nzb = grid.z / S;
-  if (psi_vectors(g))
-    vec_launch(k_stress_fwd_vec<true, 6>, grid, st, g, f, ps, lam, mu, nzb, src, shell);
-  else
-    vec_launch(k_stress_fwd_vec<false, 6>, grid, st, g, f, ps, lam, mu, nzb, src, shell);
+  auto k = parts > 1 ? (psi_vectors(g) ? k_stress_fwd_vec<true, 4, 8> : k_stress_fwd_vec<false, 4, 8>)
+                     : (psi_vectors(g) ? k_stress_fwd_vec<true, 1, 6> : k_stress_fwd_vec<false, 1, 6>);
+  vec_launch(k, grid, parts, st, g, f, ps, lam, mu, nzb, src, shell);
 }
 
 void launch_velocity_fwd_vec(int S, cudaStream_t st, const Geo &g, const Fields &f, const Psi &ps,
                              const float *buoy, const RecFuse &rec) {
-  const dim3 grid = vec_grid(g, S);
+  const int parts = vec_split(g, S) ? 3 : 1;
+  const dim3 grid = vec_grid(g, S, parts);
   const int nzb = grid.z / S;
-  if (psi_vectors(g))
-    vec_launch(k_velocity_fwd_vec<true, 5>, grid, st, g, f, ps, buoy, nzb, rec);
-  else
-    vec_launch(k_velocity_fwd_vec<false, 5>, grid, st, g, f, ps, buoy, nzb, rec);
+  auto k = parts > 1 ? (psi_vectors(g) ? k_velocity_fwd_vec<true, 3, 8> : k_velocity_fwd_vec<false, 3, 8>)
+                     : (psi_vectors(g) ? k_velocity_fwd_vec<true, 1, 5> : k_velocity_fwd_vec<false, 1, 5>);
+  vec_launch(k, grid, parts, st, g, f, ps, buoy, nzb, rec);
 }
 
 }  // namespace efwi

@@ -89,7 +89,7 @@ k_rev_velocity_vec(Geo g, Fields f, Fields a, Psi ps, const float *__restrict__ 
   const int i = c.i, sz = (int)g.sz, sx = g.sx;
   const float dt = g.dt, idz = g.idz, idx = g.idx, idy = g.idy;
   __shared__ float4 stash[10 * VEC_THREADS];
-  Stash own{stash + vec_thread()};
+  Stash<VEC_THREADS> own{stash + vec_thread()};
   enum { VZ, VX, VY, AVZ, AVX, AVY, BU, LA, MU, GR };
   own.fetch(AVZ, a.vz + i); own.fetch(AVX, a.vx + i); own.fetch(AVY, a.vy + i);
   own.fetch(BU, buoy + i);
@@ -309,7 +309,7 @@ k_rev_stress_vec(Geo g, Fields f, Fields a, Psi ps, const float *__restrict__ la
   const int i = c.i, sz = (int)g.sz, sx = g.sx;
   const float dt = g.dt, idz = g.idz, idx = g.idx, idy = g.idy;
   __shared__ float4 stash[17 * VEC_THREADS];
-  Stash own{stash + vec_thread()};
+  Stash<VEC_THREADS> own{stash + vec_thread()};
   enum { SZZ, SXX, SYY, SXZ, SXY, SYZ, AZZ, AXX, AYY, AXZ, AXY, AYZ, LA, MU, BU, GL, GM };
   own.fetch(LA, lam + i); own.fetch(MU, mu + i);
   own.fetch(AZZ, a.szz + i); own.fetch(AXX, a.sxx + i); own.fetch(AYY, a.syy + i);
@@ -557,9 +557,9 @@ void launch_rev_velocity_vec(cudaStream_t st, const Geo &g, const Fields &f, con
                              float *grho, int do_rev, int do_adj, const ShellMap &shell,
                              const RecFuse &inj) {
   if (psi_vectors(g))
-    vec_launch(k_rev_velocity_vec<true, 6>, vec_grid(g), st, g, f, a, ps, lam, mu, buoy, grho, do_rev, do_adj, shell, inj);
+    vec_launch(k_rev_velocity_vec<true, 6>, vec_grid(g), 1, st, g, f, a, ps, lam, mu, buoy, grho, do_rev, do_adj, shell, inj);
   else
-    vec_launch(k_rev_velocity_vec<false, 6>, vec_grid(g), st, g, f, a, ps, lam, mu, buoy, grho, do_rev, do_adj, shell, inj);
+    vec_launch(k_rev_velocity_vec<false, 6>, vec_grid(g), 1, st, g, f, a, ps, lam, mu, buoy, grho, do_rev, do_adj, shell, inj);
 }
 
 void launch_rev_stress_vec(cudaStream_t st, const Geo &g, const Fields &f, const Fields &a,
@@ -567,9 +567,9 @@ void launch_rev_stress_vec(cudaStream_t st, const Geo &g, const Fields &f, const
                            float *glam, float *gmu, int do_rev, int do_adj, const SrcArgs &src,
                            const ShellMap &shell) {
   if (psi_vectors(g))
-    vec_launch(k_rev_stress_vec<true, 5>, vec_grid(g), st, g, f, a, ps, lam, mu, buoy, glam, gmu, do_rev, do_adj, src, shell);
+    vec_launch(k_rev_stress_vec<true, 5>, vec_grid(g), 1, st, g, f, a, ps, lam, mu, buoy, glam, gmu, do_rev, do_adj, src, shell);
   else
-    vec_launch(k_rev_stress_vec<false, 5>, vec_grid(g), st, g, f, a, ps, lam, mu, buoy, glam, gmu, do_rev, do_adj, src, shell);
+    vec_launch(k_rev_stress_vec<false, 5>, vec_grid(g), 1, st, g, f, a, ps, lam, mu, buoy, glam, gmu, do_rev, do_adj, src, shell);
 }
 
 }  // namespace efwi

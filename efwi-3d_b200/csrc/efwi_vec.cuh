@@ -19,7 +19,15 @@ constexpr int VEC = 4;
 // through L1, and 128 threads keep the waves small.  On the 152^3 grid 16
 // vectors x 2 rows x 4 planes ran 12 % slower, 2-row or 2-plane CTAs 1-8 %,
 // 256-thread ones 3-6 %.
+//
+// A kernel has several outputs.  With enough CTAs a thread forms them one after
+// the other; on small grids (vec_split) PARTS warps of a CTA share one plane's
+// outputs, a part to each, and the latency of a launch drops to that of the
+// longest part.
 constexpr int VEC_TY = 8, VEC_TX = 4, VEC_TZ = 4, VEC_THREADS = VEC_TY * VEC_TX * VEC_TZ;
+// planes and threads of a CTA whose vectors have PARTS threads
+constexpr int vec_tz(int parts) { return parts > 1 ? 1 : VEC_TZ; }
+constexpr int vec_threads(int parts) { return VEC_TY * VEC_TX * vec_tz(parts) * parts; }
 __device__ __forceinline__ int vec_thread() {
   return (threadIdx.z * VEC_TX + threadIdx.y) * VEC_TY + threadIdx.x;
 }
@@ -316,24 +324,38 @@ __device__ __forceinline__ void mem_row_y(float *p, const Geo &g, const Pml<VA> 
 // and reads back after the differences: the bytes in flight cost no
 // registers, and as every thread reads only what it copied itself there is
 // no barrier.  `slot` is row-major over the CTA's threads (conflict-free).
+template <int THREADS>
 struct Stash {
-  float4 *slot;  // [rows][VEC_THREADS], already at the thread's column
+  float4 *slot;  // [rows][THREADS], already at the thread's column
   __device__ __forceinline__ void fetch(int r, const float *p) {
-    const uint32_t dst = (uint32_t)__cvta_generic_to_shared(slot + r * VEC_THREADS);
+    const uint32_t dst = (uint32_t)__cvta_generic_to_shared(slot + r * THREADS);
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(p) : "memory");
   }
   __device__ __forceinline__ void wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
   __device__ __forceinline__ Row get(int r) const {
-    const float4 t = slot[r * VEC_THREADS];
+    const float4 t = slot[r * THREADS];
     return Row{{t.x, t.y, t.z, t.w}};
   }
 };
 
 // Grid over the cells [2, n-3]^3 (y: vectors up to the one of cell ny-3) of S
 // shots.
-inline dim3 vec_grid(const Geo &g, int S = 1) {
-  const int nv = (g.ny - 3) / VEC + 1, nzb = (g.nz - 4 + VEC_TZ - 1) / VEC_TZ;
+inline dim3 vec_grid(const Geo &g, int S = 1, int parts = 1) {
+  const int TZ = vec_tz(parts);
+  const int nv = (g.ny - 3) / VEC + 1, nzb = (g.nz - 4 + TZ - 1) / TZ;
   return dim3((nv + VEC_TY - 1) / VEC_TY, (g.nx - 4 + VEC_TX - 1) / VEC_TX, (unsigned)(S * nzb));
+}
+// The forward kernels split their outputs over warps where the unsplit grid
+// would leave SMs short of one wave (5 CTAs of 148 SMs): launches then take one
+// thread's chain of loads, which the split shortens.  Of an isolated launch,
+// unsplit and split (us, ~6 of them the measurement): 26 x 30 x 28 K_S 10.5 /
+// 8.4; 84^3 (1200 CTAs) 22.6 / 18.5, but 45.1 / 48.2 ms for the whole gradient
+// there, whose launches overlap; 152^3 72 / 98 and 56 / 58: a split vector's
+// rows are loaded by several warps.
+constexpr int VEC_SPLIT_CTAS = 148 * 5;
+inline bool vec_split(const Geo &g, int S) {
+  const dim3 n = vec_grid(g, S);
+  return (long long)n.x * n.y * n.z < VEC_SPLIT_CTAS;
 }
 inline bool vec_fits(const Geo &g, int S) {
   return (g.nx - 4 + VEC_TX - 1) / VEC_TX <= 65535 &&
@@ -346,13 +368,13 @@ inline bool vec_fits(const Geo &g, int S) {
 // the index arithmetic, 1-2 us of a launch that takes 4 on the smallest
 // grids.
 template <class... P, class... T>
-inline void vec_launch(void (*kernel)(P...), dim3 grid, cudaStream_t st, T... args) {
+inline void vec_launch(void (*kernel)(P...), dim3 grid, int parts, cudaStream_t st, T... args) {
   cudaLaunchAttribute at{};
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at.val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t cf{};
   cf.gridDim = grid;
-  cf.blockDim = dim3(VEC_TY, VEC_TX, VEC_TZ);
+  cf.blockDim = dim3(VEC_TY, VEC_TX, vec_tz(parts) * parts);
   cf.stream = st;
   cf.attrs = &at;
   cf.numAttrs = 1;
