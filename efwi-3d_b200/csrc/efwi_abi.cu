@@ -613,7 +613,8 @@ bool use_vec(const EfwiHandle *h, const Geo &g, int S) {
 // store and the receiver gather run in the stencil kernels; otherwise as
 // separate launches.
 int forward_step(EfwiHandle *h, Fields f, Psi ps, int S, const SrcArgs &src, const RecArgs &rec,
-                 float *traces_tm, cudaStream_t st, int it, float *shell = nullptr) {
+                 float *traces_tm, cudaStream_t st, int it, float *shell = nullptr,
+                 const IllumSum &il = {}) {
   const bool vec = use_vec(h, h->geo, S);
   int nzc;
   const dim3 grid = stencil_grid(h, S, h->bx, h->zchunk, &nzc);
@@ -633,7 +634,8 @@ int forward_step(EfwiHandle *h, Fields f, Psi ps, int S, const SrcArgs &src, con
   {
     Timer t(h, K_STRESS_FWD, st, it);
     if (vec)
-      launch_stress_fwd_vec(S, st, h->geo, f, ps, h->lam.as<float>(), h->mu.as<float>(), src, shm);
+      launch_stress_fwd_vec(S, st, h->geo, f, ps, h->lam.as<float>(), h->mu.as<float>(), src, shm,
+                            il);
     else
       launch_stress_fwd(h->bx, grid, st, h->geo, f, ps, h->lam.as<float>(), h->mu.as<float>(),
                         h->zchunk, nzc, src);
@@ -641,7 +643,7 @@ int forward_step(EfwiHandle *h, Fields f, Psi ps, int S, const SrcArgs &src, con
   {
     Timer t(h, K_VELOCITY_FWD, st, it);
     if (vec)
-      launch_velocity_fwd_vec(S, st, h->geo, f, ps, h->buoy.as<float>(), rf);
+      launch_velocity_fwd_vec(S, st, h->geo, f, ps, h->buoy.as<float>(), rf, il);
     else
       launch_velocity_fwd(h->bx, grid, st, h->geo, f, ps, h->buoy.as<float>(), h->zchunk, nzc);
   }
@@ -2003,15 +2005,33 @@ int efwi_illumination(EfwiHandle *h, int n, const int *ids, float *h_lam, float 
     RecArgs norec = b.rec;
     norec.ncell = 0;
     const int ntl = nt_eff(h);
+    // Sums per shot inside the forward kernels, in the adjoint fields' memory
+    // (four shots fit in it); without room for them, a pass of its own.
+    IllumSum sums{};
+    if (use_vec(h, h->geo, S)) {
+      const size_t rest = sizeof(float) * 3 * N * (S - 1);
+      if (h->adj.ensure(std::max<size_t>(rest, sizeof(float) * 9 * N)) == cudaSuccess) {
+        CK_CUDA(h, cudaMemsetAsync(h->adj.p, 0, rest, st));
+        sums = IllumSum{il, h->adj.as<float>(), N};
+      } else {
+        cudaGetLastError();
+      }
+    }
     const dim3 grid((h->grid.ny + 31) / 32, (h->grid.nx + 3) / 4, (h->grid.nz - 4 + 7) / 8);
     for (int it = 0; it <= ntl - 2; ++it) {
       b.src.it = it;
-      rc = forward_step(h, b.f, b.ps, S, b.src, norec, nullptr, st, it);
+      rc = forward_step(h, b.f, b.ps, S, b.src, norec, nullptr, st, it, nullptr, sums);
       if (rc) return rc;
+      if (sums.first) continue;
       Timer t(h, K_OTHER, st, it);
       k_illumination<<<grid, dim3(32, 4), 0, st>>>(h->geo, b.f, b.ps, S, h->buoy.as<float>(),
                                                    it + 1 <= ntl - 2, il, im, ib);
     }
+    if (sums.first && S > 1) {
+      k_illum_reduce<<<1184, 256, 0, st>>>(sums, S, 3 * N);
+      h->launches[K_OTHER]++;
+    }
+    if (h->adj.bytes > sizeof(float) * 9 * N) h->adj.release();
   }
   const EfwiGrid &G = h->grid;
   k_buoy_to_rho_sq<<<1184, 256, 0, st>>>(ib, h->buoy.as<float>(), G.nz, G.nx, G.ny, h->py);

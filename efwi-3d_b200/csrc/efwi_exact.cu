@@ -38,6 +38,7 @@
 // issued before the plane's one barrier.
 #include "efwi_common.cuh"
 #include "efwi_exact.h"
+#include "efwi_vec.cuh"
 
 namespace efwi {
 namespace {
@@ -672,12 +673,29 @@ __global__ void k_buoy_to_rho(const float *gB, const float *buoy, float *grho, i
   }
 }
 
+// il.first += il.rest of the shots 1 .. S-1, in their order, over n values (a
+// multiple of 4).  Memory-bound, once per batch of shots.
+__global__ void k_illum_reduce(IllumSum il, int S, long long n) {
+  for (long long i = VEC * (blockIdx.x * (long long)blockDim.x + threadIdx.x); i < n;
+       i += VEC * (long long)gridDim.x * blockDim.x) {
+    Row a = ld_row(il.first + i);
+    for (int s = 1; s < S; ++s) {
+      const Row r = ld_row(il.of(s, 0) + i);
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) a.v[e] += r[e];
+    }
+    st_row(il.first + i, a);
+  }
+}
+
 // Source illumination (diagonal pseudo-Hessian of Shin et al. 2001): for the
 // state S_k after forward step k-1, adds at every cell of [2, n-3]^3, summed
 // over the S shots of the batch,
 //   hl += 3 (dt div)^2                       (d sigma_ii / d lambda = dt div)
 //   hm += dt^2 (4 sum_i e_ii^2 + sum_i<j (e_ij + e_ji)^2)
 //   hb += dt^2 |modified stress divergence|^2 (d v / d B)
+// (of the one-cell kernels, and where the four-cell ones, which form these sums
+// themselves, find no memory for a sum per shot)
 // from the C-PML-modified derivatives of the forward step: the stress-stage
 // terms of step k (velocities and stress memory variables of S_k, when
 // do_stress) and the velocity-stage terms of step k-1 (stresses and updated

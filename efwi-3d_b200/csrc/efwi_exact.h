@@ -1,6 +1,7 @@
 // Exact discrete adjoint kernels (efwi_exact.cu).
 #pragma once
 #include "efwi_common.cuh"
+#include "efwi_kernels.h"
 
 namespace efwi {
 
@@ -41,6 +42,7 @@ __global__ void k_buoy_to_rho(const float *gB, const float *buoy, float *grho, i
 __global__ void k_stf_gradient(Fields a, const long long *src_cell, const float *w2, float *out,
                                int k, float scale);
 __global__ void k_state_convert(Geo g, float *full, Fields f, Psi ps, int to_engine);
+__global__ void k_illum_reduce(IllumSum il, int S, long long n);
 __global__ void k_illumination(Geo g, Fields f, Psi ps, int S, const float *buoy, int do_stress,
                                float *hl, float *hm, float *hb);
 __global__ void k_buoy_to_rho_sq(float *hb, const float *buoy, int nz, int nx, int ny, int py);

@@ -22,10 +22,18 @@ namespace efwi {
 // the next output come from L1.  PARTS > 1: the outputs lie on different warps
 // instead (vec_split); a memory variable belongs to one derivative and so to one
 // part, and the shell's copy of an output is taken by the part that updates it.
-template <bool VA, int PARTS, int MINB>
+//
+// IL: the kernels add the step's share of the source illumination (the diagonal
+// pseudo-Hessian of k_illumination, efwi_exact.cu), whose derivatives they have
+// in registers, to the shot's own sums.  Two more rows in and out for K_S and
+// one for K_V take the place of a pass that reads the nine fields again with
+// their neighbours: 80^3, four shots, 78 us a step in all; 329 with the pass,
+// whose own 246 were one thread's chain over the shots and eight planes.
+template <bool VA, int PARTS, int MINB, bool IL = false>
 __global__ void __launch_bounds__(vec_threads(PARTS), MINB)
 k_stress_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ lam,
-                 const float *__restrict__ mu, int nzb, SrcArgs src, ShellMap shell) {
+                 const float *__restrict__ mu, int nzb, SrcArgs src, ShellMap shell, IllumSum il) {
+  static_assert(!IL || PARTS == 1, "the sums need all outputs in one thread");
   const int shot = blockIdx.z / nzb;
   constexpr int TZ = vec_tz(PARTS), T = vec_threads(PARTS);
   const int part = PARTS > 1 ? threadIdx.z / TZ : 0;
@@ -44,7 +52,7 @@ k_stress_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ lam,
   const float dt = g.dt, idz = g.idz, idx = g.idx, idy = g.idy;
   float *szz = f.szz + so, *sxx = f.sxx + so, *syy = f.syy + so;
   float *sxz = f.sxz + so, *sxy = f.sxy + so, *syz = f.syz + so;
-  __shared__ float4 stash[8 * T];
+  __shared__ float4 stash[(IL ? 10 : 8) * T];
   Stash<T> own{stash + vec_thread()};
   // outputs of the thread: 0 the normal stresses, 1 sxz, 2 sxy, 3 syz
   auto mine = [&](int k) { return PARTS == 1 || part == k; };
@@ -55,6 +63,11 @@ k_stress_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ lam,
   if (mine(2)) own.fetch(4, sxy);
   if (mine(3)) own.fetch(5, syz);
   own.fetch(7, mu + c.i);
+  float am[VEC] = {};  // IL: squared strains of hm
+  if (IL) {
+    own.fetch(8, il.of(shot, 0) + c.i);
+    own.fetch(9, il.of(shot, 1) + c.i);
+  }
 
   const Pml<VA> m = pml_of<VA>(g, c, false);
   prefetch_psi<3>(g, Psi{ps.z + (long long)shot * 6 * g.slab_z, ps.x + (long long)shot * 6 * g.slab_x,
@@ -127,6 +140,16 @@ k_stress_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ lam,
       nxx.v[e] += (le * ezz[e] + l2u * exx[e] + le * eyy[e]) * dt;
       nyy.v[e] += (le * ezz[e] + le * exx[e] + l2u * eyy[e]) * dt;
     }
+    if (IL) {
+      Row hl = own.get(8);
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) {
+        const float div = ezz[e] + exx[e] + eyy[e];
+        if (c.act[e]) hl.v[e] += 3.0f * div * div * (dt * dt);
+        am[e] = 4.0f * (ezz[e] * ezz[e] + exx[e] * exx[e] + eyy[e] * eyy[e]);
+      }
+      st_row(il.of(shot, 0) + c.i, hl);
+    }
     const long long hit = src.cell ? src.cell[shot] - c.i : -1;
     if (hit >= 0 && hit < VEC) {
       // add_source follows the stress kernel; amplitude formed in double
@@ -152,6 +175,10 @@ k_stress_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ lam,
 #pragma unroll
     for (int e = 0; e < VEC; ++e)
       if (c.act[e]) n.v[e] += u[e] * (d0[e] + d1[e]) * dt;
+    if (IL) {
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) am[e] += (d0[e] + d1[e]) * (d0[e] + d1[e]);
+    }
     st_row(dst, n);
   };
   if (mine(1)) {  // sxz
@@ -207,11 +234,20 @@ k_stress_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ lam,
     pml_y(PSI_VB1, 1, qy, dvz_dy);
     shear(5, syz, dvy_dz, dvz_dy);
   }
+  if (IL) {
+    Row hm = own.get(9);
+#pragma unroll
+    for (int e = 0; e < VEC; ++e)
+      if (c.act[e]) hm.v[e] += am[e] * (dt * dt);
+    st_row(il.of(shot, 1) + c.i, hm);
+  }
 }
 
-template <bool VA, int PARTS, int MINB>
+template <bool VA, int PARTS, int MINB, bool IL = false>
 __global__ void __launch_bounds__(vec_threads(PARTS), MINB)
-k_velocity_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ buoy, int nzb, RecFuse rec) {
+k_velocity_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ buoy, int nzb, RecFuse rec,
+                   IllumSum il) {
+  static_assert(!IL || PARTS == 1, "the sums need all outputs in one thread");
   const int shot = blockIdx.z / nzb;
   constexpr int TZ = vec_tz(PARTS), T = vec_threads(PARTS);
   const int part = PARTS > 1 ? threadIdx.z / TZ : 0;
@@ -232,7 +268,7 @@ k_velocity_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ buoy, int 
   const int sz = (int)g.sz, sx = g.sx;
   const float idz = g.idz, idx = g.idx, idy = g.idy, dt = g.dt;
   float *vz = f.vz + so, *vx = f.vx + so, *vy = f.vy + so;
-  __shared__ float4 stash[4 * T];
+  __shared__ float4 stash[(IL ? 5 : 4) * T];
   Stash<T> own{stash + vec_thread()};
   // outputs of the thread: 0 vz, 1 vx, 2 vy
   auto mine = [&](int k) { return PARTS == 1 || part == k; };
@@ -240,6 +276,8 @@ k_velocity_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ buoy, int 
   if (mine(1)) own.fetch(1, vx);
   if (mine(2)) own.fetch(2, vy);
   own.fetch(3, buoy + c.i);
+  float ab[VEC] = {};  // IL: squared stress divergence of hb
+  if (IL) own.fetch(4, il.of(shot, 2) + c.i);
   if (g.far)
     for (const float *p : {sxx, sxy, syy}) prefetch_row(p);
   // receiver map of this plane, loaded first so that its latency overlaps
@@ -274,6 +312,11 @@ k_velocity_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ buoy, int 
 #pragma unroll
     for (int e = 0; e < VEC; ++e)
       if (c.act[e]) n.v[e] += (d0[e] + d1[e] + d2[e]) * b[e] * dt;
+    if (IL) {
+#pragma unroll
+      for (int e = 0; e < VEC; ++e)
+        ab[e] += (d0[e] + d1[e] + d2[e]) * (d0[e] + d1[e] + d2[e]);
+    }
     return n;
   };
   Row nvz{}, nvx{}, nvy{};
@@ -360,6 +403,13 @@ k_velocity_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ buoy, int 
     nvy = update(2, dsyz_dz, dsxy_dx, dsyy_dy);
     st_row(vy, nvy);
   }
+  if (IL) {
+    Row hb = own.get(4);
+#pragma unroll
+    for (int e = 0; e < VEC; ++e)
+      if (c.act[e]) hb.v[e] += ab[e] * (dt * dt);
+    st_row(il.of(shot, 2) + c.i, hb);
+  }
   if (rmap >= 0) {
     const int4 u = *reinterpret_cast<const int4 *>(rec.a.map + (long long)rmap * rec.a.nxpy +
                                                    x * g.sx + y);
@@ -380,23 +430,27 @@ k_velocity_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ buoy, int 
 // with 6 is no faster where a launch has few waves (75 x 109 x 91).
 void launch_stress_fwd_vec(int S, cudaStream_t st, const Geo &g, const Fields &f, const Psi &ps,
                            const float *lam, const float *mu, const SrcArgs &src,
-                           const ShellMap &shell) {
-  const int parts = vec_split(g, S) ? 4 : 1;
+                           const ShellMap &shell, const IllumSum &il) {
+  const int parts = !il.first && vec_split(g, S) ? 4 : 1;
   const dim3 grid = vec_grid(g, S, parts);
   const int nzb = grid.z / S;
-  auto k = parts > 1 ? (psi_vectors(g) ? k_stress_fwd_vec<true, 4, 8> : k_stress_fwd_vec<false, 4, 8>)
-                     : (psi_vectors(g) ? k_stress_fwd_vec<true, 1, 6> : k_stress_fwd_vec<false, 1, 6>);
-  vec_launch(k, grid, parts, st, g, f, ps, lam, mu, nzb, src, shell);
+  const bool va = psi_vectors(g);
+  auto k = il.first ? (va ? k_stress_fwd_vec<true, 1, 5, true> : k_stress_fwd_vec<false, 1, 5, true>)
+           : parts > 1 ? (va ? k_stress_fwd_vec<true, 4, 8> : k_stress_fwd_vec<false, 4, 8>)
+                       : (va ? k_stress_fwd_vec<true, 1, 6> : k_stress_fwd_vec<false, 1, 6>);
+  vec_launch(k, grid, parts, st, g, f, ps, lam, mu, nzb, src, shell, il);
 }
 
 void launch_velocity_fwd_vec(int S, cudaStream_t st, const Geo &g, const Fields &f, const Psi &ps,
-                             const float *buoy, const RecFuse &rec) {
-  const int parts = vec_split(g, S) ? 3 : 1;
+                             const float *buoy, const RecFuse &rec, const IllumSum &il) {
+  const int parts = !il.first && vec_split(g, S) ? 3 : 1;
   const dim3 grid = vec_grid(g, S, parts);
   const int nzb = grid.z / S;
-  auto k = parts > 1 ? (psi_vectors(g) ? k_velocity_fwd_vec<true, 3, 8> : k_velocity_fwd_vec<false, 3, 8>)
-                     : (psi_vectors(g) ? k_velocity_fwd_vec<true, 1, 5> : k_velocity_fwd_vec<false, 1, 5>);
-  vec_launch(k, grid, parts, st, g, f, ps, buoy, nzb, rec);
+  const bool va = psi_vectors(g);
+  auto k = il.first ? (va ? k_velocity_fwd_vec<true, 1, 5, true> : k_velocity_fwd_vec<false, 1, 5, true>)
+           : parts > 1 ? (va ? k_velocity_fwd_vec<true, 3, 8> : k_velocity_fwd_vec<false, 3, 8>)
+                       : (va ? k_velocity_fwd_vec<true, 1, 5> : k_velocity_fwd_vec<false, 1, 5>);
+  vec_launch(k, grid, parts, st, g, f, ps, buoy, nzb, rec, il);
 }
 
 }  // namespace efwi

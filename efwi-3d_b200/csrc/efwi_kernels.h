@@ -108,15 +108,26 @@ void launch_rev_stress(int bx, dim3 grid, cudaStream_t st, const Geo &g, const F
                        const float *buoy, float *glam, float *gmu, int zchunk, int nzc,
                        int do_rev, int do_adj, const SrcArgs &src);
 
+// Illumination sums [lambda, mu, buoyancy][N] of the shots of a batch: the
+// first shot's and the others' one after the other.
+struct IllumSum {
+  float *first, *rest;
+  long long N;
+  __host__ __device__ __forceinline__ float *of(int shot, int q) const {
+    return (shot ? rest + (shot - 1) * 3 * N : first) + q * N;
+  }
+};
+
 // One thread per four cells (efwi_fwd_vec.cu), S shots per launch.  With
 // shell.rows set (one shot), K_S stores the state at the start of the step
 // into shell.store at the shell points; with rec.a.plane set, K_V records the
-// new velocities of the receiver cells at sample rec.it.
+// new velocities of the receiver cells at sample rec.it.  With il.first set
+// they add the step's illumination to the sums of each shot.
 void launch_stress_fwd_vec(int S, cudaStream_t st, const Geo &g, const Fields &f, const Psi &ps,
                            const float *lam, const float *mu, const SrcArgs &src,
-                           const ShellMap &shell);
+                           const ShellMap &shell, const IllumSum &il = {});
 void launch_velocity_fwd_vec(int S, cudaStream_t st, const Geo &g, const Fields &f, const Psi &ps,
-                             const float *buoy, const RecFuse &rec);
+                             const float *buoy, const RecFuse &rec, const IllumSum &il = {});
 
 // Reverse sweep, one thread per four cells (efwi_rev_vec.cu).  With shell.rows
 // set (do_rev), the reverse velocities (K1) and stresses (K2) are restored at
