@@ -614,8 +614,8 @@ bool use_vec(const EfwiHandle *h, const Geo &g, int S) {
 // separate launches.
 int forward_step(EfwiHandle *h, Fields f, Psi ps, int S, const SrcArgs &src, const RecArgs &rec,
                  float *traces_tm, cudaStream_t st, int it, float *shell = nullptr,
-                 const IllumSum &il = {}) {
-  const bool vec = use_vec(h, h->geo, S);
+                 const IllumSum &il = {}, const StepTo &to = {}) {
+  const bool vec = use_vec(h, h->geo, S);  // `to`: vector kernels only
   int nzc;
   const dim3 grid = stencil_grid(h, S, h->bx, h->zchunk, &nzc);
   ShellMap shm{};
@@ -635,18 +635,20 @@ int forward_step(EfwiHandle *h, Fields f, Psi ps, int S, const SrcArgs &src, con
     Timer t(h, K_STRESS_FWD, st, it);
     if (vec)
       launch_stress_fwd_vec(S, st, h->geo, f, ps, h->lam.as<float>(), h->mu.as<float>(), src, shm,
-                            il);
+                            il, to);
     else
       launch_stress_fwd(h->bx, grid, st, h->geo, f, ps, h->lam.as<float>(), h->mu.as<float>(),
                         h->zchunk, nzc, src);
   }
+  for (float **p : {&f.szz, &f.sxx, &f.syy, &f.sxz, &f.sxy, &f.syz}) *p += to.fields;
   {
     Timer t(h, K_VELOCITY_FWD, st, it);
     if (vec)
-      launch_velocity_fwd_vec(S, st, h->geo, f, ps, h->buoy.as<float>(), rf, il);
+      launch_velocity_fwd_vec(S, st, h->geo, f, ps, h->buoy.as<float>(), rf, il, to);
     else
       launch_velocity_fwd(h->bx, grid, st, h->geo, f, ps, h->buoy.as<float>(), h->zchunk, nzc);
   }
+  for (float **p : {&f.vz, &f.vx, &f.vy}) *p += to.fields;
   if (rec.ncell > 0 && !rec_fused) {
     Timer t(h, K_RECORD, st, it);
     k_record<<<(rec.ncell + 127) / 128, 128, 0, st>>>(f, h->N, rec, traces_tm, it + 1);
@@ -849,41 +851,75 @@ int exact_shot(EfwiHandle *h, int id, const float *obs, double *jdev, float *res
   CK_CUDA(h, cudaMemsetAsync(h->apsi.p, 0, sizeof(float) * 2 * P, st));
   RecArgs norec = b.rec;
   norec.ncell = 0;
-  float *state = h->fields.as<float>();  // [9N fields][P memory variables]
-  float *psi = h->psi.as<float>();
-  float *ck = h->ckpt.as<float>();
   int nzc;
   const int zc = h->zchunk_rev;
   const int bxe = h->bx;
   const dim3 grid = stencil_grid(h, 1, bxe, zc, &nzc);
   const bool vec = use_vec(h, h->geo, 1);
+  // The state is in the work buffers or in a checkpoint.  The vector kernels
+  // step from either into either (the slots are zero where no step writes):
+  // the last step before a checkpoint writes it, and a restored checkpoint is
+  // read where it lies, by the adjoint and by the first step away from it.  A
+  // slot is never stepped in place.
+  struct State {
+    float *fields, *psi;  // [9N], [P]
+  };
+  const State work{h->fields.as<float>(), h->psi.as<float>()};
+  auto slot = [&](int k) {
+    float *p = h->ckpt.as<float>() + (long long)k * SF;
+    return State{p, p + 9 * N};
+  };
+  auto copy = [&](const State &to, const State &from) {
+    CK_CUDA(h, cudaMemcpyAsync(to.fields, from.fields, sizeof(float) * 9 * N, cudaMemcpyDeviceToDevice, st));
+    CK_CUDA(h, cudaMemcpyAsync(to.psi, from.psi, sizeof(float) * P, cudaMemcpyDeviceToDevice, st));
+    return (int)EFWI_OK;
+  };
+  auto apart = [](const float *to, const float *from) {
+    return ((long long)(uintptr_t)to - (long long)(uintptr_t)from) / (long long)sizeof(float);
+  };
+  State cur = work;
+  if (vec && plan.slots_used > 0) {
+    Timer t(h, K_CHECKPOINT, st, -1);
+    CK_CUDA(h, cudaMemsetAsync(h->ckpt.p, 0, sizeof(float) * plan.slots_used * SF, st));
+  }
   int par_s = 0, par_v = 0;
   bool first = true;
-  for (const CkAction &act : plan.actions) {
+  for (size_t ia = 0; ia < plan.actions.size(); ++ia) {
+    const CkAction &act = plan.actions[ia];
     if (act.op == CK_ADVANCE) {
       for (int it = act.a; it < act.b; ++it) {
         b.src.it = it;
-        rc = forward_step(h, b.f, b.ps, 1, b.src, first ? b.rec : norec, h->traces_tm.as<float>(),
-                          st, it);
+        State to = work;
+        if (vec && it + 1 == act.b && ia + 1 < plan.actions.size() &&
+            plan.actions[ia + 1].op == CK_STORE)
+          to = slot(plan.actions[ia + 1].a);
+        rc = forward_step(h, fields_at(cur.fields, N, 1), psi_at(cur.psi, h->geo, 1), 1, b.src,
+                          first ? b.rec : norec, h->traces_tm.as<float>(), st, it, nullptr, {},
+                          StepTo{apart(to.fields, cur.fields), apart(to.psi, cur.psi)});
         if (rc) return rc;
+        cur = to;
       }
     } else if (act.op == CK_STORE) {
+      if (cur.fields == slot(act.a).fields) continue;
       Timer t(h, K_CHECKPOINT, st, -1);
-      float *dst = ck + (long long)act.a * SF;
-      CK_CUDA(h, cudaMemcpyAsync(dst, state, sizeof(float) * 9 * N, cudaMemcpyDeviceToDevice, st));
-      CK_CUDA(h, cudaMemcpyAsync(dst + 9 * N, psi, sizeof(float) * P, cudaMemcpyDeviceToDevice, st));
+      if ((rc = copy(slot(act.a), cur))) return rc;
     } else if (act.op == CK_RESTORE) {
+      if (act.a >= 0 && vec) {
+        cur = slot(act.a);
+        continue;
+      }
       Timer t(h, K_CHECKPOINT, st, -1);
-      if (act.a < 0) {
-        CK_CUDA(h, cudaMemsetAsync(state, 0, sizeof(float) * 9 * N, st));
-        CK_CUDA(h, cudaMemsetAsync(psi, 0, sizeof(float) * P, st));
+      cur = work;
+      if (act.a >= 0) {
+        if ((rc = copy(work, slot(act.a)))) return rc;
       } else {
-        const float *src = ck + (long long)act.a * SF;
-        CK_CUDA(h, cudaMemcpyAsync(state, src, sizeof(float) * 9 * N, cudaMemcpyDeviceToDevice, st));
-        CK_CUDA(h, cudaMemcpyAsync(psi, src + 9 * N, sizeof(float) * P, cudaMemcpyDeviceToDevice, st));
+        CK_CUDA(h, cudaMemsetAsync(work.fields, 0, sizeof(float) * 9 * N, st));
+        CK_CUDA(h, cudaMemsetAsync(work.psi, 0, sizeof(float) * P, st));
       }
     } else {  // CK_BLOCK
       const int k = act.a;
+      const Fields f = fields_at(cur.fields, N, 1);
+      const Psi ps = psi_at(cur.psi, h->geo, 1);
       if (first && adj_source) {
         first = false;
         if (sh.nrec > 0) {
@@ -912,7 +948,7 @@ int exact_shot(EfwiHandle *h, int id, const float *obs, double *jdev, float *res
       }
       if (k <= ntl - 2) {
         Timer t(h, K_ADJ_STRESS, st, k);
-        const ExactArgs A = exact_args(h, b.f, b.ps, a, par_s, glam, gmu);
+        const ExactArgs A = exact_args(h, f, ps, a, par_s, glam, gmu);
         if (vec) launch_adj_stress_vec(st, A);
         else launch_adj_stress_exact(bxe, grid, st, A, zc, nzc);
         par_s ^= 1;
@@ -924,7 +960,7 @@ int exact_shot(EfwiHandle *h, int id, const float *obs, double *jdev, float *res
                                                               adj_source ? 1.0f : -2.0f);
         }
         Timer t(h, K_ADJ_VELOCITY, st, k);
-        const ExactArgs A = exact_args(h, b.f, b.ps, a, par_v, gB, nullptr);
+        const ExactArgs A = exact_args(h, f, ps, a, par_v, gB, nullptr);
         if (vec) launch_adj_velocity_vec(st, A);
         else launch_adj_velocity_exact(bxe, grid, st, A, zc, nzc);
         par_v ^= 1;

@@ -16,6 +16,8 @@
 
 namespace efwi {
 
+enum { VEC_STEP, VEC_STEP_TO, VEC_ILLUM };  // what a launch does besides the step
+
 // Both kernels form one output (K_S: the normal stresses together) at a time,
 // each from its own differences, so that few values are live: registers, not
 // bandwidth, hold these kernels' occupancy down, and the rows read again for
@@ -23,17 +25,23 @@ namespace efwi {
 // instead (vec_split); a memory variable belongs to one derivative and so to one
 // part, and the shell's copy of an output is taken by the part that updates it.
 //
-// IL: the kernels add the step's share of the source illumination (the diagonal
+// VEC_STEP_TO: the results go to another state (exact gradient: a checkpoint),
+// zero where no step writes, at the cost of no copy.  A kernel of its own: with
+// the offsets in every launch, 26 x 30 x 28 and 84^3 ran 3-4 % slower.
+//
+// VEC_ILLUM: the kernels add the step's share of the source illumination (the diagonal
 // pseudo-Hessian of k_illumination, efwi_exact.cu), whose derivatives they have
 // in registers, to the shot's own sums.  Two more rows in and out for K_S and
 // one for K_V take the place of a pass that reads the nine fields again with
 // their neighbours: 80^3, four shots, 78 us a step in all; 329 with the pass,
 // whose own 246 were one thread's chain over the shots and eight planes.
-template <bool VA, int PARTS, int MINB, bool IL = false>
+template <bool VA, int PARTS, int MINB, int MODE = VEC_STEP>
 __global__ void __launch_bounds__(vec_threads(PARTS), MINB)
 k_stress_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ lam,
-                 const float *__restrict__ mu, int nzb, SrcArgs src, ShellMap shell, IllumSum il) {
+                 const float *__restrict__ mu, int nzb, SrcArgs src, ShellMap shell, IllumSum il, StepTo to) {
+  constexpr bool IL = MODE == VEC_ILLUM;
   static_assert(!IL || PARTS == 1, "the sums need all outputs in one thread");
+  const long long tf = MODE == VEC_STEP_TO ? to.fields : 0, tp = MODE == VEC_STEP_TO ? to.psi : 0;
   const int shot = blockIdx.z / nzb;
   constexpr int TZ = vec_tz(PARTS), T = vec_threads(PARTS);
   const int part = PARTS > 1 ? threadIdx.z / TZ : 0;
@@ -98,13 +106,13 @@ k_stress_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ lam,
   auto ld_x = [&](int slot) { return m.xs ? ld_psi<VA>(px + slot * g.slab_x, m.kx, c) : Row{}; };
   auto ld_y = [&](int slot) { return m.yany ? ld_psi_y(py + slot * g.slab_y, g, m, c) : Row{}; };
   auto pml_z = [&](int slot, int half, Row &r, float d[VEC]) {
-    if (m.zs) pml_row<VA>(pz + slot * g.slab_z, m.kz, r, c, g.cz + 3 * half * nz + z, nz, d);
+    if (m.zs) pml_row<VA>(pz + slot * g.slab_z + tp, m.kz, r, c, g.cz + 3 * half * nz + z, nz, d);
   };
   auto pml_x = [&](int slot, int half, Row &r, float d[VEC]) {
-    if (m.xs) pml_row<VA>(px + slot * g.slab_x, m.kx, r, c, g.cx + 3 * half * nx + x, nx, d);
+    if (m.xs) pml_row<VA>(px + slot * g.slab_x + tp, m.kx, r, c, g.cx + 3 * half * nx + x, nx, d);
   };
   auto pml_y = [&](int slot, int half, Row &r, float d[VEC]) {
-    if (m.yany) pml_row_y(py + slot * g.slab_y, r, g, m, c, half, d);
+    if (m.yany) pml_row_y(py + slot * g.slab_y + tp, r, g, m, c, half, d);
   };
 
   if (mine(0)) {  // normal stresses
@@ -165,7 +173,7 @@ k_stress_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ lam,
         nyy.v[e] = (float)((double)nyy[e] + a);
       }
     }
-    st_row(szz, nzz); st_row(sxx, nxx); st_row(syy, nyy);
+    st_row(szz + tf, nzz); st_row(sxx + tf, nxx); st_row(syy + tf, nyy);
   }
   // one shear stress from its two derivatives
   auto shear = [&](int r, float *dst, const float d0[VEC], const float d1[VEC]) {
@@ -179,7 +187,7 @@ k_stress_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ lam,
 #pragma unroll
       for (int e = 0; e < VEC; ++e) am[e] += (d0[e] + d1[e]) * (d0[e] + d1[e]);
     }
-    st_row(dst, n);
+    st_row(dst + tf, n);
   };
   if (mine(1)) {  // sxz
     Row qz = ld_z(PSI_VB1), qx = ld_x(PSI_VB1);
@@ -243,11 +251,13 @@ k_stress_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ lam,
   }
 }
 
-template <bool VA, int PARTS, int MINB, bool IL = false>
+template <bool VA, int PARTS, int MINB, int MODE = VEC_STEP>
 __global__ void __launch_bounds__(vec_threads(PARTS), MINB)
 k_velocity_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ buoy, int nzb, RecFuse rec,
-                   IllumSum il) {
+                   IllumSum il, StepTo to) {
+  constexpr bool IL = MODE == VEC_ILLUM;
   static_assert(!IL || PARTS == 1, "the sums need all outputs in one thread");
+  const long long tf = MODE == VEC_STEP_TO ? to.fields : 0, tp = MODE == VEC_STEP_TO ? to.psi : 0;
   const int shot = blockIdx.z / nzb;
   constexpr int TZ = vec_tz(PARTS), T = vec_threads(PARTS);
   const int part = PARTS > 1 ? threadIdx.z / TZ : 0;
@@ -295,13 +305,13 @@ k_velocity_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ buoy, int 
   auto ld_x = [&](int slot) { return m.xs ? ld_psi<VA>(px + slot * g.slab_x, m.kx, c) : Row{}; };
   auto ld_y = [&](int slot) { return m.yany ? ld_psi_y(py + slot * g.slab_y, g, m, c) : Row{}; };
   auto pml_z = [&](int slot, int half, Row &r, float d[VEC]) {
-    if (m.zs) pml_row<VA>(pz + slot * g.slab_z, m.kz, r, c, g.cz + 3 * half * nz + z, nz, d);
+    if (m.zs) pml_row<VA>(pz + slot * g.slab_z + tp, m.kz, r, c, g.cz + 3 * half * nz + z, nz, d);
   };
   auto pml_x = [&](int slot, int half, Row &r, float d[VEC]) {
-    if (m.xs) pml_row<VA>(px + slot * g.slab_x, m.kx, r, c, g.cx + 3 * half * nx + x, nx, d);
+    if (m.xs) pml_row<VA>(px + slot * g.slab_x + tp, m.kx, r, c, g.cx + 3 * half * nx + x, nx, d);
   };
   auto pml_y = [&](int slot, int half, Row &r, float d[VEC]) {
-    if (m.yany) pml_row_y(py + slot * g.slab_y, r, g, m, c, half, d);
+    if (m.yany) pml_row_y(py + slot * g.slab_y + tp, r, g, m, c, half, d);
   };
 
   // one velocity from its three derivatives
@@ -346,7 +356,7 @@ k_velocity_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ buoy, int 
     pml_y(PSI_SAB1, 0, qy, dsyz_dy);
     own.wait();
     nvz = update(0, dszz_dz, dsxz_dx, dsyz_dy);
-    st_row(vz, nvz);
+    st_row(vz + tf, nvz);
   }
   if (mine(1)) {  // vx
     Row qz = ld_z(PSI_SAB1), qx = ld_x(PSI_SAA), qy = ld_y(PSI_SAB2);
@@ -373,7 +383,7 @@ k_velocity_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ buoy, int 
     pml_x(PSI_SAA, 1, qx, dsxx_dx);
     pml_y(PSI_SAB2, 0, qy, dsxy_dy);
     nvx = update(1, dsxz_dz, dsxx_dx, dsxy_dy);
-    st_row(vx, nvx);
+    st_row(vx + tf, nvx);
   }
   if (mine(2)) {  // vy
     Row qz = ld_z(PSI_SAB2), qx = ld_x(PSI_SAB2), qy = ld_y(PSI_SAA);
@@ -401,7 +411,7 @@ k_velocity_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ buoy, int 
     pml_x(PSI_SAB2, 0, qx, dsxy_dx);
     pml_y(PSI_SAA, 1, qy, dsyy_dy);
     nvy = update(2, dsyz_dz, dsxy_dx, dsyy_dy);
-    st_row(vy, nvy);
+    st_row(vy + tf, nvy);
   }
   if (IL) {
     Row hb = own.get(4);
@@ -430,27 +440,31 @@ k_velocity_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ buoy, int 
 // with 6 is no faster where a launch has few waves (75 x 109 x 91).
 void launch_stress_fwd_vec(int S, cudaStream_t st, const Geo &g, const Fields &f, const Psi &ps,
                            const float *lam, const float *mu, const SrcArgs &src,
-                           const ShellMap &shell, const IllumSum &il) {
-  const int parts = !il.first && vec_split(g, S) ? 4 : 1;
+                           const ShellMap &shell, const IllumSum &il, const StepTo &to) {
+  const int mode = il.first ? VEC_ILLUM : to.fields ? VEC_STEP_TO : VEC_STEP;
+  const int parts = mode == VEC_STEP && vec_split(g, S) ? 4 : 1;
   const dim3 grid = vec_grid(g, S, parts);
   const int nzb = grid.z / S;
   const bool va = psi_vectors(g);
-  auto k = il.first ? (va ? k_stress_fwd_vec<true, 1, 5, true> : k_stress_fwd_vec<false, 1, 5, true>)
+  auto k = mode == VEC_ILLUM ? (va ? k_stress_fwd_vec<true, 1, 5, VEC_ILLUM> : k_stress_fwd_vec<false, 1, 5, VEC_ILLUM>)
+           : mode == VEC_STEP_TO ? (va ? k_stress_fwd_vec<true, 1, 6, VEC_STEP_TO> : k_stress_fwd_vec<false, 1, 6, VEC_STEP_TO>)
            : parts > 1 ? (va ? k_stress_fwd_vec<true, 4, 8> : k_stress_fwd_vec<false, 4, 8>)
                        : (va ? k_stress_fwd_vec<true, 1, 6> : k_stress_fwd_vec<false, 1, 6>);
-  vec_launch(k, grid, parts, st, g, f, ps, lam, mu, nzb, src, shell, il);
+  vec_launch(k, grid, parts, st, g, f, ps, lam, mu, nzb, src, shell, il, to);
 }
 
 void launch_velocity_fwd_vec(int S, cudaStream_t st, const Geo &g, const Fields &f, const Psi &ps,
-                             const float *buoy, const RecFuse &rec, const IllumSum &il) {
-  const int parts = !il.first && vec_split(g, S) ? 3 : 1;
+                             const float *buoy, const RecFuse &rec, const IllumSum &il, const StepTo &to) {
+  const int mode = il.first ? VEC_ILLUM : to.fields ? VEC_STEP_TO : VEC_STEP;
+  const int parts = mode == VEC_STEP && vec_split(g, S) ? 3 : 1;
   const dim3 grid = vec_grid(g, S, parts);
   const int nzb = grid.z / S;
   const bool va = psi_vectors(g);
-  auto k = il.first ? (va ? k_velocity_fwd_vec<true, 1, 5, true> : k_velocity_fwd_vec<false, 1, 5, true>)
+  auto k = mode == VEC_ILLUM ? (va ? k_velocity_fwd_vec<true, 1, 5, VEC_ILLUM> : k_velocity_fwd_vec<false, 1, 5, VEC_ILLUM>)
+           : mode == VEC_STEP_TO ? (va ? k_velocity_fwd_vec<true, 1, 5, VEC_STEP_TO> : k_velocity_fwd_vec<false, 1, 5, VEC_STEP_TO>)
            : parts > 1 ? (va ? k_velocity_fwd_vec<true, 3, 8> : k_velocity_fwd_vec<false, 3, 8>)
                        : (va ? k_velocity_fwd_vec<true, 1, 5> : k_velocity_fwd_vec<false, 1, 5>);
-  vec_launch(k, grid, parts, st, g, f, ps, buoy, nzb, rec, il);
+  vec_launch(k, grid, parts, st, g, f, ps, buoy, nzb, rec, il, to);
 }
 
 }  // namespace efwi

@@ -108,6 +108,12 @@ void launch_rev_stress(int bx, dim3 grid, cudaStream_t st, const Geo &g, const F
                        const float *buoy, float *glam, float *gmu, int zchunk, int nzc,
                        int do_rev, int do_adj, const SrcArgs &src);
 
+// Floats from the fields and memory variables that a forward step reads to
+// those it writes (0: in place).
+struct StepTo {
+  long long fields, psi;
+};
+
 // Illumination sums [lambda, mu, buoyancy][N] of the shots of a batch: the
 // first shot's and the others' one after the other.
 struct IllumSum {
@@ -122,12 +128,15 @@ struct IllumSum {
 // shell.rows set (one shot), K_S stores the state at the start of the step
 // into shell.store at the shell points; with rec.a.plane set, K_V records the
 // new velocities of the receiver cells at sample rec.it.  With il.first set
-// they add the step's illumination to the sums of each shot.
+// they add the step's illumination to the sums of each shot.  `to` (one shot): K_S
+// takes the fields and memory variables of the state before the step; K_V the
+// stresses after its K_S and all else of the state before the step.
 void launch_stress_fwd_vec(int S, cudaStream_t st, const Geo &g, const Fields &f, const Psi &ps,
                            const float *lam, const float *mu, const SrcArgs &src,
-                           const ShellMap &shell, const IllumSum &il = {});
+                           const ShellMap &shell, const IllumSum &il = {}, const StepTo &to = {});
 void launch_velocity_fwd_vec(int S, cudaStream_t st, const Geo &g, const Fields &f, const Psi &ps,
-                             const float *buoy, const RecFuse &rec, const IllumSum &il = {});
+                             const float *buoy, const RecFuse &rec, const IllumSum &il = {},
+                             const StepTo &to = {});
 
 // Reverse sweep, one thread per four cells (efwi_rev_vec.cu).  With shell.rows
 // set (do_rev), the reverse velocities (K1) and stresses (K2) are restored at
