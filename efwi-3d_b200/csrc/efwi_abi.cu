@@ -614,7 +614,7 @@ bool use_vec(const EfwiHandle *h, const Geo &g, int S) {
 // separate launches.
 int forward_step(EfwiHandle *h, Fields f, Psi ps, int S, const SrcArgs &src, const RecArgs &rec,
                  float *traces_tm, cudaStream_t st, int it, float *shell = nullptr,
-                 const IllumSum &il = {}, const StepTo &to = {}) {
+                 const IllumSum &il = {}, const StepTo &to = {}, bool chained = false) {
   const bool vec = use_vec(h, h->geo, S);  // `to`: vector kernels only
   int nzc;
   const dim3 grid = stencil_grid(h, S, h->bx, h->zchunk, &nzc);
@@ -635,7 +635,9 @@ int forward_step(EfwiHandle *h, Fields f, Psi ps, int S, const SrcArgs &src, con
     Timer t(h, K_STRESS_FWD, st, it);
     if (vec)
       launch_stress_fwd_vec(S, st, h->geo, f, ps, h->lam.as<float>(), h->mu.as<float>(), src, shm,
-                            il, to);
+                            il, to,
+                            chained && (rec.ncell == 0 || rec_fused) &&
+                                (!shell || h->npts == 0 || shm.rows));
     else
       launch_stress_fwd(h->bx, grid, st, h->geo, f, ps, h->lam.as<float>(), h->mu.as<float>(),
                         h->zchunk, nzc, src);
@@ -711,7 +713,7 @@ int run_forward_batch(EfwiHandle *h, const int *ids, int S, float *traces_tm, lo
     for (int it = 0; it <= ntl - 2; ++it) {
       b.src.it = it;
       const int r = forward_step(h, b.f, b.ps, S, b.src, b.rec, traces_tm, s, it,
-                                 shell ? shell + (size_t)it * 9 * npts : nullptr);
+                                 shell ? shell + (size_t)it * 9 * npts : nullptr, {}, {}, it > 0);
       if (r) return r;
     }
     return check_launch(h, "forward");
@@ -895,7 +897,7 @@ int exact_shot(EfwiHandle *h, int id, const float *obs, double *jdev, float *res
           to = slot(plan.actions[ia + 1].a);
         rc = forward_step(h, fields_at(cur.fields, N, 1), psi_at(cur.psi, h->geo, 1), 1, b.src,
                           first ? b.rec : norec, h->traces_tm.as<float>(), st, it, nullptr, {},
-                          StepTo{apart(to.fields, cur.fields), apart(to.psi, cur.psi)});
+                          StepTo{apart(to.fields, cur.fields), apart(to.psi, cur.psi)}, it > act.a);
         if (rc) return rc;
         cur = to;
       }
@@ -1033,7 +1035,8 @@ int window_loop_vec(EfwiHandle *h, const std::vector<Domain> &dom, const std::ve
       for (int k = gbeg[g]; k < gbeg[g + 1]; ++k) {
         const Domain &d = dom[k];
         const SrcArgs src{dsrc + k, d.stf, nt, it, it_dev};
-        launch_stress_fwd_vec(1, s, d.g, d.f, d.ps, d.lam, d.mu, src, ShellMap{});
+        launch_stress_fwd_vec(1, s, d.g, d.f, d.ps, d.lam, d.mu, src, ShellMap{}, {}, {},
+                              k > gbeg[g]);
         launch_velocity_fwd_vec(1, s, d.g, d.f, d.ps, d.buoy, RecFuse{});
       }
       const int r0 = rstart[gbeg[g]], r1 = rstart[gbeg[g + 1]];
@@ -1449,6 +1452,9 @@ static int gradient_impl(EfwiHandle *h, int n, const int *ids, const float *obs,
       }
       return m;
     };
+    // nothing but K1 and K2 in the loop: each may start in the other's tail
+    const bool chain1 = shell_fused || npts == 0;
+    const bool chain2 = chain1 && (inj_fused || rec.ncell == 0);
     auto K1 = [&](int rev, int adj, int it) {
       Timer t(h, K_REV_VELOCITY, st, it);
       const ShellMap sm = shell_at(rev, it);
@@ -1456,7 +1462,7 @@ static int gradient_impl(EfwiHandle *h, int n, const int *ids, const float *obs,
       if (inj_fused && adj) inj = RecFuse{rec, h->res_tm.as<float>(), it};
       if (vec)
         launch_rev_velocity_vec(st, h->geo, f, a, ps, h->lam.as<float>(), h->mu.as<float>(),
-                                h->buoy.as<float>(), grho, rev, adj, sm, inj);
+                                h->buoy.as<float>(), grho, rev, adj, sm, inj, rev && chain1);
       else
         launch_rev_velocity(h->bx, grid, st, h->geo, f, a, ps, h->lam.as<float>(),
                             h->mu.as<float>(), h->buoy.as<float>(), grho, zcr, nzc, rev, adj);
@@ -1466,7 +1472,8 @@ static int gradient_impl(EfwiHandle *h, int n, const int *ids, const float *obs,
       src.it = it;
       if (vec)
         launch_rev_stress_vec(st, h->geo, f, a, ps, h->lam.as<float>(), h->mu.as<float>(),
-                              h->buoy.as<float>(), glam, gmu, rev, adj, src, shell_at(rev, it));
+                              h->buoy.as<float>(), glam, gmu, rev, adj, src, shell_at(rev, it),
+                              chain2);
       else
         launch_rev_stress(h->bx, grid, st, h->geo, f, a, ps, h->lam.as<float>(), h->mu.as<float>(),
                           h->buoy.as<float>(), glam, gmu, zcr, nzc, rev, adj, src);
@@ -2056,7 +2063,8 @@ int efwi_illumination(EfwiHandle *h, int n, const int *ids, float *h_lam, float 
     const dim3 grid((h->grid.ny + 31) / 32, (h->grid.nx + 3) / 4, (h->grid.nz - 4 + 7) / 8);
     for (int it = 0; it <= ntl - 2; ++it) {
       b.src.it = it;
-      rc = forward_step(h, b.f, b.ps, S, b.src, norec, nullptr, st, it, nullptr, sums);
+      rc = forward_step(h, b.f, b.ps, S, b.src, norec, nullptr, st, it, nullptr, sums, {},
+                        sums.first && it > 0);
       if (rc) return rc;
       if (sums.first) continue;
       Timer t(h, K_OTHER, st, it);

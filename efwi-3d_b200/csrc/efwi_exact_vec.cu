@@ -536,13 +536,13 @@ __global__ void __launch_bounds__(VEC_THREADS, MINB) k_adj_velocity_vec(ExactArg
 // 92 / 85; asking for the second phase's rows before the first makes them 87
 // and 80.
 void launch_adj_stress_vec(cudaStream_t st, const ExactArgs &A) {
-  if (psi_vectors(A.g)) vec_launch(k_adj_stress_vec<true, 6>, vec_grid(A.g), 1, st, A);
-  else vec_launch(k_adj_stress_vec<false, 6>, vec_grid(A.g), 1, st, A);
+  if (psi_vectors(A.g)) vec_launch(k_adj_stress_vec<true, 6>, vec_grid(A.g), 1, true, st, A);
+  else vec_launch(k_adj_stress_vec<false, 6>, vec_grid(A.g), 1, true, st, A);
 }
 
 void launch_adj_velocity_vec(cudaStream_t st, const ExactArgs &A) {
-  if (psi_vectors(A.g)) vec_launch(k_adj_velocity_vec<true, 6>, vec_grid(A.g), 1, st, A);
-  else vec_launch(k_adj_velocity_vec<false, 6>, vec_grid(A.g), 1, st, A);
+  if (psi_vectors(A.g)) vec_launch(k_adj_velocity_vec<true, 6>, vec_grid(A.g), 1, true, st, A);
+  else vec_launch(k_adj_velocity_vec<false, 6>, vec_grid(A.g), 1, true, st, A);
 }
 
 }  // namespace efwi

@@ -51,7 +51,6 @@ k_stress_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ lam,
   const int nz = g.nz, nx = g.nx, ny = g.ny;
   if (z > nz - 3 || x > nx - 3 || y > ny - 3) return;
   const VecCell c = vec_cell(g, z, x, y);
-  vec_begin();
   const long long so = (long long)shot * g.N + c.i;
   const float *__restrict__ vz = f.vz + so;
   const float *__restrict__ vx = f.vx + so;
@@ -83,6 +82,7 @@ k_stress_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ lam,
   float *pz = ps.z + (long long)shot * 6 * g.slab_z;
   float *px = ps.x + (long long)shot * 6 * g.slab_x;
   float *py = ps.y + (long long)shot * 6 * g.slab_y;
+  vec_begin();  // up to here: nothing that the velocity kernel writes
   if (shell.rows) {  // from_bnd: the state at the start of the step
     const int srow = shell.rows[z * nx + x];
     int sk[VEC];
@@ -267,7 +267,6 @@ k_velocity_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ buoy, int 
   const int nz = g.nz, nx = g.nx, ny = g.ny;
   if (z > nz - 3 || x > nx - 3 || y > ny - 3) return;
   const VecCell c = vec_cell(g, z, x, y);
-  vec_begin();
   const long long so = (long long)shot * g.N + c.i;
   const float *__restrict__ szz = f.szz + so;
   const float *__restrict__ sxx = f.sxx + so;
@@ -299,6 +298,7 @@ k_velocity_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ buoy, int 
   float *pz = ps.z + (long long)shot * 6 * g.slab_z;
   float *px = ps.x + (long long)shot * 6 * g.slab_x;
   float *py = ps.y + (long long)shot * 6 * g.slab_y;
+  vec_begin();  // up to here: nothing that the stress kernel writes
   // memory variables `slot` of one axis, and their derivative's update (half:
   // the coefficients at half points)
   auto ld_z = [&](int slot) { return m.zs ? ld_psi<VA>(pz + slot * g.slab_z, m.kz, c) : Row{}; };
@@ -440,7 +440,7 @@ k_velocity_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ buoy, int 
 // with 6 is no faster where a launch has few waves (75 x 109 x 91).
 void launch_stress_fwd_vec(int S, cudaStream_t st, const Geo &g, const Fields &f, const Psi &ps,
                            const float *lam, const float *mu, const SrcArgs &src,
-                           const ShellMap &shell, const IllumSum &il, const StepTo &to) {
+                           const ShellMap &shell, const IllumSum &il, const StepTo &to, bool after_velocity) {
   const int mode = il.first ? VEC_ILLUM : to.fields ? VEC_STEP_TO : VEC_STEP;
   const int parts = mode == VEC_STEP && vec_split(g, S) ? 4 : 1;
   const dim3 grid = vec_grid(g, S, parts);
@@ -450,7 +450,7 @@ void launch_stress_fwd_vec(int S, cudaStream_t st, const Geo &g, const Fields &f
            : mode == VEC_STEP_TO ? (va ? k_stress_fwd_vec<true, 1, 6, VEC_STEP_TO> : k_stress_fwd_vec<false, 1, 6, VEC_STEP_TO>)
            : parts > 1 ? (va ? k_stress_fwd_vec<true, 4, 8> : k_stress_fwd_vec<false, 4, 8>)
                        : (va ? k_stress_fwd_vec<true, 1, 6> : k_stress_fwd_vec<false, 1, 6>);
-  vec_launch(k, grid, parts, st, g, f, ps, lam, mu, nzb, src, shell, il, to);
+  vec_launch(k, grid, parts, after_velocity, st, g, f, ps, lam, mu, nzb, src, shell, il, to);
 }
 
 void launch_velocity_fwd_vec(int S, cudaStream_t st, const Geo &g, const Fields &f, const Psi &ps,
@@ -464,7 +464,7 @@ void launch_velocity_fwd_vec(int S, cudaStream_t st, const Geo &g, const Fields 
            : mode == VEC_STEP_TO ? (va ? k_velocity_fwd_vec<true, 1, 5, VEC_STEP_TO> : k_velocity_fwd_vec<false, 1, 5, VEC_STEP_TO>)
            : parts > 1 ? (va ? k_velocity_fwd_vec<true, 3, 8> : k_velocity_fwd_vec<false, 3, 8>)
                        : (va ? k_velocity_fwd_vec<true, 1, 5> : k_velocity_fwd_vec<false, 1, 5>);
-  vec_launch(k, grid, parts, st, g, f, ps, buoy, nzb, rec, il, to);
+  vec_launch(k, grid, parts, true, st, g, f, ps, buoy, nzb, rec, il, to);
 }
 
 }  // namespace efwi

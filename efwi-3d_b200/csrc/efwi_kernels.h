@@ -130,10 +130,13 @@ struct IllumSum {
 // new velocities of the receiver cells at sample rec.it.  With il.first set
 // they add the step's illumination to the sums of each shot.  `to` (one shot): K_S
 // takes the fields and memory variables of the state before the step; K_V the
-// stresses after its K_S and all else of the state before the step.
+// stresses after its K_S and all else of the state before the step.  K_V
+// follows its K_S in the stream, with nothing between them; after_velocity: so
+// does K_S a K_V.
 void launch_stress_fwd_vec(int S, cudaStream_t st, const Geo &g, const Fields &f, const Psi &ps,
                            const float *lam, const float *mu, const SrcArgs &src,
-                           const ShellMap &shell, const IllumSum &il = {}, const StepTo &to = {});
+                           const ShellMap &shell, const IllumSum &il = {}, const StepTo &to = {},
+                           bool after_velocity = false);
 void launch_velocity_fwd_vec(int S, cudaStream_t st, const Geo &g, const Fields &f, const Psi &ps,
                              const float *buoy, const RecFuse &rec, const IllumSum &il = {},
                              const StepTo &to = {});
@@ -142,14 +145,16 @@ void launch_velocity_fwd_vec(int S, cudaStream_t st, const Geo &g, const Fields 
 // set (do_rev), the reverse velocities (K1) and stresses (K2) are restored at
 // the shell points from shell.store; with inj.a.plane set (do_adj), K1 adds
 // the adjoint source inj.tm at sample inj.it to the adjoint velocities.
+// after_stress, after_velocity: the launch follows the other kernel of the
+// sweep in the stream, with nothing between them.
 void launch_rev_velocity_vec(cudaStream_t st, const Geo &g, const Fields &f, const Fields &a,
                              const Psi &ps, const float *lam, const float *mu, const float *buoy,
                              float *grho, int do_rev, int do_adj, const ShellMap &shell,
-                             const RecFuse &inj);
+                             const RecFuse &inj, bool after_stress);
 void launch_rev_stress_vec(cudaStream_t st, const Geo &g, const Fields &f, const Fields &a,
                            const Psi &ps, const float *lam, const float *mu, const float *buoy,
                            float *glam, float *gmu, int do_rev, int do_adj, const SrcArgs &src,
-                           const ShellMap &shell);
+                           const ShellMap &shell, bool after_velocity);
 
 __global__ void k_prep_buoyancy(const float *rho, float *buoy, int nz, int nx, int ny, int py);
 __global__ void k_window_slice(const float *src, float *dst, int nz, int nx, int pyg, int x0,

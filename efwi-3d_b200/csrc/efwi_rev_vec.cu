@@ -84,7 +84,6 @@ k_rev_velocity_vec(Geo g, Fields f, Fields a, Psi ps, const float *__restrict__ 
   const int nz = g.nz, nx = g.nx, ny = g.ny;
   if (z > nz - 3 || x > nx - 3 || y > ny - 3) return;
   const VecCell c = vec_cell(g, z, x, y);
-  vec_begin();
   const Diff D{c};
   const int i = c.i, sz = (int)g.sz, sx = g.sx;
   const float dt = g.dt, idz = g.idz, idx = g.idx, idy = g.idy;
@@ -113,6 +112,7 @@ k_rev_velocity_vec(Geo g, Fields f, Fields a, Psi ps, const float *__restrict__ 
     own.fetch(VZ, f.vz + i); own.fetch(VX, f.vx + i); own.fetch(VY, f.vy + i);
     if (any_in) own.fetch(GR, grho + i);
   }
+  vec_begin();  // up to here: nothing that the stress kernel writes
   if (any_in || any_sk) {
     Row gi{};
     // reverse update of one velocity and its share of the rho image
@@ -304,7 +304,6 @@ k_rev_stress_vec(Geo g, Fields f, Fields a, Psi ps, const float *__restrict__ la
   const int nz = g.nz, nx = g.nx, ny = g.ny;
   if (z > nz - 3 || x > nx - 3 || y > ny - 3) return;
   const VecCell c = vec_cell(g, z, x, y);
-  vec_begin();
   const Diff D{c};
   const int i = c.i, sz = (int)g.sz, sx = g.sx;
   const float dt = g.dt, idz = g.idz, idx = g.idx, idy = g.idy;
@@ -335,6 +334,7 @@ k_rev_stress_vec(Geo g, Fields f, Fields a, Psi ps, const float *__restrict__ la
     if (any_in) { own.fetch(GL, glam + i); own.fetch(GM, gmu + i); }
   }
   if (do_adj) own.fetch(BU, buoy + i);
+  vec_begin();  // up to here: nothing that the velocity kernel writes
   if (any_rev) {
     auto restore = [&](int q, Row &n) {
       if (!any_sk) return;
@@ -555,21 +555,21 @@ k_rev_stress_vec(Geo g, Fields f, Fields a, Psi ps, const float *__restrict__ la
 void launch_rev_velocity_vec(cudaStream_t st, const Geo &g, const Fields &f, const Fields &a,
                              const Psi &ps, const float *lam, const float *mu, const float *buoy,
                              float *grho, int do_rev, int do_adj, const ShellMap &shell,
-                             const RecFuse &inj) {
+                             const RecFuse &inj, bool after_stress) {
   if (psi_vectors(g))
-    vec_launch(k_rev_velocity_vec<true, 6>, vec_grid(g), 1, st, g, f, a, ps, lam, mu, buoy, grho, do_rev, do_adj, shell, inj);
+    vec_launch(k_rev_velocity_vec<true, 6>, vec_grid(g), 1, after_stress, st, g, f, a, ps, lam, mu, buoy, grho, do_rev, do_adj, shell, inj);
   else
-    vec_launch(k_rev_velocity_vec<false, 6>, vec_grid(g), 1, st, g, f, a, ps, lam, mu, buoy, grho, do_rev, do_adj, shell, inj);
+    vec_launch(k_rev_velocity_vec<false, 6>, vec_grid(g), 1, after_stress, st, g, f, a, ps, lam, mu, buoy, grho, do_rev, do_adj, shell, inj);
 }
 
 void launch_rev_stress_vec(cudaStream_t st, const Geo &g, const Fields &f, const Fields &a,
                            const Psi &ps, const float *lam, const float *mu, const float *buoy,
                            float *glam, float *gmu, int do_rev, int do_adj, const SrcArgs &src,
-                           const ShellMap &shell) {
+                           const ShellMap &shell, bool after_velocity) {
   if (psi_vectors(g))
-    vec_launch(k_rev_stress_vec<true, 5>, vec_grid(g), 1, st, g, f, a, ps, lam, mu, buoy, glam, gmu, do_rev, do_adj, src, shell);
+    vec_launch(k_rev_stress_vec<true, 5>, vec_grid(g), 1, after_velocity, st, g, f, a, ps, lam, mu, buoy, glam, gmu, do_rev, do_adj, src, shell);
   else
-    vec_launch(k_rev_stress_vec<false, 5>, vec_grid(g), 1, st, g, f, a, ps, lam, mu, buoy, glam, gmu, do_rev, do_adj, src, shell);
+    vec_launch(k_rev_stress_vec<false, 5>, vec_grid(g), 1, after_velocity, st, g, f, a, ps, lam, mu, buoy, glam, gmu, do_rev, do_adj, src, shell);
 }
 
 }  // namespace efwi

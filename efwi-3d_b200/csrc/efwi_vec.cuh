@@ -362,13 +362,15 @@ inline bool vec_fits(const Geo &g, int S) {
          (long long)S * ((g.nz - 4 + VEC_TZ - 1) / VEC_TZ) <= 65535;
 }
 
-// Launch of a stencil kernel that may begin while the kernel before it in
-// the stream drains (programmatic dependent launch): the kernels order their
-// reads and writes with vec_begin().  What overlaps is the launch itself and
-// the index arithmetic, 1-2 us of a launch that takes 4 on the smallest
-// grids.
+// Launch of a stencil kernel.  `chained`: it may begin while the kernel before
+// it in the stream drains (programmatic dependent launch).  Then what the
+// kernel reads before vec_begin() must not be written by the kernel right
+// before it; kernels further back are complete, since that one is past its own
+// vec_begin().  Such reads are the rows of the fields that the kernel itself
+// updates, the model and the images.
 template <class... P, class... T>
-inline void vec_launch(void (*kernel)(P...), dim3 grid, int parts, cudaStream_t st, T... args) {
+inline void vec_launch(void (*kernel)(P...), dim3 grid, int parts, bool chained, cudaStream_t st,
+                       T... args) {
   cudaLaunchAttribute at{};
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at.val.programmaticStreamSerializationAllowed = 1;
@@ -377,13 +379,12 @@ inline void vec_launch(void (*kernel)(P...), dim3 grid, int parts, cudaStream_t 
   cf.blockDim = dim3(VEC_TY, VEC_TX, vec_tz(parts) * parts);
   cf.stream = st;
   cf.attrs = &at;
-  cf.numAttrs = 1;
+  cf.numAttrs = chained ? 1 : 0;
   cudaLaunchKernelEx(&cf, kernel, static_cast<P>(args)...);
 }
 // Waits until the kernels before this one are complete and their writes
 // visible, then lets the next kernel's CTAs start (once all of this grid's
-// have come here or left).  Nothing that a kernel of the time loop writes is
-// touched before it.
+// have come here or left).
 __device__ __forceinline__ void vec_begin() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
