@@ -566,7 +566,8 @@ int upload_receivers(EfwiHandle *h, const RecHost &r, cudaStream_t st, RecArgs *
       std::vector<int> maps((size_t)nmaps * nxpy, -1);
       for (size_t u = 0; u < r.ucell.size(); ++u) {
         const int m = plane[(size_t)r.ushot[u] * nz + (int)(r.ucell[u] / nxpy)];
-        maps[(size_t)m * nxpy + (size_t)(r.ucell[u] % nxpy)] = (int)u;
+        maps[(size_t)m * nxpy + (size_t)(r.ucell[u] % nxpy)] =
+            r.uptr[u + 1] - r.uptr[u] == 1 ? -2 - r.rec[r.uptr[u]] : (int)u;
       }
       const size_t pb = al(plane.size() * 4);
       CK_CUDA(h, h->recmap.ensure(pb + maps.size() * 4));

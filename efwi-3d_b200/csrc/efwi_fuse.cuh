@@ -43,37 +43,51 @@ __device__ __forceinline__ bool shell_cells(const ShellMap &s, int row, const Ve
   return any;
 }
 
-// Unique receiver cell at (shot, z, x, y), or -1.
-__device__ __forceinline__ int receiver_at(const RecArgs &r, int nz, int py, int shot, int z,
-                                           int x, int y) {
-  const int mp = r.plane[shot * nz + z];
-  if (mp < 0) return -1;
-  return r.map[(long long)mp * r.nxpy + x * py + y];
+// Map of the receiver cells in plane z of the shot, or -1.
+__device__ __forceinline__ int receiver_map(const RecArgs &r, int nz, int shot, int z) {
+  return r.plane ? r.plane[shot * nz + z] : -1;
+}
+// The map's entries at the four cells of vector c.
+__device__ __forceinline__ const float *receiver_row(const RecArgs &r, int map, const Geo &g,
+                                                     const VecCell &c) {
+  return reinterpret_cast<const float *>(r.map + (long long)map * r.nxpy + c.x * g.sx + c.y);
 }
 
-// recording (utilities.cu:481-495) of one component (0 vx, 1 vy, 2 vz) of
-// unique receiver cell u at sample it.
-__device__ __forceinline__ void record_cell(const RecArgs &rec, float *traces_tm, int it, int u,
-                                            int comp, float v) {
-  const int s = rec.ushot[u];
-  const int nr = rec.nrec[s];
-  float *t = traces_tm + rec.trace_off[s] + ((long long)it * 3 + comp) * nr;
-  for (int k = rec.uptr[u]; k < rec.uptr[u + 1]; ++k) t[rec.rec[k]] = v;
+// f(r) for the receivers r on a cell with map entry u, in their order.
+template <class F>
+__device__ __forceinline__ void receivers_of(const RecArgs &rec, int u, F f) {
+  int k = 0, end = 1;
+  if (u >= 0) { k = rec.uptr[u]; end = rec.uptr[u + 1]; }
+#pragma unroll 1
+  for (; k < end; ++k) f(u >= 0 ? rec.rec[k] : -2 - u);
 }
 
-// res_injection (utilities.cu:497-507) at unique receiver cell u: the
-// receivers on the cell are added one after the other in receiver order.
+// recording (utilities.cu:481-495) of the components wanted (x, y, z) at a
+// receiver cell of the shot (map entry u) at sample it.
+__device__ __forceinline__ void record_cell(const RecArgs &rec, float *traces_tm, int it, int shot,
+                                            int u, bool x, float vx, bool y, float vy, bool z,
+                                            float vz) {
+  const int nr = rec.nrec[shot];
+  float *t = traces_tm + rec.trace_off[shot] + (long long)it * 3 * nr;
+  receivers_of(rec, u, [&](int r) {
+    if (x) t[r] = vx;
+    if (y) t[nr + r] = vy;
+    if (z) t[2 * nr + r] = vz;
+  });
+}
+
+// res_injection (utilities.cu:497-507) at a receiver cell of shot 0 (map
+// entry u): the receivers on the cell are added one after the other in
+// receiver order.
 __device__ __forceinline__ void inject_cell(const RecArgs &rec, const float *res_tm, int it, int u,
                                             float &vz, float &vx, float &vy) {
-  const int s = rec.ushot[u];
-  const int nr = rec.nrec[s];
-  const float *t = res_tm + rec.trace_off[s] + (long long)it * 3 * nr;
-  for (int k = rec.uptr[u]; k < rec.uptr[u + 1]; ++k) {
-    const int r = rec.rec[k];
+  const int nr = rec.nrec[0];
+  const float *t = res_tm + rec.trace_off[0] + (long long)it * 3 * nr;
+  receivers_of(rec, u, [&](int r) {
     vx += t[r];
     vy += t[nr + r];
     vz += t[2 * nr + r];
-  }
+  });
 }
 
 }  // namespace efwi

@@ -277,7 +277,7 @@ k_velocity_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ buoy, int 
   const int sz = (int)g.sz, sx = g.sx;
   const float idz = g.idz, idx = g.idx, idy = g.idy, dt = g.dt;
   float *vz = f.vz + so, *vx = f.vx + so, *vy = f.vy + so;
-  __shared__ float4 stash[(IL ? 5 : 4) * T];
+  __shared__ float4 stash[(IL || PARTS > 1 ? 5 : 4) * T];
   Stash<T> own{stash + vec_thread()};
   // outputs of the thread: 0 vz, 1 vx, 2 vy
   auto mine = [&](int k) { return PARTS == 1 || part == k; };
@@ -289,8 +289,8 @@ k_velocity_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ buoy, int 
   if (IL) own.fetch(4, il.of(shot, 2) + c.i);
   if (g.far)
     for (const float *p : {sxx, sxy, syy}) prefetch_row(p);
-  // receiver map of this plane, loaded first so that its latency overlaps
-  const int rmap = rec.a.plane ? rec.a.plane[shot * nz + z] : -1;
+  const int rmap = receiver_map(rec.a, nz, shot, z);  // early: the latency overlaps
+  if (PARTS > 1 && rmap >= 0) own.fetch(4, receiver_row(rec.a, rmap, g, c));
 
   const Pml<VA> m = pml_of<VA>(g, c, true);
   prefetch_psi<3>(g, Psi{ps.z + (long long)shot * 6 * g.slab_z, ps.x + (long long)shot * 6 * g.slab_x,
@@ -421,16 +421,15 @@ k_velocity_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ buoy, int 
     st_row(il.of(shot, 2) + c.i, hb);
   }
   if (rmap >= 0) {
-    const int4 u = *reinterpret_cast<const int4 *>(rec.a.map + (long long)rmap * rec.a.nxpy +
-                                                   x * g.sx + y);
-    const int us[VEC] = {u.x, u.y, u.z, u.w};
+    // fetched ahead where a launch is one thread's chain of loads; elsewhere
+    // that only costs (84^3 misfit + 2 %)
+    const Row entry = PARTS > 1 ? own.get(4) : ld_row(receiver_row(rec.a, rmap, g, c));
 #pragma unroll
-    for (int e = 0; e < VEC; ++e)
-      if (c.act[e] && us[e] >= 0) {
-        if (mine(1)) record_cell(rec.a, rec.tm, rec.it, us[e], 0, nvx[e]);
-        if (mine(2)) record_cell(rec.a, rec.tm, rec.it, us[e], 1, nvy[e]);
-        if (mine(0)) record_cell(rec.a, rec.tm, rec.it, us[e], 2, nvz[e]);
-      }
+    for (int e = 0; e < VEC; ++e) {
+      const int u = __float_as_int(entry[e]);
+      if (c.act[e] && u != -1)
+        record_cell(rec.a, rec.tm, rec.it, shot, u, mine(1), nvx[e], mine(2), nvy[e], mine(0), nvz[e]);
+    }
   }
 }
 

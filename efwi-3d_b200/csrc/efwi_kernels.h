@@ -33,8 +33,10 @@ struct RecArgs {
   const int *nrec;      // per shot
   int ncell;
   // Cell lookup for kernels that gather or inject in their own epilogue:
-  // plane[s * nz + z] names a map [nx][py] of unique receiver cells u in
-  // plane z of shot s (-1 elsewhere), or is -1 when the plane holds none;
+  // plane[s * nz + z] names a map [nx][py] of the receiver cells in plane z
+  // of shot s, or is -1 when the plane holds none; entries: -2 - r where
+  // receiver r alone lies on the cell (no further lookup), u where several
+  // do, -1 elsewhere.
   // plane == nullptr: no lookup (separate k_record / k_inject launches).
   const int *plane;
   const int *map;

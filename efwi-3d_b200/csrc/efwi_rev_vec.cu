@@ -107,7 +107,7 @@ k_rev_velocity_vec(Geo g, Fields f, Fields a, Psi ps, const float *__restrict__ 
     const int srow = shell.rows[z * nx + x];
     if (srow >= 0) any_sk = shell_cells(shell, srow, c, sk);
   }
-  const int rmap = (do_adj && inj.a.plane) ? inj.a.plane[z] : -1;
+  const int rmap = do_adj ? receiver_map(inj.a, nz, 0, z) : -1;
   if (any_in || any_sk) {
     own.fetch(VZ, f.vz + i); own.fetch(VX, f.vx + i); own.fetch(VY, f.vy + i);
     if (any_in) own.fetch(GR, grho + i);
@@ -282,13 +282,13 @@ k_rev_velocity_vec(Geo g, Fields f, Fields a, Psi ps, const float *__restrict__ 
     feed(nay, b, PSI_SAB2, CB, PSI_SAB2, CBH, PSI_SAA);
   }
   if (rmap >= 0) {  // res_injection after the adjoint update
-    const int4 u = *reinterpret_cast<const int4 *>(inj.a.map + (long long)rmap * inj.a.nxpy +
-                                                   x * sx + y);
-    const int us[VEC] = {u.x, u.y, u.z, u.w};
+    const Row entry = ld_row(receiver_row(inj.a, rmap, g, c));
 #pragma unroll
-    for (int e = 0; e < VEC; ++e)
-      if (c.act[e] && us[e] >= 0)
-        inject_cell(inj.a, inj.tm, inj.it, us[e], naz.v[e], nax.v[e], nay.v[e]);
+    for (int e = 0; e < VEC; ++e) {
+      const int u = __float_as_int(entry[e]);
+      if (c.act[e] && u != -1)
+        inject_cell(inj.a, inj.tm, inj.it, u, naz.v[e], nax.v[e], nay.v[e]);
+    }
   }
   st_row(a.vx + i, nax); st_row(a.vz + i, naz); st_row(a.vy + i, nay);
 }
