@@ -6,11 +6,15 @@
 //
 // A CTA (8 vectors x 4 rows x 4 planes) forms the Q of its cells and of their
 // halo once into shared memory -- z-axis terms with two planes on each side,
-// x-axis terms with two rows, y-axis terms with a vector -- and after its one
-// barrier every thread gathers from there.  Forming the neighbours' Q in
-// every thread from global memory instead takes 66 row loads per thread where
-// this takes 24 and thrashes L1: 105 / 91 us per launch (stress / velocity
-// stage) at 120^3.
+// x-axis terms with two rows, y-axis terms with a vector -- and after a barrier
+// every thread gathers from there.  Forming the neighbours' Q in every thread
+// from global memory instead takes 66 row loads per thread where this takes 24
+// and thrashes L1: 105 / 91 us per launch (stress / velocity stage) at 120^3.
+//
+// A vector has two threads.  Latency bounds the kernel (a third of the DRAM and
+// L2 rates), and the images need nothing of the Q: the second half of the
+// warps forms them while the first takes the Q's items, 32 at a time, then
+// helps with what is left; after the barrier the halves share the outputs.
 #include "efwi_common.cuh"
 #include "efwi_exact.h"
 #include "efwi_vec.cuh"
@@ -25,11 +29,14 @@ struct QTile {
   float4 z[3][QZ][VEC_TX][VEC_TY];
   float4 x[3][VEC_TZ][QX][VEC_TY];
   float4 y[3][VEC_TZ][VEC_TX][QY];
+  int next;  // item of the first phase that no warp has taken yet
 };
 // Work of the first phase: the CTA's rows (QY vectors each, the outer two for
 // the y terms only), the z halo's rows, the x halo's.
 constexpr int kItemsC = VEC_TZ * VEC_TX * QY, kItemsZ = 4 * VEC_TX * VEC_TY,
               kItemsX = 4 * VEC_TZ * VEC_TY, kItems = kItemsC + kItemsZ + kItemsX;
+static_assert(kItemsC % 32 == 0 && kItemsZ % 32 == 0 && kItemsX % 32 == 0, "one kind per warp");
+constexpr int EX_THREADS = 2 * VEC_THREADS;  // two threads per vector
 
 __device__ __forceinline__ float4 to4(const Row &r) {
   return make_float4(r.v[0], r.v[1], r.v[2], r.v[3]);
@@ -98,8 +105,12 @@ template <bool VA, bool V, class Load>
 __device__ __forceinline__ void fill_q(QTile &q, const Geo &g, const Psi &lin, const Psi &lout,
                                        int x0, int y0, int z0, const Term tz[3], const Term tx[3],
                                        const Term ty[3], const Load &load) {
-#pragma unroll 1
-  for (int it = vec_thread(); it < kItems; it += VEC_THREADS) {
+  const int lane = vec_thread() & 31;
+  for (;;) {
+    // 32 items for the warp (the kinds' counts are multiples of 32)
+    int it = lane == 0 ? atomicAdd(&q.next, 32) : 0;
+    it = __shfl_sync(0xffffffffu, it, 0) + lane;
+    if (it >= kItems) break;
     // the item's row and vector relative to the CTA
     int dz, dx, v, kind;
     if (it < kItemsC) {
@@ -165,14 +176,15 @@ __device__ __forceinline__ void fill_q(QTile &q, const Geo &g, const Psi &lin, c
 struct QGather {
   const QTile &q;
   const Geo &g;
+  const int tz;
   __device__ __forceinline__ Row z(int k, int d) const {
-    return row4(q.z[k][threadIdx.z + 2 + d][threadIdx.y][threadIdx.x]);
+    return row4(q.z[k][tz + 2 + d][threadIdx.y][threadIdx.x]);
   }
   __device__ __forceinline__ Row x(int k, int d) const {
-    return row4(q.x[k][threadIdx.z][threadIdx.y + 2 + d][threadIdx.x]);
+    return row4(q.x[k][tz][threadIdx.y + 2 + d][threadIdx.x]);
   }
   __device__ __forceinline__ Span y(int k) const {
-    const float4 *p = &q.y[k][threadIdx.z][threadIdx.y][threadIdx.x + 1];
+    const float4 *p = &q.y[k][tz][threadIdx.y][threadIdx.x + 1];
     const float4 l = p[-1], m = p[0], h = p[1];
     return Span{{l.z, l.w, m.x, m.y, m.z, m.w, h.x, h.y}};
   }
@@ -244,20 +256,97 @@ __device__ __forceinline__ Row diff_my(const float *q, const VecCell &c, float i
 }  // namespace
 
 template <bool VA, int MINB>
-__global__ void __launch_bounds__(VEC_THREADS, MINB) k_adj_stress_vec(ExactArgs A) {
+__global__ void __launch_bounds__(EX_THREADS, MINB) k_adj_stress_vec(ExactArgs A) {
   const Geo &g = A.g;
   __shared__ QTile q;
   const int z0 = 2 + blockIdx.z * VEC_TZ, x0 = 2 + blockIdx.y * VEC_TX,
             y0 = VEC * blockIdx.x * VEC_TY;
-  const int z = z0 + threadIdx.z, x = x0 + threadIdx.y, y = y0 + VEC * threadIdx.x;
+  const int tz = threadIdx.z % VEC_TZ, part = threadIdx.z / VEC_TZ;
+  const int z = z0 + tz, x = x0 + threadIdx.y, y = y0 + VEC * threadIdx.x;
   const int nz = g.nz, nx = g.nx;
   const int sz = (int)g.sz, sx = g.sx;
   const float dt = g.dt, idz = g.idz, idx = g.idx, idy = g.idy;
+  if (threadIdx.x + threadIdx.y + threadIdx.z == 0) q.next = 0;
+  __syncthreads();
   vec_begin();
-  if (g.far && z <= nz - 3 && x <= nx - 3) {  // read after the barrier
-    const int i = (z * nx + x) * sx + y;
-    for (const float *p : {A.a.vz, A.a.vx, A.a.vy, A.f.vz, A.f.vx, A.f.vy}) prefetch_row(p + i);
-    if (A.g0) { prefetch_row(A.g0 + i); prefetch_row(A.g1 + i); }
+  const bool in = z <= nz - 3 && x <= nx - 3 && y <= g.ny - 3;
+  const VecCell c = vec_cell(g, z, x, y);
+  const int i = c.i;
+  if (g.far && part == 0 && in)  // read after the barrier
+    for (const float *p : {A.a.vz, A.a.vx, A.a.vy}) prefetch_row(p + i);
+  if (part == 1 && in && A.g0) {
+    const Pml<VA> m = pml_of<VA>(g, c, false);
+    const int lz = (int)g.slab_z, lx = (int)g.slab_x, ly = (int)g.slab_y;
+    const float *azz = A.a.szz + i, *axx = A.a.sxx + i, *ayy = A.a.syy + i;
+    const float *axz = A.a.sxz + i, *axy = A.a.sxy + i, *ayz = A.a.syz + i;
+    // ---- images from the forward velocities of the same step: the modified
+    // derivatives d / K + (b psi + a d)
+    auto mod = [&](Row &d, float Ki, float a, float b, const Row &p) {
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) d.v[e] = d[e] * Ki + (b * p[e] + a * d[e]);
+    };
+    auto mod_z = [&](Row &d, int slot, int half) {
+      if (!m.zs) return;
+      const float *cf = g.cz + 3 * half * nz + z;
+      mod(d, cf[CK * nz], cf[CA * nz], cf[CB * nz], ld_psi<VA>(A.ps.z + slot * lz, m.kz, c));
+    };
+    auto mod_x = [&](Row &d, int slot, int half) {
+      if (!m.xs) return;
+      const float *cf = g.cx + 3 * half * nx + x;
+      mod(d, cf[CK * nx], cf[CA * nx], cf[CB * nx], ld_psi<VA>(A.ps.x + slot * lx, m.kx, c));
+    };
+    auto mod_y = [&](Row &d, int slot, int half) {
+      if (!m.yany) return;
+      const Row K = coef_y<VA>(g, c, 3 * half + CK), a = coef_y<VA>(g, c, 3 * half + CA),
+                b = coef_y<VA>(g, c, 3 * half + CB), p = ld_psi_y(A.ps.y + slot * ly, g, m, c);
+#pragma unroll
+      for (int e = 0; e < VEC; ++e)
+        if (m.ys[e]) d.v[e] = d[e] * K[e] + (b[e] * p[e] + a[e] * d[e]);
+    };
+    const float *vz = A.f.vz + i, *vx = A.f.vx + i, *vy = A.f.vy + i;
+    Row gm;
+    {
+      Row ez = diff_m(vz, sz, idz), ex = diff_m(vx, sx, idx), ey = diff_my(vy, c, idy);
+      mod_z(ez, PSI_VA, 0);
+      mod_x(ex, PSI_VA, 0);
+      mod_y(ey, PSI_VA, 0);
+      const Row pz = ld_row(azz), px = ld_row(axx), py = ld_row(ayy);
+      Row gl = ld_row(A.g0 + i);
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) {
+        if (c.act[e]) gl.v[e] += (pz[e] + px[e] + py[e]) * (ez[e] + ex[e] + ey[e]) * dt;
+        gm.v[e] = 2.0f * (pz[e] * ez[e] + px[e] * ex[e] + py[e] * ey[e]);
+      }
+      st_row(A.g0 + i, gl);
+    }
+    auto share = [&](const float *s, const Row &d0, const Row &d1) {
+      const Row p = ld_row(s);
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) gm.v[e] += p[e] * (d0[e] + d1[e]);
+    };
+    {
+      Row d0 = diff_p(vx, sz, idz), d1 = diff_p(vz, sx, idx);
+      mod_z(d0, PSI_VB1, 1);
+      mod_x(d1, PSI_VB1, 1);
+      share(axz, d0, d1);
+    }
+    {
+      Row d0 = diff_py(vx, c, idy), d1 = diff_p(vy, sx, idx);
+      mod_y(d0, PSI_VB2, 1);
+      mod_x(d1, PSI_VB2, 1);
+      share(axy, d0, d1);
+    }
+    {
+      Row d0 = diff_p(vy, sz, idz), d1 = diff_py(vz, c, idy);
+      mod_z(d0, PSI_VB2, 1);
+      mod_y(d1, PSI_VB1, 1);
+      share(ayz, d0, d1);
+    }
+    Row g1 = ld_row(A.g1 + i);
+#pragma unroll
+    for (int e = 0; e < VEC; ++e)
+      if (c.act[e]) g1.v[e] += gm[e] * dt;
+    st_row(A.g1 + i, g1);
   }
   {
     // z: vz <- ez, vx <- xz, vy <- yz; x: vx <- ex, vz <- xz, vy <- xy;
@@ -283,14 +372,8 @@ __global__ void __launch_bounds__(VEC_THREADS, MINB) k_adj_stress_vec(ExactArgs 
     });
   }
   __syncthreads();
-  if (z > nz - 3 || x > nx - 3 || y > g.ny - 3) return;
-  const VecCell c = vec_cell(g, z, x, y);
-  const int i = c.i;
-  const QGather Q{q, g};
-  const Pml<VA> m = pml_of<VA>(g, c, false);
-  const int lz = (int)g.slab_z, lx = (int)g.slab_x, ly = (int)g.slab_y;
-  const float *azz = A.a.szz + i, *axx = A.a.sxx + i, *ayy = A.a.syy + i;
-  const float *axz = A.a.sxz + i, *axy = A.a.sxy + i, *ayz = A.a.syz + i;
+  if (!in) return;
+  const QGather Q{q, g, tz};
   auto finish = [&](float *dst, const Row &d) {
     Row n = ld_row(dst);
 #pragma unroll
@@ -298,108 +381,110 @@ __global__ void __launch_bounds__(VEC_THREADS, MINB) k_adj_stress_vec(ExactArgs 
       if (c.act[e]) n.v[e] += d[e];
     st_row(dst, n);
   };
-  {
-    Row d{};
-    Q.zp(d, 0); Q.xm(d, 1); Q.ym(d, 1);
-    finish(A.a.vz + i, d);
-  }
-  {
-    Row d{};
-    Q.xp(d, 0); Q.zm(d, 1); Q.ym(d, 2);
-    finish(A.a.vx + i, d);
-  }
-  {
-    Row d{};
-    Q.yp(d, 0); Q.xm(d, 2); Q.zm(d, 2);
-    finish(A.a.vy + i, d);
-  }
-  if (!A.g0) return;
-  // ---- images from the forward velocities of the same step: the modified
-  // derivatives d / K + (b psi + a d)
-  auto mod = [&](Row &d, float Ki, float a, float b, const Row &p) {
-#pragma unroll
-    for (int e = 0; e < VEC; ++e) d.v[e] = d[e] * Ki + (b * p[e] + a * d[e]);
-  };
-  auto mod_z = [&](Row &d, int slot, int half) {
-    if (!m.zs) return;
-    const float *cf = g.cz + 3 * half * nz + z;
-    mod(d, cf[CK * nz], cf[CA * nz], cf[CB * nz], ld_psi<VA>(A.ps.z + slot * lz, m.kz, c));
-  };
-  auto mod_x = [&](Row &d, int slot, int half) {
-    if (!m.xs) return;
-    const float *cf = g.cx + 3 * half * nx + x;
-    mod(d, cf[CK * nx], cf[CA * nx], cf[CB * nx], ld_psi<VA>(A.ps.x + slot * lx, m.kx, c));
-  };
-  auto mod_y = [&](Row &d, int slot, int half) {
-    if (!m.yany) return;
-    const Row K = coef_y<VA>(g, c, 3 * half + CK), a = coef_y<VA>(g, c, 3 * half + CA),
-              b = coef_y<VA>(g, c, 3 * half + CB), p = ld_psi_y(A.ps.y + slot * ly, g, m, c);
-#pragma unroll
-    for (int e = 0; e < VEC; ++e)
-      if (m.ys[e]) d.v[e] = d[e] * K[e] + (b[e] * p[e] + a[e] * d[e]);
-  };
-  const float *vz = A.f.vz + i, *vx = A.f.vx + i, *vy = A.f.vy + i;
-  Row gm;
-  {
-    Row ez = diff_m(vz, sz, idz), ex = diff_m(vx, sx, idx), ey = diff_my(vy, c, idy);
-    mod_z(ez, PSI_VA, 0);
-    mod_x(ex, PSI_VA, 0);
-    mod_y(ey, PSI_VA, 0);
-    const Row pz = ld_row(azz), px = ld_row(axx), py = ld_row(ayy);
-    Row gl = ld_row(A.g0 + i);
-#pragma unroll
-    for (int e = 0; e < VEC; ++e) {
-      if (c.act[e]) gl.v[e] += (pz[e] + px[e] + py[e]) * (ez[e] + ex[e] + ey[e]) * dt;
-      gm.v[e] = 2.0f * (pz[e] * ez[e] + px[e] * ex[e] + py[e] * ey[e]);
+  if (part == 0) {
+    {
+      Row d{};
+      Q.zp(d, 0); Q.xm(d, 1); Q.ym(d, 1);
+      finish(A.a.vz + i, d);
     }
-    st_row(A.g0 + i, gl);
+  } else {
+    {
+      Row d{};
+      Q.xp(d, 0); Q.zm(d, 1); Q.ym(d, 2);
+      finish(A.a.vx + i, d);
+    }
+    {
+      Row d{};
+      Q.yp(d, 0); Q.xm(d, 2); Q.zm(d, 2);
+      finish(A.a.vy + i, d);
+    }
   }
-  auto share = [&](const float *s, const Row &d0, const Row &d1) {
-    const Row p = ld_row(s);
-#pragma unroll
-    for (int e = 0; e < VEC; ++e) gm.v[e] += p[e] * (d0[e] + d1[e]);
-  };
-  {
-    Row d0 = diff_p(vx, sz, idz), d1 = diff_p(vz, sx, idx);
-    mod_z(d0, PSI_VB1, 1);
-    mod_x(d1, PSI_VB1, 1);
-    share(axz, d0, d1);
-  }
-  {
-    Row d0 = diff_py(vx, c, idy), d1 = diff_p(vy, sx, idx);
-    mod_y(d0, PSI_VB2, 1);
-    mod_x(d1, PSI_VB2, 1);
-    share(axy, d0, d1);
-  }
-  {
-    Row d0 = diff_p(vy, sz, idz), d1 = diff_py(vz, c, idy);
-    mod_z(d0, PSI_VB2, 1);
-    mod_y(d1, PSI_VB1, 1);
-    share(ayz, d0, d1);
-  }
-  Row g1 = ld_row(A.g1 + i);
-#pragma unroll
-  for (int e = 0; e < VEC; ++e)
-    if (c.act[e]) g1.v[e] += gm[e] * dt;
-  st_row(A.g1 + i, g1);
 }
 
 template <bool VA, int MINB>
-__global__ void __launch_bounds__(VEC_THREADS, MINB) k_adj_velocity_vec(ExactArgs A) {
+__global__ void __launch_bounds__(EX_THREADS, MINB) k_adj_velocity_vec(ExactArgs A) {
   const Geo &g = A.g;
   __shared__ QTile q;
   const int z0 = 2 + blockIdx.z * VEC_TZ, x0 = 2 + blockIdx.y * VEC_TX,
             y0 = VEC * blockIdx.x * VEC_TY;
-  const int z = z0 + threadIdx.z, x = x0 + threadIdx.y, y = y0 + VEC * threadIdx.x;
+  const int tz = threadIdx.z % VEC_TZ, part = threadIdx.z / VEC_TZ;
+  const int z = z0 + tz, x = x0 + threadIdx.y, y = y0 + VEC * threadIdx.x;
   const int nz = g.nz, nx = g.nx;
   const int sz = (int)g.sz, sx = g.sx;
   const float dt = g.dt, idz = g.idz, idx = g.idx, idy = g.idy;
+  if (threadIdx.x + threadIdx.y + threadIdx.z == 0) q.next = 0;
+  __syncthreads();
   vec_begin();
-  if (g.far && z <= nz - 3 && x <= nx - 3) {  // read after the barrier
-    const int i = (z * nx + x) * sx + y;
-    for (const float *p : {A.a.szz, A.a.sxx, A.a.syy, A.a.sxz, A.a.sxy, A.a.syz, A.f.szz, A.f.sxx,
-                           A.f.syy, A.f.sxz, A.f.sxy, A.f.syz}) prefetch_row(p + i);
-    if (A.g0) prefetch_row(A.g0 + i);
+  const bool in = z <= nz - 3 && x <= nx - 3 && y <= g.ny - 3;
+  const VecCell c = vec_cell(g, z, x, y);
+  const int i = c.i;
+  if (g.far && part == 0 && in)  // read after the barrier
+    for (const float *p : {A.a.szz, A.a.sxx, A.a.syy, A.a.sxz, A.a.sxy, A.a.syz}) prefetch_row(p + i);
+  if (part == 1 && in && A.g0) {
+    const Pml<VA> m = pml_of<VA>(g, c, true);
+    const int lz = (int)g.slab_z, lx = (int)g.slab_x, ly = (int)g.slab_y;
+    const float *avz = A.a.vz + i, *avx = A.a.vx + i, *avy = A.a.vy + i;
+    // ---- buoyancy image from the forward stresses of the same step: modified
+    // derivatives d / K + psi (the memory variables are the step's new ones)
+    auto mod_z = [&](Row &d, int slot, int half) {
+      if (!m.zs) return;
+      const float Ki = g.cz[(3 * half + CK) * nz + z];
+      const Row p = ld_psi<VA>(A.ps.z + slot * lz, m.kz, c);
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) d.v[e] = d[e] * Ki + p[e];
+    };
+    auto mod_x = [&](Row &d, int slot, int half) {
+      if (!m.xs) return;
+      const float Ki = g.cx[(3 * half + CK) * nx + x];
+      const Row p = ld_psi<VA>(A.ps.x + slot * lx, m.kx, c);
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) d.v[e] = d[e] * Ki + p[e];
+    };
+    auto mod_y = [&](Row &d, int slot, int half) {
+      if (!m.yany) return;
+      const Row K = coef_y<VA>(g, c, 3 * half + CK), p = ld_psi_y(A.ps.y + slot * ly, g, m, c);
+#pragma unroll
+      for (int e = 0; e < VEC; ++e)
+        if (m.ys[e]) d.v[e] = d[e] * K[e] + p[e];
+    };
+    const float *szz = A.f.szz + i, *sxx = A.f.sxx + i, *syy = A.f.syy + i;
+    const float *sxz = A.f.sxz + i, *sxy = A.f.sxy + i, *syz = A.f.syz + i;
+    Row im;
+    {
+      Row d0 = diff_p(szz, sz, idz), d1 = diff_m(sxz, sx, idx), d2 = diff_my(syz, c, idy);
+      mod_z(d0, PSI_SAA, 1);
+      mod_x(d1, PSI_SAB1, 0);
+      mod_y(d2, PSI_SAB1, 0);
+      const Row v = ld_row(avz);
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) im.v[e] = v[e] * (d0[e] + d1[e] + d2[e]);
+    }
+    {
+      Row d0 = diff_m(sxz, sz, idz), d1 = diff_p(sxx, sx, idx), d2 = diff_my(sxy, c, idy);
+      mod_z(d0, PSI_SAB1, 0);
+      mod_x(d1, PSI_SAA, 1);
+      mod_y(d2, PSI_SAB2, 0);
+      const Row v = ld_row(avx);
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) im.v[e] += v[e] * (d0[e] + d1[e] + d2[e]);
+    }
+    {
+      Row d0 = diff_m(syz, sz, idz), d1, d2 = diff_py(syy, c, idy);
+      const Row s0 = ld_row(sxy), s1 = ld_row(sxy - sx), s2 = ld_row(sxy - 2 * sx);
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) d1.v[e] = dquirk(s2[e], s1[e], s0[e]) * idx;
+      mod_z(d0, PSI_SAB2, 0);
+      mod_x(d1, PSI_SAB2, 0);
+      mod_y(d2, PSI_SAA, 1);
+      const Row v = ld_row(avy);
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) im.v[e] += v[e] * (d0[e] + d1[e] + d2[e]);
+    }
+    Row g0 = ld_row(A.g0 + i);
+#pragma unroll
+    for (int e = 0; e < VEC; ++e)
+      if (c.act[e]) g0.v[e] += im[e] * dt;
+    st_row(A.g0 + i, g0);
   }
   {
     // in the order vz, vx, vy: the stresses szz, sxz, syz (z), sxz, sxx, sxy
@@ -420,13 +505,8 @@ __global__ void __launch_bounds__(VEC_THREADS, MINB) k_adj_velocity_vec(ExactArg
     });
   }
   __syncthreads();
-  if (z > nz - 3 || x > nx - 3 || y > g.ny - 3) return;
-  const VecCell c = vec_cell(g, z, x, y);
-  const int i = c.i;
-  const QGather Q{q, g};
-  const Pml<VA> m = pml_of<VA>(g, c, true);
-  const int lz = (int)g.slab_z, lx = (int)g.slab_x, ly = (int)g.slab_y;
-  const float *avz = A.a.vz + i, *avx = A.a.vx + i, *avy = A.a.vy + i;
+  if (!in) return;
+  const QGather Q{q, g, tz};
   auto finish = [&](float *dst, const Row &d) {
     Row n = ld_row(dst);
 #pragma unroll
@@ -434,115 +514,57 @@ __global__ void __launch_bounds__(VEC_THREADS, MINB) k_adj_velocity_vec(ExactArg
       if (c.act[e]) n.v[e] += d[e];
     st_row(dst, n);
   };
-  {
-    Row d{};
-    Q.zm(d, 0);
-    finish(A.a.szz + i, d);
+  if (part == 0) {
+    {
+      Row d{};
+      Q.zm(d, 0);
+      finish(A.a.szz + i, d);
+    }
+    {
+      Row d{};
+      Q.xm(d, 1);
+      finish(A.a.sxx + i, d);
+    }
+    {
+      Row d{};
+      Q.xp(d, 0); Q.zp(d, 1);
+      finish(A.a.sxz + i, d);
+    }
+  } else {
+    {
+      Row d{};
+      Q.ym(d, 2);
+      finish(A.a.syy + i, d);
+    }
+    {
+      Row d{};
+      Q.yp(d, 0); Q.zp(d, 2);
+      finish(A.a.syz + i, d);
+    }
+    {  // sxy, with the transpose of the quirk-Q1 difference
+      Row d{};
+      Q.yp(d, 1);
+      const Row q0 = Q.x(2, 0), q1 = Q.x(2, 1), q2 = Q.x(2, 2);
+  #pragma unroll
+      for (int e = 0; e < VEC; ++e) d.v[e] += dq_t(q0[e], q1[e], q2[e]) * idx;
+      finish(A.a.sxy + i, d);
+    }
   }
-  {
-    Row d{};
-    Q.xm(d, 1);
-    finish(A.a.sxx + i, d);
-  }
-  {
-    Row d{};
-    Q.ym(d, 2);
-    finish(A.a.syy + i, d);
-  }
-  {
-    Row d{};
-    Q.xp(d, 0); Q.zp(d, 1);
-    finish(A.a.sxz + i, d);
-  }
-  {
-    Row d{};
-    Q.yp(d, 0); Q.zp(d, 2);
-    finish(A.a.syz + i, d);
-  }
-  {  // sxy, with the transpose of the quirk-Q1 difference
-    Row d{};
-    Q.yp(d, 1);
-    const Row q0 = Q.x(2, 0), q1 = Q.x(2, 1), q2 = Q.x(2, 2);
-#pragma unroll
-    for (int e = 0; e < VEC; ++e) d.v[e] += dq_t(q0[e], q1[e], q2[e]) * idx;
-    finish(A.a.sxy + i, d);
-  }
-  if (!A.g0) return;
-  // ---- buoyancy image from the forward stresses of the same step: modified
-  // derivatives d / K + psi (the memory variables are the step's new ones)
-  auto mod_z = [&](Row &d, int slot, int half) {
-    if (!m.zs) return;
-    const float Ki = g.cz[(3 * half + CK) * nz + z];
-    const Row p = ld_psi<VA>(A.ps.z + slot * lz, m.kz, c);
-#pragma unroll
-    for (int e = 0; e < VEC; ++e) d.v[e] = d[e] * Ki + p[e];
-  };
-  auto mod_x = [&](Row &d, int slot, int half) {
-    if (!m.xs) return;
-    const float Ki = g.cx[(3 * half + CK) * nx + x];
-    const Row p = ld_psi<VA>(A.ps.x + slot * lx, m.kx, c);
-#pragma unroll
-    for (int e = 0; e < VEC; ++e) d.v[e] = d[e] * Ki + p[e];
-  };
-  auto mod_y = [&](Row &d, int slot, int half) {
-    if (!m.yany) return;
-    const Row K = coef_y<VA>(g, c, 3 * half + CK), p = ld_psi_y(A.ps.y + slot * ly, g, m, c);
-#pragma unroll
-    for (int e = 0; e < VEC; ++e)
-      if (m.ys[e]) d.v[e] = d[e] * K[e] + p[e];
-  };
-  const float *szz = A.f.szz + i, *sxx = A.f.sxx + i, *syy = A.f.syy + i;
-  const float *sxz = A.f.sxz + i, *sxy = A.f.sxy + i, *syz = A.f.syz + i;
-  Row im;
-  {
-    Row d0 = diff_p(szz, sz, idz), d1 = diff_m(sxz, sx, idx), d2 = diff_my(syz, c, idy);
-    mod_z(d0, PSI_SAA, 1);
-    mod_x(d1, PSI_SAB1, 0);
-    mod_y(d2, PSI_SAB1, 0);
-    const Row v = ld_row(avz);
-#pragma unroll
-    for (int e = 0; e < VEC; ++e) im.v[e] = v[e] * (d0[e] + d1[e] + d2[e]);
-  }
-  {
-    Row d0 = diff_m(sxz, sz, idz), d1 = diff_p(sxx, sx, idx), d2 = diff_my(sxy, c, idy);
-    mod_z(d0, PSI_SAB1, 0);
-    mod_x(d1, PSI_SAA, 1);
-    mod_y(d2, PSI_SAB2, 0);
-    const Row v = ld_row(avx);
-#pragma unroll
-    for (int e = 0; e < VEC; ++e) im.v[e] += v[e] * (d0[e] + d1[e] + d2[e]);
-  }
-  {
-    Row d0 = diff_m(syz, sz, idz), d1, d2 = diff_py(syy, c, idy);
-    const Row s0 = ld_row(sxy), s1 = ld_row(sxy - sx), s2 = ld_row(sxy - 2 * sx);
-#pragma unroll
-    for (int e = 0; e < VEC; ++e) d1.v[e] = dquirk(s2[e], s1[e], s0[e]) * idx;
-    mod_z(d0, PSI_SAB2, 0);
-    mod_x(d1, PSI_SAB2, 0);
-    mod_y(d2, PSI_SAA, 1);
-    const Row v = ld_row(avy);
-#pragma unroll
-    for (int e = 0; e < VEC; ++e) im.v[e] += v[e] * (d0[e] + d1[e] + d2[e]);
-  }
-  Row g0 = ld_row(A.g0 + i);
-#pragma unroll
-  for (int e = 0; e < VEC; ++e)
-    if (c.act[e]) g0.v[e] += im[e] * dt;
-  st_row(A.g0 + i, g0);
 }
 
-// 6 resident CTAs per SM (80 registers, 32 KB of shared memory).  At 120^3 the
-// stress stage takes 104 / 94 / 90 us with 4 / 5 / 6, the velocity stage 107 /
-// 92 / 85; asking for the second phase's rows before the first makes them 87
-// and 80.
+// Resident CTAs per SM (33 KB of shared memory each).  At 120^3 (us, event
+// overhead of 6 in all) the stress stage takes 82 / 72 / 72 and the velocity
+// stage 82 / 72 / 66 with 3 / 4 / 5 CTAs; with one thread per vector for both
+// kinds of work, 6 CTAs of 128 threads, 87 and 80.  The single-cell memory
+// variables need more than the 48 registers of 5 CTAs.
 void launch_adj_stress_vec(cudaStream_t st, const ExactArgs &A) {
-  if (psi_vectors(A.g)) vec_launch(k_adj_stress_vec<true, 6>, vec_grid(A.g), 1, true, st, A);
-  else vec_launch(k_adj_stress_vec<false, 6>, vec_grid(A.g), 1, true, st, A);
+  auto k = psi_vectors(A.g) ? k_adj_stress_vec<true, 4> : k_adj_stress_vec<false, 4>;
+  vec_launch(k, vec_grid(A.g), 2 * VEC_TZ, true, st, A);
 }
 
 void launch_adj_velocity_vec(cudaStream_t st, const ExactArgs &A) {
-  if (psi_vectors(A.g)) vec_launch(k_adj_velocity_vec<true, 6>, vec_grid(A.g), 1, true, st, A);
-  else vec_launch(k_adj_velocity_vec<false, 6>, vec_grid(A.g), 1, true, st, A);
+  auto k = psi_vectors(A.g) ? k_adj_velocity_vec<true, 5> : k_adj_velocity_vec<false, 4>;
+  vec_launch(k, vec_grid(A.g), 2 * VEC_TZ, true, st, A);
 }
 
 }  // namespace efwi

@@ -449,7 +449,7 @@ void launch_stress_fwd_vec(int S, cudaStream_t st, const Geo &g, const Fields &f
            : mode == VEC_STEP_TO ? (va ? k_stress_fwd_vec<true, 1, 6, VEC_STEP_TO> : k_stress_fwd_vec<false, 1, 6, VEC_STEP_TO>)
            : parts > 1 ? (va ? k_stress_fwd_vec<true, 4, 8> : k_stress_fwd_vec<false, 4, 8>)
                        : (va ? k_stress_fwd_vec<true, 1, 6> : k_stress_fwd_vec<false, 1, 6>);
-  vec_launch(k, grid, parts, after_velocity, st, g, f, ps, lam, mu, nzb, src, shell, il, to);
+  vec_launch(k, grid, vec_tz(parts) * parts, after_velocity, st, g, f, ps, lam, mu, nzb, src, shell, il, to);
 }
 
 void launch_velocity_fwd_vec(int S, cudaStream_t st, const Geo &g, const Fields &f, const Psi &ps,
@@ -463,7 +463,7 @@ void launch_velocity_fwd_vec(int S, cudaStream_t st, const Geo &g, const Fields 
            : mode == VEC_STEP_TO ? (va ? k_velocity_fwd_vec<true, 1, 5, VEC_STEP_TO> : k_velocity_fwd_vec<false, 1, 5, VEC_STEP_TO>)
            : parts > 1 ? (va ? k_velocity_fwd_vec<true, 3, 8> : k_velocity_fwd_vec<false, 3, 8>)
                        : (va ? k_velocity_fwd_vec<true, 1, 5> : k_velocity_fwd_vec<false, 1, 5>);
-  vec_launch(k, grid, parts, true, st, g, f, ps, buoy, nzb, rec, il, to);
+  vec_launch(k, grid, vec_tz(parts) * parts, true, st, g, f, ps, buoy, nzb, rec, il, to);
 }
 
 }  // namespace efwi

@@ -557,9 +557,9 @@ void launch_rev_velocity_vec(cudaStream_t st, const Geo &g, const Fields &f, con
                              float *grho, int do_rev, int do_adj, const ShellMap &shell,
                              const RecFuse &inj, bool after_stress) {
   if (psi_vectors(g))
-    vec_launch(k_rev_velocity_vec<true, 6>, vec_grid(g), 1, after_stress, st, g, f, a, ps, lam, mu, buoy, grho, do_rev, do_adj, shell, inj);
+    vec_launch(k_rev_velocity_vec<true, 6>, vec_grid(g), VEC_TZ, after_stress, st, g, f, a, ps, lam, mu, buoy, grho, do_rev, do_adj, shell, inj);
   else
-    vec_launch(k_rev_velocity_vec<false, 6>, vec_grid(g), 1, after_stress, st, g, f, a, ps, lam, mu, buoy, grho, do_rev, do_adj, shell, inj);
+    vec_launch(k_rev_velocity_vec<false, 6>, vec_grid(g), VEC_TZ, after_stress, st, g, f, a, ps, lam, mu, buoy, grho, do_rev, do_adj, shell, inj);
 }
 
 void launch_rev_stress_vec(cudaStream_t st, const Geo &g, const Fields &f, const Fields &a,
@@ -567,9 +567,9 @@ void launch_rev_stress_vec(cudaStream_t st, const Geo &g, const Fields &f, const
                            float *glam, float *gmu, int do_rev, int do_adj, const SrcArgs &src,
                            const ShellMap &shell, bool after_velocity) {
   if (psi_vectors(g))
-    vec_launch(k_rev_stress_vec<true, 5>, vec_grid(g), 1, after_velocity, st, g, f, a, ps, lam, mu, buoy, glam, gmu, do_rev, do_adj, src, shell);
+    vec_launch(k_rev_stress_vec<true, 5>, vec_grid(g), VEC_TZ, after_velocity, st, g, f, a, ps, lam, mu, buoy, glam, gmu, do_rev, do_adj, src, shell);
   else
-    vec_launch(k_rev_stress_vec<false, 5>, vec_grid(g), 1, after_velocity, st, g, f, a, ps, lam, mu, buoy, glam, gmu, do_rev, do_adj, src, shell);
+    vec_launch(k_rev_stress_vec<false, 5>, vec_grid(g), VEC_TZ, after_velocity, st, g, f, a, ps, lam, mu, buoy, glam, gmu, do_rev, do_adj, src, shell);
 }
 
 }  // namespace efwi

@@ -369,14 +369,14 @@ inline bool vec_fits(const Geo &g, int S) {
 // vec_begin().  Such reads are the rows of the fields that the kernel itself
 // updates, the model and the images.
 template <class... P, class... T>
-inline void vec_launch(void (*kernel)(P...), dim3 grid, int parts, bool chained, cudaStream_t st,
+inline void vec_launch(void (*kernel)(P...), dim3 grid, int tz, bool chained, cudaStream_t st,
                        T... args) {
   cudaLaunchAttribute at{};
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at.val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t cf{};
   cf.gridDim = grid;
-  cf.blockDim = dim3(VEC_TY, VEC_TX, vec_tz(parts) * parts);
+  cf.blockDim = dim3(VEC_TY, VEC_TX, tz);
   cf.stream = st;
   cf.attrs = &at;
   cf.numAttrs = chained ? 1 : 0;
