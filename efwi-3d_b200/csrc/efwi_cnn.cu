@@ -699,14 +699,21 @@ k_conv3d_fwd_tc2(const __grid_constant__ CUtensorMap xmap, const __nv_bfloat16 *
 // tile of plane z'-1 is complete: the warps read it, set its columns to zero
 // for plane z'+2 and hand over to the next MMAs before they store.  A plane's
 // sums see the taps in the same order as in the forms above (the same bits).
-// Waits inside a CTA are filled by the other CTAs of the SM (six: 35 KB of
-// shared memory and 64 TMEM columns each).
+// What bounds it now is the tensor cores' reads of shared memory (44 of the
+// SM's cycles per MMA: 25 us of the 39 at 128^3) and, with few tiles in flight,
+// the chain from one plane's MMAs over its drain to the next plane's.  So a CTA
+// has four tiles of four warps each that share the weights and nothing else
+// (a barrier of their own per tile): 70 KB of shared memory, two CTAs or eight
+// tiles per SM, all 512 TMEM columns.  One tile per CTA fits six times: 49 /
+// 118 us at 128^3 / 192^3, 41 at 93 x 117 x 141; two per CTA 40 / 108, 36; four
+// 39 / 106, 33; a third stage changes nothing.
 constexpr int kZmStages = 2;
 constexpr int kZmPlane = kTcSY * kTcSX * 32;                     // a staged plane
 constexpr int kZmStage = (kZmPlane + 255) / 256 * 256;
 constexpr int kZmWTap = 2 * 5 * kC * 16;                         // weights of one (dy, dx)
 constexpr int kZmWBytes = 9 * kZmWTap;
-constexpr int kZmSmem = kZmStages * kZmStage + kZmWBytes + 256;  // + alignment slack
+constexpr int kZmTiles = 4;                                      // tiles of a CTA
+constexpr int kZmSmem = kZmTiles * kZmStages * kZmStage + kZmWBytes + 256;  // + alignment slack
 
 // kind::f16, FP32 accumulator, BF16 K-major operands, N = 48, M = 128.
 constexpr uint32_t kZmIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((48u >> 3) << 17) |
@@ -747,22 +754,47 @@ __device__ __forceinline__ void tc_zero16(uint32_t taddr) {
   asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 
-__global__ void __launch_bounds__(128)
+// Barriers of a tile's four warps; sync_and returns whether `ok` held for all
+// their threads.  The warps leave them converged, as tcgen05.ld and .st need.
+__device__ __forceinline__ void sync_128(int id) {
+  __syncwarp();
+  asm volatile("bar.sync %0, 128;" ::"r"(id) : "memory");
+}
+__device__ __forceinline__ bool sync_and(int id, bool ok) {
+  int r;
+  __syncwarp();
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %1, 0;\n\t"
+      "bar.red.and.pred q, %2, 128, p;\n\tselp.b32 %0, 1, 0, q;\n\t}\n"
+      : "=r"(r)
+      : "r"((int)ok), "r"(id)
+      : "memory");
+  return r != 0;
+}
+
+__global__ void __launch_bounds__(128 * kZmTiles)
 k_conv3d_fwd_zm(const __grid_constant__ CUtensorMap xmap, const __nv_bfloat16 *__restrict__ w,
-                const float *__restrict__ bias, int D, int H, int W, int zlen, int relu,
-                __nv_bfloat16 *__restrict__ yb, float *__restrict__ yf, float *__restrict__ y0c) {
+                const float *__restrict__ bias, int D, int H, int W, int zlen, int units,
+                int relu, __nv_bfloat16 *__restrict__ yb, float *__restrict__ yf,
+                float *__restrict__ y0c) {
   extern __shared__ unsigned char smem_raw[];
-  __shared__ __align__(8) uint64_t full[kZmStages], done;
+  __shared__ __align__(8) uint64_t s_full[kZmTiles][kZmStages], s_done[kZmTiles];
   __shared__ uint32_t tmem_slot;
-  __shared__ int s_abort;
+  __shared__ int s_abort_of[kZmTiles];
   unsigned char *smem = smem_raw + ((256u - (smem_u32(smem_raw) & 255u)) & 255u);
-  unsigned char *swt = smem + kZmStages * kZmStage;  // [dy][dx][half][5 dz blocks][co] x 16 B
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  // weights [dy][dx][half][5 dz blocks][co] x 16 B
+  unsigned char *swt = smem + kZmTiles * kZmStages * kZmStage;
+  const int tile = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 7), 0);
+  const int tid = threadIdx.x & 127, warp = tid >> 5, lane = tid & 31;
+  smem += tile * kZmStages * kZmStage;
+  uint64_t *full = s_full[tile], &done = s_done[tile];
+  int &s_abort = s_abort_of[tile];
+  const int unit = (int)blockIdx.x * kZmTiles + tile;
   const int ntx = (W + kTcX - 1) / kTcX, nty = (H + kTcY - 1) / kTcY;
-  const int x0 = (int)(blockIdx.x % ntx) * kTcX;
-  const int rest = (int)(blockIdx.x / ntx);
+  const int x0 = unit % ntx * kTcX;
+  const int rest = unit / ntx;
   const int y0 = rest % nty * kTcY, zb = rest / nty * zlen, ze = min(zb + zlen, D);
-  const int nj = ze - zb + 2;  // input planes zb-1 .. ze
+  const int nj = unit < units ? ze - zb + 2 : 0;  // input planes zb-1 .. ze
   auto issue = [&](int j) {    // thread 0: input plane zb-1+j into stage j % kZmStages
     const int s = j % kZmStages;
     mbar_arrive_expect_tx(&full[s], kZmPlane);
@@ -776,15 +808,16 @@ k_conv3d_fwd_zm(const __grid_constant__ CUtensorMap xmap, const __nv_bfloat16 *_
     s_abort = 0;
     for (; n_tma < kZmStages && n_tma < nj; ++n_tma) issue(n_tma);
   }
-  for (int k = tid; k < 9 * 2 * 5 * kC; k += blockDim.x) {
+  for (int k = threadIdx.x; k < 9 * 2 * 5 * kC; k += blockDim.x) {
     const int co = k % kC, b = k / kC % 5, h = k / (kC * 5) % 2, t = k / (kC * 10);
     const int dz = (5 - b) % 3;  // blocks in the order 2 1 0 2 1
     *reinterpret_cast<uint4 *>(swt + k * 16) =
         *reinterpret_cast<const uint4 *>(w + ((dz * 9 + t) * kC + co) * kC + h * 8);
   }
-  if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 64;" ::"r"(
-                     smem_u32(&tmem_slot))
+  if (threadIdx.x < 32) {  // one allocation: the permit is the CTA's
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                     smem_u32(&tmem_slot)),
+                 "n"(64 * kZmTiles)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
@@ -792,7 +825,8 @@ k_conv3d_fwd_zm(const __grid_constant__ CUtensorMap xmap, const __nv_bfloat16 *_
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem = tmem_slot, tlane = tmem + ((uint32_t)(warp * 32) << 16);
+  const uint32_t tmem = tmem_slot + (uint32_t)(64 * tile),
+                 tlane = tmem + ((uint32_t)(warp * 32) << 16);
   const uint32_t swa = smem_u32(swt);
   for (int s = 0; s < 3; ++s) tc_zero16(tlane + (uint32_t)(s * kC));
   float bv[16];
@@ -820,11 +854,11 @@ k_conv3d_fwd_zm(const __grid_constant__ CUtensorMap xmap, const __nv_bfloat16 *_
     tc_commit(&done);
     n_mma = j + 1;
   };
-  if (tid == 0) mma(0);
+  if (tid == 0 && nj > 0) mma(0);
   bool ok = true;
   for (int j = 0; j < nj; ++j) {
     // every thread takes the same branch: tcgen05.ld is warp-collective
-    ok = __syncthreads_and(!s_abort && mbar_wait_bounded(&done, (uint32_t)(j & 1)));
+    ok = sync_and(tile + 1, !s_abort && mbar_wait_bounded(&done, (uint32_t)(j & 1)));
     if (!ok) break;
     if (tid == 0 && n_tma < nj) { issue(n_tma); ++n_tma; }  // into plane j's stage
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -835,7 +869,7 @@ k_conv3d_fwd_zm(const __grid_constant__ CUtensorMap xmap, const __nv_bfloat16 *_
     if (j + 1 < nj) {
       tc_zero16(col);
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      __syncthreads();
+      sync_128(tile + 1);
       if (tid == 0) mma(j + 1);
     }
     if (p >= zb && inside) {
@@ -876,8 +910,10 @@ k_conv3d_fwd_zm(const __grid_constant__ CUtensorMap xmap, const __nv_bfloat16 *_
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (warp == 0)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 64;" ::"r"(tmem) : "memory");
+  if (threadIdx.x < 32)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_slot),
+                 "n"(64 * kZmTiles)
+                 : "memory");
 }
 
 
@@ -1376,10 +1412,10 @@ int zm_launch(const CUtensorMap &map, const void *w, const float *bias, int D, i
               int relu, void *y_bf16, float *y_f32, float *y0c, cudaStream_t st) {
   int sms = 0;
   if (!conv_sms(&sms)) return 2;
-  // planes per CTA: the fewest steps (waves of 6 CTAs per SM times the planes
-  // that a CTA reads)
+  // planes per tile: the fewest steps (waves of 8 tiles per SM times the planes
+  // that a tile reads)
   const long long cols = (long long)((W + kTcX - 1) / kTcX) * ((H + kTcY - 1) / kTcY);
-  const long long slots = 6LL * sms;
+  const long long slots = 8LL * sms;
   long long best = -1;
   int zlen = D;
   for (int n = 1; n <= D; ++n) {
@@ -1389,11 +1425,11 @@ int zm_launch(const CUtensorMap &map, const void *w, const float *bias, int D, i
     if (best < 0 || steps < best) { best = steps; zlen = len; }
     if (ctas > 8 * slots) break;
   }
-  const long long ctas = cols * ((D + zlen - 1) / zlen);
-  if (ctas > 0x7fffffffLL) return 1;
+  const long long units = cols * ((D + zlen - 1) / zlen), ctas = (units + kZmTiles - 1) / kZmTiles;
+  if (units > 0x7fffffffLL - kZmTiles) return 1;
   set_smem_once(k_conv3d_fwd_zm, kZmSmem, g_tc2_smem_set);
-  k_conv3d_fwd_zm<<<(unsigned)ctas, 128, kZmSmem, st>>>(map, (const __nv_bfloat16 *)w, bias, D, H,
-                                                        W, zlen, relu, (__nv_bfloat16 *)y_bf16,
+  k_conv3d_fwd_zm<<<(unsigned)ctas, 128 * kZmTiles, kZmSmem, st>>>(map, (const __nv_bfloat16 *)w, bias, D, H,
+                                                        W, zlen, (int)units, relu, (__nv_bfloat16 *)y_bf16,
                                                         y_f32, y0c);
   return 0;
 }

@@ -58,7 +58,8 @@ def test_backward_keeps_infinities_and_nans():
     assert torch.equal(db[:3], ref[:3])
 
 
-@pytest.mark.parametrize("shape", [(1, 1, 1), (2, 17, 9), (40, 15, 8), (70, 33, 7), (1, 300, 200)])
+@pytest.mark.parametrize("shape", [(1, 1, 1), (2, 17, 9), (40, 15, 8), (70, 33, 7), (1, 300, 200),
+                                   (20, 300, 297)])
 def test_z_march_matches_single_tap_form(shape):
     from efwi.cnn import conv3d_raw, conv3d_status, set_conv_kernel
     g = torch.Generator(device="cuda").manual_seed(sum(shape))
