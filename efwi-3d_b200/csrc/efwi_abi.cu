@@ -492,6 +492,21 @@ Psi psi_at(float *base, const Geo &g, int S) {
   return p;
 }
 
+// Row pitch of a grid's volumes: a multiple of 4 cells, so that the kernels'
+// 16-byte vectors are aligned; whole 128-byte lines where they add at most a
+// sixth to the volumes: a CTA reads 128 bytes of a row, one line instead of
+// parts of two.  Misfit and gradient at 84^3 (84 -> 96) 12.7 -> 11.8 and 43.1
+// -> 41.4 ms, exact gradient at 120^3 (128) 48.6 -> 47.4.  Beyond a sixth the
+// larger volumes cost as much in L2 (illumination at 80^3, 80 -> 96: 11.65 ->
+// 12.3), the latency-bound small grids lose 1-4 % (26 x 30 x 28), and grids
+// beyond 2^26 cells (5 GB a state) are left the memory.
+int y_pitch(int nz, int nx, int ny) {
+  const int vec = (ny + 3) & ~3, line = (ny + 31) & ~31;
+  const bool pays = (long long)nz * nx * ny >= (1LL << 18) &&
+                    (long long)nz * nx * line <= (1LL << 26) && 6LL * line <= 7LL * ny;
+  return pays ? line : vec;
+}
+
 // Receivers of a batch, grouped by (shot, cell).
 struct RecHost {
   std::vector<long long> ucell, trace_off;
@@ -778,13 +793,19 @@ int misfit_shot(EfwiHandle *h, const ShotHost &sh, const float *obs, const float
   return check_launch(h, "misfit");
 }
 
-// Floats of one checkpoint: 9 fields and the memory variables of one shot.
-long long state_floats(const EfwiHandle *h) { return 9 * h->N + psi_per_shot(h->geo); }
+// Floats of one checkpoint, 9 fields and the memory variables of one shot: as
+// stored, and as the budget and efwi_state_bytes count them, without the rows'
+// padding to whole lines (at most a sixth).
+long long stored_floats(const EfwiHandle *h) { return 9 * h->N + psi_per_shot(h->geo); }
+long long state_floats(const EfwiHandle *h) {
+  const EfwiGrid &g = h->grid;
+  return 9LL * g.nz * g.nx * ((g.ny + 3) & ~3) + psi_per_shot(h->geo);
+}
 
-// Checkpoint slots the budget allows for a run of `blocks` states
-// (S_0 is the zero state and needs none).
-int checkpoint_slots(const EfwiHandle *h, int blocks) {
-  const long long per = state_floats(h) * (long long)sizeof(float);
+// Checkpoint slots of `floats` each that the budget allows for a run of
+// `blocks` states (S_0 is the zero state and needs none).
+int checkpoint_slots(const EfwiHandle *h, int blocks, long long floats) {
+  const long long per = floats * (long long)sizeof(float);
   long long s = per > 0 ? h->ck_budget / per : 0;
   if (s > blocks - 1) s = blocks - 1;
   return (int)std::max(s, 0LL);
@@ -834,15 +855,22 @@ int exact_shot(EfwiHandle *h, int id, const float *obs, double *jdev, float *res
   CK_CUDA(h, h->adj.ensure(sizeof(float) * 9 * N));
   CK_CUDA(h, h->apsi.ensure(sizeof(float) * 2 * P));
 
-  const int slots = checkpoint_slots(h, ntl);
+  const long long SF = stored_floats(h);
   CkPlan plan;
-  plan.build(ntl, slots, 64LL * ntl + 4096);
-  if (plan.too_long || plan.forward_steps > 16LL * ntl)
-    return fail(h, EFWI_ERR_TOO_LARGE,
-                "checkpoint budget of %lld bytes (%d slots of %lld bytes) is too small for %d steps",
-                h->ck_budget, slots, state_floats(h) * 4, ntl);
-  const long long SF = state_floats(h);
-  CK_CUDA(h, h->ckpt.ensure(sizeof(float) * std::max(1LL, (long long)plan.slots_used * SF)));
+  cudaError_t room = cudaSuccess;
+  for (const long long floats : {state_floats(h), SF}) {
+    const int slots = checkpoint_slots(h, ntl, floats);
+    plan.build(ntl, slots, 64LL * ntl + 4096);
+    if (plan.too_long || plan.forward_steps > 16LL * ntl)
+      return fail(h, EFWI_ERR_TOO_LARGE,
+                  "checkpoint budget of %lld bytes (%d slots of %lld bytes) is too small for %d steps",
+                  h->ck_budget, slots, floats * 4, ntl);
+    room = h->ckpt.ensure(sizeof(float) * std::max(1LL, (long long)plan.slots_used * SF));
+    // no room for the padding as well: the slots that fit the budget with it
+    if (room != cudaErrorMemoryAllocation || floats == SF) break;
+    cudaGetLastError();
+  }
+  CK_CUDA(h, room);
   h->ck_forward_steps = plan.forward_steps;
   h->ck_slots = plan.slots_used;
 
@@ -1121,7 +1149,7 @@ int efwi_create(const EfwiGrid *g, EfwiHandle **out) {
     return rc;
   }
   h->grid = *g;
-  h->py = (g->ny + 3) & ~3;
+  h->py = y_pitch(g->nz, g->nx, g->ny);
   h->N = (long long)g->nz * g->nx * h->py;
   if (h->N >= (1LL << 31)) {
     *out = h;
@@ -1765,7 +1793,7 @@ int efwi_forward_windows(EfwiHandle *h, int n, const int *ids, const EfwiWindow 
     if (lx < 2 || lx > w.nx - 3 || ly < 2 || ly > w.ny - 3)
       return fail(h, EFWI_ERR_ARG, "shot %d: source outside the updated part of its window", ids[k]);
     Domain &d = dom[k];
-    const int pyw = (w.ny + 3) & ~3;
+    const int pyw = y_pitch(h->grid.nz, w.nx, w.ny);
     Geo &g = d.g;
     g = h->geo;
     g.nx = w.nx; g.ny = w.ny;

@@ -3,8 +3,8 @@
 // Layout (HBM): every volume is [nz][nx][py] float32, y fastest -- the
 // torch-native C order of the caller's tensors (the reference transposes to
 // z-fastest on the host, libCUFD.cu:72-80), with the y pitch py = ny rounded
-// up to a multiple of 4 so that every row starts on a 16-byte boundary (the
-// alignment of bulk tensor copies).  Shots of one batch are stacked with
+// up to a multiple of 4, so that every row starts on a 16-byte boundary, or of
+// 32, a 128-byte line (y_pitch in efwi_abi.cu).  Shots of one batch are stacked with
 // stride N = nz*nx*py.
 //
 // C-PML memory variables live only in their slabs (the reference keeps 18

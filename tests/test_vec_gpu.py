@@ -3,8 +3,9 @@ L1 kernels (variant 0): the same bits, at the edges of their vectors, tiles
 and slabs.  ny runs over every remainder by the vector length; C-PML widths
 and ny that are not multiples of it take the single-cell memory variables,
 the others the vector ones; nx and nz run over the remainders of the 4 x 4
-row and plane tile; the smallest grid has one updated cell.  On all but the last two grids the
-forward kernels split their outputs over warps."""
+row and plane tile; the smallest grid has one updated cell.  On all but the last four grids the
+forward kernels split their outputs over warps; the last two have rows of
+whole lines."""
 import numpy as np
 import pytest
 import torch
@@ -38,7 +39,7 @@ def _problem(nz, nx, ny, npml, nt=40):
 
 SIZES = [(5, 5, 5, 2), (14, 13, 12, 4), (15, 14, 33, 4), (16, 17, 34, 5), (17, 18, 35, 6),
          (18, 19, 36, 8), (23, 22, 40, 4), (22, 23, 64, 8), (13, 24, 69, 6),
-         (61, 70, 66, 7), (62, 71, 68, 8)]
+         (61, 70, 66, 7), (62, 71, 68, 8), (56, 57, 90, 5), (46, 61, 124, 8)]
 
 
 def _run(g, shots, stf, model, obs, variant, graphs):
