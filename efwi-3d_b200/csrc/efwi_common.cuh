@@ -81,10 +81,21 @@ __device__ __forceinline__ float dquirk(float m2, float m1, float p0) {
 }
 
 // Arithmetic of the reverse sweep, rounded as written (the compiler would
-// fuse the products of a sum differently from kernel to kernel): both kernel
-// families use these, so their images are the same bits.
+// fuse the products of a sum differently from kernel to kernel).  Both kernel
+// families use these, so their images are the same bits, and the choice of the
+// product that a sum leaves unrounded is the one that these images have always
+// had: a long reverse sweep through the absorbing layers amplifies roundings
+// up to 1e3 times, so that another choice moves an image by up to 2e-4.
 __device__ __forceinline__ float sum3(float a, float b, float c) {
   return __fadd_rn(__fadd_rn(a, b), c);
+}
+// a / ha + b / hb + c / hc of three differences (ia: 1 / ha)
+__device__ __forceinline__ float sum3d(float a, float ia, float b, float ib, float c, float ic) {
+  return __fmaf_rn(c, ic, __fmaf_rn(a, ia, __fmul_rn(b, ib)));
+}
+// a / ha + b / hb of two differences
+__device__ __forceinline__ float sum2d(float a, float ia, float b, float ib) {
+  return __fmaf_rn(a, ia, __fmul_rn(b, ib));
 }
 // v - d b dt
 __device__ __forceinline__ float undo(float v, float d, float b, float dt) {
@@ -98,9 +109,16 @@ __device__ __forceinline__ float add4(float s, float a, float d, float K, float 
 __device__ __forceinline__ float add3(float s, float a, float b, float dt) {
   return __fmaf_rn(__fmul_rn(a, b), dt, s);
 }
+// (v1 d1 + v2 d2 + v3 d3) dt n
+__device__ __forceinline__ float img3(float v1, float d1, float v2, float d2, float v3, float d3,
+                                      float dt, float n) {
+  const float p1 = __fmul_rn(__fmul_rn(v1, d1), dt), p2 = __fmul_rn(__fmul_rn(v2, d2), dt),
+              p3 = __fmul_rn(__fmul_rn(v3, d3), dt);
+  return __fmaf_rn(p3, n, __fmaf_rn(p1, n, __fmul_rn(p2, n)));
+}
 // c1 e1 + c2 e2 + c3 e3
 __device__ __forceinline__ float dot3(float c1, float e1, float c2, float e2, float c3, float e3) {
-  return __fmaf_rn(c3, e3, __fmaf_rn(c2, e2, __fmul_rn(c1, e1)));
+  return __fmaf_rn(c3, e3, __fmaf_rn(c1, e1, __fmul_rn(c2, e2)));
 }
 
 __device__ __forceinline__ bool slab_s(int i, int n, int np) { return i < np || i > n - np - 1; }

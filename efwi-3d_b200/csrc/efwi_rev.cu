@@ -102,21 +102,20 @@ k_rev_velocity(Geo g, Fields f, Fields a, Psi ps, const float *__restrict__ lam,
     const float b = buoy[i];
     const float avz0 = a.vz[i], avx0 = a.vx[i], avy0 = a.vy[i];
     if (do_rev && xin && yin && z >= np && z <= nz - 1 - np) {
-      const float dz_ = sum3(__fmul_rn(dplus(szz[i - sz], szz[i], szz[i + sz], szz[i + 2 * sz]), idz),
-                             __fmul_rn(dminus(sxz[i - 2 * sx], sxz[i - sx], sxz[i], sxz[i + sx]), idx),
-                             __fmul_rn(dminus(syz[i - 2], syz[i - 1], syz[i], syz[i + 1]), idy));
-      const float dx_ = sum3(__fmul_rn(dminus(sxz[i - 2 * sz], sxz[i - sz], sxz[i], sxz[i + sz]), idz),
-                             __fmul_rn(dplus(sxx[i - sx], sxx[i], sxx[i + sx], sxx[i + 2 * sx]), idx),
-                             __fmul_rn(dminus(sxy[i - 2], sxy[i - 1], sxy[i], sxy[i + 1]), idy));
-      const float dy_ = sum3(__fmul_rn(dminus(syz[i - 2 * sz], syz[i - sz], syz[i], syz[i + sz]), idz),
-                             __fmul_rn(dquirk(sxy[i - 2 * sx], sxy[i - sx], sxy[i]), idx),
-                             __fmul_rn(dplus(syy[i - 1], syy[i], syy[i + 1], syy[i + 2]), idy));
+      const float dz_ = sum3d(dplus(szz[i - sz], szz[i], szz[i + sz], szz[i + 2 * sz]), idz,
+                             dminus(sxz[i - 2 * sx], sxz[i - sx], sxz[i], sxz[i + sx]), idx,
+                             dminus(syz[i - 2], syz[i - 1], syz[i], syz[i + 1]), idy);
+      const float dx_ = sum3d(dminus(sxz[i - 2 * sz], sxz[i - sz], sxz[i], sxz[i + sz]), idz,
+                             dplus(sxx[i - sx], sxx[i], sxx[i + sx], sxx[i + 2 * sx]), idx,
+                             dminus(sxy[i - 2], sxy[i - 1], sxy[i], sxy[i + 1]), idy);
+      const float dy_ = sum3d(dminus(syz[i - 2 * sz], syz[i - sz], syz[i], syz[i + sz]), idz,
+                             dquirk(sxy[i - 2 * sx], sxy[i - sx], sxy[i]), idx,
+                             dplus(syy[i - 1], syy[i], syy[i + 1], syy[i + 2]), idy);
       f.vz[i] = undo(f.vz[i], dz_, b, dt);
       f.vx[i] = undo(f.vx[i], dx_, b, dt);
       f.vy[i] = undo(f.vy[i], dy_, b, dt);
       const float nb2 = -(b * b);
-      grho[i] = __fadd_rn(grho[i], -add4(add4(add4(0.f, avz0, dz_, dt, nb2), avx0, dx_, dt, nb2),
-                                         avy0, dy_, dt, nb2));
+      grho[i] = __fadd_rn(grho[i], -img3(avz0, dz_, avx0, dx_, avy0, dy_, dt, nb2));
     }
     if (!do_adj) continue;
     const bool zs = slab_s(z, nz, np);
@@ -140,9 +139,9 @@ k_rev_velocity(Geo g, Fields f, Fields a, Psi ps, const float *__restrict__ lam,
       if (ys) acc = __fmaf_rn(cy.ah, __fmul_rn(nym(g, psy + PSI_VB2 * g.slab_y, z, x, y), idy), acc);
       const float v = __fadd_rn(avx0, acc);
       a.vx[i] = v;
-      if (xs) { const long long k = PSI_SAA * g.slab_x + psi_x_idx(g, z, x, y); px[k] = __fmaf_rn(cx.bh, px[k], __fmul_rn(__fmul_rn(b, v), dt)); }
-      if (zs) { const long long k = PSI_SAB1 * g.slab_z + psi_z_idx(g, z, x, y); pz[k] = __fmaf_rn(cz.b, pz[k], __fmul_rn(__fmul_rn(b, v), dt)); }
-      if (ys) { const long long k = PSI_SAB2 * g.slab_y + psi_y_idx(g, z, x, y); py[k] = __fmaf_rn(cy.b, py[k], __fmul_rn(__fmul_rn(b, v), dt)); }
+      if (xs) { const long long k = PSI_SAA * g.slab_x + psi_x_idx(g, z, x, y); px[k] = add3(__fmul_rn(cx.bh, px[k]), b, v, dt); }
+      if (zs) { const long long k = PSI_SAB1 * g.slab_z + psi_z_idx(g, z, x, y); pz[k] = add3(__fmul_rn(cz.b, pz[k]), b, v, dt); }
+      if (ys) { const long long k = PSI_SAB2 * g.slab_y + psi_y_idx(g, z, x, y); py[k] = add3(__fmul_rn(cy.b, py[k]), b, v, dt); }
     }
     // ---- adjoint vz
     {
@@ -163,8 +162,8 @@ k_rev_velocity(Geo g, Fields f, Fields a, Psi ps, const float *__restrict__ lam,
       const float v = __fadd_rn(avz0, acc);
       a.vz[i] = v;
       if (xs) { const long long k = PSI_SAB1 * g.slab_x + psi_x_idx(g, z, x, y); px[k] = __fmaf_rn(cx.b, px[k], __fmul_rn(__fmul_rn(b, v), dt)); }
-      if (zs) { const long long k = PSI_SAA * g.slab_z + psi_z_idx(g, z, x, y); pz[k] = __fmaf_rn(cz.bh, pz[k], __fmul_rn(__fmul_rn(b, v), dt)); }
-      if (ys) { const long long k = PSI_SAB1 * g.slab_y + psi_y_idx(g, z, x, y); py[k] = __fmaf_rn(cy.b, py[k], __fmul_rn(__fmul_rn(b, v), dt)); }
+      if (zs) { const long long k = PSI_SAA * g.slab_z + psi_z_idx(g, z, x, y); pz[k] = add3(__fmul_rn(cz.bh, pz[k]), b, v, dt); }
+      if (ys) { const long long k = PSI_SAB1 * g.slab_y + psi_y_idx(g, z, x, y); py[k] = add3(__fmul_rn(cy.b, py[k]), b, v, dt); }
     }
     // ---- adjoint vy
     {
@@ -174,8 +173,8 @@ k_rev_velocity(Geo g, Fields f, Fields a, Psi ps, const float *__restrict__ lam,
       const float dsxy_dx = __fmul_rn(-dminus(asxy[i - 2 * sx], asxy[i - sx], asxy[i], asxy[i + sx]), idx);
       const float dsyz_dz = __fmul_rn(-dminus(asyz[i - 2 * sz], asyz[i - sz], asyz[i], asyz[i + sz]), idz);
       float acc = 0.f;
-      acc = add4(acc, l2u, dsyy_dy, cy.K, dt);
       acc = add4(acc, l, dsxx_dy, cy.K, dt);
+      acc = add4(acc, l2u, dsyy_dy, cy.K, dt);
       acc = add4(acc, l, dszz_dy, cy.K, dt);
       acc = add4(acc, u, cx.Kh, dsxy_dx, dt);
       acc = add4(acc, u, cz.Kh, dsyz_dz, dt);
@@ -184,9 +183,9 @@ k_rev_velocity(Geo g, Fields f, Fields a, Psi ps, const float *__restrict__ lam,
       if (zs) acc = __fmaf_rn(cz.ah, __fmul_rn(nzm(g, psz + PSI_VB2 * g.slab_z, z, x, y), idz), acc);
       const float v = __fadd_rn(avy0, acc);
       a.vy[i] = v;
-      if (xs) { const long long k = PSI_SAB2 * g.slab_x + psi_x_idx(g, z, x, y); px[k] = __fmaf_rn(cx.b, px[k], __fmul_rn(__fmul_rn(b, v), dt)); }
-      if (zs) { const long long k = PSI_SAB2 * g.slab_z + psi_z_idx(g, z, x, y); pz[k] = __fmaf_rn(cz.bh, pz[k], __fmul_rn(__fmul_rn(b, v), dt)); }
-      if (ys) { const long long k = PSI_SAA * g.slab_y + psi_y_idx(g, z, x, y); py[k] = __fmaf_rn(cy.b, py[k], __fmul_rn(__fmul_rn(b, v), dt)); }
+      if (xs) { const long long k = PSI_SAB2 * g.slab_x + psi_x_idx(g, z, x, y); px[k] = add3(__fmul_rn(cx.b, px[k]), b, v, dt); }
+      if (zs) { const long long k = PSI_SAB2 * g.slab_z + psi_z_idx(g, z, x, y); pz[k] = add3(__fmul_rn(cz.bh, pz[k]), b, v, dt); }
+      if (ys) { const long long k = PSI_SAA * g.slab_y + psi_y_idx(g, z, x, y); py[k] = add3(__fmul_rn(cy.b, py[k]), b, v, dt); }
     }
   }
 }
@@ -242,20 +241,20 @@ k_rev_stress(Geo g, Fields f, Fields a, Psi ps, const float *__restrict__ lam,
         szz = __fmaf_rn(-dot3(l2u, ezz, l, exx, l, eyy), dt, szz);
         sxx = __fmaf_rn(-dot3(l, ezz, l2u, exx, l, eyy), dt, sxx);
         syy = __fmaf_rn(-dot3(l, ezz, l, exx, l2u, eyy), dt, syy);
-        const float dvx_dz = __fmul_rn(dplus(vx[i - sz], vx[i], vx[i + sz], vx[i + 2 * sz]), idz);
-        const float dvx_dy = __fmul_rn(dplus(vx[i - 1], vx[i], vx[i + 1], vx[i + 2]), idy);
-        const float dvz_dx = __fmul_rn(dplus(vz[i - sx], vz[i], vz[i + sx], vz[i + 2 * sx]), idx);
-        const float dvz_dy = __fmul_rn(dplus(vz[i - 1], vz[i], vz[i + 1], vz[i + 2]), idy);
-        const float dvy_dx = __fmul_rn(dplus(vy[i - sx], vy[i], vy[i + sx], vy[i + 2 * sx]), idx);
-        const float dvy_dz = __fmul_rn(dplus(vy[i - sz], vy[i], vy[i + sz], vy[i + 2 * sz]), idz);
-        f.sxz[i] = undo(f.sxz[i], __fadd_rn(dvx_dz, dvz_dx), u, dt);
-        f.sxy[i] = undo(f.sxy[i], __fadd_rn(dvx_dy, dvy_dx), u, dt);
-        f.syz[i] = undo(f.syz[i], __fadd_rn(dvy_dz, dvz_dy), u, dt);
+        const float exz = sum2d(dplus(vx[i - sz], vx[i], vx[i + sz], vx[i + 2 * sz]), idz,
+                                dplus(vz[i - sx], vz[i], vz[i + sx], vz[i + 2 * sx]), idx);
+        const float exy = sum2d(dplus(vx[i - 1], vx[i], vx[i + 1], vx[i + 2]), idy,
+                                dplus(vy[i - sx], vy[i], vy[i + sx], vy[i + 2 * sx]), idx);
+        const float eyz = sum2d(dplus(vy[i - sz], vy[i], vy[i + sz], vy[i + 2 * sz]), idz,
+                                dplus(vz[i - 1], vz[i], vz[i + 1], vz[i + 2]), idy);
+        f.sxz[i] = undo(f.sxz[i], exz, u, dt);
+        f.sxy[i] = undo(f.sxy[i], exy, u, dt);
+        f.syz[i] = undo(f.syz[i], eyz, u, dt);
         glam[i] = undo(glam[i], sum3(azz0, axx0, ayy0), sum3(ezz, exx, eyy), dt);
         float gm = dot3(2.0f * azz0, ezz, 2.0f * axx0, exx, 2.0f * ayy0, eyy);
-        gm = __fmaf_rn(axz0, __fadd_rn(dvx_dz, dvz_dx), gm);
-        gm = __fmaf_rn(ayz0, __fadd_rn(dvy_dz, dvz_dy), gm);
-        gm = __fmaf_rn(axy0, __fadd_rn(dvx_dy, dvy_dx), gm);
+        gm = __fmaf_rn(axz0, exz, gm);
+        gm = __fmaf_rn(ayz0, eyz, gm);
+        gm = __fmaf_rn(axy0, exy, gm);
         gmu[i] = __fmaf_rn(-gm, dt, gmu[i]);
       }
       f.szz[i] = szz; f.sxx[i] = sxx; f.syy[i] = syy;
@@ -275,22 +274,22 @@ k_rev_stress(Geo g, Fields f, Fields a, Psi ps, const float *__restrict__ lam,
       if (zs) acc = __fmaf_rn(cz.a, __fmul_rn(nzp(g, psz + PSI_SAB1 * g.slab_z, z, x, y), idz), acc);
       const float s = __fadd_rn(axz0, acc);
       a.sxz[i] = s;
-      if (xs) { const long long k = PSI_VB1 * g.slab_x + psi_x_idx(g, z, x, y); px[k] = __fmaf_rn(cx.bh, px[k], __fmul_rn(__fmul_rn(s, u), dt)); }
-      if (zs) { const long long k = PSI_VB1 * g.slab_z + psi_z_idx(g, z, x, y); pz[k] = __fmaf_rn(cz.bh, pz[k], __fmul_rn(__fmul_rn(s, u), dt)); }
+      if (xs) { const long long k = PSI_VB1 * g.slab_x + psi_x_idx(g, z, x, y); px[k] = add3(__fmul_rn(cx.bh, px[k]), s, u, dt); }
+      if (zs) { const long long k = PSI_VB1 * g.slab_z + psi_z_idx(g, z, x, y); pz[k] = add3(__fmul_rn(cz.bh, pz[k]), s, u, dt); }
     }
     // ---- sxy
     {
       const float dvy_dx = __fmul_rn(-dplus(avy[i - sx], avy[i], avy[i + sx], avy[i + 2 * sx]), idx);
       const float dvx_dy = __fmul_rn(-dplus(avx[i - 1], avx[i], avx[i + 1], avx[i + 2]), idy);
       float acc = 0.f;
-      acc = add4(acc, dvy_dx, cx.K, b, dt);
       acc = add4(acc, dvx_dy, cy.K, b, dt);
+      acc = add4(acc, dvy_dx, cx.K, b, dt);
       if (xs) acc = __fmaf_rn(cx.a, __fmul_rn(nxp(g, psx + PSI_SAB2 * g.slab_x, z, x, y), idx), acc);
       if (ys) acc = __fmaf_rn(cy.a, __fmul_rn(nyp(g, psy + PSI_SAB2 * g.slab_y, z, x, y), idy), acc);
       const float s = __fadd_rn(axy0, acc);
       a.sxy[i] = s;
-      if (ys) { const long long k = PSI_VB2 * g.slab_y + psi_y_idx(g, z, x, y); py[k] = __fmaf_rn(cy.bh, py[k], __fmul_rn(__fmul_rn(s, u), dt)); }
-      if (xs) { const long long k = PSI_VB2 * g.slab_x + psi_x_idx(g, z, x, y); px[k] = __fmaf_rn(cx.bh, px[k], __fmul_rn(__fmul_rn(s, u), dt)); }
+      if (ys) { const long long k = PSI_VB2 * g.slab_y + psi_y_idx(g, z, x, y); py[k] = add3(__fmul_rn(cy.bh, py[k]), s, u, dt); }
+      if (xs) { const long long k = PSI_VB2 * g.slab_x + psi_x_idx(g, z, x, y); px[k] = add3(__fmul_rn(cx.bh, px[k]), s, u, dt); }
     }
     // ---- syz
     {
@@ -303,8 +302,8 @@ k_rev_stress(Geo g, Fields f, Fields a, Psi ps, const float *__restrict__ lam,
       if (zs) acc = __fmaf_rn(cz.a, __fmul_rn(nzp(g, psz + PSI_SAB2 * g.slab_z, z, x, y), idz), acc);
       const float s = __fadd_rn(ayz0, acc);
       a.syz[i] = s;
-      if (ys) { const long long k = PSI_VB1 * g.slab_y + psi_y_idx(g, z, x, y); py[k] = __fmaf_rn(cy.bh, py[k], __fmul_rn(__fmul_rn(s, u), dt)); }
-      if (zs) { const long long k = PSI_VB2 * g.slab_z + psi_z_idx(g, z, x, y); pz[k] = __fmaf_rn(cz.bh, pz[k], __fmul_rn(__fmul_rn(s, u), dt)); }
+      if (ys) { const long long k = PSI_VB1 * g.slab_y + psi_y_idx(g, z, x, y); py[k] = add3(__fmul_rn(cy.bh, py[k]), s, u, dt); }
+      if (zs) { const long long k = PSI_VB2 * g.slab_z + psi_z_idx(g, z, x, y); pz[k] = add3(__fmul_rn(cz.bh, pz[k]), s, u, dt); }
     }
     // ---- normal stresses
     {

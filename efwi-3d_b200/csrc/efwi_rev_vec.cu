@@ -115,7 +115,7 @@ k_rev_velocity_vec(Geo g, Fields f, Fields a, Psi ps, const float *__restrict__ 
   vec_begin();  // up to here: nothing that the stress kernel writes
   if (any_in || any_sk) {
     Row gi{};
-    // reverse update of one velocity and its share of the rho image
+    // reverse update of one velocity and its share of the rho image (img3)
     auto reverse = [&](int r, int ra, int q, float *dst, const Row &d) {
       Row n = own.get(r);
       const Row b = own.get(BU), av = own.get(ra);
@@ -124,7 +124,9 @@ k_rev_velocity_vec(Geo g, Fields f, Fields a, Psi ps, const float *__restrict__ 
         const float nb2 = -(b[e] * b[e]);
         if (any_in && in[e]) {
           n.v[e] = undo(n[e], d[e], b[e], dt);
-          gi.v[e] = add4(gi[e], av[e], d[e], dt, nb2);
+          const float p = __fmul_rn(__fmul_rn(av[e], d[e]), dt);
+          gi.v[e] = r == VZ ? p : r == VX ? __fmaf_rn(gi[e], nb2, __fmul_rn(p, nb2))
+                                          : __fmaf_rn(p, nb2, gi[e]);
         }
         if (sk[e] >= 0) n.v[e] = shell.store[(size_t)q * shell.npts + sk[e]];
       }
@@ -132,24 +134,24 @@ k_rev_velocity_vec(Geo g, Fields f, Fields a, Psi ps, const float *__restrict__ 
     };
     Row d{};
     if (any_in) {
-      const Row d0 = D.p(f.szz + i, sz, idz), d1 = D.m(f.sxz + i, sx, idx), d2 = D.my(f.syz + i, idy);
+      const Row d0 = D.p(f.szz + i, sz, 1.f), d1 = D.m(f.sxz + i, sx, 1.f), d2 = D.my(f.syz + i, 1.f);
 #pragma unroll
-      for (int e = 0; e < VEC; ++e) d.v[e] = sum3(d0[e], d1[e], d2[e]);
+      for (int e = 0; e < VEC; ++e) d.v[e] = sum3d(d0[e], idz, d1[e], idx, d2[e], idy);
     }
     own.wait();
     reverse(VZ, AVZ, 6, f.vz + i, d);
     if (any_in) {
-      const Row d0 = D.m(f.sxz + i, sz, idz), d1 = D.p(f.sxx + i, sx, idx), d2 = D.my(f.sxy + i, idy);
+      const Row d0 = D.m(f.sxz + i, sz, 1.f), d1 = D.p(f.sxx + i, sx, 1.f), d2 = D.my(f.sxy + i, 1.f);
 #pragma unroll
-      for (int e = 0; e < VEC; ++e) d.v[e] = sum3(d0[e], d1[e], d2[e]);
+      for (int e = 0; e < VEC; ++e) d.v[e] = sum3d(d0[e], idz, d1[e], idx, d2[e], idy);
     }
     reverse(VX, AVX, 7, f.vx + i, d);
     if (any_in) {
-      const Row d0 = D.m(f.syz + i, sz, idz), d2 = D.py(f.syy + i, idy);
+      const Row d0 = D.m(f.syz + i, sz, 1.f), d2 = D.py(f.syy + i, 1.f);
       const Row m0 = ld_row(f.sxy + i), m1 = ld_row(f.sxy + i - sx), m2 = ld_row(f.sxy + i - 2 * sx);
 #pragma unroll
       for (int e = 0; e < VEC; ++e)
-        d.v[e] = sum3(d0[e], __fmul_rn(dquirk(m2[e], m1[e], m0[e]), idx), d2[e]);
+        d.v[e] = sum3d(d0[e], idz, dquirk(m2[e], m1[e], m0[e]), idx, d2[e], idy);
     }
     reverse(VY, AVY, 8, f.vy + i, d);
     if (any_in) {
@@ -172,10 +174,12 @@ k_rev_velocity_vec(Geo g, Fields f, Fields a, Psi ps, const float *__restrict__ 
   auto feed = [&](const Row &v, const Row &b, int slx, int bx, int slz, int bz, int sly) {
     Row add;
 #pragma unroll
-    for (int e = 0; e < VEC; ++e) add.v[e] = __fmul_rn(__fmul_rn(b[e], v[e]), dt);
-    if (m.xs) mem_row<VA>(px + slx * lx, m.kx, c, g.cx[bx * nx + x], add);
-    if (m.zs) mem_row<VA>(pz + slz * lz, m.kz, c, g.cz[bz * nz + z], add);
-    if (m.yany) mem_row_y(py + sly * ly, g, m, c, coef_y<VA>(g, c, CB), add);
+    for (int e = 0; e < VEC; ++e) add.v[e] = __fmul_rn(b[e], v[e]);
+    if (m.xs && slx == PSI_SAB1)
+      mem_row<VA, true>(px + slx * lx, m.kx, c, g.cx[bx * nx + x], add, dt);
+    if (m.xs && slx != PSI_SAB1) mem_row<VA>(px + slx * lx, m.kx, c, g.cx[bx * nx + x], add, dt);
+    if (m.zs) mem_row<VA>(pz + slz * lz, m.kz, c, g.cz[bz * nz + z], add, dt);
+    if (m.yany) mem_row_y(py + sly * ly, g, m, c, coef_y<VA>(g, c, CB), add, dt);
   };
   Row nax, naz, nay;
   own.wait();
@@ -257,8 +261,8 @@ k_rev_velocity_vec(Geo g, Fields f, Fields a, Psi ps, const float *__restrict__ 
 #pragma unroll
       for (int e = 0; e < VEC; ++e) {
         const float l2u = l[e] + 2.0f * u[e];
-        acc.v[e] = add4(0.f, l2u, s2[e], K[e], dt);
-        acc.v[e] = add4(acc[e], l[e], s1[e], K[e], dt);
+        acc.v[e] = add4(0.f, l[e], s1[e], K[e], dt);
+        acc.v[e] = add4(acc[e], l2u, s2[e], K[e], dt);
         acc.v[e] = add4(acc[e], l[e], s0[e], K[e], dt);
         acc.v[e] = add4(acc[e], u[e], Kx, t0[e], dt);
         acc.v[e] = add4(acc[e], u[e], Kz, t1[e], dt);
@@ -384,13 +388,14 @@ k_rev_stress_vec(Geo g, Fields f, Fields a, Psi ps, const float *__restrict__ la
     }
     if (any_in || any_sk) {
       // one shear stress from its two derivatives, and its share of the mu image
-      auto shear = [&](int r, int ra, int q, float *dst, const Row &d0, const Row &d1) {
+      auto shear = [&](int r, int ra, int q, float *dst, const Row &d0, float i0, const Row &d1,
+                       float i1) {
         Row n = own.get(r);
         const Row u = own.get(MU), as = own.get(ra);
 #pragma unroll
         for (int e = 0; e < VEC; ++e) {
           if (!any_in || !in[e]) continue;
-          const float s = __fadd_rn(d0[e], d1[e]);
+          const float s = sum2d(d0[e], i0, d1[e], i1);
           n.v[e] = undo(n[e], s, u[e], dt);
           gm.v[e] = __fmaf_rn(as[e], s, gm[e]);
         }
@@ -398,12 +403,12 @@ k_rev_stress_vec(Geo g, Fields f, Fields a, Psi ps, const float *__restrict__ la
         st_row(dst, n);
       };
       Row d0{}, d1{};
-      if (any_in) { d0 = D.p(f.vx + i, sz, idz); d1 = D.p(f.vz + i, sx, idx); }
-      shear(SXZ, AXZ, 1, f.sxz + i, d0, d1);
-      if (any_in) { d0 = D.p(f.vy + i, sz, idz); d1 = D.py(f.vz + i, idy); }
-      shear(SYZ, AYZ, 5, f.syz + i, d0, d1);
-      if (any_in) { d0 = D.py(f.vx + i, idy); d1 = D.p(f.vy + i, sx, idx); }
-      shear(SXY, AXY, 4, f.sxy + i, d0, d1);
+      if (any_in) { d0 = D.p(f.vx + i, sz, 1.f); d1 = D.p(f.vz + i, sx, 1.f); }
+      shear(SXZ, AXZ, 1, f.sxz + i, d0, idz, d1, idx);
+      if (any_in) { d0 = D.p(f.vy + i, sz, 1.f); d1 = D.py(f.vz + i, 1.f); }
+      shear(SYZ, AYZ, 5, f.syz + i, d0, idz, d1, idy);
+      if (any_in) { d0 = D.py(f.vx + i, 1.f); d1 = D.p(f.vy + i, sx, 1.f); }
+      shear(SXY, AXY, 4, f.sxy + i, d0, idy, d1, idx);
       if (any_in) {
         Row gr = own.get(GM);
 #pragma unroll
@@ -422,11 +427,11 @@ k_rev_stress_vec(Geo g, Fields f, Fields a, Psi ps, const float *__restrict__ la
   auto cfx = [&](int k, float out) { return m.xs ? g.cx[k * nx + x] : out; };
   auto cfy = [&](int k, float out) { return m.yany ? coef_y<VA>(g, c, k) : fill(out); };
   own.wait();
-  auto scaled = [&](const Row &s) {  // s * mu * dt, what a shear stress feeds
+  auto scaled = [&](const Row &s) {  // s * mu, what a shear stress feeds
     const Row u = own.get(MU);
     Row r;
 #pragma unroll
-    for (int e = 0; e < VEC; ++e) r.v[e] = __fmul_rn(__fmul_rn(s[e], u[e]), dt);
+    for (int e = 0; e < VEC; ++e) r.v[e] = __fmul_rn(s[e], u[e]);
     return r;
   };
   auto add_k = [&](Row &acc, float k, const Row &q) {
@@ -460,8 +465,8 @@ k_rev_stress_vec(Geo g, Fields f, Fields a, Psi ps, const float *__restrict__ la
     if (m.xs) add_k(acc, cfx(CA, 0.f), G.dpx(px + PSI_SAB1 * lx));
     if (m.zs) add_k(acc, cfz(CA, 0.f), G.dpz(pz + PSI_SAB1 * lz));
     const Row s = finish(AXZ, a.sxz + i, acc);
-    if (m.xs) mem_row<VA>(px + PSI_VB1 * lx, m.kx, c, g.cx[CBH * nx + x], scaled(s));
-    if (m.zs) mem_row<VA>(pz + PSI_VB1 * lz, m.kz, c, g.cz[CBH * nz + z], scaled(s));
+    if (m.xs) mem_row<VA>(px + PSI_VB1 * lx, m.kx, c, g.cx[CBH * nx + x], scaled(s), dt);
+    if (m.zs) mem_row<VA>(pz + PSI_VB1 * lz, m.kz, c, g.cz[CBH * nz + z], scaled(s), dt);
   }
   {  // sxy
     const Row d0 = D.np(a.vy + i, sx, idx), d1 = D.npy(a.vx + i, idy);
@@ -470,14 +475,14 @@ k_rev_stress_vec(Geo g, Fields f, Fields a, Psi ps, const float *__restrict__ la
     Row acc;
 #pragma unroll
     for (int e = 0; e < VEC; ++e) {
-      acc.v[e] = add4(0.f, d0[e], K0, b[e], dt);
-      acc.v[e] = add4(acc[e], d1[e], K1[e], b[e], dt);
+      acc.v[e] = add4(0.f, d1[e], K1[e], b[e], dt);
+      acc.v[e] = add4(acc[e], d0[e], K0, b[e], dt);
     }
     if (m.xs) add_k(acc, cfx(CA, 0.f), G.dpx(px + PSI_SAB2 * lx));
     if (m.yany) add_y(acc, CA, G.dpy(py + PSI_SAB2 * ly));
     const Row s = finish(AXY, a.sxy + i, acc);
-    if (m.yany) mem_row_y(py + PSI_VB2 * ly, g, m, c, coef_y<VA>(g, c, CBH), scaled(s));
-    if (m.xs) mem_row<VA>(px + PSI_VB2 * lx, m.kx, c, g.cx[CBH * nx + x], scaled(s));
+    if (m.yany) mem_row_y(py + PSI_VB2 * ly, g, m, c, coef_y<VA>(g, c, CBH), scaled(s), dt);
+    if (m.xs) mem_row<VA>(px + PSI_VB2 * lx, m.kx, c, g.cx[CBH * nx + x], scaled(s), dt);
   }
   {  // syz
     const Row d0 = D.npy(a.vz + i, idy), d1 = D.np(a.vy + i, sz, idz);
@@ -492,8 +497,8 @@ k_rev_stress_vec(Geo g, Fields f, Fields a, Psi ps, const float *__restrict__ la
     if (m.yany) add_y(acc, CA, G.dpy(py + PSI_SAB1 * ly));
     if (m.zs) add_k(acc, cfz(CA, 0.f), G.dpz(pz + PSI_SAB2 * lz));
     const Row s = finish(AYZ, a.syz + i, acc);
-    if (m.yany) mem_row_y(py + PSI_VB1 * ly, g, m, c, coef_y<VA>(g, c, CBH), scaled(s));
-    if (m.zs) mem_row<VA>(pz + PSI_VB2 * lz, m.kz, c, g.cz[CBH * nz + z], scaled(s));
+    if (m.yany) mem_row_y(py + PSI_VB1 * ly, g, m, c, coef_y<VA>(g, c, CBH), scaled(s), dt);
+    if (m.zs) mem_row<VA>(pz + PSI_VB2 * lz, m.kz, c, g.cz[CBH * nz + z], scaled(s), dt);
   }
   {  // normal stresses
     const Row b = own.get(BU);
@@ -529,8 +534,8 @@ k_rev_stress_vec(Geo g, Fields f, Fields a, Psi ps, const float *__restrict__ la
 #pragma unroll
         for (int e = 0; e < VEC; ++e)
           if (c.act[e])
-            r.v[e] = add3(add3(add3(__fmul_rn(bz, r[e]), cz[e], szz[e], dt), cx[e], sxx[e], dt),
-                          cy[e], syy[e], dt);
+            r.v[e] = add3(add3(add3(__fmul_rn(bz, r[e]), cz[e], szz[e], dt), cx[e],
+                               sxx[e], dt), cy[e], syy[e], dt);
         st_psi<VA>(p, k, r, c);
       };
       if (m.xs) feed(px + PSI_VA * lx, m.kx, g.cx[CB * nx + x], l, l2, l);
@@ -542,8 +547,8 @@ k_rev_stress_vec(Geo g, Fields f, Fields a, Psi ps, const float *__restrict__ la
 #pragma unroll
         for (int e = 0; e < VEC; ++e)
           if (m.ys[e])
-            r.v[e] = add3(add3(add3(__fmul_rn(bz[e], r[e]), l[e], szz[e], dt), l[e], sxx[e], dt),
-                          l2[e], syy[e], dt);
+            r.v[e] = add3(add3(add3(__fmul_rn(bz[e], r[e]), l[e], szz[e], dt), l[e],
+                               sxx[e], dt), l2[e], syy[e], dt);
         st_psi_y(p, r, m, g, c);
       }
     }

@@ -298,24 +298,27 @@ struct PsiGather {
   }
 };
 
-// Memory-variable update m = b m + add of a z or x slab row, or of a y slab
-// row with the coefficients b of its cells.
-template <bool VA>
+// Memory-variable update m = b m + add dt of a z or x slab row, or of a y slab
+// row with the coefficients b of its cells.  OLD: the product with the old
+// value is the one that the sum's rounding takes in.
+template <bool VA, bool OLD = false>
 __device__ __forceinline__ void mem_row(float *p, int k, const VecCell &c, float b,
-                                        const Row &add) {
+                                        const Row &add, float dt) {
   Row r = ld_psi<VA>(p, k, c);
 #pragma unroll
   for (int e = 0; e < VEC; ++e)
-    if (c.act[e]) r.v[e] = __fmaf_rn(b, r[e], add[e]);
+    if (c.act[e])
+      r.v[e] = OLD ? __fmaf_rn(b, r[e], __fmul_rn(add[e], dt)) : __fmaf_rn(add[e], dt, __fmul_rn(b, r[e]));
   st_psi<VA>(p, k, r, c);
 }
 template <bool VA>
 __device__ __forceinline__ void mem_row_y(float *p, const Geo &g, const Pml<VA> &m,
-                                          const VecCell &c, const Row &b, const Row &add) {
+                                          const VecCell &c, const Row &b, const Row &add,
+                                          float dt) {
   Row r = ld_psi_y(p, g, m, c);
 #pragma unroll
   for (int e = 0; e < VEC; ++e)
-    if (m.ys[e]) r.v[e] = __fmaf_rn(b[e], r[e], add[e]);
+    if (m.ys[e]) r.v[e] = __fmaf_rn(add[e], dt, __fmul_rn(b[e], r[e]));
   st_psi_y(p, r, m, g, c);
 }
 
