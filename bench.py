@@ -195,9 +195,9 @@ def kernel_bytes(grid, nshot_launch=1):
 # padded grid (128^3 model, C-PML 12), one shot per launch, from one ncu
 # capture of each kernel (dram__bytes_read.sum + dram__bytes_write.sum);
 # other grids report no traffic.
-TRAFFIC_152 = {"rev_velocity": 423.3e6, "rev_stress": 514.7e6,
-               "stress_fwd": 236.5e6, "velocity_fwd": 185.5e6,
-               "adj_velocity": 356.6e6, "adj_stress": 324.9e6}
+TRAFFIC_152 = {"rev_velocity": 409.6e6, "rev_stress": 475.2e6,
+               "stress_fwd": 227.3e6, "velocity_fwd": 190.5e6,
+               "adj_velocity": 364.9e6, "adj_stress": 324.5e6}
 
 
 def algorithmic_step_bytes(grid, nmodel):
@@ -445,7 +445,7 @@ def run_windows(a):
     """Config 4: 64 shots on uneven windows, forward modelling of all
     windows per call; the autotuner picks the stencil variant and launch
     shape (L1-served multi-domain launch per half-step with the time loop
-    in a CUDA graph, or per-window TMA launches on 8 streams); one JSON
+    in a CUDA graph, or per-window launches on 8 streams); one JSON
     line."""
     import torch
     from efwi import synthetic
@@ -492,7 +492,7 @@ def run_windows(a):
         "graph": True,
         "graph_form": "one persistent multi-domain launch per half-step, whole time loop in one "
                       "graph" if tune["variant"] == "l1" else
-                      "per-window TMA launches on 8 streams, one time step captured as a graph "
+                      "per-window launches on 8 streams, one time step captured as a graph "
                       "(parallel branches) and replayed per step",
         "clocks": clocks}))
     P.close()

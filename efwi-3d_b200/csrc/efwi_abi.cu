@@ -145,7 +145,7 @@ struct EfwiHandle {
   long long N = 0;  // cells of one pitched volume
   int py = 0;       // y pitch
   int if_win = 0, bx = 4, zchunk = 8, max_batch = 4;
-  int variant = 1;  // 0: L1-served stencils, 1: four cells per thread (exact: TMA-staged)
+  int variant = 1;  // 0: L1-served stencils, 1: four cells per thread
   int zchunk_rev = 8;  // z planes per CTA of the exact adjoint kernels
   int nt_limit = 0;        // > 0: time loops stop early (timing probes)
   std::string err;

@@ -436,7 +436,11 @@ k_velocity_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ buoy, int 
 // Registers decide the resident CTAs per SM: K_S 6 (80 registers), K_V 5 (96).
 // At 152^3, one shot of a gradient (microseconds, event overhead of 6 in all):
 // K_S 94 / 82 / 79 / 89 and K_V 68 / 64 / 62 / 68 with 4 / 5 / 6 / 7 CTAs; K_V
-// with 6 is no faster where a launch has few waves (75 x 109 x 91).
+// with 6 is no faster where a launch has few waves (75 x 109 x 91).  With the
+// own rows fetched ahead of the kernel before, K_S takes 72 and K_V 55 (126 and
+// 91 in z-marching kernels on bulk copies); four shots 203 and 181 (408, 280),
+// 0.84 and 0.77 of the copy bandwidth: DRAM bounds batches, the tail of each
+// launch and the loads' latency single shots.
 void launch_stress_fwd_vec(int S, cudaStream_t st, const Geo &g, const Fields &f, const Psi &ps,
                            const float *lam, const float *mu, const SrcArgs &src,
                            const ShellMap &shell, const IllumSum &il, const StepTo &to, bool after_velocity) {

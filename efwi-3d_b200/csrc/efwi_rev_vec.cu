@@ -556,7 +556,12 @@ k_rev_stress_vec(Geo g, Fields f, Fields a, Psi ps, const float *__restrict__ la
 }
 
 // K1 6 and K2 5 resident CTAs per SM (80 and 93 registers).  At 152^3 K1 takes
-// 150 / 144 / 137 us with 4 / 5 / 6 CTAs, K2 138 / 139 / 152.
+// 150 / 144 / 137 us with 4 / 5 / 6 CTAs, K2 138 / 139 / 152; with the own rows
+// fetched ahead of the kernel before, both 130 (271 and 289 in z-marching
+// kernels on bulk copies).  Latency bounds them: DRAM at 0.5 of the copy
+// bandwidth, L1's data pipe 55-60 % busy at a hit rate of 47 %, 20-24 warps per
+// SM.  More warps do not help: the reverse and the adjoint half on different
+// warps, 32 per SM, take 170 and 149.
 void launch_rev_velocity_vec(cudaStream_t st, const Geo &g, const Fields &f, const Fields &a,
                              const Psi &ps, const float *lam, const float *mu, const float *buoy,
                              float *grho, int do_rev, int do_adj, const ShellMap &shell,

@@ -1,5 +1,5 @@
 // Four-cell vectors of the direct stencil kernels (efwi_fwd_vec.cu,
-// efwi_rev_vec.cu).
+// efwi_rev_vec.cu, efwi_exact_vec.cu).
 //
 // A thread owns the four cells y .. y+3 (y a multiple of 4, so every row
 // access is one aligned 16-byte load: the pitch is a multiple of 4) of one row

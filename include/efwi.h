@@ -79,7 +79,7 @@ int efwi_set_variant(EfwiHandle *h, int variant);
 /* CUDA graphs of the time loops (default on): the forward time loop of a
  * batch and the reverse time loop of a reference-mode gradient shot are
  * captured once and replayed while their launch parameters (buffers,
- * tensor maps, tuning, time axis) are unchanged, across shots and calls.
+ * tuning, time axis) are unchanged, across shots and calls.
  * on = 0 launches them one by one (results are bitwise the same).  Runs with
  * kernel-event sampling (efwi_profile) launch eagerly.  No reference
  * counterpart (the reference launches about 25 kernels per step from the
