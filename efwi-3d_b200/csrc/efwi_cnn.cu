@@ -200,10 +200,11 @@ k_conv3d_wgrad(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restr
 }
 
 // out[i] = sum over the CTAs' partial sums, in a fixed order: warp w of a CTA
-// adds the partials w, w + 8, ... of 32 outputs (one 128-byte line each), the
-// eight warps' sums are added in warp order.  One thread per output, reading
-// all partials one after the other, took 40 us for 592 of them.
-constexpr int kRedWarps = 8;
+// adds the partials w, w + 32, ... of 32 outputs (one 128-byte line each), the
+// warps' sums are added in warp order.  Latency bounds it: one thread per
+// output, reading all partials one after the other, took 40 us for 592 of
+// them; 8 warps 9 us for 296, 32 warps 5.
+constexpr int kRedWarps = 32;
 struct Partials {
   const float *p;  // [parts][n]
   int parts, n;
