@@ -569,6 +569,12 @@ int upload_receivers(EfwiHandle *h, const RecHost &r, cudaStream_t st, RecArgs *
   const int nz = h->grid.nz;
   const long long nxpy = (long long)h->grid.nx * h->py;
   out->nxpy = (int)nxpy;
+  out->outer = 0;
+  for (const long long c : r.ucell) {
+    const EfwiGrid &g = h->grid;
+    const int y = (int)(c % h->py), x = (int)(c / h->py % g.nx), z = (int)(c / nxpy);
+    if (z < 2 || z > nz - 3 || x < 2 || x > g.nx - 3 || y < 2 || y > g.ny - 3) out->outer = 1;
+  }
   const int S = (int)r.trace_off.size();
   if (h->variant == 1 && !r.ucell.empty()) {
     std::vector<int> plane((size_t)S * nz, -1);
@@ -1470,9 +1476,11 @@ static int gradient_impl(EfwiHandle *h, int n, const int *ids, const float *obs,
     const int zcr = h->zchunk;
     const dim3 grid = stencil_grid(h, 1, h->bx, zcr, &nzc);
     // On the vector kernels the shell restore and the adjoint-source
-    // injection run inside K1 and K2; otherwise as separate launches.
+    // injection run inside K1 and K2; otherwise as separate launches.  K1
+    // reaches the cells it updates: a survey with receivers on others injects
+    // with a launch of its own (the adjoint stresses read those cells).
     const bool shell_fused = vec && h->shell_fused && npts > 0;
-    const bool inj_fused = vec && rec.ncell > 0 && rec.plane;
+    const bool inj_fused = vec && rec.ncell > 0 && rec.plane && !rec.outer;
     auto shell_at = [&](int rev, int it) {
       ShellMap m{};
       if (shell_fused && rev) {
@@ -1536,8 +1544,8 @@ static int gradient_impl(EfwiHandle *h, int n, const int *ids, const float *obs,
     KeyBytes key;
     key.add(f).add(a).add(ps).add(grho).add(glam).add(gmu).add(shell).add(npts).rec(rec)
         .src(src).add(h->res_tm.p).add(zcr).add(h->bx).add(vec).add(shell_fused)
-        .add(inj_fused).add(ntl).geo(h->geo).shell(h->shm).add(h->lam.p).add(h->mu.p)
-        .add(h->buoy.p);
+        .add(inj_fused).add(inj_fused ? 0 : rec.ncell)  // the separate launch bakes it in
+        .add(ntl).geo(h->geo).shell(h->shm).add(h->lam.p).add(h->mu.p).add(h->buoy.p);
     cudaStream_t caller = st;
     rc = run_graphed(h, h->g_rev, key.s, caller, loop);
     st = caller;

@@ -41,6 +41,7 @@ struct RecArgs {
   const int *plane;
   const int *map;
   int nxpy;
+  int outer;  // a receiver lies outside the cells [2, n-3]^3 that the steps update
 };
 
 // Boundary-shell save/restore inside the stencil kernels (efwi_fuse.cuh):
