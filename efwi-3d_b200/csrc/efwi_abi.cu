@@ -538,6 +538,13 @@ RecHost group_receivers(const EfwiHandle *h, const int *ids, int S, long long *t
   return r;
 }
 
+// Whether a launch over S shots of grid g runs on the vector kernels: variant
+// 1, within the grid limits of a launch (65535 CTAs along x rows and along
+// planes; larger grids take the L1-served kernels, whose CTAs march z).
+bool use_vec(const EfwiHandle *h, const Geo &g, int S) {
+  return h->variant == 1 && vec_fits(g, S);
+}
+
 // Uploads the grouping into h->recbuf and returns device views.
 int upload_receivers(EfwiHandle *h, const RecHost &r, cudaStream_t st, RecArgs *out) {
   auto al = [](size_t b) { return (b + 255) & ~size_t(255); };
@@ -576,7 +583,7 @@ int upload_receivers(EfwiHandle *h, const RecHost &r, cudaStream_t st, RecArgs *
     if (z < 2 || z > nz - 3 || x < 2 || x > g.nx - 3 || y < 2 || y > g.ny - 3) out->outer = 1;
   }
   const int S = (int)r.trace_off.size();
-  if (h->variant == 1 && !r.ucell.empty()) {
+  if (use_vec(h, h->geo, S) && !r.ucell.empty()) {
     std::vector<int> plane((size_t)S * nz, -1);
     int nmaps = 0;
     for (size_t u = 0; u < r.ucell.size(); ++u) {
@@ -620,13 +627,6 @@ dim3 stencil_grid(const EfwiHandle *h, int S, int bx, int zchunk, int *nzc) {
 
 int nt_eff(const EfwiHandle *h) {
   return h->nt_limit > 0 && h->nt_limit < h->grid.nt ? std::max(h->nt_limit, 2) : h->grid.nt;
-}
-
-// Whether a launch over S shots of grid g runs on the vector kernels: variant
-// 1, within the grid limits of a launch (65535 CTAs along x rows and along
-// planes; larger grids take the L1-served kernels, whose CTAs march z).
-bool use_vec(const EfwiHandle *h, const Geo &g, int S) {
-  return h->variant == 1 && vec_fits(g, S);
 }
 
 // One forward time step of a batch: stress (+ source), velocity, receivers.

@@ -83,3 +83,28 @@ def test_window_gradient_with_receivers_on_its_edge():
     for u, v in zip(*out):
         assert float(u.abs().max()) > 0
         assert torch.equal(u, v)
+
+
+def test_receiver_cells_of_shots_in_turn_beyond_the_launch_limits():
+    """More planes than one launch of the vector kernels takes: the one-cell
+    kernels run, and the captured time loop's separate receiver launch covers
+    the cells of the shot at hand (3, then 30, for as many receivers)."""
+    from efwi.engine import Grid, Propagator, Shot
+    nz, n, nt = 4 * 65535 + 20, 30, 24
+    g = Grid(nz, 5, 5, 2, nt, 10.0, 10.0, 10.0, 8e-4, 25.0)
+    model = [torch.full((nz, 5, 5), v) for v in (1.2e6, 1e6, 1.6)]
+    two = np.full(n, 2, np.int32)
+    shots = [Shot(src=(nz // 2, 2, 2), z_rec=(nz // 2 - 15 + r % cells).astype(np.int32), x_rec=two,
+                  y_rec=two) for cells, r in ((3, np.arange(n)), (n, np.arange(n)))]
+    stf = np.random.default_rng(0).standard_normal((2, nt)).astype(np.float32)
+    out = []
+    for graphs in (False, True):
+        P = Propagator(g)
+        P.set_graphs(graphs)
+        P.set_survey(shots, stf)
+        P.set_model(*model)
+        out.append([P.forward([k]).view(3, n, nt) for k in (0, 1, 0)])
+        P.close()
+    for u, v in zip(*out):
+        assert torch.equal(u, v)
+    assert bool((out[1][1][2].abs().amax(1) > 0).all())
