@@ -96,9 +96,9 @@ __device__ __forceinline__ void qs_z(const ExactArgs &A, int zn, int x, int y, f
     const int k = psi32_z(g, zn, x, y);
     const float *c = g.cz;
     const int nz = g.nz;
-    qez = qpml(G.ez, true, A.lin.z[PSI_VA * (int)g.slab_z + k], c[CK * nz + zn], c[CA * nz + zn]);
-    qvx = qpml(G.xz, true, A.lin.z[PSI_VB1 * (int)g.slab_z + k], c[CKH * nz + zn], c[CAH * nz + zn]);
-    qvy = qpml(G.yz, true, A.lin.z[PSI_VB2 * (int)g.slab_z + k], c[CKH * nz + zn], c[CAH * nz + zn]);
+    qez = qpml(G.ez, true, A.lin.z[PSI_VA * g.slab_z + k], c[CK * nz + zn], c[CA * nz + zn]);
+    qvx = qpml(G.xz, true, A.lin.z[PSI_VB1 * g.slab_z + k], c[CKH * nz + zn], c[CAH * nz + zn]);
+    qvy = qpml(G.yz, true, A.lin.z[PSI_VB2 * g.slab_z + k], c[CKH * nz + zn], c[CAH * nz + zn]);
   } else {
     qez = G.ez; qvx = G.xz; qvy = G.yz;
   }
@@ -115,9 +115,9 @@ __device__ __forceinline__ void qs_x(const ExactArgs &A, int z, int xn, int y, f
     const int k = psi32_x(g, z, xn, y);
     const float *c = g.cx;
     const int nx = g.nx;
-    qex = qpml(G.ex, true, A.lin.x[PSI_VA * (int)g.slab_x + k], c[CK * nx + xn], c[CA * nx + xn]);
-    qvz = qpml(G.xz, true, A.lin.x[PSI_VB1 * (int)g.slab_x + k], c[CKH * nx + xn], c[CAH * nx + xn]);
-    qvy = qpml(G.xy, true, A.lin.x[PSI_VB2 * (int)g.slab_x + k], c[CKH * nx + xn], c[CAH * nx + xn]);
+    qex = qpml(G.ex, true, A.lin.x[PSI_VA * g.slab_x + k], c[CK * nx + xn], c[CA * nx + xn]);
+    qvz = qpml(G.xz, true, A.lin.x[PSI_VB1 * g.slab_x + k], c[CKH * nx + xn], c[CAH * nx + xn]);
+    qvy = qpml(G.xy, true, A.lin.x[PSI_VB2 * g.slab_x + k], c[CKH * nx + xn], c[CAH * nx + xn]);
   } else {
     qex = G.ex; qvz = G.xz; qvy = G.xy;
   }
@@ -134,9 +134,9 @@ __device__ __forceinline__ void qs_y(const ExactArgs &A, int z, int x, int yn, f
     const int k = psi32_y(g, z, x, yn);
     const float *c = g.cy;
     const int ny = g.ny;
-    qey = qpml(G.ey, true, A.lin.y[PSI_VA * (int)g.slab_y + k], c[CK * ny + yn], c[CA * ny + yn]);
-    qvz = qpml(G.yz, true, A.lin.y[PSI_VB1 * (int)g.slab_y + k], c[CKH * ny + yn], c[CAH * ny + yn]);
-    qvx = qpml(G.xy, true, A.lin.y[PSI_VB2 * (int)g.slab_y + k], c[CKH * ny + yn], c[CAH * ny + yn]);
+    qey = qpml(G.ey, true, A.lin.y[PSI_VA * g.slab_y + k], c[CK * ny + yn], c[CA * ny + yn]);
+    qvz = qpml(G.yz, true, A.lin.y[PSI_VB1 * g.slab_y + k], c[CKH * ny + yn], c[CAH * ny + yn]);
+    qvx = qpml(G.xy, true, A.lin.y[PSI_VB2 * g.slab_y + k], c[CKH * ny + yn], c[CAH * ny + yn]);
   } else {
     qey = G.ey; qvz = G.yz; qvx = G.xy;
   }
@@ -151,9 +151,9 @@ __device__ __forceinline__ GS qs_own(const ExactArgs &A, int z, int x, int y, fl
     const int k = psi32_x(g, z, x, y);
     const float *c = g.cx;
     const int nx = g.nx;
-    qx[0] = qpml(G.ex, true, A.lin.x[PSI_VA * (int)g.slab_x + k], c[CK * nx + x], c[CA * nx + x]);
-    qx[1] = qpml(G.xz, true, A.lin.x[PSI_VB1 * (int)g.slab_x + k], c[CKH * nx + x], c[CAH * nx + x]);
-    qx[2] = qpml(G.xy, true, A.lin.x[PSI_VB2 * (int)g.slab_x + k], c[CKH * nx + x], c[CAH * nx + x]);
+    qx[0] = qpml(G.ex, true, A.lin.x[PSI_VA * g.slab_x + k], c[CK * nx + x], c[CA * nx + x]);
+    qx[1] = qpml(G.xz, true, A.lin.x[PSI_VB1 * g.slab_x + k], c[CKH * nx + x], c[CAH * nx + x]);
+    qx[2] = qpml(G.xy, true, A.lin.x[PSI_VB2 * g.slab_x + k], c[CKH * nx + x], c[CAH * nx + x]);
   } else {
     qx[0] = G.ex; qx[1] = G.xz; qx[2] = G.xy;
   }
@@ -161,9 +161,9 @@ __device__ __forceinline__ GS qs_own(const ExactArgs &A, int z, int x, int y, fl
     const int k = psi32_y(g, z, x, y);
     const float *c = g.cy;
     const int ny = g.ny;
-    qy[0] = qpml(G.ey, true, A.lin.y[PSI_VA * (int)g.slab_y + k], c[CK * ny + y], c[CA * ny + y]);
-    qy[1] = qpml(G.yz, true, A.lin.y[PSI_VB1 * (int)g.slab_y + k], c[CKH * ny + y], c[CAH * ny + y]);
-    qy[2] = qpml(G.xy, true, A.lin.y[PSI_VB2 * (int)g.slab_y + k], c[CKH * ny + y], c[CAH * ny + y]);
+    qy[0] = qpml(G.ey, true, A.lin.y[PSI_VA * g.slab_y + k], c[CK * ny + y], c[CA * ny + y]);
+    qy[1] = qpml(G.yz, true, A.lin.y[PSI_VB1 * g.slab_y + k], c[CKH * ny + y], c[CAH * ny + y]);
+    qy[2] = qpml(G.xy, true, A.lin.y[PSI_VB2 * g.slab_y + k], c[CKH * ny + y], c[CAH * ny + y]);
   } else {
     qy[0] = G.ey; qy[1] = G.yz; qy[2] = G.xy;
   }
@@ -296,12 +296,12 @@ __global__ void __launch_bounds__(32 * BX) k_adj_stress_exact(ExactArgs A, int z
         const float Kzh = c[CKH * nz + z], azh = c[CAH * nz + z], bzh = c[CBH * nz + z];
         const int k = psi32_z(g, z, x, y);
         const float *p = A.ps.z;
-        ezz = ezz * Kz + (bz * p[PSI_VA * (int)g.slab_z + k] + az * ezz);
-        dvx_dz = dvx_dz * Kzh + (bzh * p[PSI_VB1 * (int)g.slab_z + k] + azh * dvx_dz);
-        dvy_dz = dvy_dz * Kzh + (bzh * p[PSI_VB2 * (int)g.slab_z + k] + azh * dvy_dz);
-        A.lout.z[PSI_VA * (int)g.slab_z + k] = bz * (A.lin.z[PSI_VA * (int)g.slab_z + k] + G.ez);
-        A.lout.z[PSI_VB1 * (int)g.slab_z + k] = bzh * (A.lin.z[PSI_VB1 * (int)g.slab_z + k] + G.xz);
-        A.lout.z[PSI_VB2 * (int)g.slab_z + k] = bzh * (A.lin.z[PSI_VB2 * (int)g.slab_z + k] + G.yz);
+        ezz = ezz * Kz + (bz * p[PSI_VA * g.slab_z + k] + az * ezz);
+        dvx_dz = dvx_dz * Kzh + (bzh * p[PSI_VB1 * g.slab_z + k] + azh * dvx_dz);
+        dvy_dz = dvy_dz * Kzh + (bzh * p[PSI_VB2 * g.slab_z + k] + azh * dvy_dz);
+        A.lout.z[PSI_VA * g.slab_z + k] = bz * (A.lin.z[PSI_VA * g.slab_z + k] + G.ez);
+        A.lout.z[PSI_VB1 * g.slab_z + k] = bzh * (A.lin.z[PSI_VB1 * g.slab_z + k] + G.xz);
+        A.lout.z[PSI_VB2 * g.slab_z + k] = bzh * (A.lin.z[PSI_VB2 * g.slab_z + k] + G.yz);
       }
       if (xs) {
         const float *c = g.cx;
@@ -309,12 +309,12 @@ __global__ void __launch_bounds__(32 * BX) k_adj_stress_exact(ExactArgs A, int z
         const float Kxh = c[CKH * nx + x], axh = c[CAH * nx + x], bxh = c[CBH * nx + x];
         const int k = psi32_x(g, z, x, y);
         const float *p = A.ps.x;
-        exx = exx * Kx + (bx * p[PSI_VA * (int)g.slab_x + k] + ax * exx);
-        dvz_dx = dvz_dx * Kxh + (bxh * p[PSI_VB1 * (int)g.slab_x + k] + axh * dvz_dx);
-        dvy_dx = dvy_dx * Kxh + (bxh * p[PSI_VB2 * (int)g.slab_x + k] + axh * dvy_dx);
-        A.lout.x[PSI_VA * (int)g.slab_x + k] = bx * (A.lin.x[PSI_VA * (int)g.slab_x + k] + G.ex);
-        A.lout.x[PSI_VB1 * (int)g.slab_x + k] = bxh * (A.lin.x[PSI_VB1 * (int)g.slab_x + k] + G.xz);
-        A.lout.x[PSI_VB2 * (int)g.slab_x + k] = bxh * (A.lin.x[PSI_VB2 * (int)g.slab_x + k] + G.xy);
+        exx = exx * Kx + (bx * p[PSI_VA * g.slab_x + k] + ax * exx);
+        dvz_dx = dvz_dx * Kxh + (bxh * p[PSI_VB1 * g.slab_x + k] + axh * dvz_dx);
+        dvy_dx = dvy_dx * Kxh + (bxh * p[PSI_VB2 * g.slab_x + k] + axh * dvy_dx);
+        A.lout.x[PSI_VA * g.slab_x + k] = bx * (A.lin.x[PSI_VA * g.slab_x + k] + G.ex);
+        A.lout.x[PSI_VB1 * g.slab_x + k] = bxh * (A.lin.x[PSI_VB1 * g.slab_x + k] + G.xz);
+        A.lout.x[PSI_VB2 * g.slab_x + k] = bxh * (A.lin.x[PSI_VB2 * g.slab_x + k] + G.xy);
       }
       if (ys) {
         const float *c = g.cy;
@@ -322,12 +322,12 @@ __global__ void __launch_bounds__(32 * BX) k_adj_stress_exact(ExactArgs A, int z
         const float Kyh = c[CKH * ny + y], ayh = c[CAH * ny + y], byh = c[CBH * ny + y];
         const int k = psi32_y(g, z, x, y);
         const float *p = A.ps.y;
-        eyy = eyy * Ky + (by * p[PSI_VA * (int)g.slab_y + k] + ay * eyy);
-        dvz_dy = dvz_dy * Kyh + (byh * p[PSI_VB1 * (int)g.slab_y + k] + ayh * dvz_dy);
-        dvx_dy = dvx_dy * Kyh + (byh * p[PSI_VB2 * (int)g.slab_y + k] + ayh * dvx_dy);
-        A.lout.y[PSI_VA * (int)g.slab_y + k] = by * (A.lin.y[PSI_VA * (int)g.slab_y + k] + G.ey);
-        A.lout.y[PSI_VB1 * (int)g.slab_y + k] = byh * (A.lin.y[PSI_VB1 * (int)g.slab_y + k] + G.yz);
-        A.lout.y[PSI_VB2 * (int)g.slab_y + k] = byh * (A.lin.y[PSI_VB2 * (int)g.slab_y + k] + G.xy);
+        eyy = eyy * Ky + (by * p[PSI_VA * g.slab_y + k] + ay * eyy);
+        dvz_dy = dvz_dy * Kyh + (byh * p[PSI_VB1 * g.slab_y + k] + ayh * dvz_dy);
+        dvx_dy = dvx_dy * Kyh + (byh * p[PSI_VB2 * g.slab_y + k] + ayh * dvx_dy);
+        A.lout.y[PSI_VA * g.slab_y + k] = by * (A.lin.y[PSI_VA * g.slab_y + k] + G.ey);
+        A.lout.y[PSI_VB1 * g.slab_y + k] = byh * (A.lin.y[PSI_VB1 * g.slab_y + k] + G.yz);
+        A.lout.y[PSI_VB2 * g.slab_y + k] = byh * (A.lin.y[PSI_VB2 * g.slab_y + k] + G.xy);
       }
       if (A.g0) {
         const float azz = A.a.szz[i], axx = A.a.sxx[i], ayy = A.a.syy[i];
@@ -375,9 +375,9 @@ __device__ __forceinline__ void qv_z(const ExactArgs &A, int zn, int x, int y, f
     const int k = psi32_z(g, zn, x, y);
     const float *c = g.cz;
     const int nz = g.nz;
-    qzz = qpml(gz, true, A.lin.z[PSI_SAA * (int)g.slab_z + k], c[CKH * nz + zn], c[CAH * nz + zn]);
-    qxz = qpml(gx, true, A.lin.z[PSI_SAB1 * (int)g.slab_z + k], c[CK * nz + zn], c[CA * nz + zn]);
-    qyz = qpml(gy, true, A.lin.z[PSI_SAB2 * (int)g.slab_z + k], c[CK * nz + zn], c[CA * nz + zn]);
+    qzz = qpml(gz, true, A.lin.z[PSI_SAA * g.slab_z + k], c[CKH * nz + zn], c[CAH * nz + zn]);
+    qxz = qpml(gx, true, A.lin.z[PSI_SAB1 * g.slab_z + k], c[CK * nz + zn], c[CA * nz + zn]);
+    qyz = qpml(gy, true, A.lin.z[PSI_SAB2 * g.slab_z + k], c[CK * nz + zn], c[CA * nz + zn]);
   } else {
     qzz = gz; qxz = gx; qyz = gy;
   }
@@ -395,9 +395,9 @@ __device__ __forceinline__ void qv_x(const ExactArgs &A, int z, int xn, int y, f
     const int k = psi32_x(g, z, xn, y);
     const float *c = g.cx;
     const int nx = g.nx;
-    qxz = qpml(gz, true, A.lin.x[PSI_SAB1 * (int)g.slab_x + k], c[CK * nx + xn], c[CA * nx + xn]);
-    qxx = qpml(gx, true, A.lin.x[PSI_SAA * (int)g.slab_x + k], c[CKH * nx + xn], c[CAH * nx + xn]);
-    qxy = qpml(gy, true, A.lin.x[PSI_SAB2 * (int)g.slab_x + k], c[CK * nx + xn], c[CA * nx + xn]);
+    qxz = qpml(gz, true, A.lin.x[PSI_SAB1 * g.slab_x + k], c[CK * nx + xn], c[CA * nx + xn]);
+    qxx = qpml(gx, true, A.lin.x[PSI_SAA * g.slab_x + k], c[CKH * nx + xn], c[CAH * nx + xn]);
+    qxy = qpml(gy, true, A.lin.x[PSI_SAB2 * g.slab_x + k], c[CK * nx + xn], c[CA * nx + xn]);
   } else {
     qxz = gz; qxx = gx; qxy = gy;
   }
@@ -415,9 +415,9 @@ __device__ __forceinline__ void qv_y(const ExactArgs &A, int z, int x, int yn, f
     const int k = psi32_y(g, z, x, yn);
     const float *c = g.cy;
     const int ny = g.ny;
-    qyz = qpml(gz, true, A.lin.y[PSI_SAB1 * (int)g.slab_y + k], c[CK * ny + yn], c[CA * ny + yn]);
-    qxy = qpml(gx, true, A.lin.y[PSI_SAB2 * (int)g.slab_y + k], c[CK * ny + yn], c[CA * ny + yn]);
-    qyy = qpml(gy, true, A.lin.y[PSI_SAA * (int)g.slab_y + k], c[CKH * ny + yn], c[CAH * ny + yn]);
+    qyz = qpml(gz, true, A.lin.y[PSI_SAB1 * g.slab_y + k], c[CK * ny + yn], c[CA * ny + yn]);
+    qxy = qpml(gx, true, A.lin.y[PSI_SAB2 * g.slab_y + k], c[CK * ny + yn], c[CA * ny + yn]);
+    qyy = qpml(gy, true, A.lin.y[PSI_SAA * g.slab_y + k], c[CKH * ny + yn], c[CAH * ny + yn]);
   } else {
     qyz = gz; qxy = gx; qyy = gy;
   }
@@ -433,9 +433,9 @@ __device__ __forceinline__ void qv_own(const ExactArgs &A, int z, int x, int y, 
     const int k = psi32_x(g, z, x, y);
     const float *c = g.cx;
     const int nx = g.nx;
-    qx[0] = qpml(gz, true, A.lin.x[PSI_SAB1 * (int)g.slab_x + k], c[CK * nx + x], c[CA * nx + x]);
-    qx[1] = qpml(gx, true, A.lin.x[PSI_SAA * (int)g.slab_x + k], c[CKH * nx + x], c[CAH * nx + x]);
-    qx[2] = qpml(gy, true, A.lin.x[PSI_SAB2 * (int)g.slab_x + k], c[CK * nx + x], c[CA * nx + x]);
+    qx[0] = qpml(gz, true, A.lin.x[PSI_SAB1 * g.slab_x + k], c[CK * nx + x], c[CA * nx + x]);
+    qx[1] = qpml(gx, true, A.lin.x[PSI_SAA * g.slab_x + k], c[CKH * nx + x], c[CAH * nx + x]);
+    qx[2] = qpml(gy, true, A.lin.x[PSI_SAB2 * g.slab_x + k], c[CK * nx + x], c[CA * nx + x]);
   } else {
     qx[0] = gz; qx[1] = gx; qx[2] = gy;
   }
@@ -443,9 +443,9 @@ __device__ __forceinline__ void qv_own(const ExactArgs &A, int z, int x, int y, 
     const int k = psi32_y(g, z, x, y);
     const float *c = g.cy;
     const int ny = g.ny;
-    qy[0] = qpml(gz, true, A.lin.y[PSI_SAB1 * (int)g.slab_y + k], c[CK * ny + y], c[CA * ny + y]);
-    qy[1] = qpml(gx, true, A.lin.y[PSI_SAB2 * (int)g.slab_y + k], c[CK * ny + y], c[CA * ny + y]);
-    qy[2] = qpml(gy, true, A.lin.y[PSI_SAA * (int)g.slab_y + k], c[CKH * ny + y], c[CAH * ny + y]);
+    qy[0] = qpml(gz, true, A.lin.y[PSI_SAB1 * g.slab_y + k], c[CK * ny + y], c[CA * ny + y]);
+    qy[1] = qpml(gx, true, A.lin.y[PSI_SAB2 * g.slab_y + k], c[CK * ny + y], c[CA * ny + y]);
+    qy[2] = qpml(gy, true, A.lin.y[PSI_SAA * g.slab_y + k], c[CKH * ny + y], c[CAH * ny + y]);
   } else {
     qy[0] = gz; qy[1] = gx; qy[2] = gy;
   }
@@ -571,36 +571,36 @@ __global__ void __launch_bounds__(32 * BX) k_adj_velocity_exact(ExactArgs A, int
         const float Kz = c[CK * nz + z], bz = c[CB * nz + z], Kzh = c[CKH * nz + z], bzh = c[CBH * nz + z];
         const int k = psi32_z(g, z, x, y);
         const float *p = A.ps.z;
-        dszz_dz = dszz_dz * Kzh + p[PSI_SAA * (int)g.slab_z + k];
-        dsxz_dz = dsxz_dz * Kz + p[PSI_SAB1 * (int)g.slab_z + k];
-        dsyz_dz = dsyz_dz * Kz + p[PSI_SAB2 * (int)g.slab_z + k];
-        A.lout.z[PSI_SAA * (int)g.slab_z + k] = bzh * (A.lin.z[PSI_SAA * (int)g.slab_z + k] + gz);
-        A.lout.z[PSI_SAB1 * (int)g.slab_z + k] = bz * (A.lin.z[PSI_SAB1 * (int)g.slab_z + k] + gx);
-        A.lout.z[PSI_SAB2 * (int)g.slab_z + k] = bz * (A.lin.z[PSI_SAB2 * (int)g.slab_z + k] + gy);
+        dszz_dz = dszz_dz * Kzh + p[PSI_SAA * g.slab_z + k];
+        dsxz_dz = dsxz_dz * Kz + p[PSI_SAB1 * g.slab_z + k];
+        dsyz_dz = dsyz_dz * Kz + p[PSI_SAB2 * g.slab_z + k];
+        A.lout.z[PSI_SAA * g.slab_z + k] = bzh * (A.lin.z[PSI_SAA * g.slab_z + k] + gz);
+        A.lout.z[PSI_SAB1 * g.slab_z + k] = bz * (A.lin.z[PSI_SAB1 * g.slab_z + k] + gx);
+        A.lout.z[PSI_SAB2 * g.slab_z + k] = bz * (A.lin.z[PSI_SAB2 * g.slab_z + k] + gy);
       }
       if (xs) {
         const float *c = g.cx;
         const float Kx = c[CK * nx + x], bx = c[CB * nx + x], Kxh = c[CKH * nx + x], bxh = c[CBH * nx + x];
         const int k = psi32_x(g, z, x, y);
         const float *p = A.ps.x;
-        dsxz_dx = dsxz_dx * Kx + p[PSI_SAB1 * (int)g.slab_x + k];
-        dsxx_dx = dsxx_dx * Kxh + p[PSI_SAA * (int)g.slab_x + k];
-        dsxy_dx = dsxy_dx * Kx + p[PSI_SAB2 * (int)g.slab_x + k];
-        A.lout.x[PSI_SAB1 * (int)g.slab_x + k] = bx * (A.lin.x[PSI_SAB1 * (int)g.slab_x + k] + gz);
-        A.lout.x[PSI_SAA * (int)g.slab_x + k] = bxh * (A.lin.x[PSI_SAA * (int)g.slab_x + k] + gx);
-        A.lout.x[PSI_SAB2 * (int)g.slab_x + k] = bx * (A.lin.x[PSI_SAB2 * (int)g.slab_x + k] + gy);
+        dsxz_dx = dsxz_dx * Kx + p[PSI_SAB1 * g.slab_x + k];
+        dsxx_dx = dsxx_dx * Kxh + p[PSI_SAA * g.slab_x + k];
+        dsxy_dx = dsxy_dx * Kx + p[PSI_SAB2 * g.slab_x + k];
+        A.lout.x[PSI_SAB1 * g.slab_x + k] = bx * (A.lin.x[PSI_SAB1 * g.slab_x + k] + gz);
+        A.lout.x[PSI_SAA * g.slab_x + k] = bxh * (A.lin.x[PSI_SAA * g.slab_x + k] + gx);
+        A.lout.x[PSI_SAB2 * g.slab_x + k] = bx * (A.lin.x[PSI_SAB2 * g.slab_x + k] + gy);
       }
       if (ys) {
         const float *c = g.cy;
         const float Ky = c[CK * ny + y], by = c[CB * ny + y], Kyh = c[CKH * ny + y], byh = c[CBH * ny + y];
         const int k = psi32_y(g, z, x, y);
         const float *p = A.ps.y;
-        dsyz_dy = dsyz_dy * Ky + p[PSI_SAB1 * (int)g.slab_y + k];
-        dsxy_dy = dsxy_dy * Ky + p[PSI_SAB2 * (int)g.slab_y + k];
-        dsyy_dy = dsyy_dy * Kyh + p[PSI_SAA * (int)g.slab_y + k];
-        A.lout.y[PSI_SAB1 * (int)g.slab_y + k] = by * (A.lin.y[PSI_SAB1 * (int)g.slab_y + k] + gz);
-        A.lout.y[PSI_SAB2 * (int)g.slab_y + k] = by * (A.lin.y[PSI_SAB2 * (int)g.slab_y + k] + gx);
-        A.lout.y[PSI_SAA * (int)g.slab_y + k] = byh * (A.lin.y[PSI_SAA * (int)g.slab_y + k] + gy);
+        dsyz_dy = dsyz_dy * Ky + p[PSI_SAB1 * g.slab_y + k];
+        dsxy_dy = dsxy_dy * Ky + p[PSI_SAB2 * g.slab_y + k];
+        dsyy_dy = dsyy_dy * Kyh + p[PSI_SAA * g.slab_y + k];
+        A.lout.y[PSI_SAB1 * g.slab_y + k] = by * (A.lin.y[PSI_SAB1 * g.slab_y + k] + gz);
+        A.lout.y[PSI_SAB2 * g.slab_y + k] = by * (A.lin.y[PSI_SAB2 * g.slab_y + k] + gx);
+        A.lout.y[PSI_SAA * g.slab_y + k] = byh * (A.lin.y[PSI_SAA * g.slab_y + k] + gy);
       }
       if (A.g0) {
         A.g0[i] += (A.a.vz[i] * (dszz_dz + dsxz_dx + dsyz_dy) + A.a.vx[i] * (dsxz_dz + dsxx_dx + dsxy_dy) +
@@ -735,21 +735,21 @@ k_illumination(Geo g, Fields f, Psi ps, int S, const float *buoy, int do_stress,
         float dvy_dx = dplus(vy[i - sx], vy[i], vy[i + sx], vy[i + 2 * sx]) * idx;
         if (zs) {
           const float *c = g.cz;
-          const int k = psi32_z(g, z, x, y), sl = (int)g.slab_z;
+          const long long k = psi32_z(g, z, x, y), sl = g.slab_z;
           ezz = ezz * c[CK * nz + z] + (c[CB * nz + z] * pz[PSI_VA * sl + k] + c[CA * nz + z] * ezz);
           dvx_dz = dvx_dz * c[CKH * nz + z] + (c[CBH * nz + z] * pz[PSI_VB1 * sl + k] + c[CAH * nz + z] * dvx_dz);
           dvy_dz = dvy_dz * c[CKH * nz + z] + (c[CBH * nz + z] * pz[PSI_VB2 * sl + k] + c[CAH * nz + z] * dvy_dz);
         }
         if (xs) {
           const float *c = g.cx;
-          const int k = psi32_x(g, z, x, y), sl = (int)g.slab_x;
+          const long long k = psi32_x(g, z, x, y), sl = g.slab_x;
           exx = exx * c[CK * nx + x] + (c[CB * nx + x] * px[PSI_VA * sl + k] + c[CA * nx + x] * exx);
           dvz_dx = dvz_dx * c[CKH * nx + x] + (c[CBH * nx + x] * px[PSI_VB1 * sl + k] + c[CAH * nx + x] * dvz_dx);
           dvy_dx = dvy_dx * c[CKH * nx + x] + (c[CBH * nx + x] * px[PSI_VB2 * sl + k] + c[CAH * nx + x] * dvy_dx);
         }
         if (ys) {
           const float *c = g.cy;
-          const int k = psi32_y(g, z, x, y), sl = (int)g.slab_y;
+          const long long k = psi32_y(g, z, x, y), sl = g.slab_y;
           eyy = eyy * c[CK * ny + y] + (c[CB * ny + y] * py[PSI_VA * sl + k] + c[CA * ny + y] * eyy);
           dvz_dy = dvz_dy * c[CKH * ny + y] + (c[CBH * ny + y] * py[PSI_VB1 * sl + k] + c[CAH * ny + y] * dvz_dy);
           dvx_dy = dvx_dy * c[CKH * ny + y] + (c[CBH * ny + y] * py[PSI_VB2 * sl + k] + c[CAH * ny + y] * dvx_dy);
@@ -772,21 +772,21 @@ k_illumination(Geo g, Fields f, Psi ps, int S, const float *buoy, int do_stress,
       float dsyy_dy = dplus(syy[i - 1], syy[i], syy[i + 1], syy[i + 2]) * idy;
       if (zs) {
         const float *c = g.cz;
-        const int k = psi32_z(g, z, x, y), sl = (int)g.slab_z;
+        const long long k = psi32_z(g, z, x, y), sl = g.slab_z;
         dszz_dz = dszz_dz * c[CKH * nz + z] + pz[PSI_SAA * sl + k];
         dsxz_dz = dsxz_dz * c[CK * nz + z] + pz[PSI_SAB1 * sl + k];
         dsyz_dz = dsyz_dz * c[CK * nz + z] + pz[PSI_SAB2 * sl + k];
       }
       if (xv) {
         const float *c = g.cx;
-        const int k = psi32_x(g, z, x, y), sl = (int)g.slab_x;
+        const long long k = psi32_x(g, z, x, y), sl = g.slab_x;
         dsxz_dx = dsxz_dx * c[CK * nx + x] + px[PSI_SAB1 * sl + k];
         dsxx_dx = dsxx_dx * c[CKH * nx + x] + px[PSI_SAA * sl + k];
         dsxy_dx = dsxy_dx * c[CK * nx + x] + px[PSI_SAB2 * sl + k];
       }
       if (yv) {
         const float *c = g.cy;
-        const int k = psi32_y(g, z, x, y), sl = (int)g.slab_y;
+        const long long k = psi32_y(g, z, x, y), sl = g.slab_y;
         dsyz_dy = dsyz_dy * c[CK * ny + y] + py[PSI_SAB1 * sl + k];
         dsxy_dy = dsxy_dy * c[CK * ny + y] + py[PSI_SAB2 * sl + k];
         dsyy_dy = dsyy_dy * c[CKH * ny + y] + py[PSI_SAA * sl + k];

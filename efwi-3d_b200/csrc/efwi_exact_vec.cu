@@ -276,7 +276,6 @@ __global__ void __launch_bounds__(EX_THREADS, MINB) k_adj_stress_vec(ExactArgs A
     for (const float *p : {A.a.vz, A.a.vx, A.a.vy}) prefetch_row(p + i);
   if (part == 1 && in && A.g0) {
     const Pml<VA> m = pml_of<VA>(g, c, false);
-    const int lz = (int)g.slab_z, lx = (int)g.slab_x, ly = (int)g.slab_y;
     const float *azz = A.a.szz + i, *axx = A.a.sxx + i, *ayy = A.a.syy + i;
     const float *axz = A.a.sxz + i, *axy = A.a.sxy + i, *ayz = A.a.syz + i;
     // ---- images from the forward velocities of the same step: the modified
@@ -288,17 +287,17 @@ __global__ void __launch_bounds__(EX_THREADS, MINB) k_adj_stress_vec(ExactArgs A
     auto mod_z = [&](Row &d, int slot, int half) {
       if (!m.zs) return;
       const float *cf = g.cz + 3 * half * nz + z;
-      mod(d, cf[CK * nz], cf[CA * nz], cf[CB * nz], ld_psi<VA>(A.ps.z + slot * lz, m.kz, c));
+      mod(d, cf[CK * nz], cf[CA * nz], cf[CB * nz], ld_psi<VA>(A.ps.z, slot, g.slab_z, m.kz, c));
     };
     auto mod_x = [&](Row &d, int slot, int half) {
       if (!m.xs) return;
       const float *cf = g.cx + 3 * half * nx + x;
-      mod(d, cf[CK * nx], cf[CA * nx], cf[CB * nx], ld_psi<VA>(A.ps.x + slot * lx, m.kx, c));
+      mod(d, cf[CK * nx], cf[CA * nx], cf[CB * nx], ld_psi<VA>(A.ps.x, slot, g.slab_x, m.kx, c));
     };
     auto mod_y = [&](Row &d, int slot, int half) {
       if (!m.yany) return;
       const Row K = coef_y<VA>(g, c, 3 * half + CK), a = coef_y<VA>(g, c, 3 * half + CA),
-                b = coef_y<VA>(g, c, 3 * half + CB), p = ld_psi_y(A.ps.y + slot * ly, g, m, c);
+                b = coef_y<VA>(g, c, 3 * half + CB), p = ld_psi_y(A.ps.y, slot, g, m, c);
 #pragma unroll
       for (int e = 0; e < VEC; ++e)
         if (m.ys[e]) d.v[e] = d[e] * K[e] + (b[e] * p[e] + a[e] * d[e]);
@@ -422,27 +421,26 @@ __global__ void __launch_bounds__(EX_THREADS, MINB) k_adj_velocity_vec(ExactArgs
     for (const float *p : {A.a.szz, A.a.sxx, A.a.syy, A.a.sxz, A.a.sxy, A.a.syz}) prefetch_row(p + i);
   if (part == 1 && in && A.g0) {
     const Pml<VA> m = pml_of<VA>(g, c, true);
-    const int lz = (int)g.slab_z, lx = (int)g.slab_x, ly = (int)g.slab_y;
     const float *avz = A.a.vz + i, *avx = A.a.vx + i, *avy = A.a.vy + i;
     // ---- buoyancy image from the forward stresses of the same step: modified
     // derivatives d / K + psi (the memory variables are the step's new ones)
     auto mod_z = [&](Row &d, int slot, int half) {
       if (!m.zs) return;
       const float Ki = g.cz[(3 * half + CK) * nz + z];
-      const Row p = ld_psi<VA>(A.ps.z + slot * lz, m.kz, c);
+      const Row p = ld_psi<VA>(A.ps.z, slot, g.slab_z, m.kz, c);
 #pragma unroll
       for (int e = 0; e < VEC; ++e) d.v[e] = d[e] * Ki + p[e];
     };
     auto mod_x = [&](Row &d, int slot, int half) {
       if (!m.xs) return;
       const float Ki = g.cx[(3 * half + CK) * nx + x];
-      const Row p = ld_psi<VA>(A.ps.x + slot * lx, m.kx, c);
+      const Row p = ld_psi<VA>(A.ps.x, slot, g.slab_x, m.kx, c);
 #pragma unroll
       for (int e = 0; e < VEC; ++e) d.v[e] = d[e] * Ki + p[e];
     };
     auto mod_y = [&](Row &d, int slot, int half) {
       if (!m.yany) return;
-      const Row K = coef_y<VA>(g, c, 3 * half + CK), p = ld_psi_y(A.ps.y + slot * ly, g, m, c);
+      const Row K = coef_y<VA>(g, c, 3 * half + CK), p = ld_psi_y(A.ps.y, slot, g, m, c);
 #pragma unroll
       for (int e = 0; e < VEC; ++e)
         if (m.ys[e]) d.v[e] = d[e] * K[e] + p[e];

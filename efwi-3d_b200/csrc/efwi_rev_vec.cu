@@ -166,7 +166,7 @@ k_rev_velocity_vec(Geo g, Fields f, Fields a, Psi ps, const float *__restrict__ 
 
   const PsiGather<VA> G{g, c, m};
   float *pz = ps.z, *px = ps.x, *py = ps.y;
-  const int lz = (int)g.slab_z, lx = (int)g.slab_x, ly = (int)g.slab_y;
+  const long long lz = g.slab_z, lx = g.slab_x, ly = g.slab_y;
   auto cfz = [&](int k, float out) { return m.zs ? g.cz[k * nz + z] : out; };
   auto cfx = [&](int k, float out) { return m.xs ? g.cx[k * nx + x] : out; };
   auto cfy = [&](int k, float out) { return m.yany ? coef_y<VA>(g, c, k) : fill(out); };
@@ -422,7 +422,7 @@ k_rev_stress_vec(Geo g, Fields f, Fields a, Psi ps, const float *__restrict__ la
 
   const PsiGather<VA> G{g, c, m};
   float *pz = ps.z, *px = ps.x, *py = ps.y;
-  const int lz = (int)g.slab_z, lx = (int)g.slab_x, ly = (int)g.slab_y;
+  const long long lz = g.slab_z, lx = g.slab_x, ly = g.slab_y;
   auto cfz = [&](int k, float out) { return m.zs ? g.cz[k * nz + z] : out; };
   auto cfx = [&](int k, float out) { return m.xs ? g.cx[k * nx + x] : out; };
   auto cfy = [&](int k, float out) { return m.yany ? coef_y<VA>(g, c, k) : fill(out); };

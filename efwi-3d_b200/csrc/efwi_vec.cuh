@@ -139,6 +139,15 @@ __device__ __forceinline__ void st_psi(float *p, int k, const Row &r, const VecC
   for (int e = 0; e < VEC; ++e)
     if (c.act[e]) p[k + e] = r.v[e];
 }
+// The same of memory variable `slot` of an axis with slabs of `slab` cells.  Its
+// offset passes 2^31 cells on large grids; whole vectors are counted in 32 bits.
+template <bool VA>
+__device__ __forceinline__ Row ld_psi(const float *p, int slot, long long slab, int k,
+                                      const VecCell &c) {
+  if (VA)
+    return ld_row(p + (size_t)(slot * ((unsigned)slab / VEC) + (unsigned)k / VEC) * VEC);
+  return ld_psi<VA>(p + slot * slab, k, c);
+}
 // Four cells of a y slab.
 template <bool VA>
 __device__ __forceinline__ int psi_y_cell(const Geo &g, const Pml<VA> &m, const VecCell &c, int e) {
@@ -152,6 +161,12 @@ __device__ __forceinline__ Row ld_psi_y(const float *p, const Geo &g, const Pml<
 #pragma unroll
   for (int e = 0; e < VEC; ++e) r.v[e] = m.ys[e] ? p[psi_y_cell(g, m, c, e)] : 0.f;
   return r;
+}
+template <bool VA>
+__device__ __forceinline__ Row ld_psi_y(const float *p, int slot, const Geo &g, const Pml<VA> &m,
+                                        const VecCell &c) {
+  if (VA) return ld_psi<VA>(p, slot, g.slab_y, m.ky, c);
+  return ld_psi_y(p + slot * g.slab_y, g, m, c);
 }
 template <bool VA>
 __device__ __forceinline__ void st_psi_y(float *p, const Row &r, const Pml<VA> &m, const Geo &g,
