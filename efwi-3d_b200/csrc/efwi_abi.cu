@@ -664,7 +664,10 @@ int forward_step(EfwiHandle *h, Fields f, Psi ps, int S, const SrcArgs &src, con
       launch_stress_fwd(h->bx, grid, st, h->geo, f, ps, h->lam.as<float>(), h->mu.as<float>(),
                         h->zchunk, nzc, src);
   }
-  for (float **p : {&f.szz, &f.sxx, &f.syy, &f.sxz, &f.sxy, &f.syz}) *p += to.fields;
+  Fields done = f;  // of the state written
+  if (to.out) done = fields_at(to.out, (long long)h->grid.nz * h->grid.nx * to.pitch_out, 1);
+  f.szz = done.szz; f.sxx = done.sxx; f.syy = done.syy;
+  f.sxz = done.sxz; f.sxy = done.sxy; f.syz = done.syz;
   {
     Timer t(h, K_VELOCITY_FWD, st, it);
     if (vec)
@@ -672,10 +675,11 @@ int forward_step(EfwiHandle *h, Fields f, Psi ps, int S, const SrcArgs &src, con
     else
       launch_velocity_fwd(h->bx, grid, st, h->geo, f, ps, h->buoy.as<float>(), h->zchunk, nzc);
   }
-  for (float **p : {&f.vz, &f.vx, &f.vy}) *p += to.fields;
   if (rec.ncell > 0 && !rec_fused) {
+    // (a state whose rows differ from the grid's never comes here: the maps of a
+    // grid with padded rows are within their limit)
     Timer t(h, K_RECORD, st, it);
-    k_record<<<(rec.ncell + 127) / 128, 128, 0, st>>>(f, h->N, rec, traces_tm, it + 1);
+    k_record<<<(rec.ncell + 127) / 128, 128, 0, st>>>(done, h->N, rec, traces_tm, it + 1);
   }
   return check_launch(h, "forward step");
 }
@@ -799,30 +803,30 @@ int misfit_shot(EfwiHandle *h, const ShotHost &sh, const float *obs, const float
   return check_launch(h, "misfit");
 }
 
-// Floats of one checkpoint, 9 fields and the memory variables of one shot: as
-// stored, and as the budget and efwi_state_bytes count them, without the rows'
-// padding to whole lines (at most a sixth).
-long long stored_floats(const EfwiHandle *h) { return 9 * h->N + psi_per_shot(h->geo); }
+// Row pitch and floats of one checkpoint, 9 fields and the memory variables of
+// one shot: the budget is the caller's, so that the rows are not padded to whole
+// lines as those of the work buffers may be (y_pitch).
+int state_pitch(const EfwiHandle *h) { return (h->grid.ny + 3) & ~3; }
 long long state_floats(const EfwiHandle *h) {
-  const EfwiGrid &g = h->grid;
-  return 9LL * g.nz * g.nx * ((g.ny + 3) & ~3) + psi_per_shot(h->geo);
+  return 9LL * h->grid.nz * h->grid.nx * state_pitch(h) + psi_per_shot(h->geo);
 }
 
-// Checkpoint slots of `floats` each that the budget allows for a run of
-// `blocks` states (S_0 is the zero state and needs none).
-int checkpoint_slots(const EfwiHandle *h, int blocks, long long floats) {
-  const long long per = floats * (long long)sizeof(float);
+// Checkpoint slots the budget allows for a run of `blocks` states
+// (S_0 is the zero state and needs none).
+int checkpoint_slots(const EfwiHandle *h, int blocks) {
+  const long long per = state_floats(h) * (long long)sizeof(float);
   long long s = per > 0 ? h->ck_budget / per : 0;
   if (s > blocks - 1) s = blocks - 1;
   return (int)std::max(s, 0LL);
 }
 
 // Adjoint kernels' arguments over the engine's single-shot buffers.
-ExactArgs exact_args(EfwiHandle *h, const Fields &f, const Psi &ps, const Fields &a, int par,
-                     float *g0, float *g1) {
+ExactArgs exact_args(EfwiHandle *h, const Fields &f, int pitch_f, const Psi &ps, const Fields &a,
+                     int par, float *g0, float *g1) {
   ExactArgs A;
   A.g = h->geo;
   A.f = f;
+  A.pitch_f = pitch_f;
   A.ps = ps;
   A.a = a;
   const long long P = psi_per_shot(h->geo);
@@ -861,22 +865,15 @@ int exact_shot(EfwiHandle *h, int id, const float *obs, double *jdev, float *res
   CK_CUDA(h, h->adj.ensure(sizeof(float) * 9 * N));
   CK_CUDA(h, h->apsi.ensure(sizeof(float) * 2 * P));
 
-  const long long SF = stored_floats(h);
+  const int slots = checkpoint_slots(h, ntl);
   CkPlan plan;
-  cudaError_t room = cudaSuccess;
-  for (const long long floats : {state_floats(h), SF}) {
-    const int slots = checkpoint_slots(h, ntl, floats);
-    plan.build(ntl, slots, 64LL * ntl + 4096);
-    if (plan.too_long || plan.forward_steps > 16LL * ntl)
-      return fail(h, EFWI_ERR_TOO_LARGE,
-                  "checkpoint budget of %lld bytes (%d slots of %lld bytes) is too small for %d steps",
-                  h->ck_budget, slots, floats * 4, ntl);
-    room = h->ckpt.ensure(sizeof(float) * std::max(1LL, (long long)plan.slots_used * SF));
-    // no room for the padding as well: the slots that fit the budget with it
-    if (room != cudaErrorMemoryAllocation || floats == SF) break;
-    cudaGetLastError();
-  }
-  CK_CUDA(h, room);
+  plan.build(ntl, slots, 64LL * ntl + 4096);
+  if (plan.too_long || plan.forward_steps > 16LL * ntl)
+    return fail(h, EFWI_ERR_TOO_LARGE,
+                "checkpoint budget of %lld bytes (%d slots of %lld bytes) is too small for %d steps",
+                h->ck_budget, slots, state_floats(h) * 4, ntl);
+  const long long SF = state_floats(h);
+  CK_CUDA(h, h->ckpt.ensure(sizeof(float) * std::max(1LL, (long long)plan.slots_used * SF)));
   h->ck_forward_steps = plan.forward_steps;
   h->ck_slots = plan.slots_used;
 
@@ -899,20 +896,26 @@ int exact_shot(EfwiHandle *h, int id, const float *obs, double *jdev, float *res
   // read where it lies, by the adjoint and by the first step away from it.  A
   // slot is never stepped in place.
   struct State {
-    float *fields, *psi;  // [9N], [P]
+    float *fields, *psi;  // nine volumes of rows of
+    int pitch;            // this pitch, [P]
   };
-  const State work{h->fields.as<float>(), h->psi.as<float>()};
+  const State work{h->fields.as<float>(), h->psi.as<float>(), h->py};
+  const long long rows = (long long)h->grid.nz * h->grid.nx;
   auto slot = [&](int k) {
     float *p = h->ckpt.as<float>() + (long long)k * SF;
-    return State{p, p + 9 * N};
+    return State{p, p + SF - P, state_pitch(h)};
   };
+  auto fields_of = [&](const State &s) { return fields_at(s.fields, rows * s.pitch, 1); };
+  // (the work buffers' padding is zero and stays so)
   auto copy = [&](const State &to, const State &from) {
-    CK_CUDA(h, cudaMemcpyAsync(to.fields, from.fields, sizeof(float) * 9 * N, cudaMemcpyDeviceToDevice, st));
+    if (to.pitch == from.pitch)
+      CK_CUDA(h, cudaMemcpyAsync(to.fields, from.fields, sizeof(float) * 9 * N, cudaMemcpyDeviceToDevice, st));
+    else
+      CK_CUDA(h, cudaMemcpy2DAsync(to.fields, sizeof(float) * to.pitch, from.fields,
+                                   sizeof(float) * from.pitch, sizeof(float) * state_pitch(h),
+                                   9 * (size_t)rows, cudaMemcpyDeviceToDevice, st));
     CK_CUDA(h, cudaMemcpyAsync(to.psi, from.psi, sizeof(float) * P, cudaMemcpyDeviceToDevice, st));
     return (int)EFWI_OK;
-  };
-  auto apart = [](const float *to, const float *from) {
-    return ((long long)(uintptr_t)to - (long long)(uintptr_t)from) / (long long)sizeof(float);
   };
   State cur = work;
   if (vec && plan.slots_used > 0) {
@@ -930,9 +933,14 @@ int exact_shot(EfwiHandle *h, int id, const float *obs, double *jdev, float *res
         if (vec && it + 1 == act.b && ia + 1 < plan.actions.size() &&
             plan.actions[ia + 1].op == CK_STORE)
           to = slot(plan.actions[ia + 1].a);
-        rc = forward_step(h, fields_at(cur.fields, N, 1), psi_at(cur.psi, h->geo, 1), 1, b.src,
+        StepTo dest{};
+        if (to.fields != work.fields || cur.fields != work.fields) {
+          const long long psi = (long long)(uintptr_t)to.psi - (long long)(uintptr_t)cur.psi;
+          dest = StepTo{to.fields, psi / (long long)sizeof(float), cur.pitch, to.pitch};
+        }
+        rc = forward_step(h, fields_of(cur), psi_at(cur.psi, h->geo, 1), 1, b.src,
                           first ? b.rec : norec, h->traces_tm.as<float>(), st, it, nullptr, {},
-                          StepTo{apart(to.fields, cur.fields), apart(to.psi, cur.psi)}, it > act.a);
+                          dest, it > act.a);
         if (rc) return rc;
         cur = to;
       }
@@ -955,7 +963,7 @@ int exact_shot(EfwiHandle *h, int id, const float *obs, double *jdev, float *res
       }
     } else {  // CK_BLOCK
       const int k = act.a;
-      const Fields f = fields_at(cur.fields, N, 1);
+      const Fields f = fields_of(cur);
       const Psi ps = psi_at(cur.psi, h->geo, 1);
       if (first && adj_source) {
         first = false;
@@ -985,7 +993,7 @@ int exact_shot(EfwiHandle *h, int id, const float *obs, double *jdev, float *res
       }
       if (k <= ntl - 2) {
         Timer t(h, K_ADJ_STRESS, st, k);
-        const ExactArgs A = exact_args(h, f, ps, a, par_s, glam, gmu);
+        const ExactArgs A = exact_args(h, f, cur.pitch, ps, a, par_s, glam, gmu);
         if (vec) launch_adj_stress_vec(st, A);
         else launch_adj_stress_exact(bxe, grid, st, A, zc, nzc);
         par_s ^= 1;
@@ -997,7 +1005,7 @@ int exact_shot(EfwiHandle *h, int id, const float *obs, double *jdev, float *res
                                                               adj_source ? 1.0f : -2.0f);
         }
         Timer t(h, K_ADJ_VELOCITY, st, k);
-        const ExactArgs A = exact_args(h, f, ps, a, par_v, gB, nullptr);
+        const ExactArgs A = exact_args(h, f, cur.pitch, ps, a, par_v, gB, nullptr);
         if (vec) launch_adj_velocity_vec(st, A);
         else launch_adj_velocity_exact(bxe, grid, st, A, zc, nzc);
         par_v ^= 1;
@@ -2203,8 +2211,8 @@ int efwi_step(EfwiHandle *h, float *state, int transpose, void *stream) {
     k_state_convert<<<1184, 256, 0, st>>>(h->geo, state, a, ap, 1);
     int nzc;
     const dim3 grid = stencil_grid(h, 1, h->bx, h->zchunk_rev, &nzc);
-    launch_adj_velocity_exact(h->bx, grid, st, exact_args(h, f, ps, a, 0, nullptr, nullptr), h->zchunk_rev, nzc);
-    launch_adj_stress_exact(h->bx, grid, st, exact_args(h, f, ps, a, 0, nullptr, nullptr), h->zchunk_rev, nzc);
+    launch_adj_velocity_exact(h->bx, grid, st, exact_args(h, f, h->py, ps, a, 0, nullptr, nullptr), h->zchunk_rev, nzc);
+    launch_adj_stress_exact(h->bx, grid, st, exact_args(h, f, h->py, ps, a, 0, nullptr, nullptr), h->zchunk_rev, nzc);
     Psi out = psi_at(h->apsi.as<float>() + P, h->geo, 1);
     k_state_convert<<<1184, 256, 0, st>>>(h->geo, state, a, out, 0);
   }

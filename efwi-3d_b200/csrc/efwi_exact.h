@@ -18,7 +18,8 @@ __device__ __forceinline__ float dq_t(float p0, float p1, float p2) {
 
 struct ExactArgs {
   Geo g;
-  Fields f;        // forward state S_k (read)
+  Fields f;        // forward state S_k (read), rows of
+  int pitch_f;     // this pitch (the one-cell kernels: the grid's)
   Psi ps;          // forward memory variables of S_k (read)
   Fields a;        // adjoint fields (updated in place)
   Psi lin, lout;   // adjoint memory variables: read from lin, written to lout

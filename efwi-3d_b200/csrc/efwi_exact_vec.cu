@@ -264,7 +264,6 @@ __global__ void __launch_bounds__(EX_THREADS, MINB) k_adj_stress_vec(ExactArgs A
   const int tz = threadIdx.z % VEC_TZ, part = threadIdx.z / VEC_TZ;
   const int z = z0 + tz, x = x0 + threadIdx.y, y = y0 + VEC * threadIdx.x;
   const int nz = g.nz, nx = g.nx;
-  const int sz = (int)g.sz, sx = g.sx;
   const float dt = g.dt, idz = g.idz, idx = g.idx, idy = g.idy;
   if (threadIdx.x + threadIdx.y + threadIdx.z == 0) q.next = 0;
   __syncthreads();
@@ -302,10 +301,12 @@ __global__ void __launch_bounds__(EX_THREADS, MINB) k_adj_stress_vec(ExactArgs A
       for (int e = 0; e < VEC; ++e)
         if (m.ys[e]) d.v[e] = d[e] * K[e] + (b[e] * p[e] + a[e] * d[e]);
     };
-    const float *vz = A.f.vz + i, *vx = A.f.vx + i, *vy = A.f.vy + i;
+    const VecCell cf = vec_cell(g, z, x, y, A.pitch_f);  // in the forward state
+    const int fx = A.pitch_f, fz = nx * fx;
+    const float *vz = A.f.vz + cf.i, *vx = A.f.vx + cf.i, *vy = A.f.vy + cf.i;
     Row gm;
     {
-      Row ez = diff_m(vz, sz, idz), ex = diff_m(vx, sx, idx), ey = diff_my(vy, c, idy);
+      Row ez = diff_m(vz, fz, idz), ex = diff_m(vx, fx, idx), ey = diff_my(vy, cf, idy);
       mod_z(ez, PSI_VA, 0);
       mod_x(ex, PSI_VA, 0);
       mod_y(ey, PSI_VA, 0);
@@ -324,19 +325,19 @@ __global__ void __launch_bounds__(EX_THREADS, MINB) k_adj_stress_vec(ExactArgs A
       for (int e = 0; e < VEC; ++e) gm.v[e] += p[e] * (d0[e] + d1[e]);
     };
     {
-      Row d0 = diff_p(vx, sz, idz), d1 = diff_p(vz, sx, idx);
+      Row d0 = diff_p(vx, fz, idz), d1 = diff_p(vz, fx, idx);
       mod_z(d0, PSI_VB1, 1);
       mod_x(d1, PSI_VB1, 1);
       share(axz, d0, d1);
     }
     {
-      Row d0 = diff_py(vx, c, idy), d1 = diff_p(vy, sx, idx);
+      Row d0 = diff_py(vx, cf, idy), d1 = diff_p(vy, fx, idx);
       mod_y(d0, PSI_VB2, 1);
       mod_x(d1, PSI_VB2, 1);
       share(axy, d0, d1);
     }
     {
-      Row d0 = diff_p(vy, sz, idz), d1 = diff_py(vz, c, idy);
+      Row d0 = diff_p(vy, fz, idz), d1 = diff_py(vz, cf, idy);
       mod_z(d0, PSI_VB2, 1);
       mod_y(d1, PSI_VB1, 1);
       share(ayz, d0, d1);
@@ -409,7 +410,6 @@ __global__ void __launch_bounds__(EX_THREADS, MINB) k_adj_velocity_vec(ExactArgs
   const int tz = threadIdx.z % VEC_TZ, part = threadIdx.z / VEC_TZ;
   const int z = z0 + tz, x = x0 + threadIdx.y, y = y0 + VEC * threadIdx.x;
   const int nz = g.nz, nx = g.nx;
-  const int sz = (int)g.sz, sx = g.sx;
   const float dt = g.dt, idz = g.idz, idx = g.idx, idy = g.idy;
   if (threadIdx.x + threadIdx.y + threadIdx.z == 0) q.next = 0;
   __syncthreads();
@@ -445,11 +445,13 @@ __global__ void __launch_bounds__(EX_THREADS, MINB) k_adj_velocity_vec(ExactArgs
       for (int e = 0; e < VEC; ++e)
         if (m.ys[e]) d.v[e] = d[e] * K[e] + p[e];
     };
-    const float *szz = A.f.szz + i, *sxx = A.f.sxx + i, *syy = A.f.syy + i;
-    const float *sxz = A.f.sxz + i, *sxy = A.f.sxy + i, *syz = A.f.syz + i;
+    const VecCell cf = vec_cell(g, z, x, y, A.pitch_f);  // in the forward state
+    const int fx = A.pitch_f, fz = nx * fx;
+    const float *szz = A.f.szz + cf.i, *sxx = A.f.sxx + cf.i, *syy = A.f.syy + cf.i;
+    const float *sxz = A.f.sxz + cf.i, *sxy = A.f.sxy + cf.i, *syz = A.f.syz + cf.i;
     Row im;
     {
-      Row d0 = diff_p(szz, sz, idz), d1 = diff_m(sxz, sx, idx), d2 = diff_my(syz, c, idy);
+      Row d0 = diff_p(szz, fz, idz), d1 = diff_m(sxz, fx, idx), d2 = diff_my(syz, cf, idy);
       mod_z(d0, PSI_SAA, 1);
       mod_x(d1, PSI_SAB1, 0);
       mod_y(d2, PSI_SAB1, 0);
@@ -458,7 +460,7 @@ __global__ void __launch_bounds__(EX_THREADS, MINB) k_adj_velocity_vec(ExactArgs
       for (int e = 0; e < VEC; ++e) im.v[e] = v[e] * (d0[e] + d1[e] + d2[e]);
     }
     {
-      Row d0 = diff_m(sxz, sz, idz), d1 = diff_p(sxx, sx, idx), d2 = diff_my(sxy, c, idy);
+      Row d0 = diff_m(sxz, fz, idz), d1 = diff_p(sxx, fx, idx), d2 = diff_my(sxy, cf, idy);
       mod_z(d0, PSI_SAB1, 0);
       mod_x(d1, PSI_SAA, 1);
       mod_y(d2, PSI_SAB2, 0);
@@ -467,8 +469,8 @@ __global__ void __launch_bounds__(EX_THREADS, MINB) k_adj_velocity_vec(ExactArgs
       for (int e = 0; e < VEC; ++e) im.v[e] += v[e] * (d0[e] + d1[e] + d2[e]);
     }
     {
-      Row d0 = diff_m(syz, sz, idz), d1, d2 = diff_py(syy, c, idy);
-      const Row s0 = ld_row(sxy), s1 = ld_row(sxy - sx), s2 = ld_row(sxy - 2 * sx);
+      Row d0 = diff_m(syz, fz, idz), d1, d2 = diff_py(syy, cf, idy);
+      const Row s0 = ld_row(sxy), s1 = ld_row(sxy - fx), s2 = ld_row(sxy - 2 * fx);
 #pragma unroll
       for (int e = 0; e < VEC; ++e) d1.v[e] = dquirk(s2[e], s1[e], s0[e]) * idx;
       mod_z(d0, PSI_SAB2, 0);

@@ -18,6 +18,12 @@ namespace efwi {
 
 enum { VEC_STEP, VEC_STEP_TO, VEC_ILLUM };  // what a launch does besides the step
 
+// The thread's vector in volume q of the state that a step writes.
+__device__ __forceinline__ float *step_to(const StepTo &to, const Geo &g, int q, int z, int x, int y) {
+  const long long n = (long long)g.nz * g.nx * to.pitch_out;
+  return to.out + q * n + (z * g.nx + x) * to.pitch_out + y;
+}
+
 // Both kernels form one output (K_S: the normal stresses together) at a time,
 // each from its own differences, so that few values are live: registers, not
 // bandwidth, hold these kernels' occupancy down, and the rows read again for
@@ -26,8 +32,9 @@ enum { VEC_STEP, VEC_STEP_TO, VEC_ILLUM };  // what a launch does besides the st
 // part, and the shell's copy of an output is taken by the part that updates it.
 //
 // VEC_STEP_TO: the results go to another state (exact gradient: a checkpoint),
-// zero where no step writes, at the cost of no copy.  A kernel of its own: with
-// the offsets in every launch, 26 x 30 x 28 and 84^3 ran 3-4 % slower.
+// zero where no step writes, at the cost of no copy.  A checkpoint's rows have
+// no padding to whole lines.  A kernel of its own: with the offsets in every
+// launch, 26 x 30 x 28 and 84^3 ran 3-4 % slower.
 //
 // VEC_ILLUM: the kernels add the step's share of the source illumination (the diagonal
 // pseudo-Hessian of k_illumination, efwi_exact.cu), whose derivatives they have
@@ -41,7 +48,7 @@ k_stress_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ lam,
                  const float *__restrict__ mu, int nzb, SrcArgs src, ShellMap shell, IllumSum il, StepTo to) {
   constexpr bool IL = MODE == VEC_ILLUM;
   static_assert(!IL || PARTS == 1, "the sums need all outputs in one thread");
-  const long long tf = MODE == VEC_STEP_TO ? to.fields : 0, tp = MODE == VEC_STEP_TO ? to.psi : 0;
+  const long long tp = MODE == VEC_STEP_TO ? to.psi : 0;
   const int shot = blockIdx.z / nzb;
   constexpr int TZ = vec_tz(PARTS), T = vec_threads(PARTS);
   const int part = PARTS > 1 ? threadIdx.z / TZ : 0;
@@ -51,14 +58,20 @@ k_stress_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ lam,
   const int nz = g.nz, nx = g.nx, ny = g.ny;
   if (z > nz - 3 || x > nx - 3 || y > ny - 3) return;
   const VecCell c = vec_cell(g, z, x, y);
-  const long long so = (long long)shot * g.N + c.i;
+  const VecCell r = MODE == VEC_STEP_TO ? vec_cell(g, z, x, y, to.pitch_in) : c;  // in the state read
+  const long long so = (long long)shot * g.N + r.i;
   const float *__restrict__ vz = f.vz + so;
   const float *__restrict__ vx = f.vx + so;
   const float *__restrict__ vy = f.vy + so;
-  const int sz = (int)g.sz, sx = g.sx;
+  const int sx = MODE == VEC_STEP_TO ? to.pitch_in : g.sx;
+  const int sz = MODE == VEC_STEP_TO ? nx * sx : (int)g.sz;
   const float dt = g.dt, idz = g.idz, idx = g.idx, idy = g.idy;
   float *szz = f.szz + so, *sxx = f.sxx + so, *syy = f.syy + so;
   float *sxz = f.sxz + so, *sxy = f.sxy + so, *syz = f.syz + so;
+  // where output volume q (in the order of Fields) of a field at p goes
+  auto dest = [&](float *p, int q) {
+    return MODE == VEC_STEP_TO ? step_to(to, g, q, z, x, y) : p;
+  };
   __shared__ float4 stash[(IL ? 10 : 8) * T];
   Stash<T> own{stash + vec_thread()};
   // outputs of the thread: 0 the normal stresses, 1 sxz, 2 sxy, 3 syz
@@ -130,7 +143,7 @@ k_stress_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ lam,
       for (int e = 0; e < VEC; ++e) exx[e] = dminus(a[e], b[e], x0[e], d[e]) * idx;
     }
     {
-      const Span w = ld_span(vy, y0, c);
+      const Span w = ld_span(vy, y0, r);
 #pragma unroll
       for (int e = 0; e < VEC; ++e) eyy[e] = dminus(w(e, -2), w(e, -1), y0[e], w(e, 1)) * idy;
     }
@@ -173,12 +186,12 @@ k_stress_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ lam,
         nyy.v[e] = (float)((double)nyy[e] + a);
       }
     }
-    st_row(szz + tf, nzz); st_row(sxx + tf, nxx); st_row(syy + tf, nyy);
+    st_row(dest(szz, 3), nzz); st_row(dest(sxx, 4), nxx); st_row(dest(syy, 5), nyy);
   }
   // one shear stress from its two derivatives
-  auto shear = [&](int r, float *dst, const float d0[VEC], const float d1[VEC]) {
+  auto shear = [&](int k, float *dst, const float d0[VEC], const float d1[VEC]) {
     if (PARTS > 1) own.wait();
-    Row n = own.get(r);
+    Row n = own.get(k);
     const Row u = own.get(7);
 #pragma unroll
     for (int e = 0; e < VEC; ++e)
@@ -187,7 +200,7 @@ k_stress_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ lam,
 #pragma unroll
       for (int e = 0; e < VEC; ++e) am[e] += (d0[e] + d1[e]) * (d0[e] + d1[e]);
     }
-    st_row(dst + tf, n);
+    st_row(dst, n);
   };
   if (mine(1)) {  // sxz
     Row qz = ld_z(PSI_VB1), qx = ld_x(PSI_VB1);
@@ -204,14 +217,14 @@ k_stress_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ lam,
     }
     pml_z(PSI_VB1, 1, qz, dvx_dz);
     pml_x(PSI_VB1, 1, qx, dvz_dx);
-    shear(3, sxz, dvx_dz, dvz_dx);
+    shear(3, dest(sxz, 6), dvx_dz, dvz_dx);
   }
   if (mine(2)) {  // sxy
     Row qx = ld_x(PSI_VB2), qy = ld_y(PSI_VB2);
     float dvx_dy[VEC], dvy_dx[VEC];
     {
       const Row m = ld_row(vx);
-      const Span w = ld_span(vx, m, c);
+      const Span w = ld_span(vx, m, r);
 #pragma unroll
       for (int e = 0; e < VEC; ++e) dvx_dy[e] = dplus(w(e, -1), m[e], w(e, 1), w(e, 2)) * idy;
     }
@@ -222,7 +235,7 @@ k_stress_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ lam,
     }
     pml_x(PSI_VB2, 1, qx, dvy_dx);
     pml_y(PSI_VB2, 1, qy, dvx_dy);
-    shear(4, sxy, dvx_dy, dvy_dx);
+    shear(4, dest(sxy, 7), dvx_dy, dvy_dx);
   }
   if (mine(3)) {  // syz
     Row qz = ld_z(PSI_VB2), qy = ld_y(PSI_VB1);
@@ -234,13 +247,13 @@ k_stress_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ lam,
     }
     {
       const Row m = ld_row(vz);
-      const Span w = ld_span(vz, m, c);
+      const Span w = ld_span(vz, m, r);
 #pragma unroll
       for (int e = 0; e < VEC; ++e) dvz_dy[e] = dplus(w(e, -1), m[e], w(e, 1), w(e, 2)) * idy;
     }
     pml_z(PSI_VB2, 1, qz, dvy_dz);
     pml_y(PSI_VB1, 1, qy, dvz_dy);
-    shear(5, syz, dvy_dz, dvz_dy);
+    shear(5, dest(syz, 8), dvy_dz, dvz_dy);
   }
   if (IL) {
     Row hm = own.get(9);
@@ -257,7 +270,7 @@ k_velocity_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ buoy, int 
                    IllumSum il, StepTo to) {
   constexpr bool IL = MODE == VEC_ILLUM;
   static_assert(!IL || PARTS == 1, "the sums need all outputs in one thread");
-  const long long tf = MODE == VEC_STEP_TO ? to.fields : 0, tp = MODE == VEC_STEP_TO ? to.psi : 0;
+  const long long tp = MODE == VEC_STEP_TO ? to.psi : 0;
   const int shot = blockIdx.z / nzb;
   constexpr int TZ = vec_tz(PARTS), T = vec_threads(PARTS);
   const int part = PARTS > 1 ? threadIdx.z / TZ : 0;
@@ -267,16 +280,23 @@ k_velocity_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ buoy, int 
   const int nz = g.nz, nx = g.nx, ny = g.ny;
   if (z > nz - 3 || x > nx - 3 || y > ny - 3) return;
   const VecCell c = vec_cell(g, z, x, y);
-  const long long so = (long long)shot * g.N + c.i;
+  // in the stresses: its K_S's output
+  const VecCell r = MODE == VEC_STEP_TO ? vec_cell(g, z, x, y, to.pitch_out) : c;
+  const long long so = (long long)shot * g.N + r.i;
   const float *__restrict__ szz = f.szz + so;
   const float *__restrict__ sxx = f.sxx + so;
   const float *__restrict__ syy = f.syy + so;
   const float *__restrict__ sxz = f.sxz + so;
   const float *__restrict__ sxy = f.sxy + so;
   const float *__restrict__ syz = f.syz + so;
-  const int sz = (int)g.sz, sx = g.sx;
+  const int sx = MODE == VEC_STEP_TO ? to.pitch_out : g.sx;
+  const int sz = MODE == VEC_STEP_TO ? nx * sx : (int)g.sz;
   const float idz = g.idz, idx = g.idx, idy = g.idy, dt = g.dt;
-  float *vz = f.vz + so, *vx = f.vx + so, *vy = f.vy + so;
+  const long long vo = MODE == VEC_STEP_TO ? (z * nx + x) * to.pitch_in + y : so;
+  float *vz = f.vz + vo, *vx = f.vx + vo, *vy = f.vy + vo;
+  auto dest = [&](float *p, int q) {
+    return MODE == VEC_STEP_TO ? step_to(to, g, q, z, x, y) : p;
+  };
   __shared__ float4 stash[(IL || PARTS > 1 ? 5 : 4) * T];
   Stash<T> own{stash + vec_thread()};
   // outputs of the thread: 0 vz, 1 vx, 2 vy
@@ -315,9 +335,9 @@ k_velocity_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ buoy, int 
   };
 
   // one velocity from its three derivatives
-  auto update = [&](int r, const float d0[VEC], const float d1[VEC], const float d2[VEC]) {
+  auto update = [&](int k, const float d0[VEC], const float d1[VEC], const float d2[VEC]) {
     if (PARTS > 1) own.wait();
-    Row n = own.get(r);
+    Row n = own.get(k);
     const Row b = own.get(3);
 #pragma unroll
     for (int e = 0; e < VEC; ++e)
@@ -347,7 +367,7 @@ k_velocity_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ buoy, int 
     }
     {
       const Row m = ld_row(syz);
-      const Span w = ld_span(syz, m, c);
+      const Span w = ld_span(syz, m, r);
 #pragma unroll
       for (int e = 0; e < VEC; ++e) dsyz_dy[e] = dminus(w(e, -2), w(e, -1), m[e], w(e, 1)) * idy;
     }
@@ -356,7 +376,7 @@ k_velocity_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ buoy, int 
     pml_y(PSI_SAB1, 0, qy, dsyz_dy);
     own.wait();
     nvz = update(0, dszz_dz, dsxz_dx, dsyz_dy);
-    st_row(vz + tf, nvz);
+    st_row(dest(vz, 0), nvz);
   }
   if (mine(1)) {  // vx
     Row qz = ld_z(PSI_SAB1), qx = ld_x(PSI_SAA), qy = ld_y(PSI_SAB2);
@@ -375,7 +395,7 @@ k_velocity_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ buoy, int 
     }
     {
       const Row m = ld_row(sxy);
-      const Span w = ld_span(sxy, m, c);
+      const Span w = ld_span(sxy, m, r);
 #pragma unroll
       for (int e = 0; e < VEC; ++e) dsxy_dy[e] = dminus(w(e, -2), w(e, -1), m[e], w(e, 1)) * idy;
     }
@@ -383,7 +403,7 @@ k_velocity_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ buoy, int 
     pml_x(PSI_SAA, 1, qx, dsxx_dx);
     pml_y(PSI_SAB2, 0, qy, dsxy_dy);
     nvx = update(1, dsxz_dz, dsxx_dx, dsxy_dy);
-    st_row(vx + tf, nvx);
+    st_row(dest(vx, 1), nvx);
   }
   if (mine(2)) {  // vy
     Row qz = ld_z(PSI_SAB2), qx = ld_x(PSI_SAB2), qy = ld_y(PSI_SAA);
@@ -403,7 +423,7 @@ k_velocity_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ buoy, int 
     }
     {
       const Row m = ld_row(syy);
-      const Span w = ld_span(syy, m, c);
+      const Span w = ld_span(syy, m, r);
 #pragma unroll
       for (int e = 0; e < VEC; ++e) dsyy_dy[e] = dplus(w(e, -1), m[e], w(e, 1), w(e, 2)) * idy;
     }
@@ -411,7 +431,7 @@ k_velocity_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ buoy, int 
     pml_x(PSI_SAB2, 0, qx, dsxy_dx);
     pml_y(PSI_SAA, 1, qy, dsyy_dy);
     nvy = update(2, dsyz_dz, dsxy_dx, dsyy_dy);
-    st_row(vy + tf, nvy);
+    st_row(dest(vy, 2), nvy);
   }
   if (IL) {
     Row hb = own.get(4);
@@ -444,7 +464,7 @@ k_velocity_fwd_vec(Geo g, Fields f, Psi ps, const float *__restrict__ buoy, int 
 void launch_stress_fwd_vec(int S, cudaStream_t st, const Geo &g, const Fields &f, const Psi &ps,
                            const float *lam, const float *mu, const SrcArgs &src,
                            const ShellMap &shell, const IllumSum &il, const StepTo &to, bool after_velocity) {
-  const int mode = il.first ? VEC_ILLUM : to.fields ? VEC_STEP_TO : VEC_STEP;
+  const int mode = il.first ? VEC_ILLUM : to.out ? VEC_STEP_TO : VEC_STEP;
   const int parts = mode == VEC_STEP && vec_split(g, S) ? 4 : 1;
   const dim3 grid = vec_grid(g, S, parts);
   const int nzb = grid.z / S;
@@ -458,7 +478,7 @@ void launch_stress_fwd_vec(int S, cudaStream_t st, const Geo &g, const Fields &f
 
 void launch_velocity_fwd_vec(int S, cudaStream_t st, const Geo &g, const Fields &f, const Psi &ps,
                              const float *buoy, const RecFuse &rec, const IllumSum &il, const StepTo &to) {
-  const int mode = il.first ? VEC_ILLUM : to.fields ? VEC_STEP_TO : VEC_STEP;
+  const int mode = il.first ? VEC_ILLUM : to.out ? VEC_STEP_TO : VEC_STEP;
   const int parts = mode == VEC_STEP && vec_split(g, S) ? 3 : 1;
   const dim3 grid = vec_grid(g, S, parts);
   const int nzb = grid.z / S;

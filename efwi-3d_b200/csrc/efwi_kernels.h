@@ -111,10 +111,13 @@ void launch_rev_stress(int bx, dim3 grid, cudaStream_t st, const Geo &g, const F
                        const float *buoy, float *glam, float *gmu, int zchunk, int nzc,
                        int do_rev, int do_adj, const SrcArgs &src);
 
-// Floats from the fields and memory variables that a forward step reads to
-// those it writes (0: in place).
+// Where a forward step's results go (out null: in place).  The state that it
+// reads and the one that it writes may have rows of their own pitch; the model
+// and the receiver maps have the grid's.
 struct StepTo {
-  long long fields, psi;
+  float *out;       // nine volumes of nz * nx * pitch_out floats, in the order of Fields
+  long long psi;    // floats from the memory variables read to those written
+  int pitch_in, pitch_out;
 };
 
 // Illumination sums [lambda, mu, buoyancy][N] of the shots of a batch: the

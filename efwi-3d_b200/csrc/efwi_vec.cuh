@@ -66,15 +66,18 @@ struct VecCell {
   bool act[VEC];      // cells of [2, ny-3]
 };
 
-__device__ __forceinline__ VecCell vec_cell(const Geo &g, int z, int x, int y) {
+__device__ __forceinline__ VecCell vec_cell(const Geo &g, int z, int x, int y, int pitch) {
   VecCell c;
   c.z = z; c.x = x; c.y = y;
-  c.i = (z * g.nx + x) * g.sx + y;
+  c.i = (z * g.nx + x) * pitch + y;
   c.lo = y > 0;
-  c.hi = y + VEC < g.sx;
+  c.hi = y + VEC < pitch;
 #pragma unroll
   for (int e = 0; e < VEC; ++e) c.act[e] = y + e >= 2 && y + e <= g.ny - 3;
   return c;
+}
+__device__ __forceinline__ VecCell vec_cell(const Geo &g, int z, int x, int y) {
+  return vec_cell(g, z, x, y, g.sx);
 }
 
 // The vector m at p with its neighbours; cells outside the row (only ever

@@ -200,8 +200,7 @@ int efwi_illumination(EfwiHandle *h, int n, const int *shot_ids, float *h_lam, f
 /* Exact-gradient checkpoints (no reference counterpart; the reference keeps
  * only the boundary shell, Boundary.cu).  bytes: HBM for checkpoint slots
  * (default 4 GiB); one slot holds one state of efwi_state_bytes(h) bytes.
- * (On some grids rows are padded to whole 128-byte lines, at most a sixth of
- * the volume, which neither number counts.)
+ * The slots of a call, over all its lanes, take no more than the budget.
  * efwi_checkpoint_stats: forward steps and slots of the last exact
  * gradient's shot.  efwi_checkpoint_plan (host only, no handle): the
  * schedule for nt time steps and `slots` slots -- total forward steps,
