@@ -104,21 +104,31 @@ def conv3d_wgrad(x: torch.Tensor, dy: torch.Tensor, nparts: int = 592) -> torch.
     return dw
 
 
+def _dense(t: torch.Tensor, dtype) -> torch.Tensor:
+    """t as the kernels read it: of `dtype`, contiguous, on a 16-byte boundary
+    (what saved-tensor hooks hand back need not be)."""
+    if t.dtype == dtype and t.is_contiguous() and not t.data_ptr() & 15:
+        return t
+    t = t.to(dtype).contiguous()
+    return t.clone() if t.data_ptr() & 15 else t
+
+
 def conv3d_backward(x: torch.Tensor, wb: torch.Tensor, gy: torch.Tensor, y, want_dx: bool,
                     nparts: int = 592):
     """(dx or None, dw, db) of one layer: g = gy * (y > 0) in float32 (y None:
     no ReLU), dx and dw from g in BF16, db = sum of g over the voxels.  A gy
     [D, H, W] is the gradient of channel 0 alone."""
     D, H, W = x.shape[:3]
+    bf16 = torch.bfloat16
+    x, wb = _dense(x, bf16), _dense(wb, bf16)
     if gy.dim() == 3:
-        gy, kind = gy.float().contiguous(), 2
+        gy, kind = _dense(gy, torch.float32), 2
     else:
-        if gy.dtype != torch.bfloat16:
-            gy = gy.float()
-        gy, kind = gy.contiguous(), int(gy.dtype == torch.float32)
-    if gy.data_ptr() & 15:
-        gy = gy.clone()
+        kind = int(gy.dtype != bf16)
+        gy = _dense(gy, torch.float32 if kind else bf16)
     relu = int(y is not None)
+    if relu:
+        y = _dense(y, bf16 if y.dtype == bf16 else torch.float32)
     L = lib()
     n = L.efwi_conv3d_backward_scratch(D, H, W, nparts, kind, relu)
     scratch = torch.empty(n, device=x.device, dtype=torch.uint8)

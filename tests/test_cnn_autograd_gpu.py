@@ -1,0 +1,62 @@
+"""Autograd features around the preconditioner's convolutions."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module", autouse=True)
+def _ready():
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+
+
+def _layer(shape, seed=5):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    x = torch.randn(*shape, 16, device="cuda", generator=g).to(torch.bfloat16)
+    w = 0.2 * torch.randn(27, 16, 16, device="cuda", generator=g)
+    b = torch.randn(16, device="cuda", generator=g)
+    gy = torch.randn(*shape, 16, device="cuda", generator=g)
+    return [t.requires_grad_(True) for t in (x, w, b)], gy
+
+
+def _shift(t):  # on a 2- or 4-byte boundary
+    buf = torch.empty(t.numel() + 1, dtype=t.dtype, device=t.device)
+    buf[1:] = t.reshape(-1)
+    return buf[1:].view(t.shape)
+
+
+HOOKS = {
+    "permuted": (lambda t: t.transpose(0, 1).contiguous(), lambda t: t.transpose(0, 1)),
+    "unaligned": (lambda t: t, _shift),
+    "float64": (lambda t: t.double(), lambda t: t),
+}
+
+
+@pytest.mark.parametrize("hook", sorted(HOOKS))
+@pytest.mark.parametrize("relu,out_f32", [(True, False), (True, True), (False, False)])
+def test_layer_backward_under_saved_tensor_hooks(hook, relu, out_f32):
+    """Whatever strides, alignment and type the hooks hand back."""
+    from efwi.cnn import Conv3dBF16
+    (x, w, b), gy = _layer((5, 7, 9))
+    out = []
+    for pack, unpack in ((lambda t: t, lambda t: t), HOOKS[hook]):
+        with torch.autograd.graph.saved_tensors_hooks(pack, unpack):
+            y = Conv3dBF16.apply(x, w, b, relu, out_f32)
+        out.append(torch.autograd.grad(y, [x, w, b], gy.to(y.dtype)))
+    for u, v in zip(*out):
+        assert torch.equal(u, v)
+
+
+@pytest.mark.parametrize("hook", sorted(HOOKS))
+def test_network_backward_under_saved_tensor_hooks(hook):
+    from efwi.cnn import Preconditioner
+    net = Preconditioner(seed=2).cuda()
+    feats = torch.randn(3, 5, 7, 9, device="cuda")
+    out = []
+    for pack, unpack in ((lambda t: t, lambda t: t), HOOKS[hook]):
+        with torch.autograd.graph.saved_tensors_hooks(pack, unpack):
+            y = net(feats)
+        out.append(torch.autograd.grad(y, list(net.parameters()), torch.ones_like(y)))
+    for u, v in zip(*out):
+        assert torch.equal(u, v)
