@@ -14,6 +14,7 @@ import ctypes as C
 import math
 
 import torch
+from torch.autograd import forward_ad
 
 from ._lib import lib
 
@@ -226,11 +227,20 @@ class _ChannelsLast(torch.autograd.Function):
         return gx[..., :ctx.c].permute(3, 0, 1, 2).to(torch.float32)
 
 
+def _transformed(t: torch.Tensor) -> bool:
+    """Whether t takes part in a functorch transform, forward-mode
+    differentiation or a trace, which see torch operations only."""
+    return (type(t) not in (torch.Tensor, torch.nn.Parameter)
+            or torch._C._are_functorch_transforms_active()
+            or forward_ad.unpack_dual(t).tangent is not None
+            or torch.jit.is_tracing() or torch.compiler.is_compiling())
+
+
 def to_channels_last(feats: torch.Tensor) -> torch.Tensor:
     """[C, D, H, W] f32 -> [D, H, W, 16] bf16 (channels zero-padded)."""
     c = feats.shape[0]
     if (feats.is_cuda and feats.dtype == torch.float32 and feats.dim() == 4 and 1 <= c <= C16
-            and feats.numel() > 0):
+            and feats.numel() > 0 and not _transformed(feats)):
         return _ChannelsLast.apply(feats)
     x = torch.zeros(feats.shape[1:] + (C16,), device=feats.device, dtype=torch.bfloat16)
     x[..., :c] = feats.permute(1, 2, 3, 0).to(torch.bfloat16)

@@ -60,3 +60,40 @@ def test_network_backward_under_saved_tensor_hooks(hook):
         out.append(torch.autograd.grad(y, list(net.parameters()), torch.ones_like(y)))
     for u, v in zip(*out):
         assert torch.equal(u, v)
+
+
+def _chain(feats):  # torch operations
+    x = torch.zeros(feats.shape[1:] + (16,), device=feats.device, dtype=torch.bfloat16)
+    x[..., :feats.shape[0]] = feats.permute(1, 2, 3, 0).to(torch.bfloat16)
+    return x
+
+
+def _dual(fn, a, t):
+    from torch.autograd import forward_ad
+    with forward_ad.dual_level():
+        return forward_ad.unpack_dual(fn(forward_ad.make_dual(a, t))).tangent
+
+
+TRANSFORMS = {
+    "values": lambda fn, a, t: fn(a),
+    "backward": lambda fn, a, t: torch.autograd.grad(fn(a.requires_grad_(True)).float().pow(2).sum(), a)[0],
+    "grad": lambda fn, a, t: torch.func.grad(lambda v: fn(v).float().pow(2).sum())(a),
+    "jvp": lambda fn, a, t: torch.func.jvp(fn, (a,), (t,))[1],
+    "forward mode": _dual,
+    "jacfwd": lambda fn, a, t: torch.func.jacfwd(lambda v: fn(v).float())(a),
+    "jacrev": lambda fn, a, t: torch.func.jacrev(lambda v: fn(v).float())(a),
+    "hvp": lambda fn, a, t: torch.autograd.functional.hvp(lambda v: fn(v).float().pow(3).sum(), a, t)[1],
+    "trace": lambda fn, a, t: torch.jit.trace(fn, (a + 1,))(a),
+}
+
+
+@pytest.mark.parametrize("how", sorted(TRANSFORMS))
+@pytest.mark.filterwarnings("ignore")
+def test_channels_last_copy_under_transforms(how):
+    from efwi.cnn import to_channels_last
+    g = torch.Generator(device="cuda").manual_seed(1)
+    a, t = (torch.randn(3, 2, 4, 5, device="cuda", generator=g) for _ in range(2))
+    fn = TRANSFORMS[how]
+    out, ref = fn(to_channels_last, a.clone(), t), fn(_chain, a.clone(), t)
+    assert out.dtype == ref.dtype and torch.equal(out, ref)
+    assert float(ref.abs().max()) > 0
