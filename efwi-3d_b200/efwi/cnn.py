@@ -167,10 +167,11 @@ class _Network(torch.autograd.Function):
     """The network's layers as one node: ReLU layers, then channel 0 of the
     last layer, [D, H, W] f32 (its other channels are neither written nor
     differentiated).  Same kernels and sums as a chain of Conv3dBF16; what
-    it saves is the host work between their launches."""
+    it saves is the host work between their launches.  `keep`: a backward pass
+    may follow; otherwise an activation lives until the next one is there."""
 
     @staticmethod
-    def forward(ctx, x, n, *params):
+    def forward(ctx, x, n, keep, *params):
         ws, bs = params[:n], params[n:]
         if any(p.device != x.device for p in params):
             raise ValueError("the network's parameters and input are on different devices")
@@ -185,7 +186,8 @@ class _Network(torch.autograd.Function):
                 y = torch.empty_like(x)
                 rc = rc or L.efwi_conv3d_forward(_ptr(h), _ptr(wb[k]), _ptr(bias[k]), D, H, W, 1,
                                                  _ptr(y), None, st)
-                acts.append(y)
+                if keep:
+                    acts.append(y)
                 h = y
             out = torch.empty(D, H, W, device=x.device, dtype=torch.float32)
             head = rc or L.efwi_conv3d_forward_head(_ptr(h), _ptr(wb[n - 1]), _ptr(bias[n - 1]), D,
@@ -194,7 +196,8 @@ class _Network(torch.autograd.Function):
             raise RuntimeError(f"a convolution of the network failed ({rc or head})")
         if head == 3:  # another kernel form is selected
             out = conv3d_raw(h, wb[n - 1], bs[n - 1], False, True)[..., 0].contiguous()
-        ctx.save_for_backward(x, wb, *acts)
+        if keep:
+            ctx.save_for_backward(x, wb, *acts)
         return out
 
     @staticmethod
@@ -206,7 +209,7 @@ class _Network(torch.autograd.Function):
             g, dws[k], dbs[k] = conv3d_backward(acts[k - 1] if k else x, wb[k], g,
                                                 acts[k] if k < n - 1 else None,
                                                 k > 0 or ctx.needs_input_grad[0])
-        return (g, None, *dws, *dbs)
+        return (g, None, None, *dws, *dbs)
 
 
 class _ChannelsLast(torch.autograd.Function):
@@ -270,4 +273,6 @@ class Preconditioner(torch.nn.Module):
     def forward(self, feats: torch.Tensor) -> torch.Tensor:
         """feats [C, D, H, W] f32 on a GPU -> [D, H, W] f32."""
         h = to_channels_last(feats)
-        return _Network.apply(h, len(self.w), *self.w, *self.b)
+        params = (*self.w, *self.b)
+        keep = torch.is_grad_enabled() and (h.requires_grad or any(p.requires_grad for p in params))
+        return _Network.apply(h, len(self.w), keep, *params)

@@ -97,3 +97,26 @@ def test_channels_last_copy_under_transforms(how):
     out, ref = fn(to_channels_last, a.clone(), t), fn(_chain, a.clone(), t)
     assert out.dtype == ref.dtype and torch.equal(out, ref)
     assert float(ref.abs().max()) > 0
+
+
+@pytest.mark.parametrize("frozen", [True, False])
+def test_inference_memory_does_not_grow_with_the_layers(frozen):
+    """Without a backward pass to come (no_grad, or nothing to differentiate)
+    the input copy and two activations of 2 * 16 bytes a voxel are alive."""
+    from efwi.cnn import Preconditioner
+    shape = (64, 64, 64)
+    feats = torch.randn(3, *shape, device="cuda")
+    unit = 32 * 64 ** 3
+    for layers in (4, 12):
+        net = Preconditioner(seed=2, layers=layers).cuda().requires_grad_(not frozen)
+        with torch.set_grad_enabled(frozen):
+            net(feats)
+            torch.cuda.synchronize()
+            base = torch.cuda.memory_allocated()
+            torch.cuda.reset_peak_memory_stats()
+            y = net(feats)
+            torch.cuda.synchronize()
+        assert not y.requires_grad
+        # and the output, a float a voxel, and the weights' BF16 copies
+        assert torch.cuda.max_memory_allocated() - base <= 3 * unit + unit // 8 + (1 << 20)
+        del y
