@@ -159,8 +159,11 @@ class Conv3dBF16(torch.autograd.Function):
     @staticmethod
     def backward(ctx, gy):
         x, wb, y = ctx.saved_tensors
-        return (*conv3d_backward(x, wb, gy, y if ctx.relu else None, ctx.needs_input_grad[0]),
-                None, None)
+        dx, dw, db = conv3d_backward(x, wb, gy, y if ctx.relu else None, ctx.needs_input_grad[0])
+        if torch.is_grad_enabled():  # create_graph: db stays a function of gy
+            g = gy.float()
+            db = (g * (y > 0) if ctx.relu else g).sum(dim=(0, 1, 2))
+        return dx, dw, db, None, None
 
 
 class _Network(torch.autograd.Function):
@@ -209,6 +212,8 @@ class _Network(torch.autograd.Function):
             g, dws[k], dbs[k] = conv3d_backward(acts[k - 1] if k else x, wb[k], g,
                                                 acts[k] if k < n - 1 else None,
                                                 k > 0 or ctx.needs_input_grad[0])
+        if torch.is_grad_enabled():  # create_graph: the head's db stays a function of gy
+            dbs[-1] = torch.nn.functional.pad(gy.float().sum().reshape(1), (0, C16 - 1))
         return (g, None, None, *dws, *dbs)
 
 

@@ -120,3 +120,30 @@ def test_inference_memory_does_not_grow_with_the_layers(frozen):
         # and the output, a float a voxel, and the weights' BF16 copies
         assert torch.cuda.max_memory_allocated() - base <= 3 * unit + unit // 8 + (1 << 20)
         del y
+
+
+@pytest.mark.parametrize("relu", [True, False])
+def test_bias_gradient_can_be_differentiated_again(relu):
+    """d/db sum_v (y_v)^2 = 2 sum_v m_v y_v (m: behind the ReLU), and again:
+    2 times the number of open voxels.  Whole numbers in float32."""
+    from efwi.cnn import Conv3dBF16
+    (x, w, b), _ = _layer((5, 7, 9))
+    y = Conv3dBF16.apply(x, w, b, relu, True)
+    (db,) = torch.autograd.grad(y.pow(2).sum(), b, create_graph=True)
+    ref = 2 * y.detach().double().sum(dim=(0, 1, 2))
+    # sums of 315 terms in any order, each product rounded once
+    size = 2 * y.detach().double().abs().sum(dim=(0, 1, 2))
+    assert bool(((db.double() - ref).abs() <= 316 * 2.0 ** -24 * size).all())
+    (d2,) = torch.autograd.grad(db.sum(), b)
+    opened = (y > 0).sum(dim=(0, 1, 2)) if relu else torch.full((16,), 5 * 7 * 9, device="cuda")
+    assert torch.equal(d2, 2.0 * opened)
+
+
+def test_head_bias_gradient_can_be_differentiated_again():
+    from efwi.cnn import Preconditioner
+    net = Preconditioner(seed=2).cuda()
+    y = net(torch.randn(3, 5, 7, 9, device="cuda"))
+    b = net.b[-1]
+    (db,) = torch.autograd.grad(y.pow(2).sum(), b, create_graph=True)
+    (d2,) = torch.autograd.grad(db.sum(), b)
+    assert torch.equal(d2, torch.tensor([630.0] + 15 * [0.0], device="cuda"))
