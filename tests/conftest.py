@@ -20,3 +20,13 @@ def cuda_ok():
         return torch.cuda.is_available()
     except Exception:
         return False
+
+
+@pytest.fixture(autouse=True)
+def _reference_checker(monkeypatch):
+    """Tests that compare with the reference's own kernels compiled for the CPU
+    are skipped where its sources are not there to build them from."""
+    import oracle
+    if not oracle.ref_available():
+        monkeypatch.setattr(oracle, "ref", lambda: pytest.skip(
+            "oracle/_ref is not built: the reference's sources are not here"))
