@@ -278,6 +278,8 @@ class Preconditioner(torch.nn.Module):
     def forward(self, feats: torch.Tensor) -> torch.Tensor:
         """feats [C, D, H, W] f32 on a GPU -> [D, H, W] f32."""
         h = to_channels_last(feats)
+        if not len(self.w):
+            return h[..., 0]
         params = (*self.w, *self.b)
         keep = torch.is_grad_enabled() and (h.requires_grad or any(p.requires_grad for p in params))
         return _Network.apply(h, len(self.w), keep, *params)
