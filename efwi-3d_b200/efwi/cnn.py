@@ -120,16 +120,9 @@ def conv3d_backward(x: torch.Tensor, wb: torch.Tensor, gy: torch.Tensor, y, want
     no ReLU), dx and dw from g in BF16, db = sum of g over the voxels.  A gy
     [D, H, W] is the gradient of channel 0 alone."""
     D, H, W = x.shape[:3]
-    bf16 = torch.bfloat16
-    x, wb = _dense(x, bf16), _dense(wb, bf16)
-    if gy.dim() == 3:
-        gy, kind = _dense(gy, torch.float32), 2
-    else:
-        kind = int(gy.dtype != bf16)
-        gy = _dense(gy, torch.float32 if kind else bf16)
+    kind = 2 if gy.dim() == 3 else int(gy.dtype != torch.bfloat16)
+    gy = _dense(gy, torch.float32 if kind else torch.bfloat16)
     relu = int(y is not None)
-    if relu:
-        y = _dense(y, bf16 if y.dtype == bf16 else torch.float32)
     L = lib()
     n = L.efwi_conv3d_backward_scratch(D, H, W, nparts, kind, relu)
     scratch = torch.empty(n, device=x.device, dtype=torch.uint8)
@@ -159,7 +152,11 @@ class Conv3dBF16(torch.autograd.Function):
     @staticmethod
     def backward(ctx, gy):
         x, wb, y = ctx.saved_tensors
-        dx, dw, db = conv3d_backward(x, wb, gy, y if ctx.relu else None, ctx.needs_input_grad[0])
+        bf16 = torch.bfloat16
+        dx, dw, db = conv3d_backward(
+            _dense(x, bf16), _dense(wb, bf16), gy,
+            _dense(y, bf16 if y.dtype == bf16 else torch.float32) if ctx.relu else None,
+            ctx.needs_input_grad[0])
         if torch.is_grad_enabled():  # create_graph: db stays a function of gy
             g = gy.float()
             db = (g * (y > 0) if ctx.relu else g).sum(dim=(0, 1, 2))
@@ -205,7 +202,7 @@ class _Network(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, gy):
-        x, wb, *acts = ctx.saved_tensors
+        x, wb, *acts = (_dense(t, torch.bfloat16) for t in ctx.saved_tensors)
         n = wb.shape[0]
         dws, dbs, g = [None] * n, [None] * n, gy
         for k in range(n - 1, -1, -1):
@@ -278,8 +275,8 @@ class Preconditioner(torch.nn.Module):
     def forward(self, feats: torch.Tensor) -> torch.Tensor:
         """feats [C, D, H, W] f32 on a GPU -> [D, H, W] f32."""
         h = to_channels_last(feats)
-        if not len(self.w):
-            return h[..., 0]
         params = (*self.w, *self.b)
+        if not params:
+            return h[..., 0]
         keep = torch.is_grad_enabled() and (h.requires_grad or any(p.requires_grad for p in params))
-        return _Network.apply(h, len(self.w), keep, *params)
+        return _Network.apply(h, len(params) // 2, keep, *params)
