@@ -12,17 +12,21 @@
 // transposed convolution).
 //
 // Kernels (efwi_conv3d_set_kernel / efwi_conv3d_set_wgrad_kernel choose):
-//   k_conv3d_fwd_tc2  forward on tcgen05.mma (the default): per tile of
-//                     128 voxels one MMA per tap, accumulator in tensor
-//                     memory, input tiles staged by bulk tensor copies
+//   k_conv3d_fwd_zm   forward on tcgen05.mma (the default): tiles of 8 x 16
+//                     voxels march through z, one MMA per (dy, dx) for the
+//                     three dz, accumulators in tensor memory, input planes
+//                     staged by bulk tensor copies
+//   k_conv3d_fwd_tc2  per tile of 128 voxels one MMA per tap, input tiles
+//                     staged by bulk tensor copies
 //   k_conv3d_fwd_ws   the same, warp-specialised (copy + MMA warp, four
 //                     epilogue warps)
 //   k_conv3d_fwd_tc   the same MMAs, tiles staged by plain loads
 //   k_conv3d_fwd      forward on mma.sync.m16n8k16: per output row of 16
 //                     voxels one warp, A fragments by ldmatrix
 //   k_conv3d_wgrad_tc dW[t][co][ci] = sum_u dy[u - off_t][co] x[u][ci] on
-//                     tcgen05.mma (the default): eight taps stacked on the
-//                     MMA's rows, K = voxels
+//                     tcgen05.mma (the default): the (dy, dz) of the taps
+//                     stacked on the MMA's rows, the dx on its columns,
+//                     K = voxels
 //   k_conv3d_wgrad    the same on mma.sync: one warp per tap
 // Both weight gradients leave per-CTA partial sums that k_reduce_partials
 // adds in a fixed order.
@@ -512,11 +516,9 @@ k_conv3d_fwd_tc(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__rest
 // The same tile and MMAs with the input staged by bulk tensor copies and
 // the work software-pipelined: while the warps drain tile j's accumulator,
 // the tensor cores already work on tile j+1 (two accumulators of 16 TMEM
-// columns, used in turn) and the copy engine fills stages ahead.  With NS
-// stages the copies of tile j+NS-1 are issued as soon as their stage is
-// free: for NS = 3 right after tile j+1's MMAs (the stage last held tile
-// j-1, whose MMAs completed in the previous iteration), for NS = 2 once tile
-// j's MMAs completed.  The tensor map views x as [D][H][W][2 halves][8
+// columns, used in turn) and the copy engine fills stages ahead: the copies of
+// tile j+2 are issued right after tile j+1's MMAs, into the third stage (it
+// last held tile j-1, whose MMAs completed in the previous iteration).  The tensor map views x as [D][H][W][2 halves][8
 // channels]; a box of 8 x 1 x 10 x 18 x 3 is one channel-half plane of the
 // staged tile in exactly the layout above (zeros outside the volume), so
 // each stage takes two copies.  Half planes start 128-byte aligned.
@@ -536,12 +538,11 @@ __device__ __forceinline__ void tma_load_5d(void *dst, const CUtensorMap *map, u
       : "memory");
 }
 
-template <int NS>
 __global__ void __launch_bounds__(128)
 k_conv3d_fwd_tc2(const __grid_constant__ CUtensorMap xmap, const __nv_bfloat16 *__restrict__ w,
                  const float *__restrict__ bias, int D, int H, int W, int relu,
                  __nv_bfloat16 *__restrict__ yb, float *__restrict__ yf) {
-  static_assert(NS == 2 || NS == 3, "two or three stages");
+  constexpr int NS = 3;  // stages
   extern __shared__ unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t full[NS];  // stage filled (copies landed)
   __shared__ __align__(8) uint64_t done[2];   // accumulator b complete
@@ -624,7 +625,7 @@ k_conv3d_fwd_tc2(const __grid_constant__ CUtensorMap xmap, const __nv_bfloat16 *
         if (mma(j + 1)) n_mma = j + 2;
         else s_abort = 1;
       }
-      if (NS == 3 && !s_abort && j + 2 < nj) {
+      if (!s_abort && j + 2 < nj) {
         issue(j + 2);
         n_tma = j + 3;
       }
@@ -632,10 +633,6 @@ k_conv3d_fwd_tc2(const __grid_constant__ CUtensorMap xmap, const __nv_bfloat16 *
     // every thread takes the same branch: tcgen05.ld is warp-collective
     const bool got =
         __syncthreads_and(mbar_wait_bounded(&done[j & 1], (uint32_t)((j >> 1) & 1)));
-    if (NS == 2 && tid == 0 && got && !s_abort && j + 2 < nj) {
-      issue(j + 2);  // stage j % 2: tile j's MMAs completed
-      n_tma = j + 3;
-    }
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     if (got) {
       int x0, y0, z;
@@ -1111,7 +1108,7 @@ k_conv3d_fwd_ws(const __grid_constant__ CUtensorMap xmap, const __nv_bfloat16 *_
 // with the number of MMAs added in one go (at 93 x 117 x 141 the sums are
 // 6e-6 off when a CTA's units stay in TMEM to the end).  The CTA's 27 x 16
 // x 16 sums go to partial[cta] for the fixed-order reduction.  One thread of a
-// fifth warp runs the copies (two stages) and the MMAs; every wait is
+// fifth warp runs the copies (three stages) and the MMAs; every wait is
 // bounded, and on a timeout the CTA sets the status flag and writes NaN
 // partial sums.
 constexpr int kWgX = 8, kWgY = 16, kWgZ = 2;          // voxels of a unit
@@ -1307,9 +1304,10 @@ k_channels_last(const float *__restrict__ feats, int c, long long vox, __nv_bflo
 using namespace efwi;
 
 namespace {
-// 0: mma.sync; 1: tcgen05, tile staged by loads; 2 / 3: tcgen05, tiles
-// staged by bulk tensor copies two / three stages deep; 4 / 5: the same,
-// warp-specialised (copy + MMA warp, four epilogue warps), two / three stages
+// 0: mma.sync; 1: tcgen05, one MMA per tap, tile staged by loads; 2: tcgen05,
+// z-marching; 3: as 1 with the tiles staged by bulk tensor copies three stages
+// deep; 4 / 5: as 3, warp-specialised (copy + MMA warp, four epilogue warps),
+// two / three stages
 std::atomic<int> g_conv_kernel{2};
 std::atomic<unsigned long long> g_tc_smem_set{0}, g_tc2_smem_set{0}, g_tc3_smem_set{0},
     g_ws2_smem_set{0}, g_ws3_smem_set{0};
@@ -1488,9 +1486,9 @@ extern "C" int efwi_conv3d_forward(const void *x, const void *w, const float *bi
         const int rc = zm_launch(map, w, bias, D, H, W, relu, y_bf16, y_f32, nullptr, st);
         if (rc) return rc;
       } else {  // three stages, 66 KB: 3 CTAs per SM
-        set_smem_once(k_conv3d_fwd_tc2<3>, tc2_smem<3>(), g_tc3_smem_set);
+        set_smem_once(k_conv3d_fwd_tc2, tc2_smem<3>(), g_tc3_smem_set);
         const int blocks = (int)std::min<long long>(tiles, 3LL * sms);
-        k_conv3d_fwd_tc2<3><<<blocks, 128, tc2_smem<3>(), st>>>(
+        k_conv3d_fwd_tc2<<<blocks, 128, tc2_smem<3>(), st>>>(
             map, (const __nv_bfloat16 *)w, bias, D, H, W, relu, (__nv_bfloat16 *)y_bf16, y_f32);
       }
     } else {
