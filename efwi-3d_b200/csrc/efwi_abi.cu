@@ -146,7 +146,7 @@ struct EfwiHandle {
   int py = 0;       // y pitch
   int if_win = 0, bx = 4, zchunk = 8, max_batch = 4;
   int variant = 1;  // 0: L1-served stencils, 1: four cells per thread
-  int zchunk_rev = 8;  // z planes per CTA of the exact adjoint kernels
+  int zchunk_rev = 8;  // z planes per CTA of the one-cell exact adjoint kernels
   int nt_limit = 0;        // > 0: time loops stop early (timing probes)
   std::string err;
 
@@ -496,7 +496,8 @@ Psi psi_at(float *base, const Geo &g, int S) {
 // 16-byte vectors are aligned; whole 128-byte lines where they add at most a
 // sixth to the volumes: a CTA reads 128 bytes of a row, one line instead of
 // parts of two.  Misfit and gradient at 84^3 (84 -> 96) 12.7 -> 11.8 and 43.1
-// -> 41.4 ms, exact gradient at 120^3 (128) 48.6 -> 47.4.  Beyond a sixth the
+// -> 41.4 ms, exact gradient at 120^3 (128) 48.6 -> 48.4: its checkpoints, which
+// count against the caller's budget, have rows without it.  Beyond a sixth the
 // larger volumes cost as much in L2 (illumination at 80^3, 80 -> 96: 11.65 ->
 // 12.3), the latency-bound small grids lose 1-4 % (26 x 30 x 28), and grids
 // beyond 2^26 cells (5 GB a state) are left the memory.

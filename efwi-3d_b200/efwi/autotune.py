@@ -5,8 +5,9 @@ problem the tuner runs short gradient probes (the time loops stopped after
 `nt_probe` steps) on the handle's real grid, model and survey, reads the
 per-kernel CUDA-event timings of the engine, and keeps the fastest.  The
 vector kernels of variant 1 choose their own launch shape, so by default one
-configuration of each knob is probed; callers may pass more (zchunk_rev is
-the z march of the exact adjoint kernels, zchunk_fwd that of variant 0).
+configuration of each knob is probed.  Callers may pass more; of those,
+zchunk_fwd is the z march of variant 0, zchunk_rev that of its exact adjoint,
+and the cfg numbers change nothing.
 """
 from __future__ import annotations
 
@@ -110,7 +111,9 @@ def autotune_windows(P, shot_ids, windows, nt_probe: int = 16, bxs=(4, 8), zchun
     """Stencil variant and launch shape of the window forward, the fastest
     over short probes (time loop stopped after `nt_probe` steps, CUDA events
     on the current stream): the L1-served multi-domain launch over
-    (tile_bx, zchunk) and the per-window vector kernels (reported as "tma").
+    (tile_bx, zchunk) and the per-window vector kernels (reported as "tma", the
+    name of this choice in saved results; fwd_cfgs and tma_zchunks change
+    nothing there).
     Sets the choice on P (its variant included: the windows' results do not
     depend on it)."""
     def probe():

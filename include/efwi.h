@@ -70,10 +70,12 @@ const char *efwi_version(void);
 int efwi_set_options(EfwiHandle *h, int if_win, int tile_bx, int zchunk, int max_batch);
 
 /* Kernel family of the stencil sweeps: 1 (default) updates four cells per
- * thread with 16-byte accesses (exact gradients: planes staged in shared
- * memory by bulk tensor copies); 0 marches z one cell per thread.  Both give
- * identical results; grids beyond 65535 CTAs along x or z run as 0.  No
- * reference counterpart (the reference has one plain kernel per update). */
+ * thread with 16-byte accesses (the exact adjoint: with its terms staged in
+ * shared memory); 0 marches z one cell per thread.  Both give the same traces,
+ * misfits and reference gradients to the bit; exact gradients and the
+ * illumination, whose sums are ordered or fused differently, agree to 5e-6 and
+ * 1e-5.  Grids beyond 65535 CTAs along x or z run as 0.  No reference
+ * counterpart (the reference has one plain kernel per update). */
 int efwi_set_variant(EfwiHandle *h, int variant);
 
 /* CUDA graphs of the time loops (default on): the forward time loop of a
@@ -88,7 +90,8 @@ int efwi_set_graphs(EfwiHandle *h, int on);
 
 /* Launch configuration (the autotuner's knobs; results do not depend on
  * them): zchunk_fwd > 0 sets the z planes per CTA of variant 0, zchunk_rev
- * > 0 those of the exact adjoint kernels (0 keeps).  fwd_cfg in 0..3 and
+ * > 0 those of its exact adjoint kernels, which efwi_step's transpose runs on
+ * either variant (0 keeps).  fwd_cfg in 0..3 and
  * rev_cfg in 0..7 are accepted and have no effect: the vector kernels choose
  * their own launch shape.  No reference counterpart. */
 int efwi_set_tuning(EfwiHandle *h, int fwd_cfg, int zchunk_fwd, int rev_cfg, int zchunk_rev);
