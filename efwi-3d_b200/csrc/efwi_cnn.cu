@@ -86,7 +86,11 @@ k_conv3d_fwd(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restric
   __shared__ __align__(16) unsigned char sx[kTileVox * kVoxPitch];
   const int tid = threadIdx.x;
   const int x0 = blockIdx.x * kTileX, y0 = blockIdx.y * kRowsFwd, z = blockIdx.z;
-  for (int k = tid; k < 27 * kC * kC / 2; k += blockDim.x) sw[k] = ld32(w + 2 * k);
+  // w and yb may lie on 2-byte boundaries (the tcgen05 forms' unaligned calls
+  // come here)
+  const bool w4 = ((uintptr_t)w & 3) == 0, y4 = ((uintptr_t)yb & 3) == 0;
+  for (int k = tid; k < 27 * kC * kC / 2; k += blockDim.x)
+    sw[k] = w4 ? ld32(w + 2 * k) : ld16(w + 2 * k) | (ld16(w + 2 * k + 1) << 16);
   for (int c = tid; c < 2 * kTileVox; c += blockDim.x) {
     const int v = c >> 1, h = c & 1;
     const int xx = v % (kTileX + 2), t = v / (kTileX + 2);
@@ -137,7 +141,12 @@ k_conv3d_fwd(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restric
       float o0 = c[nt][2 * hh] + b0, o1 = c[nt][2 * hh + 1] + b1;
       if (relu) { o0 = fmaxf(o0, 0.f); o1 = fmaxf(o1, 0.f); }
       const long long off = (((long long)z * H + y) * W + xv) * kC + co;
-      if (yb) *reinterpret_cast<__nv_bfloat162 *>(yb + off) = __floats2bfloat162_rn(o0, o1);
+      if (yb && y4) {
+        *reinterpret_cast<__nv_bfloat162 *>(yb + off) = __floats2bfloat162_rn(o0, o1);
+      } else if (yb) {
+        yb[off] = __float2bfloat16_rn(o0);
+        yb[off + 1] = __float2bfloat16_rn(o1);
+      }
       if (yf) { yf[off] = o0; yf[off + 1] = o1; }
     }
   }
